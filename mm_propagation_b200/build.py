@@ -4,7 +4,7 @@
 
 Objects go to mm_propagation_b200/_build/; the shared library lands next to
 this file so it travels with the source tree. kern_inst.cu is compiled once per
-(precision, log2 NT) with -D switches so the unrolled FFT kernels build in
+(precision, log2 NT, row split) with -D switches so the unrolled FFT kernels build in
 parallel. Rebuilds only what is older than its sources.
 """
 from __future__ import annotations
@@ -30,9 +30,11 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompil
 CXX = os.environ.get("MMP_CXX", "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++")
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-Wall", "-I", INCLUDE]
 LOGN_RANGE = range(6, 17)
-# row-split variants (kernel_table.h kSplit*): log2 NT ranges per precision
-SPLIT_F32 = range(12, 17)
-SPLIT_F64 = range(11, 15)
+
+
+def _max_split(fp64: bool, L: int) -> int:
+    """kernel_table.h max_split: row splits built for rows of 2^L samples."""
+    return 0 if L < 11 else 2 if L == 11 else 3 if L <= 13 else (16 - L if fp64 else 3 if L == 14 else 17 - L)
 
 
 def nvcc() -> str:
@@ -57,9 +59,9 @@ def _stale(target: str, deps) -> bool:
 def _units():
     units = []
     inst = os.path.join(CSRC, "kern_inst.cu")
-    for tag, real, split in (("f32", "float", SPLIT_F32), ("f64", "double", SPLIT_F64)):
-        for L in LOGN_RANGE:
-            for xc in ((0, 1) if L in split else (0,)):
+    for tag, real in (("f32", "float"), ("f64", "double")):
+        for L in reversed(LOGN_RANGE):  # the longest compilations first
+            for xc in range(_max_split(real == "double", L) + 1):
                 obj = os.path.join(BUILD, f"kern_{tag}_{L}_x{xc}.o")
                 units.append((inst, obj, [f"-DMMP_REAL={real}", f"-DMMP_LOGN={L}", f"-DMMP_TAG={tag}",
                                           f"-DMMP_XC={xc}"]))

@@ -1,34 +1,31 @@
-// fft.cuh — shared-memory Stockham FFT for one row per CTA, or one row per
-// thread-block cluster (rows larger than 128 KB), built for sm_100a.
+// fft.cuh — the transform of one row of N = 2^LOGN complex samples (precision T) by one CTA or
+// by a thread-block cluster of C CTAs, built for sm_100a.
 //
-// Row of N = 2^LOGN complex samples in precision T (float or double).
-//  * C = 2^LOGC CTAs (a cluster) share a row when N * sizeof(T2) > 128 KB.
-//    The row is cut into runs of G consecutive samples, G * sizeof(T2) = 32 bytes (one
-//    DRAM sector: G = 4 in FP32, 2 in FP64), dealt out to the CTAs in turn: CTA r holds
-//    the samples t = g + G (r + C v), g < G, v < NL/G (NL = N / C), so that its global
-//    loads and stores move whole sectors. In shared memory they are G rows of NL/G:
-//    row g is the sub-sequence x_g[s] = x[g + G s] at s = r + C v, decimated over the
-//    cluster. Forward: every CTA transforms its G rows locally (NL/G points each); a
-//    radix-(C G) butterfly combines, per frequency, the partial spectra of the G rows
-//    of all C CTAs, read through distributed shared memory (decimation in time over
-//    the C G sub-sequences x[n + C G u]). The inverse runs the same steps backwards.
-//    With C = 1, G = 1 and the row is one local transform.
-//  * The local transform is an in-place Stockham autosort FFT in padded
-//    shared memory: each thread keeps E = 2^LOGE samples in registers per pass,
-//    runs radix-2^r butterflies on them, and writes them back in Stockham order,
-//    so no bit reversal is needed and input and output are both in natural order.
-//  * Twiddles come from per-size tables w_n[m] = exp(-2 pi i m / n), computed in
-//    FP64 on the host and rounded to T.
+// N = A B, both powers of two. Forward (decimation in frequency):
+//   first pass   thread i < B takes the A samples x[i + B r] straight from global memory (a
+//                warp's loads are consecutive), a radix-A butterfly in registers, the twiddles
+//                w_N^{i k_1}, and hands output k_1 to sub-row k_1 in shared memory;
+//   row passes   sub-row k_1 (B samples y_{k_1}) is transformed in place by B / A threads, up to
+//                8192 samples a warp or less: radices R_1, ..., R_m, each pass reading
+//                and writing the same positions, so that one synchronisation of those
+//                threads separates two passes;
+//   last pass    leaves X[k_1 + A k_2] in registers, where the caller works on it.
+// The inverse runs the same steps backwards with conjugate twiddles, from registers to
+// registers: x[i + B r] ends in the thread that stores it. A spectrum is never put in natural
+// order: it is stored in the order of the last pass (SpecLayout, radix_plan.h).
 //
-// Frequency-domain samples stay in shared memory in the "combined layout" (Geo::freq_of:
-// C G spans of CH consecutive frequencies per CTA). Time-domain samples: local row g,
-// column v holds time g + G (rank + C v); kernels walk them in time order with
-// Geo::time_of_w / Geo::local_of_w, so that a warp's accesses cover whole sectors.
+// With C > 1 the CTA of rank c takes i in [c B/C, (c+1) B/C) in the first pass and keeps the
+// sub-rows [c A/C, (c+1) A/C): the first pass's outputs go to their owners through
+// distributed shared memory, and the inverse's last step reads them back. Every sample sees the same
+// operations in the same order whatever C is, so the bits of a transform do not depend on how
+// many CTAs share the row, and C may follow the number of rows at hand.
+// (What it measured: see k_nu.)
 #pragma once
 
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "radix_plan.h"
 
 namespace mmp {
 namespace cg = cooperative_groups;
@@ -81,6 +78,14 @@ __device__ __forceinline__ V twiddle_const(V v) {
   }
 }
 
+// Complex sums as one packed two-lane operation in FP32 (add.rn.f32x2, and fma.rn.f32x2 by
+// -1, which rounds as the subtraction does); the rotated pair of a radix-4 butterfly crosses
+// the lanes and stays scalar.
+__device__ __forceinline__ float2 pk_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 pk_sub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ double2 pk_add(double2 a, double2 b) { return cadd(a, b); }
+__device__ __forceinline__ double2 pk_sub(double2 a, double2 b) { return csub(a, b); }
+
 // In-register DFT of size R (power of two <= 32), natural order in and out.
 template <int R, bool INV> struct RegDFT;
 
@@ -90,18 +95,18 @@ template <bool INV> struct RegDFT<1, INV> {
 template <bool INV> struct RegDFT<2, INV> {
   template <typename V> __device__ __forceinline__ static void run(V* v) {
     const V a = v[0], b = v[1];
-    v[0] = cadd(a, b);
-    v[1] = csub(a, b);
+    v[0] = pk_add(a, b);
+    v[1] = pk_sub(a, b);
   }
 };
 template <bool INV> struct RegDFT<4, INV> {
   template <typename V> __device__ __forceinline__ static void run(V* v) {
     const V a = v[0], b = v[1], c = v[2], d = v[3];
-    const V apc = cadd(a, c), amc = csub(a, c), bpd = cadd(b, d);
-    const V rot = crot<INV>(csub(b, d));  // forward: -i (b-d); inverse: +i (b-d)
-    v[0] = cadd(apc, bpd);
+    const V apc = pk_add(a, c), amc = pk_sub(a, c), bpd = pk_add(b, d);
+    const V rot = crot<INV>(pk_sub(b, d));  // forward: -i (b-d); inverse: +i (b-d)
+    v[0] = pk_add(apc, bpd);
     v[1] = cadd(amc, rot);
-    v[2] = csub(apc, bpd);
+    v[2] = pk_sub(apc, bpd);
     v[3] = csub(amc, rot);
   }
 };
@@ -145,311 +150,223 @@ template <int R, bool INV> struct RegDFT {
   }
 };
 
-
-// Twiddle tables: tw.f[L] / tw.d[L] point at 2^L entries exp(-2 pi i m / 2^L).
-// cf[L][xc] / cd[L][xc]: the cluster combine's twiddles of a split row of 2^L samples
-// (row split xc), [n][kl] = exp(-2 pi i n kl / 2^L) for n < CG, kl < 2^L / CG (CG = C G of
-// that geometry), so that a warp's lanes (consecutive kl) read consecutive entries; null
-// where not built (the combine then reads the 2^L table at n kl).
-struct TwTables {
-  const float2* f[17];
-  const double2* d[17];
-  const float2* cf[17][2];
-  const double2* cd[17][2];
-};
-template <typename T> __device__ __forceinline__ const c2<T>* tw_table(const TwTables& t, int L);
-template <> __device__ __forceinline__ const float2* tw_table<float>(const TwTables& t, int L) { return t.f[L]; }
-template <> __device__ __forceinline__ const double2* tw_table<double>(const TwTables& t, int L) { return t.d[L]; }
-template <typename T> __device__ __forceinline__ const c2<T>* cmb_table(const TwTables& t, int L, int xc);
-template <> __device__ __forceinline__ const float2* cmb_table<float>(const TwTables& t, int L, int xc) { return t.cf[L][xc]; }
-template <> __device__ __forceinline__ const double2* cmb_table<double>(const TwTables& t, int L, int xc) { return t.cd[L][xc]; }
-
-// Geometry of one row transform.
+// Geometry of one row transform; the minimal cluster keeps at most 128 KB of a row per CTA,
+// XC widens it 2^XC times.
 template <typename T, int LOGN_, int XC_ = 0> struct Geo {
   using Real = T;
+  static constexpr bool FP64 = sizeof(T) == 8;
   static constexpr int LOGN = LOGN_;
   static constexpr int N = 1 << LOGN;
-  static constexpr int LOGSZ = sizeof(c2<T>) == 8 ? 3 : 4;
-  static constexpr int LOGC = ((LOGN + LOGSZ > 17) ? (LOGN + LOGSZ - 17) : 0) + XC_;  // <= 128 KB of row per CTA, times 2^XC_ CTAs
+  static constexpr int LOGSZ = FP64 ? 4 : 3;
+  static constexpr int LOGC = ((LOGN + LOGSZ > 17) ? (LOGN + LOGSZ - 17) : 0) + XC_;
   static constexpr int C = 1 << LOGC;
-  static constexpr int LOGL = LOGN - LOGC;
-  static constexpr int NL = 1 << LOGL;
-  // runs of G samples (32 bytes) per CTA on split rows; G rows of NLG in shared memory
-  static constexpr int LOGG = LOGC > 0 ? 5 - LOGSZ : 0;
-  static constexpr int G = 1 << LOGG;
-  static constexpr int LOGNLG = LOGL - LOGG;
-  static constexpr int NLG = 1 << LOGNLG;
-  static constexpr int LOGE_PREF = (sizeof(T) == 4 && LOGL >= 13) ? 5 : 4;
-  static constexpr int LOGE_CAP = LOGL - 5 > 1 ? LOGL - 5 : 1;  // keep >= 32 threads
-  static constexpr int LOGE = LOGE_PREF < LOGE_CAP ? LOGE_PREF : LOGE_CAP;
-  static constexpr int E = 1 << LOGE;
-  static constexpr int NTHR = NL / E;
-  static constexpr int LOGCH = LOGNLG - LOGC;
-  static constexpr int CH = 1 << LOGCH;  // frequencies per span: C G spans per CTA
-  // twiddle table of the local size in shared memory: half a wave (one sign flip per
-  // lookup) where that is at most 32 KB, else a quarter wave (a quadrant fold per lookup;
-  // a 64 KB table cost the 16384-sample single-CTA rows ~5% in loading it)
-  static constexpr bool TW_HALF = (NLG / 2) * (int)sizeof(c2<T>) <= 32 * 1024;
-  static constexpr int LOGH = TW_HALF ? LOGNLG - 1 : LOGNLG - 2;  // log2 of the table's entries
-  static constexpr int NTW = 1 << LOGH;
-  // rows g > 0 start SKEW elements later (mod 128 bytes), so that a warp walking the
-  // samples in time order (row g = lane mod G) reads and writes without bank conflicts
-  static constexpr int SKEW = LOGG > 0 ? 4 : 0;
-  static constexpr int DATA_BYTES = (padded_len(NL) + (G - 1) * SKEW) * (int)sizeof(c2<T>);
-  static constexpr int TW_BYTES = padded_len(NTW) * (int)sizeof(c2<T>);
-  static constexpr int SMEM_BYTES = DATA_BYTES + TW_BYTES;
-  // split rows (XC_ > 0) are sized so that two CTAs share an SM
-  static constexpr int MIN_BLOCKS = (XC_ > 0 && SMEM_BYTES <= 110 * 1024 && NTHR <= 512) ? 2 : 1;
-  static_assert(LOGE >= LOGC + LOGG, "each thread must combine at least one frequency per CTA");
-  static_assert(LOGNLG - LOGE >= 5 || LOGG == 0, "a warp's butterflies stay within one row");
-  static_assert(NTHR >= 32 && NTHR <= 1024, "block size");
-  static_assert(DATA_BYTES % 16 == 0, "twiddle table alignment");
+  static constexpr int NL = N / C;
+  static constexpr RadixPlan PLAN = radix_plan(LOGN);
+  static constexpr int NP = PLAN.n;          // passes
+  static constexpr int LOGA = PLAN.r[0], A = 1 << LOGA;
+  static constexpr int E = A;                // samples per thread
+  static constexpr int LOGB = LOGN - LOGA, B = 1 << LOGB;
+  static constexpr int LOGRM = PLAN.r[NP - 1], RM = 1 << LOGRM;  // last pass
+  static constexpr int NBF = E / RM;         // its butterflies per thread
+  static constexpr int RPC = A / C;          // sub-rows per CTA
+  static constexpr int TPR = B / E;          // threads per sub-row
+  static constexpr int NTHR = RPC * TPR;     // = B / C
+  // length (log2) of the blocks row pass p works on
+  __host__ __device__ static constexpr int loglen(int p) {
+    int l = LOGB;
+    for (int i = 1; i < p; ++i) l -= PLAN.r[i];
+    return l;
+  }
+  // Shared positions are padded by one sample per bank row (16 samples in FP32, 8 in FP64), so
+  // that a pass reading and writing at any power-of-two stride spreads over the banks; rows
+  // served by less than a bank row of threads start TPR banks apart.
+  static constexpr int SLOTS = FP64 ? 8 : 16;
+  __host__ __device__ static constexpr int pad(int x) { return x + x / SLOTS; }
+  static constexpr int RS0 = pad(B);
+  static constexpr int RS = TPR < SLOTS ? RS0 + ((TPR - RS0) % SLOTS + SLOTS) % SLOTS : RS0;
+  static constexpr int SMEM_BYTES = RPC * RS * (int)sizeof(c2<T>);
+  // 64 registers a thread in FP32 (1024 threads on an SM), 128 in FP64
+  static constexpr int REG_BLOCKS = (FP64 ? 512 : 1024) / NTHR;
+  static constexpr int MEM_BLOCKS = 222 * 1024 / (SMEM_BYTES + 2048);
+  static constexpr int MIN_BLOCKS = REG_BLOCKS < MEM_BLOCKS ? (REG_BLOCKS < 16 ? REG_BLOCKS : 16) : MEM_BLOCKS;
+  static constexpr int SYNC_ROWS = RPC > 15 ? 2 : 1;  // sub-rows that share a named barrier
+  static_assert(RPC >= 1 && TPR >= 1 && NTHR >= 32 && REG_BLOCKS >= 1, "block size");
+  static_assert(MEM_BLOCKS >= 1, "the row fits");
 
-  // shared-memory offset of local index i (row i >> LOGNLG)
-  __host__ __device__ __forceinline__ static int sidx(int i) { return pad(i) + (i >> LOGNLG) * SKEW; }
-  // Spectrum layout in shared memory after a forward transform ("combined layout"):
-  // local index i holds frequency rank*CH + (i mod CH) + NLG*(i div CH); for C = 1
-  // that is just i.
-  __device__ __forceinline__ static int freq_of(int rank, int i) {
-    if constexpr (C == 1) return i;
-    else return rank * CH + (i & (CH - 1)) + NLG * (i >> LOGCH);
+  // The last pass's butterfly b (q_1, ..., q_{m-1}, q_1 most significant): the frequencies
+  // it produces are freq0(k1, b) + r KSTR, stored at spec0(k1, b) + r SSTR, r < RM.
+  static constexpr int KSTR = N / RM;
+  static constexpr int SSTR = B / RM;
+  template <int P = 1, int POS = 0, int LOW = LOGB - LOGRM> __device__ __forceinline__ static int digits(int b) {
+    if constexpr (P < NP - 1) {  // digits of b from the top
+      constexpr int R = PLAN.r[P];
+      return (((b >> (LOW - R)) & ((1 << R) - 1)) << POS) + digits<P + 1, POS + R, LOW - R>(b);
+    } else {
+      return 0;
+    }
   }
-  // The CTA's time samples in time order, w < NL: time and local index of the w-th.
-  __device__ __forceinline__ static int time_of_w(int rank, int w) {
-    if constexpr (C == 1) return w;
-    else return ((((w >> LOGG) << LOGC) + rank) << LOGG) + (w & (G - 1));
-  }
-  __device__ __forceinline__ static int local_of_w(int w) {
-    if constexpr (C == 1) return w;
-    else return ((w & (G - 1)) << LOGNLG) + (w >> LOGG);
-  }
+  __device__ __forceinline__ static int freq0(int k1, int b) { return k1 + (digits(b) << LOGA); }
+  __device__ __forceinline__ static int spec0(int k1, int b) { return (k1 << LOGB) + b; }
 };
 
-// exp(-2 pi i m / NLG) (conjugated for INV), m < NLG, from the table
-// sh[pad(m')] = exp(-2 pi i m' / NLG), m' < 2^LOGH: a half wave (w(m) = -sh[m - NLG/2] from
-// NLG/2 on) or a quarter wave (w(m) = (-i)^(m div NLG/4) sh[m mod NLG/4]).
-// The table uses the same padded index as the data: the Stockham passes read it at
-// strides of 2^a entries, which would otherwise land in one bank.
-template <typename V, bool INV, bool HALF, int LOGH>
-__device__ __forceinline__ V tw_lookup(const V* __restrict__ sh, int m) {
-  const int q = m >> LOGH;
-  V w = sh[pad(m & ((1 << LOGH) - 1))];
-  if constexpr (HALF) {
-    if (q) { w.x = -w.x; w.y = -w.y; }
-  } else {
-    const V w0 = w;
-    w.x = (q & 1) ? w0.y : w0.x;
-    w.y = (q & 1) ? -w0.x : w0.y;
-    if (q & 2) { w.x = -w.x; w.y = -w.y; }
+// Where frequency k of a spectrum in storage order `l` lies (kernels that meet another
+// geometry's order; the stage kernels step through their own).
+__device__ __forceinline__ int spec_pos(const SpecLayout& l, int k) {
+  if (l.n == 0) return k;
+  const int k1 = k & ((1 << l.loga) - 1);
+  int rest = k >> l.loga, b = 0;
+  for (int p = 0; p + 1 < l.n; ++p) {
+    b = (b << l.r[p]) | (rest & ((1 << l.r[p]) - 1));
+    rest >>= l.r[p];
   }
-  if (INV) w.y = -w.y;
-  return w;
+  return (k1 << l.logb) + (rest << (l.logb - l.r[l.n - 1])) + b;
 }
 
-// Copy the first 2^LOGH entries of the local transform's table (NLG points) into shared memory.
-template <typename T, int LOGN, int XC>
-__device__ __forceinline__ c2<T>* load_twiddles(unsigned char* smem_raw, const TwTables& tw) {
-  using Gm = Geo<T, LOGN, XC>;
-  c2<T>* sq = reinterpret_cast<c2<T>*>(smem_raw + Gm::DATA_BYTES);
-  const c2<T>* g = tw_table<T>(tw, Gm::LOGNLG);
-#pragma unroll 4
-  for (int m = threadIdx.x; m < Gm::NTW; m += Gm::NTHR) sq[pad(m)] = __ldg(&g[m]);
-  return sq;
+template <bool CONJ, typename V> __device__ __forceinline__ V twiddle(V v, V w) {
+  return CONJ ? cmulc(v, w) : cmul(v, w);
 }
 
-// One in-place Stockham pass of radix 2^LOGR at stride Ns = 2^logns (runtime) over the
-// rows of Gm (G rows of NLG samples; a thread's butterflies j < NL/R, row j / (NLG/R)).
-// Shared-memory offsets: where a butterfly's R elements lie 32·c apart within a row, the
-// padded offset advances by a constant (pad(i + 32c) = pad(i) + 33c), so only the first
-// is computed.
-template <typename Gm, int LOGR, bool INV>
-__device__ __forceinline__ void stockham_pass(c2<typename Gm::Real>* __restrict__ s,
-                                              const c2<typename Gm::Real>* __restrict__ sq, int logns) {
-  using V = c2<typename Gm::Real>;
-  constexpr int LOGB = Gm::LOGNLG;  // row length
-  constexpr int NB = 1 << LOGB, E = Gm::E, NTHR = Gm::NTHR;
-  constexpr int R = 1 << LOGR, NBF = E / R;
-  constexpr int LOGJ = LOGB - LOGR;  // butterflies per row
-  constexpr int S = NB / R;          // read stride
-  const int tid = threadIdx.x;
-  V v[E];
-#pragma unroll
-  for (int bf = 0; bf < NBF; ++bf) {
-    const int ja = tid + bf * NTHR;
-    const int base = (ja >> LOGJ) << LOGB, j = ja & ((1 << LOGJ) - 1);
-    if constexpr (S % 32 == 0) {
-      const int a0 = Gm::sidx(base + j);
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[bf * R + r] = s[a0 + r * (S + S / 32)];
-    } else {
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[bf * R + r] = s[Gm::sidx(base + j + r * S)];
-    }
-  }
-  __syncthreads();
-  const int nsm = (1 << logns) - 1;
-#pragma unroll
-  for (int bf = 0; bf < NBF; ++bf) {
-    const int ja = tid + bf * NTHR;
-    const int base = (ja >> LOGJ) << LOGB, j = ja & ((1 << LOGJ) - 1);
-    const int jm = j & nsm;
-    if (logns > 0) {
-      const int step = jm << (LOGB - logns - LOGR);  // jm * NB / (Ns * R)
-#pragma unroll
-      for (int r = 1; r < R; ++r) v[bf * R + r] = cmul(v[bf * R + r], tw_lookup<V, INV, Gm::TW_HALF, Gm::LOGH>(sq, r * step));
-    }
-    RegDFT<R, INV>::run(&v[bf * R]);
-    const int idxD = ((j >> logns) << (logns + LOGR)) + jm;
-    const int w0 = Gm::sidx(base + idxD);
-    if (logns >= 5) {  // R elements Ns apart, Ns a multiple of 32
-      const int st = (1 << logns) + (1 << (logns - 5));
-#pragma unroll
-      for (int r = 0; r < R; ++r) s[w0 + r * st] = v[bf * R + r];
-    } else if (logns == 0) {  // R consecutive elements from a multiple of R (R <= 32)
-#pragma unroll
-      for (int r = 0; r < R; ++r) s[w0 + r] = v[bf * R + r];
-    } else {
-#pragma unroll
-      for (int r = 0; r < R; ++r) s[Gm::sidx(base + idxD + (r << logns))] = v[bf * R + r];
-    }
-  }
-  __syncthreads();
+// Cluster-wide barrier in two halves (every thread of every CTA arrives, then waits).
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// A row kernel on a cluster announces that it runs, before any peer writes to its shared memory
+// (row_first waits for that), and leaves only when no peer reads it any more (row_leave).
+template <typename Gm> __device__ __forceinline__ void row_enter() {
+  if constexpr (Gm::C > 1) cluster_arrive();
+}
+template <typename Gm> __device__ __forceinline__ void row_leave() {
+  if constexpr (Gm::C > 1) cluster_wait();
 }
 
-// Local transform of the G rows of NLG samples in shared memory (natural order in and
-// out, unnormalised). One pass body per radix keeps the instruction footprint small.
-template <typename T, int LOGN, int XC, bool INV>
-__device__ __noinline__ void local_fft(c2<T>* __restrict__ s, const c2<T>* __restrict__ sq) {
-  using Gm = Geo<T, LOGN, XC>;
-  constexpr int FULL = Gm::LOGNLG / Gm::LOGE, REM = Gm::LOGNLG % Gm::LOGE;
-  __syncthreads();
-  int logns = 0;
-#pragma unroll 1
-  for (int p = 0; p < FULL; ++p) {
-    stockham_pass<Gm, Gm::LOGE, INV>(s, sq, logns);
-    logns += Gm::LOGE;
-  }
-  if constexpr (REM > 0) stockham_pass<Gm, REM, INV>(s, sq, logns);
+// Threads of one sub-row: between two of its passes.
+template <typename Gm> __device__ __forceinline__ void row_sync() {
+  if constexpr (Gm::TPR <= 32) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / (Gm::TPR * Gm::SYNC_ROWS)), "n"(Gm::TPR * Gm::SYNC_ROWS) : "memory");
 }
 
-// w[n] = w_N^{n kl}, 0 < n < CG: row n of the combine table at kl, or the N-point table
-// at n kl where no combine table is given.
+// First pass, forward: v[r] = x[i + B r], i = rank NTHR + tid, into the sub-rows. Ends at a
+// barrier of all the row's threads (which also publishes whatever else the CTA has staged).
 template <typename Gm>
-__device__ __forceinline__ void combine_twiddles(c2<typename Gm::Real>* w, const c2<typename Gm::Real>* twc,
-                                                 const c2<typename Gm::Real>* twN, int kl) {
-  constexpr int CG = Gm::C * Gm::G;
-  if (twc) {
+__device__ __forceinline__ void row_first(c2<typename Gm::Real>* v, c2<typename Gm::Real>* s,
+                                          const c2<typename Gm::Real>* __restrict__ tw, int rank) {
+  using V = c2<typename Gm::Real>;
+  const int i = rank * Gm::NTHR + (int)threadIdx.x;
+  const V* w = tw + i;
+  RegDFT<Gm::A, false>::run(v);
 #pragma unroll
-    for (int n = 1; n < CG; ++n) w[n] = __ldg(&twc[n * Gm::NLG + kl]);
-  } else {
+  for (int k = 1; k < Gm::A; ++k) v[k] = twiddle<false>(v[k], __ldg(w + k * Gm::B));
+  if constexpr (Gm::C == 1) {
+    V* d = s + Gm::pad(i);
 #pragma unroll
-    for (int n = 1; n < CG; ++n) w[n] = __ldg(&twN[n * kl]);
-  }
-}
-
-// Forward transform of the time samples in shared memory (row g, column v: time
-// g + G (rank + C v)); leaves the spectrum in shared memory in the combined layout
-// (Geo::freq_of). Row g of CTA c is the sub-sequence x[n + CG u], n = g + G c, u < NLG
-// (CG = C G), so with F_n its local NLG-point spectrum (decimation in time):
-//   X[kl + NLG j] = sum_n w_CG^{n j} w_N^{n kl} F_n[kl],  kl < NLG, j < CG.
-// A thread handles K = E / CG values kl = rank CH + i, i = tid + jj NTHR: CG inputs each
-// (G rows in each of the C CTAs), one radix-CG DFT, CG outputs, all of them frequencies
-// this CTA keeps (span j, offset i). Every remote read is issued before the cluster
-// barrier that lets the CTAs overwrite their rows. Out of line: its registers are its own.
-template <typename T, int LOGN, int XC>
-__device__ __noinline__ void combine_fwd(c2<T>* __restrict__ s, const TwTables& tw) {
-  using Gm = Geo<T, LOGN, XC>;
-  using V = c2<T>;
-  if constexpr (Gm::C > 1) {
-    constexpr int C = Gm::C, G = Gm::G, CG = C * G, K = Gm::E / CG;
-    cg::cluster_group cl = cg::this_cluster();
-    const int rank = (int)cl.block_rank();
-    const int tid = threadIdx.x;
-    const V* twN = tw_table<T>(tw, Gm::LOGN);
-    V v[K][CG];
-    cl.sync();  // every CTA finished its local transforms
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      const V* peer = cl.map_shared_rank(s, c);
-#pragma unroll
-      for (int jj = 0; jj < K; ++jj) {
-        const int kl = rank * Gm::CH + tid + jj * Gm::NTHR;
-#pragma unroll
-        for (int g = 0; g < G; ++g) v[jj][g + G * c] = peer[Gm::sidx(g * Gm::NLG + kl)];
-      }
-    }
-    const V* twc = cmb_table<T>(tw, Gm::LOGN, XC);
-#pragma unroll
-    for (int jj = 0; jj < K; ++jj) {
-      const int kl = rank * Gm::CH + tid + jj * Gm::NTHR;
-      V w[CG];
-      combine_twiddles<Gm>(w, twc, twN, kl);
-#pragma unroll
-      for (int n = 1; n < CG; ++n) v[jj][n] = cmul(v[jj][n], w[n]);
-      RegDFT<CG, false>::run(v[jj]);
-    }
-    cl.sync();  // all peer reads done before shared memory is overwritten
-#pragma unroll
-    for (int jj = 0; jj < K; ++jj) {
-      const int i = tid + jj * Gm::NTHR;
-#pragma unroll
-      for (int j = 0; j < CG; ++j) s[Gm::sidx(j * Gm::CH + i)] = v[jj][j];
-    }
+    for (int k = 0; k < Gm::A; ++k) d[k * Gm::RS] = v[k];
     __syncthreads();
+  } else {
+    cg::cluster_group cl = cg::this_cluster();
+    cluster_wait();  // every CTA of the cluster runs
+#pragma unroll
+    for (int c = 0; c < Gm::C; ++c) {
+      V* d = cl.map_shared_rank(s, c) + Gm::pad(i);
+#pragma unroll
+      for (int k = 0; k < Gm::RPC; ++k) d[k * Gm::RS] = v[c * Gm::RPC + k];
+    }
+    cluster_arrive();
+    cluster_wait();
   }
-}
-template <typename T, int LOGN, int XC>
-__device__ __forceinline__ void forward(c2<T>* __restrict__ s, const c2<T>* __restrict__ sq, const TwTables& tw) {
-  local_fft<T, LOGN, XC, false>(s, sq);
-  if constexpr (Geo<T, LOGN, XC>::C > 1) combine_fwd<T, LOGN, XC>(s, tw);
 }
 
-// Inverse transform of a spectrum in shared memory in the combined layout; leaves
-// the (unnormalised) time samples in shared memory (row g, column v: time
-// g + G (rank + C v)): the forward steps backwards with conjugate twiddles.
-template <typename T, int LOGN, int XC>
-__device__ __noinline__ void combine_inv(c2<T>* __restrict__ s, const TwTables& tw) {
-  using Gm = Geo<T, LOGN, XC>;
-  using V = c2<T>;
-  if constexpr (Gm::C > 1) {
-    constexpr int C = Gm::C, G = Gm::G, CG = C * G, K = Gm::E / CG;
-    cg::cluster_group cl = cg::this_cluster();
-    const int rank = (int)cl.block_rank();
-    const int tid = threadIdx.x;
-    const V* twN = tw_table<T>(tw, Gm::LOGN);
-    V v[K][CG];
-    __syncthreads();  // the caller's writes of the spectrum are complete
-    const V* twc = cmb_table<T>(tw, Gm::LOGN, XC);
+// Row pass P (1 <= P < NP - 1) over this thread's share of its sub-row sr (u-th of TPR).
+template <typename Gm, int P, bool INV>
+__device__ __forceinline__ void row_pass(c2<typename Gm::Real>* sr,
+                                         const c2<typename Gm::Real>* __restrict__ tw, int u) {
+  using V = c2<typename Gm::Real>;
+  constexpr int LOGR = Gm::PLAN.r[P], R = 1 << LOGR;
+  constexpr int LOGL = Gm::loglen(P), LOGS = LOGL - LOGR, S = 1 << LOGS;
 #pragma unroll
-    for (int jj = 0; jj < K; ++jj) {
-      const int i = tid + jj * Gm::NTHR;
-      const int kl = rank * Gm::CH + i;
+  for (int bf = 0; bf < Gm::E / R; ++bf) {
+    const int b = u + Gm::TPR * bf;
+    const int j = b & (S - 1);
+    V* d = sr + Gm::pad(((b >> LOGS) << LOGL) + j);
+    const V* w = tw + j;
+    V v[R];
 #pragma unroll
-      for (int j = 0; j < CG; ++j) v[jj][j] = s[Gm::sidx(j * Gm::CH + i)];
-      RegDFT<CG, true>::run(v[jj]);
-      V w[CG];
-      combine_twiddles<Gm>(w, twc, twN, kl);
+    for (int r = 0; r < R; ++r) v[r] = d[Gm::pad(r * S)];
+    if constexpr (INV) {
 #pragma unroll
-      for (int n = 1; n < CG; ++n) v[jj][n] = cmulc(v[jj][n], w[n]);
+      for (int q = 1; q < R; ++q) v[q] = twiddle<true>(v[q], __ldg(w + q * S));
     }
-    cl.sync();  // every CTA is running and has read its own spectrum
+    RegDFT<R, INV>::run(v);
+    if constexpr (!INV) {
 #pragma unroll
-    for (int c = 0; c < C; ++c) {
-      V* peer = cl.map_shared_rank(s, c);
-#pragma unroll
-      for (int jj = 0; jj < K; ++jj) {
-        const int kl = rank * Gm::CH + tid + jj * Gm::NTHR;
-#pragma unroll
-        for (int g = 0; g < G; ++g) peer[Gm::sidx(g * Gm::NLG + kl)] = v[jj][g + G * c];
-      }
+      for (int q = 1; q < R; ++q) v[q] = twiddle<false>(v[q], __ldg(w + q * S));
     }
-    cl.sync();  // all peer writes landed
+#pragma unroll
+    for (int r = 0; r < R; ++r) d[Gm::pad(r * S)] = v[r];
   }
 }
-template <typename T, int LOGN, int XC>
-__device__ __forceinline__ void inverse(c2<T>* __restrict__ s, const c2<T>* __restrict__ sq, const TwTables& tw) {
-  if constexpr (Geo<T, LOGN, XC>::C > 1) combine_inv<T, LOGN, XC>(s, tw);
-  local_fft<T, LOGN, XC, true>(s, sq);
+
+// All row passes but the last, forward, each followed by its synchronisation; tw points at
+// the row's whole table. OFF: the pass's offset in it.
+template <typename Gm, int P = 1, int OFF = Gm::N>
+__device__ __forceinline__ void rows_fwd(c2<typename Gm::Real>* sr,
+                                         const c2<typename Gm::Real>* __restrict__ tw, int u) {
+  if constexpr (P < Gm::NP - 1) {
+    row_pass<Gm, P, false>(sr, tw + OFF, u);
+    row_sync<Gm>();
+    rows_fwd<Gm, P + 1, OFF + (1 << Gm::loglen(P))>(sr, tw, u);
+  }
+}
+// ... inverse, in the opposite order, each preceded by its synchronisation.
+template <typename Gm, int P = 1, int OFF = Gm::N>
+__device__ __forceinline__ void rows_inv(c2<typename Gm::Real>* sr,
+                                         const c2<typename Gm::Real>* __restrict__ tw, int u) {
+  if constexpr (P < Gm::NP - 1) {
+    rows_inv<Gm, P + 1, OFF + (1 << Gm::loglen(P))>(sr, tw, u);
+    row_sync<Gm>();
+    row_pass<Gm, P, true>(sr, tw + OFF, u);
+  }
+}
+
+// The last pass's butterflies of this thread: f(butterfly b, its RM values in shared memory,
+// value r at pad(r)).
+// f runs the forward or inverse radix-RM step (or both) on them.
+template <typename Gm, typename F>
+__device__ __forceinline__ void rows_last(c2<typename Gm::Real>* sr, int u, F&& f) {
+#pragma unroll 1
+  for (int bf = 0; bf < Gm::NBF; ++bf) {
+    const int b = u + Gm::TPR * bf;
+    f(b, sr + Gm::pad(b * Gm::RM));
+  }
+}
+
+// Last step, inverse: v[r] = x[i + B r] (unnormalised), i = rank NTHR + tid. Starts with the
+// barrier after the row passes; the CTA's shared memory must stay until row_leave.
+template <typename Gm>
+__device__ __forceinline__ void row_last_inv(c2<typename Gm::Real>* v, c2<typename Gm::Real>* s,
+                                             const c2<typename Gm::Real>* __restrict__ tw, int rank) {
+  using V = c2<typename Gm::Real>;
+  const int i = rank * Gm::NTHR + (int)threadIdx.x;
+  const V* w = tw + i;
+  if constexpr (Gm::C == 1) {
+    __syncthreads();
+    const V* d = s + Gm::pad(i);
+#pragma unroll
+    for (int k = 0; k < Gm::A; ++k) v[k] = d[k * Gm::RS];
+  } else {
+    cg::cluster_group cl = cg::this_cluster();
+    cluster_arrive();
+    cluster_wait();
+#pragma unroll
+    for (int c = 0; c < Gm::C; ++c) {
+      const V* d = cl.map_shared_rank(s, c) + Gm::pad(i);
+#pragma unroll
+      for (int k = 0; k < Gm::RPC; ++k) v[c * Gm::RPC + k] = d[k * Gm::RS];
+    }
+  }
+#pragma unroll
+  for (int k = 1; k < Gm::A; ++k) v[k] = twiddle<true>(v[k], __ldg(w + k * Gm::B));
+  if constexpr (Gm::C > 1) cluster_arrive();  // this thread has read its peers
+  RegDFT<Gm::A, true>::run(v);
 }
 
 }  // namespace mmp

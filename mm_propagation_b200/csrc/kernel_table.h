@@ -2,6 +2,8 @@
 // (precision, log2 NT) pair by kern_inst.cu.
 #pragma once
 
+#include "radix_plan.h"
+
 namespace mmp {
 
 struct KernelSet {
@@ -21,12 +23,11 @@ struct KernelSet {
   int xc = 0;     // rows split over 2^xc times the minimal number of CTAs
 };
 
-constexpr int kMinLogN = 6;
-constexpr int kMaxLogN = 16;
-
-// Row-split variants built besides xc = 0 (FP32 / FP64 ranges of log2 NT).
-constexpr int kSplitMinLogN32 = 12, kSplitMaxLogN32 = 16;
-constexpr int kSplitMinLogN64 = 11, kSplitMaxLogN64 = 14;
+// Row splits built for rows of 2^logn samples: xc = 0 .. max_split, clusters of 2^xc times the
+// minimal number of CTAs, up to 8 CTAs and down to 32 threads each.
+constexpr int max_split(bool fp64, int logn) {
+  return logn < 11 ? 0 : logn == 11 ? 2 : logn <= 13 ? 3 : fp64 ? 16 - logn : logn == 14 ? 3 : 17 - logn;
+}
 
 // Defined in the kern_inst.cu objects; returns an empty set for variants not built.
 KernelSet kernels_for(int fp64, int logn, int xc = 0);

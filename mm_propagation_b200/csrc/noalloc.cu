@@ -14,8 +14,7 @@
 // the FP64 and FP32 twiddle tables for every supported size followed by a
 // staging buffer of kMaxSamples complex FP64 samples. Every GPU that loads this
 // library holds the array until the process exits. The transform runs in place
-// in the staging buffer (each row is read whole into shared memory before any
-// of it is written), so no second buffer is needed.
+// in the staging buffer (each row is read whole before any of it is written), so no second buffer is needed.
 //
 // Set-up: the first call on a device, with that device current, looks up the
 // array's device address with cudaGetSymbolAddress (host code may not use the
@@ -43,33 +42,38 @@ using namespace mmp;
 
 namespace {
 
-constexpr size_t kTwEntries = ((size_t)1 << (kMaxLogN + 1)) - 2;  // sum over L = 1..16 of 2^L
 constexpr size_t kMaxSamples = (size_t)1 << 20;                  // complex FP64 staging samples
-constexpr size_t kTwD = kTwEntries * sizeof(double2);
-constexpr size_t kTwF = kTwEntries * sizeof(float2);
+constexpr size_t kTwD = kTwiddles * sizeof(double2);
+constexpr size_t kTwF = kTwiddles * sizeof(float2);
 constexpr size_t kStageOff = ((kTwD + kTwF) + 255) & ~(size_t)255;
 constexpr size_t kArenaBytes = kStageOff + kMaxSamples * sizeof(double2);
 
 static __device__ __align__(256) unsigned char g_noalloc_arena[kArenaBytes];
 
-// w_L[m] = exp(-2 pi i m / 2^L) for L = 1..16; table L starts at entry 2^L - 2.
+// The tables of radix_plan.h. One block column per (precision, size).
 __global__ void k_fill_twiddles(double2* d, float2* f) {
-  for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < kTwEntries;
-       g += (size_t)gridDim.x * blockDim.x) {
-    int L = 1;
-    while (((size_t)1 << (L + 1)) - 2 <= g) ++L;
-    const size_t m = g - (((size_t)1 << L) - 2);
-    double s, c;
-    sincospi(-2.0 * (double)m / (double)((size_t)1 << L), &s, &c);
-    d[g] = make_double2(c, s);
-    f[g] = make_float2((float)c, (float)s);
+  const bool fp64 = blockIdx.y != 0;
+  const int L = kMinLogN + (int)blockIdx.z;
+  const RadixPlan pl = radix_plan(L);
+  size_t off = twiddle_offset(L);
+  int len = L;
+  for (int p = 0; p + 1 < pl.n; ++p) {
+    const size_t S = (size_t)1 << (len - pl.r[p]), n = (size_t)1 << len;
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+      double sn, cs;
+      sincospi(-2.0 * (double)((e % S) * (e / S)) / (double)n, &sn, &cs);
+      if (fp64) d[off + e] = make_double2(cs, sn);
+      else f[off + e] = make_float2((float)cs, (float)sn);
+    }
+    off += n;
+    len -= pl.r[p];
   }
 }
 
 struct NoallocDevice {
   bool ready = false;
   unsigned char* base = nullptr;
-  TwTables tw{};
+  const void* tw[2][kMaxLogN + 1] = {};
 };
 std::mutex g_mu;
 constexpr int kMaxDevices = 64;
@@ -100,14 +104,14 @@ int setup(int dev, NoallocDevice** out) {
   r.base = static_cast<unsigned char*>(p);
   double2* d = reinterpret_cast<double2*>(r.base);
   float2* f = reinterpret_cast<float2*>(r.base + kTwD);
-  k_fill_twiddles<<<256, 256>>>(d, f);
+  k_fill_twiddles<<<dim3(32, 2, kMaxLogN - kMinLogN + 1), 256>>>(d, f);
   e = cudaGetLastError();
   if (e == cudaSuccess) mmp_detail::count_launch();
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return fail(MMP_ECUDA, cudaGetErrorString(e));
-  for (int L = 0; L <= kMaxLogN; ++L) {
-    r.tw.d[L] = L ? d + (((size_t)1 << L) - 2) : nullptr;
-    r.tw.f[L] = L ? f + (((size_t)1 << L) - 2) : nullptr;
+  for (int L = kMinLogN; L <= kMaxLogN; ++L) {
+    r.tw[1][L] = d + twiddle_offset(L);
+    r.tw[0][L] = f + twiddle_offset(L);
   }
   for (int fp64 = 0; fp64 < 2; ++fp64)
     for (int L = kMinLogN; L <= kMaxLogN; ++L) {
@@ -151,7 +155,7 @@ int mmp_dft_noalloc(uint32_t n, uint32_t rows, int direction, int fp64, const do
     a.out = stage;
     a.rows = (int)rows;
     a.scale = direction < 0 ? 1.0 : 1.0 / (double)n;
-    a.tw = r->tw;
+    a.tw = r->tw[fp64 ? 1 : 0][lg];
     void* args[] = {&a};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows * (unsigned)ks.C, 1, 1);

@@ -31,43 +31,31 @@ using namespace mmp;
 // ---------------------------------------------------------------------------------------
 // instantiated kernel sets (kern_inst.cu objects)
 #define MMP_DECL(tag, L, X) KernelSet make_kernels_##tag##_##L##_##X();
-#define MMP_DECL_ALL(tag) \
-  MMP_DECL(tag, 6, 0) MMP_DECL(tag, 7, 0) MMP_DECL(tag, 8, 0) MMP_DECL(tag, 9, 0) MMP_DECL(tag, 10, 0) \
-  MMP_DECL(tag, 11, 0) MMP_DECL(tag, 12, 0) MMP_DECL(tag, 13, 0) MMP_DECL(tag, 14, 0) MMP_DECL(tag, 15, 0) \
-  MMP_DECL(tag, 16, 0)
+// every kernel set built: X(tag, log2 NT, row split), max_split(precision, log2 NT) splits each
+#define MMP_SETS_F32(X) \
+  X(f32, 6, 0) X(f32, 7, 0) X(f32, 8, 0) X(f32, 9, 0) X(f32, 10, 0) X(f32, 11, 0) X(f32, 11, 1) X(f32, 11, 2) \
+  X(f32, 12, 0) X(f32, 12, 1) X(f32, 12, 2) X(f32, 12, 3) X(f32, 13, 0) X(f32, 13, 1) X(f32, 13, 2) X(f32, 13, 3) \
+  X(f32, 14, 0) X(f32, 14, 1) X(f32, 14, 2) X(f32, 14, 3) X(f32, 15, 0) X(f32, 15, 1) X(f32, 15, 2) X(f32, 16, 0) \
+  X(f32, 16, 1)
+#define MMP_SETS_F64(X) \
+  X(f64, 6, 0) X(f64, 7, 0) X(f64, 8, 0) X(f64, 9, 0) X(f64, 10, 0) X(f64, 11, 0) X(f64, 11, 1) X(f64, 11, 2) \
+  X(f64, 12, 0) X(f64, 12, 1) X(f64, 12, 2) X(f64, 12, 3) X(f64, 13, 0) X(f64, 13, 1) X(f64, 13, 2) X(f64, 13, 3) \
+  X(f64, 14, 0) X(f64, 14, 1) X(f64, 14, 2) X(f64, 15, 0) X(f64, 15, 1) X(f64, 16, 0)
 namespace mmp {
-MMP_DECL_ALL(f32)
-MMP_DECL_ALL(f64)
-MMP_DECL(f32, 12, 1) MMP_DECL(f32, 13, 1) MMP_DECL(f32, 14, 1) MMP_DECL(f32, 15, 1) MMP_DECL(f32, 16, 1)
-MMP_DECL(f64, 11, 1) MMP_DECL(f64, 12, 1) MMP_DECL(f64, 13, 1) MMP_DECL(f64, 14, 1)
+MMP_SETS_F32(MMP_DECL)
+MMP_SETS_F64(MMP_DECL)
 
 KernelSet kernels_for(int fp64, int logn, int xc) {
-#define MMP_CASE(tag, L, X) case L: return make_kernels_##tag##_##L##_##X();
-  if (xc == 1) {
-    if (fp64) {
-      switch (logn) {
-        MMP_CASE(f64, 11, 1) MMP_CASE(f64, 12, 1) MMP_CASE(f64, 13, 1) MMP_CASE(f64, 14, 1)
-        default: return KernelSet();
-      }
-    }
-    switch (logn) {
-      MMP_CASE(f32, 12, 1) MMP_CASE(f32, 13, 1) MMP_CASE(f32, 14, 1) MMP_CASE(f32, 15, 1) MMP_CASE(f32, 16, 1)
-      default: return KernelSet();
-    }
-  }
-  if (xc != 0) return KernelSet();
+#define MMP_CASE(tag, L, X) case 4 * L + X: return make_kernels_##tag##_##L##_##X();
+  if (xc < 0 || xc > 3) return KernelSet();
   if (fp64) {
-    switch (logn) {
-      MMP_CASE(f64, 6, 0) MMP_CASE(f64, 7, 0) MMP_CASE(f64, 8, 0) MMP_CASE(f64, 9, 0) MMP_CASE(f64, 10, 0)
-      MMP_CASE(f64, 11, 0) MMP_CASE(f64, 12, 0) MMP_CASE(f64, 13, 0) MMP_CASE(f64, 14, 0) MMP_CASE(f64, 15, 0)
-      MMP_CASE(f64, 16, 0)
+    switch (4 * logn + xc) {
+      MMP_SETS_F64(MMP_CASE)
       default: return KernelSet();
     }
   }
-  switch (logn) {
-    MMP_CASE(f32, 6, 0) MMP_CASE(f32, 7, 0) MMP_CASE(f32, 8, 0) MMP_CASE(f32, 9, 0) MMP_CASE(f32, 10, 0)
-    MMP_CASE(f32, 11, 0) MMP_CASE(f32, 12, 0) MMP_CASE(f32, 13, 0) MMP_CASE(f32, 14, 0) MMP_CASE(f32, 15, 0)
-    MMP_CASE(f32, 16, 0)
+  switch (4 * logn + xc) {
+    MMP_SETS_F32(MMP_CASE)
     default: return KernelSet();
   }
 #undef MMP_CASE
@@ -164,12 +152,13 @@ void dev_free(void* p, cudaStream_t st = nullptr, bool pooled = false) {
 constexpr int kScanSmem = padded_len(128 * 1024 / 8) * 8;
 // Dynamic shared memory k_contract may take (the 227 KB per block, less its static part)
 constexpr size_t kContractSmemMax = 226 * 1024;
+constexpr int kSMs = 148;  // of a B200
 
 // ---- per-device resources: twiddle tables, kernel attributes ------------------------------
 struct DeviceRes {
   bool ready = false;
-  TwTables tw{};
   void* tw_mem = nullptr;
+  const void* tw[2][kMaxLogN + 1] = {};  // [precision][log2 size]: twiddle tables (radix_plan.h)
 };
 std::mutex g_dev_mu;
 std::map<int, DeviceRes> g_dev;
@@ -182,81 +171,55 @@ int ensure_device(int dev, DeviceRes** out) {
   CUDA_TRY(cudaGetDeviceProperties(&prop, dev));
   if (prop.major < 10) return fail(MMP_ENODEV, "device is not sm_100 (compute capability " +
                                    std::to_string(prop.major) + "." + std::to_string(prop.minor) + ")");
-  // twiddle tables w_L[m] = exp(-2 pi i m / 2^L), L = 1..16, in FP64 and FP32
-  size_t n_tot = 0;
-  for (int L = 1; L <= kMaxLogN; ++L) n_tot += (size_t)1 << L;
-  std::vector<double2> hd(n_tot);
-  std::vector<float2> hf(n_tot);
-  size_t off = 0;
-  std::vector<size_t> offs(kMaxLogN + 1, 0);
-  for (int L = 1; L <= kMaxLogN; ++L) {
-    offs[L] = off;
-    const size_t n = (size_t)1 << L;
-    for (size_t m = 0; m < n; ++m) {
-      const double a = -2.0 * M_PI * (double)m / (double)n;
-      hd[off + m] = make_double2(std::cos(a), std::sin(a));
-      hf[off + m] = make_float2((float)hd[off + m].x, (float)hd[off + m].y);
+  // w[m] = exp(-2 pi i m / 2^kMaxLogN); every table entry is one of them
+  constexpr size_t kWave = (size_t)1 << kMaxLogN;
+  std::vector<double2> wave(kWave);
+  for (size_t m = 0; m < kWave; ++m) {
+    const double a = -2.0 * M_PI * (double)m / (double)kWave;
+    wave[m] = make_double2(std::cos(a), std::sin(a));
+  }
+  std::vector<double2> hd(kTwiddles);
+  std::vector<float2> hf(kTwiddles);
+  for (int L = kMinLogN; L <= kMaxLogN; ++L) {
+    const RadixPlan pl = radix_plan(L);
+    size_t e = twiddle_offset(L);
+    int len = L;
+    for (int p = 0; p + 1 < pl.n; ++p) {
+      const size_t S = (size_t)1 << (len - pl.r[p]), R = (size_t)1 << pl.r[p];
+      for (size_t q = 0; q < R; ++q)
+        for (size_t jj = 0; jj < S; ++jj, ++e) {
+          hd[e] = wave[(jj * q) << (kMaxLogN - len)];
+          hf[e] = make_float2((float)hd[e].x, (float)hd[e].y);
+        }
+      len -= pl.r[p];
     }
-    off += n;
   }
-  // the split rows' combine tables, [n][kl] = w_L[n kl] (n < CG, kl < 2^L / CG), gathered
-  // from the tables above, so that they hold the same values
-  struct Cmb { int fp64, L, xc; size_t off; };
-  std::vector<Cmb> cm;
-  size_t cbytes = 0;
-  for (int fp64 = 0; fp64 < 2; ++fp64)
-    for (int L = kMinLogN; L <= kMaxLogN; ++L)
-      for (int xc = 0; xc < 2; ++xc) {
-        const KernelSet ks = kernels_for(fp64, L, xc);
-        if (!ks.prime || ks.C < 2) continue;
-        cm.push_back({fp64, L, xc, cbytes});
-        cbytes += ((size_t)1 << L) * (fp64 ? sizeof(double2) : sizeof(float2));
-      }
-  std::vector<unsigned char> hc(cbytes);
-  for (const Cmb& c : cm) {
-    const KernelSet ks = kernels_for(c.fp64, c.L, c.xc);
-    const size_t n = (size_t)1 << c.L;
-    const size_t CG = (size_t)ks.C * (c.fp64 ? 2 : 4);  // C times the run length G (32 bytes)
-    for (size_t kl = 0; kl < n / CG; ++kl)
-      for (size_t q = 0; q < CG; ++q) {
-        const size_t m = q * kl, e = q * (n / CG) + kl;
-        if (c.fp64) reinterpret_cast<double2*>(hc.data() + c.off)[e] = hd[offs[c.L] + m];
-        else reinterpret_cast<float2*>(hc.data() + c.off)[e] = hf[offs[c.L] + m];
-      }
-  }
-  // one allocation: FP64 tables | FP32 tables | combine tables
+  // one allocation: FP64 tables | FP32 tables
   void* mem = nullptr;
-  CUDA_TRY(dev_malloc(&mem, n_tot * (sizeof(double2) + sizeof(float2)) + cbytes));
+  CUDA_TRY(dev_malloc(&mem, kTwiddles * (sizeof(double2) + sizeof(float2))));
   double2* dd = (double2*)mem;
-  float2* df = (float2*)(dd + n_tot);
-  unsigned char* dc = (unsigned char*)(df + n_tot);
-  cudaError_t ce = cudaMemcpy(dd, hd.data(), n_tot * sizeof(double2), cudaMemcpyHostToDevice);
-  if (ce == cudaSuccess) ce = cudaMemcpy(df, hf.data(), n_tot * sizeof(float2), cudaMemcpyHostToDevice);
-  if (ce == cudaSuccess && cbytes) ce = cudaMemcpy(dc, hc.data(), cbytes, cudaMemcpyHostToDevice);
+  float2* df = (float2*)(dd + kTwiddles);
+  cudaError_t ce = cudaMemcpy(dd, hd.data(), kTwiddles * sizeof(double2), cudaMemcpyHostToDevice);
+  if (ce == cudaSuccess) ce = cudaMemcpy(df, hf.data(), kTwiddles * sizeof(float2), cudaMemcpyHostToDevice);
   if (ce != cudaSuccess) {
     dev_free(mem);
     return fail(MMP_ECUDA, std::string("twiddle upload: ") + cudaGetErrorString(ce));
   }
-  for (int L = 0; L <= kMaxLogN; ++L) {
-    r.tw.d[L] = L ? dd + offs[L] : nullptr;
-    r.tw.f[L] = L ? df + offs[L] : nullptr;
-  }
-  for (const Cmb& c : cm) {
-    if (c.fp64) r.tw.cd[c.L][c.xc] = (const double2*)(dc + c.off);
-    else r.tw.cf[c.L][c.xc] = (const float2*)(dc + c.off);
+  for (int L = kMinLogN; L <= kMaxLogN; ++L) {
+    r.tw[1][L] = dd + twiddle_offset(L);
+    r.tw[0][L] = df + twiddle_offset(L);
   }
   r.tw_mem = mem;
   // dynamic shared memory opt-in for every instantiated kernel
   for (int fp64 = 0; fp64 < 2; ++fp64)
     for (int L = kMinLogN; L <= kMaxLogN; ++L)
-      for (int xc = 0; xc < 2; ++xc) {
+      for (int xc = 0; xc <= max_split(fp64 != 0, L); ++xc) {
         KernelSet ks = kernels_for(fp64, L, xc);
-        if (!ks.prime) continue;
         std::vector<const void*> fns = {ks.prime, ks.pair, ks.nu, ks.result, ks.dft_fwd, ks.dft_inv};
-        for (const void* f : ks.nu_mid) if (f) fns.push_back(f);
-        for (const void* f : ks.nu_last) if (f) fns.push_back(f);
+        for (const void* f : ks.nu_mid) fns.push_back(f);
+        for (const void* f : ks.nu_last) fns.push_back(f);
         for (const void* f : fns)
-          CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, ks.smem));
+          if (f) CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, ks.smem));
       }
   const void* contract_fns[] = {(const void*)&k_contract<float, 0>,  (const void*)&k_contract<float, 1>,
                                 (const void*)&k_contract<float, 2>,  (const void*)&k_contract<double, 0>,
@@ -701,6 +664,7 @@ struct mmp_batch {
   bool tc = false;  // dense form on the tensor cores (k_contract_tc)
   int pchunk = 0;   // > 0: pair fields per chunk of the pair-chunked contraction (k_contract_pc)
   bool sr = false;  // serial-recurrence contraction in sub-blocks (k_contract_sr)
+  int xc_req = -1;   // row split asked for by MMP_ROW_SPLIT or the autotuner (-1: row_split's)
   int tile_req = 0;  // contraction tile asked for by the autotuner (0: batch_shape's own)
   int tuned = 0;     // 1: launch parameters chosen by timing (autotune)
   std::vector<cudaStream_t> branch;
@@ -769,20 +733,32 @@ int grow_monitors(mmp_batch* b, Member& s, unsigned long long need) {
 }
 
 // launch helpers ------------------------------------------------------------------------
-KParams kparams(mmp_batch* b, int stage, const SolveDesc* descs) {
-  KParams kp;
-  std::memset(&kp, 0, sizeof(kp));
-  kp.descs = descs;
-  kp.tw = b->dev->tw;
-  kp.tab = b->tab;
-  kp.stage = stage;
-  return kp;
+StageArgs stage_args(const Tableau& tab, int i) {
+  StageArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.stage = i;
+  a.last = i == tab.s - 1;
+  for (int j = 0; j < tab.s; ++j) {
+    const double c = a.last ? (j != i ? tab.b[j] : 0.0) : (j < i ? tab.a[i + 1][j] : 0.0);
+    if (c == 0.0) continue;
+    a.jq[a.nq] = j;
+    a.cq[a.nq++] = c;
+  }
+  a.cself = a.last ? tab.b[i] : tab.a[i + 1][i];
+  a.c_this = tab.c[i];
+  a.c_next = a.last ? 1.0 : tab.c[i + 1];
+  return a;
 }
 
 int launch_row_kernel(mmp_batch* b, const KernelSet& ks, const void* fn, int rows, int nsolves, int stage,
                       const SolveDesc* descs, cudaStream_t st = nullptr) {
   if (rows <= 0 || nsolves <= 0) return MMP_OK;
-  KParams kp = kparams(b, stage, descs);
+  KParams kp;
+  std::memset(&kp, 0, sizeof(kp));
+  kp.descs = descs;
+  kp.tw = b->dev->tw[ks.fp64][ks.logn];
+  kp.st = stage_args(b->tab, stage);
+  kp.lay = spec_layout(b->logn);
   void* args[] = {&kp};
   dim3 grid((unsigned)(rows * ks.C), (unsigned)nsolves, 1);
   CUDA_TRY(launch(fn, grid, ks.nthr, ks.smem, ks.C, st ? st : b->stream, args));
@@ -826,19 +802,12 @@ int launch_contract(mmp_batch* b, uint32_t first = 0, uint32_t count = ~0u, cuda
   return MMP_OK;
 }
 
-// The k_nu instantiation for stage i: a stage whose count of stored N_hat_j terms (the
-// count k_nu's thread 0 derives) has a specialised body built takes it; every other
-// stage the generic one.
+// The k_nu instantiation for stage i: the body built for its count of stored N_hat_j, or the
+// any-stage one.
 const void* nu_kernel(const KernelSet& ks, const Tableau& tab, int i) {
-  const bool last = i == tab.s - 1;
-  int nq = 0;
-  if (last) {
-    for (int j = 0; j < tab.s; ++j) nq += (j != i && tab.b[j] != 0.0);
-  } else {
-    for (int j = 0; j < i; ++j) nq += (tab.a[i + 1][j] != 0.0);
-  }
-  if (!last && nq < 6 && ks.nu_mid[nq]) return ks.nu_mid[nq];
-  if (last && nq < 5 && ks.nu_last[nq]) return ks.nu_last[nq];
+  const StageArgs a = stage_args(tab, i);
+  if (!a.last && a.nq < 6 && ks.nu_mid[a.nq]) return ks.nu_mid[a.nq];
+  if (a.last && a.nq < 5 && ks.nu_last[a.nq]) return ks.nu_last[a.nq];
   return ks.nu;
 }
 
@@ -1062,7 +1031,8 @@ int member_set_fields(mmp_batch* b, uint32_t idx, const double* phi0) {
   a.out = s.desc.psi_hat;
   a.rows = (int)s.M;
   a.scale = s.cf;
-  a.tw = b->dev->tw;
+  a.tw = b->dev->tw[1][b->logn];
+  a.lay = spec_layout(b->logn);
   void* args[] = {&a};
   CUDA_TRY(launch(b->ks64.dft_fwd, dim3((unsigned)(s.M * b->ks64.C), 1, 1), b->ks64.nthr, b->ks64.smem,
                   b->ks64.C, b->stream, args));
@@ -1095,10 +1065,9 @@ int batch_open(mmp_batch* b, const mmp_params* p0, const Tableau& tab0) {
   b->nt = p0->nt;
   b->logn = ilog2_exact(p0->nt);
   b->tab = tab0;
-  b->ks = kernels_for(b->fp64 ? 1 : 0, b->logn);
-  if (const char* env = std::getenv("MMP_ROW_SPLIT"))  // 1: rows split over twice the CTAs, where built
-    if (std::atoi(env) == 1 && kernels_for(b->fp64 ? 1 : 0, b->logn, 1).prime)
-      b->ks = kernels_for(b->fp64 ? 1 : 0, b->logn, 1);
+  if (const char* env = std::getenv("MMP_ROW_SPLIT"))  // fixes the row split (where built)
+    if (*env) b->xc_req = std::min(std::max(std::atoi(env), 0), max_split(b->fp64, b->logn));
+  b->ks = kernels_for(b->fp64 ? 1 : 0, b->logn, std::max(b->xc_req, 0));
   b->ks64 = kernels_for(1, b->logn);
   if (!b->ks.prime || !b->ks64.prime) return fail(MMP_ENOTSUP, "no kernels built for this nt");
   b->kernels_per_step = b->tab.s * ((b->raman ? 1 : 0) + 2);
@@ -1410,7 +1379,8 @@ int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
     a.out = h64;
     a.rows = 1;
     a.scale = s.delta_t * s.T0 * s.fR / (double)nt;
-    a.tw = b->dev->tw;
+    a.tw = b->dev->tw[1][b->logn];
+    a.lay = spec_layout(b->logn);
     void* args[] = {&a};
     CUDA_TRY(launch(b->ks64.dft_fwd, dim3((unsigned)b->ks64.C, 1, 1), b->ks64.nthr, b->ks64.smem, b->ks64.C, b->stream, args));
     const void* conv = b->fp64 ? (const void*)&k_to_t2<double> : (const void*)&k_to_t2<float>;
@@ -1640,9 +1610,25 @@ bool joins_same_kernels(const mmp_batch* b, const SolveCounts& c) {
   return empty || same_kernels(choose_shape(b, batch_stats(b)), w);
 }
 
+// Row split for a launch of `rows` rows: the widest cluster that still leaves an SM to every
+// CTA. A transform's bits do not depend on it (fft.cuh), so it may follow what a served pool
+// holds. Measured, microseconds a step (RK4, one branch), C = 1 / 2 / 4 / 8: 6 rows of 16384
+// samples 157 / 133 / 118 / 111; 2 rows of 4096 in FP64 98 / 91 / 83 / 81; 27 rows of 8192
+// 116 / 107 / 102 / 103; 192 rows of 16384 499 / 485 / 495 / 541. A row of 2048 is quicker in
+// one CTA (64 against 73 / 71 for a single-mode solve): nothing shorter than 4096 is split.
+int row_split(bool fp64, int logn, int rows) {
+  int xc = 0;
+  const int c0 = kernels_for(fp64 ? 1 : 0, logn).C;
+  while (logn >= 12 && xc < max_split(fp64, logn) && rows * c0 * (2 << xc) <= kSMs) ++xc;
+  return xc;
+}
+
 bool batch_shape(mmp_batch* b) {
   const Shape sh = choose_shape(b, batch_stats(b));
-  const bool changed = sh.Mmax != b->Mmax || sh.Pmax != b->Pmax || sh.TT != b->TT || sh.smem != b->contract_smem ||
+  const int xc = b->xc_req >= 0 ? b->xc_req : row_split(b->fp64, b->logn, sh.Mmax * (int)sh.span);
+  const bool resplit = xc != b->ks.xc;
+  if (resplit) b->ks = kernels_for(b->fp64 ? 1 : 0, b->logn, xc);
+  const bool changed = resplit || sh.Mmax != b->Mmax || sh.Pmax != b->Pmax || sh.TT != b->TT || sh.smem != b->contract_smem ||
                        sh.stage_terms != b->stage_terms || sh.span != b->span || sh.iir != b->raman_iir ||
                        sh.fused != b->raman_fused || sh.dense != b->dense || sh.tc != b->tc ||
                        sh.pchunk != b->pchunk || sh.sr != b->sr;
@@ -1671,9 +1657,8 @@ bool batch_shape(mmp_batch* b) {
 // Three launch parameters are chosen by timing whole RK steps of this batch on its own
 // buffers, one parameter after the other (each timed with the others at their current
 // choice):
-//   1. the per-mode transform kernels: each row on the minimal set of CTAs, or split over
-//      twice as many (a cluster twice as wide: one more radix-2 exchange across CTAs and
-//      half the shared memory per CTA, so two CTAs share an SM), where that set is built;
+//   1. the CTAs a row is spread over: row_split's choice for the batch's rows, half and twice
+//      as many, where built;
 //   2. the contraction tile: samples per CTA of k_contract (64 / 128 / 256, as many as fit
 //      its shared memory) or of k_contract_sr (64 / 128 / 256);
 //   3. the graph branches: the batch's solves split into 1, 2 or 4 independent kernel
@@ -1739,22 +1724,23 @@ int restore_members(mmp_batch* b, const mmp_params* const* params) {
 
 int autotune(mmp_batch* b, const mmp_params* const* params) {
   mmp_detail::Range range("mmp.autotune");
-  const KernelSet base = kernels_for(b->fp64 ? 1 : 0, b->logn, 0);
-  const KernelSet alt = kernels_for(b->fp64 ? 1 : 0, b->logn, 1);
-  std::vector<int> xcs = {0}, tiles = tile_candidates(b), gs = {1};
-  if (alt.prime) xcs.push_back(1);
+  std::vector<int> xcs, tiles = tile_candidates(b), gs = {1};
+  const int xc0 = b->ks.xc;  // row_split's choice, and its neighbours
+  xcs = {xc0};
+  for (int x = std::max(0, xc0 - 1); x <= std::min(xc0 + 1, max_split(b->fp64, b->logn)); ++x)
+    if (x != xc0) xcs.push_back(x);
   const int g0 = b->span >= 16 ? 4 : (b->span >= 4 ? 2 : 1);  // the untuned default
   gs = {g0};
   for (int g : {1, 2, 4})
     if (g != g0 && (uint32_t)g <= b->span) gs.push_back(g);
   if (const char* env = std::getenv("MMP_ROW_SPLIT"))
-    if (*env) xcs = {std::atoi(env) == 1 && alt.prime ? 1 : 0};
+    if (*env) xcs = {b->xc_req};
   if (const char* env = std::getenv("MMP_CONTRACT_TILE"))
     if (*env) tiles = {std::atoi(env)};
   if (const char* env = std::getenv("MMP_GROUPS"))
     if (*env) gs = {std::max(1, std::atoi(env))};
   auto apply = [&](const TuneChoice& c) {
-    b->ks = c.xc ? alt : base;
+    b->xc_req = c.xc;
     b->tile_req = c.tile;
     batch_shape(b);
     b->groups = (uint32_t)c.groups;
@@ -2198,7 +2184,7 @@ int mmp_dft(uint32_t n, uint32_t rows, int direction, int fp64, const double* in
     a.out = d_out;
     a.rows = (int)rows;
     a.scale = direction < 0 ? 1.0 : 1.0 / (double)n;
-    a.tw = res->tw;
+    a.tw = res->tw[fp64 ? 1 : 0][lg];
     void* args[] = {&a};
     e = launch(direction < 0 ? ks.dft_fwd : ks.dft_inv, dim3(rows * (unsigned)ks.C, 1, 1), ks.nthr,
                ks.smem, ks.C, st, args);

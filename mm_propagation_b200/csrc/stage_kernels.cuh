@@ -35,12 +35,25 @@
 
 namespace mmp {
 
+// One stage of the tableau as its k_nu needs it (host: stage_args). Stored N_hat_j entering
+// x_hat of the next stage, or at the last stage psi_{n+1} = psi_n + h sum_j b_j N_j
+// (src/MultimodePropagation_CPU.cpp:75-85), with their coefficients a or b; N_hat_i itself
+// comes from registers (cself).
+struct StageArgs {
+  int stage;
+  int last;  // 1: the final stage
+  int nq;
+  int jq[kMaxStages];
+  double cq[kMaxStages];
+  double cself;
+  double c_this, c_next;  // z at this stage and the next, in steps beyond z_n
+};
+
 struct KParams {
   const SolveDesc* descs;
-  TwTables tw;
-  Tableau tab;
-  int stage;
-  int pad_;
+  const void* tw;    // twiddle table of the kernel's precision and size (radix_plan.h)
+  StageArgs st;
+  SpecLayout lay;    // psi_hat's storage order (kernels of another geometry)
 };
 
 // Im L_p(alpha) by Horner over the per-mode polynomial (FP64).
@@ -68,8 +81,8 @@ __device__ __forceinline__ double alpha_of(int k, int nt, double alpha_scale) {
 // no conversion instruction; valid for |theta 2/pi| < 2^51), then the Taylor
 // series of sin and cos to x^9 and x^10 (truncation below 2e-9 on that interval),
 // evaluated by Horner in x^2 in FP32; the quadrant swaps and negates. Short, branch-free
-// code with no large-argument path (the argument is already small). FP64: reduced by
-// 2 pi, then sincos.
+// code with no large-argument path (the argument is already small). FP64: the same reduction
+// and the series to x^17 and x^16 (truncation below 1e-19 and 2e-18).
 template <typename T> __device__ __forceinline__ c2<T> expi(double theta) {
   if constexpr (sizeof(T) == 4) {
     constexpr double k2OverPi = 0.63661977236758134308;
@@ -91,15 +104,28 @@ template <typename T> __device__ __forceinline__ c2<T> expi(double theta) {
     const float c = (q & 1) ? sp : cp, s = (q & 1) ? cp : sp;
     return make_float2((q == 1 || q == 2) ? -c : c, (q >= 2) ? -s : s);
   } else {
-    constexpr double kInv2Pi = 0.15915494309189533577;
-    constexpr double kTwoPiHi = 6.28318530717958623200;   // nearest double to 2 pi
-    constexpr double kTwoPiLo = 2.4492935982947063697e-16;  // 2 pi - kTwoPiHi
-    const double n = rint(theta * kInv2Pi);
-    double r = fma(-n, kTwoPiHi, theta);
-    r = fma(-n, kTwoPiLo, r);
-    double s, c;
-    sincos(r, &s, &c);
-    return make_double2(c, s);
+    constexpr double k2OverPi = 0.63661977236758134308;
+    constexpr double kHalfPiHi = 1.57079632679489655800;
+    constexpr double kHalfPiLo = 6.12323399573676603587e-17;
+    constexpr double kRound = 6755399441055744.0;
+    const double t = fma(theta, k2OverPi, kRound);
+    const double n = t - kRound;
+    const double x = fma(-n, kHalfPiLo, fma(-n, kHalfPiHi, theta)), x2 = x * x;
+    double sp = 1.0 / 355687428096000.0, cp = 1.0 / 20922789888000.0;  // 1/17!, 1/16!
+    constexpr double sc[7] = {-1.0 / 1307674368000.0, 1.0 / 6227020800.0, -1.0 / 39916800.0, 1.0 / 362880.0,
+                              -1.0 / 5040.0, 1.0 / 120.0, -1.0 / 6.0};
+    constexpr double cc[7] = {-1.0 / 87178291200.0, 1.0 / 479001600.0, -1.0 / 3628800.0, 1.0 / 40320.0,
+                              -1.0 / 720.0, 1.0 / 24.0, -0.5};
+#pragma unroll
+    for (int j = 0; j < 7; ++j) {
+      sp = fma(sp, x2, sc[j]);
+      cp = fma(cp, x2, cc[j]);
+    }
+    sp = fma(sp * x2, x, x);
+    cp = fma(cp, x2, 1.0);
+    const int q = __double2loint(t) & 3;
+    const double c = (q & 1) ? sp : cp, s = (q & 1) ? cp : sp;
+    return make_double2((q == 1 || q == 2) ? -c : c, (q >= 2) ? -s : s);
   }
 }
 
@@ -128,19 +154,23 @@ __device__ __forceinline__ void st2<float>(float2* p, float2 a, float2 b) {
   *reinterpret_cast<float4*>(p) = make_float4(a.x, a.y, b.x, b.y);
 }
 
-__device__ __forceinline__ void load_poly(double* poly, const SolveDesc& d, int p) {
-  if (threadIdx.x < d.n_beta) poly[threadIdx.x] = d.poly[p * d.n_beta + threadIdx.x];
-  __syncthreads();
-}
-
-// One warp copies this CTA's solve descriptor into shared memory in a single round
-// trip, instead of every field becoming its own dependent global load. The caller
-// synchronises before reading it.
+// The CTA copies its solve descriptor and mode p's dispersion polynomial into shared memory
+// instead of every field becoming its own dependent global load. Published by the caller's
+// next barrier.
 static_assert(sizeof(SolveDesc) % 8 == 0, "descriptor copied in 8-byte words");
+// a pointer field of a descriptor in global memory (constant while kernels run)
+template <typename P> __device__ __forceinline__ P* ldg_ptr(P* const* f) {
+  return reinterpret_cast<P*>(__ldg(reinterpret_cast<const unsigned long long*>(f)));
+}
 __device__ __forceinline__ void stage_desc(SolveDesc* dst, const SolveDesc* src) {
   constexpr int W = (int)(sizeof(SolveDesc) / 8);
   for (int i = threadIdx.x; i < W; i += blockDim.x)
     reinterpret_cast<unsigned long long*>(dst)[i] = __ldg(reinterpret_cast<const unsigned long long*>(src) + i);
+}
+__device__ __forceinline__ void stage_poly(double* poly, const SolveDesc* gd, int p) {
+  const int nb = __ldg(&gd->n_beta);
+  const double* src = ldg_ptr(&gd->poly);
+  if ((int)threadIdx.x < nb) poly[threadIdx.x] = __ldg(src + p * nb + threadIdx.x);
 }
 
 // Ask the TMA engine to pull [p, p + bytes) into L2 without waiting for it
@@ -161,15 +191,6 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
   const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem_src) : "memory");
 }
-__device__ __forceinline__ void cp_async8(void* smem_dst, const void* gmem_src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(gmem_src) : "memory");
-}
-// one complex value of T
-template <typename T> __device__ __forceinline__ void cp_async_c2(c2<T>* smem_dst, const c2<T>* gmem_src) {
-  if constexpr (sizeof(c2<T>) == 8) cp_async8(smem_dst, gmem_src);
-  else cp_async16(smem_dst, gmem_src);
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
@@ -180,54 +201,63 @@ template <typename G> __device__ __forceinline__ int cluster_rank() {
   else return (int)cg::this_cluster().block_rank();
 }
 
-// Common start of a row kernel: shared memory (the row, then the twiddle table).
-#define MMP_ROW_SMEM()                                                 \
-  extern __shared__ __align__(128) unsigned char smem_raw[];            \
-  V* s = reinterpret_cast<V*>(smem_raw);
+// A streamed value (used once by this kernel: kept out of L1, which holds the twiddles)
+__device__ __forceinline__ float2 ld_stream(const float2* p) { return __ldcg(p); }
+__device__ __forceinline__ double2 ld_stream(const double2* p) { return __ldcg(p); }
 
-// ---- k_prime: U for stage `stage` from psi_hat (and the stored N_hat_j) -------------------
+// Common names of a row kernel: this CTA's sub-rows and the thread's place in its own.
+#define MMP_ROW_SETUP()                                              \
+  extern __shared__ __align__(128) unsigned char smem_raw[];          \
+  V* s = reinterpret_cast<V*>(smem_raw);                              \
+  const int rank = cluster_rank<Gm>();                                \
+  const int tid = threadIdx.x;                                        \
+  const int u = tid % Gm::TPR, lrow = tid / Gm::TPR;                  \
+  const int k1 = rank * Gm::RPC + lrow;                               \
+  V* sr = s + lrow * Gm::RS;                                          \
+  const int i0 = rank * Gm::NTHR + tid;
+
+// ---- k_prime: U for stage 0 from psi_hat --------------------------------------------------
 template <typename T, int LOGN, int XC>
 __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_BLOCKS) k_prime(const KParams kp) {
   using Gm = Geo<T, LOGN, XC>;
   using V = c2<T>;
-  MMP_ROW_SMEM();
+  MMP_ROW_SETUP();
   __shared__ double poly[kMaxBeta];
   __shared__ SolveDesc sdesc;
-  stage_desc(&sdesc, kp.descs + blockIdx.y);
-  const V* sq = load_twiddles<T, LOGN, XC>(smem_raw, kp.tw);
+  const SolveDesc* gd = kp.descs + blockIdx.y;
+  const int p = blockIdx.x / Gm::C;
+  if (p >= __ldg(&gd->M)) return;  // uniform over the cluster
+  stage_desc(&sdesc, gd);
+  stage_poly(poly, gd, p);
   __syncthreads();
   const SolveDesc& d = sdesc;
-  const int p = blockIdx.x / Gm::C;
-  if (p >= d.M) return;  // uniform over the cluster
-  const int rank = cluster_rank<Gm>();
-  const int tid = threadIdx.x;
-  load_poly(poly, d, p);
-  const int i = kp.stage;
+  const V* tw = static_cast<const V*>(kp.tw);
   const unsigned long long n = __ldcg(d.step);
-  const double zs = ((double)n + kp.tab.c[i]) * d.dz;
+  const double zs = ((double)n + kp.st.c_this) * d.dz;
   const size_t row = (size_t)p * Gm::N;
-  const size_t mstride = (size_t)d.M * Gm::N;
-  const V* Nh = as_t2<T>(d.Nh);
-#pragma unroll 2
-  for (int li = tid; li < Gm::NL; li += Gm::NTHR) {
-    const int k = Gm::freq_of(rank, li);
-    double2 x = d.psi_hat[row + k];
-    for (int j = 0; j < i; ++j) {
-      const double aij = kp.tab.a[i][j];
-      if (aij != 0.0) {
-        const double2 nj = to_d2(Nh[(size_t)j * mstride + row + k]);
-        x.x = fma(aij * d.dz, nj.x, x.x);
-        x.y = fma(aij * d.dz, nj.y, x.y);
-      }
+  rows_last<Gm>(sr, u, [&](int b, V* x) {
+    const double2* ps = d.psi_hat + row + Gm::spec0(k1, b);
+    const int k0 = Gm::freq0(k1, b);
+    V v[Gm::RM];
+#pragma unroll
+    for (int r = 0; r < Gm::RM; ++r) v[r] = from_d2<T>(__ldcg(ps + r * Gm::SSTR));
+#pragma unroll
+    for (int r = 0; r < Gm::RM; ++r) {
+      const double th = im_L(poly, d.n_beta, alpha_of(k0 + r * Gm::KSTR, Gm::N, d.alpha_scale)) * zs;
+      v[r] = cmul(v[r], expi<T>(th));
     }
-    const double th = im_L(poly, d.n_beta, alpha_of(k, Gm::N, d.alpha_scale)) * zs;
-    s[Gm::sidx(li)] = cmul(from_d2<T>(x), expi<T>(th));
-  }
-  inverse<T, LOGN, XC>(s, sq, kp.tw);
-  V* U = as_t2<T>(d.U);
+    RegDFT<Gm::RM, true>::run(v);
+#pragma unroll
+    for (int r = 0; r < Gm::RM; ++r) x[Gm::pad(r)] = v[r];
+  });
+  rows_inv<Gm>(sr, tw, u);
+  V v[Gm::E];
+  row_last_inv<Gm>(v, s, tw, rank);
+  V* U = as_t2<T>(d.U) + row + i0;
   const T inv = (T)d.inv_nt;
-#pragma unroll 8
-  for (int w = tid; w < Gm::NL; w += Gm::NTHR) U[row + Gm::time_of_w(rank, w)] = cscale(s[Gm::sidx(Gm::local_of_w(w))], inv);
+#pragma unroll
+  for (int r = 0; r < Gm::E; ++r) U[r * Gm::B] = cscale(v[r], inv);
+  row_leave<Gm>();
 }
 
 // ---- k_pair: R_q = IFFT(FFT(V_q) * H), V_q = U_l conj(U_m) -------------------------------
@@ -235,56 +265,47 @@ template <typename T, int LOGN, int XC>
 __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_BLOCKS) k_pair(const KParams kp) {
   using Gm = Geo<T, LOGN, XC>;
   using V = c2<T>;
-  MMP_ROW_SMEM();
-  __shared__ SolveDesc sdesc;
-  stage_desc(&sdesc, kp.descs + blockIdx.y);
-  const V* sq = load_twiddles<T, LOGN, XC>(smem_raw, kp.tw);
-  __syncthreads();
-  const SolveDesc& d = sdesc;
+  MMP_ROW_SETUP();
+  const SolveDesc* gd = kp.descs + blockIdx.y;
   const int q = blockIdx.x / Gm::C;
-  if (q >= d.P || __ldcg(d.step) >= d.step_limit) return;  // uniform over the cluster
-  const int rank = cluster_rank<Gm>();
-  const int tid = threadIdx.x;
-  const int2 lm = d.pairs[q];
-  const V* U = as_t2<T>(d.U);
-  const size_t rl = (size_t)lm.x * Gm::N, rm = (size_t)lm.y * Gm::N;
-  if constexpr (Gm::C == 1 && sizeof(T) == 4) {
-    // one CTA per row: two consecutive samples per 16-byte load
-    const float4* Ul = reinterpret_cast<const float4*>(U + rl);
-    const float4* Um = reinterpret_cast<const float4*>(U + rm);
-#pragma unroll 8
-    for (int u2 = tid; u2 < Gm::NL / 2; u2 += Gm::NTHR) {
-      const float4 a = Ul[u2], b = Um[u2];
-      s[pad(2 * u2)] = cmulc(make_float2(a.x, a.y), make_float2(b.x, b.y));
-      s[pad(2 * u2 + 1)] = cmulc(make_float2(a.z, a.w), make_float2(b.z, b.w));
-    }
-  } else {
-#pragma unroll 8
-    for (int w = tid; w < Gm::NL; w += Gm::NTHR) {
-      const int t = Gm::time_of_w(rank, w);
-      s[Gm::sidx(Gm::local_of_w(w))] = cmulc(U[rl + t], U[rm + t]);
-    }
+  if (q >= __ldg(&gd->P)) return;  // uniform over the cluster
+  const unsigned long long* step = ldg_ptr(&gd->step);
+  const V* U = as_t2<T>(static_cast<const void*>(ldg_ptr(&gd->U))) + i0;
+  const V* H = as_t2<T>(static_cast<const void*>(ldg_ptr(&gd->H)));
+  V* W = as_t2<T>(ldg_ptr(&gd->W));
+  const int2 lm = __ldg(ldg_ptr(&gd->pairs) + q);
+  if (__ldcg(step) >= __ldg(&gd->step_limit)) return;  // uniform over the cluster
+  row_enter<Gm>();
+  const V* tw = static_cast<const V*>(kp.tw);
+  V v[Gm::E];
+  {
+    const V* Ul = U + (size_t)lm.x * Gm::N;
+    const V* Um = U + (size_t)lm.y * Gm::N;
+#pragma unroll
+    for (int r = 0; r < Gm::E; ++r) v[r] = cmulc(ld_stream(Ul + r * Gm::B), ld_stream(Um + r * Gm::B));
   }
-  forward<T, LOGN, XC>(s, sq, kp.tw);
-  const V* H = as_t2<T>(d.H);
-  if constexpr (Gm::C == 1 && sizeof(T) == 4) {
-    const float4* H4 = reinterpret_cast<const float4*>(H);
-#pragma unroll 8
-    for (int k2 = tid; k2 < Gm::NL / 2; k2 += Gm::NTHR) {
-      const float4 hh = __ldg(&H4[k2]);
-      s[pad(2 * k2)] = cmul(s[pad(2 * k2)], make_float2(hh.x, hh.y));
-      s[pad(2 * k2 + 1)] = cmul(s[pad(2 * k2 + 1)], make_float2(hh.z, hh.w));
-    }
-  } else {
-#pragma unroll 4
-    for (int li = tid; li < Gm::NL; li += Gm::NTHR) s[Gm::sidx(li)] = cmul(s[Gm::sidx(li)], __ldg(&H[Gm::freq_of(rank, li)]));
-  }
-  inverse<T, LOGN, XC>(s, sq, kp.tw);
+  row_first<Gm>(v, s, tw, rank);
+  rows_fwd<Gm>(sr, tw, u);
+  rows_last<Gm>(sr, u, [&](int b, V* x) {
+    const V* h = H + Gm::spec0(k1, b);
+    V w[Gm::RM];
+#pragma unroll
+    for (int r = 0; r < Gm::RM; ++r) w[r] = x[Gm::pad(r)];
+    RegDFT<Gm::RM, false>::run(w);
+#pragma unroll
+    for (int r = 0; r < Gm::RM; ++r) w[r] = cmul(w[r], __ldg(h + r * Gm::SSTR));
+    RegDFT<Gm::RM, true>::run(w);
+#pragma unroll
+    for (int r = 0; r < Gm::RM; ++r) x[Gm::pad(r)] = w[r];
+  });
+  rows_inv<Gm>(sr, tw, u);
+  row_last_inv<Gm>(v, s, tw, rank);
   // R_q = (H_R conv V_q); the Kerr part (1 - fR) V_q is formed by the contraction from
   // the U tile it already holds
-  V* R = as_t2<T>(d.W) + (size_t)q * Gm::N;
-#pragma unroll 8
-  for (int w = tid; w < Gm::NL; w += Gm::NTHR) R[Gm::time_of_w(rank, w)] = s[Gm::sidx(Gm::local_of_w(w))];
+  V* R = W + (size_t)q * Gm::N + i0;
+#pragma unroll
+  for (int r = 0; r < Gm::E; ++r) R[r * Gm::B] = v[r];
+  row_leave<Gm>();
 }
 
 // ---- k_raman_scan: R_q = h_R (*) V_q as a periodic linear recurrence ----------------------
@@ -501,295 +522,228 @@ __global__ void __launch_bounds__(512) k_raman_scan(const SolveDesc* __restrict_
 // (BODY = n), of a last stage that reads n (BODY = kNuLastBody + n), or of any stage (-1).
 // The host launches the instantiation that matches each stage of its tableau (RK4: 0 at
 // the intermediate stages, kNuLastBody + 3 at the last), so each kernel carries one body.
+//
+// What bounds it: instruction issue and shared memory, then the row's global traffic. sigma goes
+// from global memory into the first pass's registers, the stage arithmetic runs between the
+// forward and the inverse radix step of the last pass (straight in its registers where the
+// radix is 4; else chunk by chunk through the thread's own shared positions, so that the code
+// stays one short loop), and U leaves from the last pass's registers: two block- or
+// cluster-wide barriers a stage. Measured on a B200, a launch, against Stockham passes with
+// block barriers between them and one layout per cluster size:
+//   192 rows of 16384, FP32, intermediate stage   64-69 -> 49-53 us, 22.6-25.2 -> 16.3-19.0
+//                                                 million warp instructions
+//   6 rows of 16384, FP32 (one solve)             30-39 -> 12-15 us (6 -> 48 CTAs)
+//   6 rows of 8192, FP64, order 8                 35-49 -> 12-15 us (6 -> 48 CTAs)
+//   1 row of 2048, FP32                           9.1 -> 5.9 us
+//   56 rows of 65536, FP32                        170-217 -> 118-156 us
 constexpr int kNuLastBody = 10;
 template <typename T, int LOGN, int XC, int BODY>
 __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_BLOCKS) k_nu(const KParams kp) {
   using Gm = Geo<T, LOGN, XC>;
   using V = c2<T>;
-  MMP_ROW_SMEM();
+  MMP_ROW_SETUP();
   __shared__ double poly[kMaxBeta];
   __shared__ double red[2][32];
   __shared__ SolveDesc sdesc;
+  const SolveDesc* gd = kp.descs + blockIdx.y;
   const int p = blockIdx.x / Gm::C;
-  const int rank = cluster_rank<Gm>();
-  const int tid = threadIdx.x;
-  // The sigma row and the twiddle table start on their way first, as asynchronous copies
-  // into shared memory (all of a thread's elements in flight, no registers held): the row's
-  // address and the mode count come straight from the descriptor in global memory, so
-  // the descriptor and polynomial round trips below overlap the row's.
-  V* sq = reinterpret_cast<V*>(smem_raw + Gm::DATA_BYTES);
-  {
-    const c2<T>* g = tw_table<T>(kp.tw, Gm::LOGNLG);
-    for (int m = tid; m < Gm::NTW; m += Gm::NTHR) cp_async_c2<T>(&sq[pad(m)], &g[m]);
-    const SolveDesc* gd = kp.descs + blockIdx.y;
-    if (p < __ldg(&gd->M)) {
-      const V* sg = as_t2<T>(reinterpret_cast<const void*>(__ldg(reinterpret_cast<const unsigned long long*>(&gd->sigma)))) +
-                    (size_t)p * Gm::N;
-      for (int w = tid; w < Gm::NL; w += Gm::NTHR)
-        cp_async_c2<T>(&s[Gm::sidx(Gm::local_of_w(w))], sg + Gm::time_of_w(rank, w));
-    }
-    cp_async_commit();
-  }
-  stage_desc(&sdesc, kp.descs + blockIdx.y);
-  __syncthreads();
-  const SolveDesc& d = sdesc;
-  if (p >= d.M) {  // empty slot (its descriptor is zero); uniform over the cluster
-    cp_async_wait<0>();  // no copy may land after the CTA has left
-    return;
-  }
-  // the step counters in one round trip, shared by the finished-solve check and thread
-  // 0's setup below
-  const unsigned long long n_step = __ldcg(d.step), n_total = __ldcg(d.total);
-  if (n_step >= d.step_limit) {  // finished solve; uniform over the cluster
-    cp_async_wait<0>();
-    return;
-  }
-  load_poly(poly, d, p);
-  // Scalars needed after the forward transform live in shared memory rather than in
-  // registers, so the (out-of-line) transform call has little to save and restore.
-  __shared__ unsigned long long s_cnt[2];  // step since z reset, steps since creation
-  __shared__ double s_z[2];               // z at this stage, z at the next stage
-  // Stage-combination list: the stored N_hat_j entering x_hat (or, at the last stage,
-  // psi_{n+1} = psi_n + h sum_j b_j N_j, src/MultimodePropagation_CPU.cpp:75-85) with
-  // their coefficients h*a or h*b; N_hat_i itself comes from registers (cself).
-  // Once the sigma loads are issued, the CTA's threads start L2 prefetches of the psi_hat
-  // the cluster reads after its forward transform, so it arrives while the transform runs.
-  __shared__ int s_jq[kMaxStages];
-  __shared__ double s_cq[kMaxStages];
-  __shared__ int s_nq;
-  if (tid == 0) {
-    const int i = kp.stage;
-    const int S = kp.tab.s;
-    const bool last = (i == S - 1);
-    const double h = d.dz;
-    const unsigned long long n = n_step;
-    s_cnt[0] = n;
-    s_cnt[1] = n_total;
-    s_z[0] = ((double)n + kp.tab.c[i]) * h;
-    s_z[1] = last ? ((double)(n + 1)) * h : ((double)n + kp.tab.c[i + 1]) * h;
-    int nq = 0;
-    if (last) {
-      for (int j = 0; j < S; ++j)
-        if (j != i && kp.tab.b[j] != 0.0) { s_jq[nq] = j; s_cq[nq] = kp.tab.b[j] * h; ++nq; }
-    } else {
-      for (int j = 0; j < i; ++j)
-        if (kp.tab.a[i + 1][j] != 0.0) { s_jq[nq] = j; s_cq[nq] = kp.tab.a[i + 1][j] * h; ++nq; }
-    }
-    s_nq = nq;
-  }
-  {
-    // the row's psi_hat (FP64 at the last stage, in T at the others), 1/C of it per CTA of
-    // the cluster (together the frequencies every CTA reads), one piece of at most 32 KB
-    // per thread. The N_hat_j are not prefetched: a wave's rows of them do not fit in L2
-    // beside the rest, and measured, prefetching them too was slower.
-    const bool lastp = kp.stage == kp.tab.s - 1;
-    const unsigned esz = lastp ? (unsigned)sizeof(double2) : (unsigned)sizeof(V);
-    const unsigned bytes = Gm::NL * esz;
-    const unsigned piece = bytes < 32u * 1024u ? bytes : 32u * 1024u;
-    const char* base = reinterpret_cast<const char*>(lastp ? (const void*)d.psi_hat : d.psi_t) +
-                       ((size_t)p * Gm::N + (size_t)rank * Gm::NL) * esz;
-    for (unsigned t = tid; t < bytes / piece; t += Gm::NTHR) prefetch_l2(base + (size_t)t * piece, piece);
-  }
-  cp_async_wait<0>();                  // this thread's sigma and twiddle copies
-  forward<T, LOGN, XC>(s, sq, kp.tw);  // its barriers publish them and the values thread 0 wrote
-  const int i = kp.stage;
-  const int S = kp.tab.s;
+  if (p >= __ldg(&gd->M)) return;  // also an empty slot (its descriptor is zero); uniform over the cluster
+  const unsigned long long* stepp = ldg_ptr(&gd->step);
+  const unsigned long long* totalp = ldg_ptr(&gd->total);
+  const V* sg = as_t2<T>(static_cast<const void*>(ldg_ptr(&gd->sigma))) + (size_t)p * Gm::N + i0;
+  const unsigned long long limit = __ldg(&gd->step_limit);
+  const double h = __ldg(&gd->dz);
+  stage_desc(&sdesc, gd);
+  stage_poly(poly, gd, p);
+  const unsigned long long n_step = __ldcg(stepp), n_total = __ldcg(totalp);
+  V v[Gm::E];
+#pragma unroll
+  for (int r = 0; r < Gm::E; ++r) v[r] = ld_stream(sg + r * Gm::B);
   // a specialised BODY serves intermediate or last stages only: fixed at compile time, so
   // each instantiation carries only its half of the stage arithmetic
-  const bool last = BODY < 0 ? (i == S - 1) : (BODY >= kNuLastBody);
-  const double h = d.dz;
+  const bool last = BODY < 0 ? kp.st.last != 0 : (BODY >= kNuLastBody);
+  {
+    // the row's psi_hat (FP64 at the last stage, in T at the others), 1/C of it per CTA (the
+    // part the CTA reads), on its way to L2 while the forward passes run, one piece of at
+    // most 32 KB per thread. The N_hat_j are not prefetched: a wave's rows of them do not
+    // fit in L2 beside the rest.
+    const unsigned esz = last ? (unsigned)sizeof(double2) : (unsigned)sizeof(V);
+    const unsigned bytes = Gm::NL * esz;
+    const unsigned piece = bytes < 32u * 1024u ? bytes : 32u * 1024u;
+    const void* src = last ? static_cast<const void*>(ldg_ptr(&gd->psi_hat)) : static_cast<const void*>(ldg_ptr(&gd->psi_t));
+    const char* base = static_cast<const char*>(src) + ((size_t)p * Gm::N + (size_t)rank * Gm::NL) * esz;
+    for (unsigned t = tid; t < bytes / piece; t += Gm::NTHR) prefetch_l2(base + (size_t)t * piece, piece);
+  }
+  if (n_step >= limit) return;  // finished solve; uniform over the cluster
+  row_enter<Gm>();
+  const V* tw = static_cast<const V*>(kp.tw);
+  row_first<Gm>(v, s, tw, rank);  // its barrier publishes the descriptor and the polynomial
+  rows_fwd<Gm>(sr, tw, u);
+  const SolveDesc& d = sdesc;
+  const int i = kp.st.stage;
   const size_t row = (size_t)p * Gm::N;
   const size_t mstride = (size_t)d.M * Gm::N;
-  V* Nh = as_t2<T>(d.Nh);
-  V* psiT = as_t2<T>(d.psi_t);
   // FP32 stage bodies of one kind read psi_hat's T copy at the intermediate stages; the
   // FP64 ones (psi_t is psi_hat) and the any-stage body read psi_hat
   constexpr bool kReadT = sizeof(T) == 4 && BODY >= 0;
-  const double zi = s_z[0], znext = s_z[1];
+  const double zi = ((double)n_step + kp.st.c_this) * h, znext = ((double)n_step + kp.st.c_next) * h;
   double e_part = 0.0, p_part = 0.0;
+  float p_part_f = 0.0f;
   bool finite = true;
-  const int nq = s_nq;
-  const double cself = (last ? kp.tab.b[i] : kp.tab.a[i + 1][i]) * h;
-  // spectrum entering the inverse transform: conjugated when it runs as a forward one
-  auto spec_in = [](V v) { return Gm::C == 1 ? cconj(v) : v; };
-  constexpr int MAXQ = 6;
-  // Fast path, one body per count of stored terms (no predicated dead work): all loads
-  // of a chunk of frequencies are issued before its math. Intermediate stages combine
-  // x_hat in T (it only feeds the nonlinearity, which runs in T); the last stage
-  // accumulates psi_{n+1} in FP64.
+  const double cself = kp.st.cself * h;
   // E_{i+1} = E_i when z does not move between the stages (RK4: c_2 = c_3, c_4 = 1)
   const bool same_z = zi == znext;
-  float p_part_f = 0.0f;
   const float w0f = (float)d.omega0_T0, asf = (float)d.alpha_scale;
-  // NQ: the (compile-time) most stored terms the body reads; nqr: how many it reads
-  auto body = [&](auto nqc, int nqr) {
-    constexpr int NQ = decltype(nqc)::value;
-    // frequencies per chunk: all of a chunk's loads are in flight together (8 when the
-    // stage reads only psi_hat; 4 also with 4 or 5 stored terms, where 2 was measured 3%
-    // slower on the 28-mode sweep and 2% on the 6-mode order-6 batch)
-    constexpr int CHK0 = NQ == 0 ? 8 : 4;
-    constexpr int CHK = CHK0 < Gm::E ? CHK0 : Gm::E;
-    const double nb3 = d.n_beta == 3;
-#pragma unroll 1
-    for (int e0 = 0; e0 < Gm::E; e0 += CHK) {
-      int kk[CHK];
-      double2 ps[CHK];  // last stage: psi_hat in FP64
-      V pt[CHK];        // other stages: psi_hat in T
-      V sv[CHK];
-      V nj[CHK][NQ > 0 ? NQ : 1];
+  const bool nb3 = d.n_beta == 3;
+  // stored terms: their count at compile time, or (any-stage body) at run time
+  constexpr int NQ = BODY < 0 ? -1 : (BODY >= kNuLastBody ? BODY - kNuLastBody : BODY);
+  constexpr int NQR = NQ > 0 ? NQ : 1;
+  double cq[NQR];
+#pragma unroll
+  for (int q = 0; q < NQR; ++q) cq[q] = NQ > 0 ? kp.st.cq[q] * h : 0.0;
+  // frequencies per chunk: a chunk's loads are all in flight before its arithmetic
+  constexpr int CHK0 = NQ <= (sizeof(T) == 8 ? 0 : 2) ? 4 : 2;
+  constexpr int CHK = CHK0 < Gm::RM ? CHK0 : Gm::RM;
+  rows_last<Gm>(sr, u, [&](int b, V* x) {
+    const size_t at = row + Gm::spec0(k1, b);
+    const int k0 = Gm::freq0(k1, b);
+    double2 ps[CHK];  // last stage (and FP64): psi_hat in FP64
+    V pt[CHK];        // other stages: psi_hat in T
+    V nj[CHK][NQR];
+    auto fetch = [&](int c0) {
 #pragma unroll
       for (int c = 0; c < CHK; ++c) {
-        const int li = tid + (e0 + c) * Gm::NTHR;
-        kk[c] = Gm::freq_of(rank, li);
-        if constexpr (!kReadT) ps[c] = d.psi_hat[row + kk[c]];
-        else if (last) ps[c] = d.psi_hat[row + kk[c]];
-        else pt[c] = psiT[row + kk[c]];
-        sv[c] = s[Gm::sidx(li)];
+        const size_t f = at + (c0 + c) * Gm::SSTR;
+        if (!kReadT || last) ps[c] = __ldcg(d.psi_hat + f);
+        else pt[c] = __ldcg(as_t2<T>(d.psi_t) + f);
+        if constexpr (NQ > 0) {
 #pragma unroll
-        for (int q = 0; q < NQ; ++q)
-          if (q < nqr) nj[c][q] = Nh[(size_t)s_jq[q] * mstride + row + kk[c]];
+          for (int q = 0; q < NQ; ++q) nj[c][q] = __ldcg(as_t2<T>(d.Nh) + (size_t)kp.st.jq[q] * mstride + f);
+        }
       }
+    };
+    // the chunk's values w become the spectrum entering the inverse
+    auto chunk = [&](V* w, int c0) {
 #pragma unroll
       for (int c = 0; c < CHK; ++c) {
-        const int li = tid + (e0 + c) * Gm::NTHR;
-        const int k = kk[c];
+        const int r = c0 + c;
+        const size_t f = at + r * Gm::SSTR;
+        const int k = k0 + r * Gm::KSTR;
         const double alpha = alpha_of(k, Gm::N, d.alpha_scale);
         const double L = nb3 ? fma(fma(poly[2], alpha, poly[1]), alpha, poly[0]) : im_L(poly, d.n_beta, alpha);
         // N_hat_i = i sgn(gamma) conj(E_i) FFT(sigma)   (src/MultimodePropagation_CPU.cpp:231-237)
         const V ei = expi<T>(L * zi);
-        const V xe = cmulc(sv[c], ei);
+        const V xe = cmulc(w[c], ei);
         V nh;
         nh.x = (T)(-d.sgn_gamma) * xe.y;
         nh.y = (T)(d.sgn_gamma) * xe.x;
-        Nh[(size_t)i * mstride + row + k] = nh;
+        as_t2<T>(d.Nh)[(size_t)i * mstride + f] = nh;
         V xt;
-        if (last && sizeof(T) == 4) {
-          // psi_{n+1} = psi_n + inc in FP64; the increment h sum_j b_j N_j is formed in
-          // FP32 from the FP32 N_j (its rounding is that of the N_j themselves), so the
-          // only conversions are inc -> FP64 and psi_{n+1} -> FP32
-          V inc = mk<T>((T)cself * nh.x, (T)cself * nh.y);
+        if (last || BODY < 0) {
+          // FP32 bodies of the last stage: the increment h sum_j b_j N_j is formed in FP32 from
+          // the FP32 N_j (its rounding is that of the N_j themselves); psi_{n+1} = psi_n + inc
+          // in FP64. FP64 and the any-stage body accumulate in FP64 throughout.
+          double2 y = ps[c];
+          if constexpr (sizeof(T) == 4 && BODY >= 0) {
+            V inc = mk<T>((T)cself * nh.x, (T)cself * nh.y);
 #pragma unroll
-          for (int q = 0; q < NQ; ++q) {
-            if (q < nqr) {
-              const T cq = (T)s_cq[q];
-              inc.x = fma(cq, nj[c][q].x, inc.x);
-              inc.y = fma(cq, nj[c][q].y, inc.y);
+            for (int q = 0; q < NQ; ++q) {
+              inc.x = fma((T)cq[q], nj[c][q].x, inc.x);
+              inc.y = fma((T)cq[q], nj[c][q].y, inc.y);
+            }
+            y = make_double2(y.x + (double)inc.x, y.y + (double)inc.y);
+          } else {
+            const double2 nhd = to_d2(nh);
+            y.x = fma(cself, nhd.x, y.x);
+            y.y = fma(cself, nhd.y, y.y);
+            if constexpr (NQ >= 0) {
+#pragma unroll
+              for (int q = 0; q < NQ; ++q) {
+                const double2 nv = to_d2(nj[c][q]);
+                y.x = fma(cq[q], nv.x, y.x);
+                y.y = fma(cq[q], nv.y, y.y);
+              }
+            } else {
+              for (int q = 0; q < kp.st.nq; ++q) {
+                const double2 nv = to_d2(__ldcg(as_t2<T>(d.Nh) + (size_t)kp.st.jq[q] * mstride + f));
+                const double cr = kp.st.cq[q] * h;
+                y.x = fma(cr, nv.x, y.x);
+                y.y = fma(cr, nv.y, y.y);
+              }
             }
           }
-          const double2 x = make_double2(ps[c].x + (double)inc.x, ps[c].y + (double)inc.y);
-          d.psi_hat[row + k] = x;
-          const double a2 = x.x * x.x + x.y * x.y;
-          finite = finite && isfinite(a2);
-          e_part += a2;
-          xt = from_d2<T>(x);
-          psiT[row + k] = xt;
-          // photon monitor in FP32 (per-thread partial sums; FP64 across threads)
-          if (w0f != 0.0f) {
-            const int kk = (k <= (Gm::N >> 1)) ? k : k - Gm::N;
-            const float af = __int_as_float(0x4B400000 + kk) - 12582912.0f;  // kk as float, exact
-            p_part_f += __fdividef(xt.x * xt.x + xt.y * xt.y, fmaf(asf, af, w0f));
-          }
-        } else if (last) {
-          const double2 nhd = to_d2(nh);
-          double2 x = ps[c];
-          x.x = fma(cself, nhd.x, x.x);
-          x.y = fma(cself, nhd.y, x.y);
-#pragma unroll
-          for (int q = 0; q < NQ; ++q) {
-            if (q < nqr) {
-              const double2 v = to_d2(nj[c][q]);
-              x.x = fma(s_cq[q], v.x, x.x);
-              x.y = fma(s_cq[q], v.y, x.y);
+          xt = from_d2<T>(y);
+          if (last) {
+            d.psi_hat[f] = y;
+            if constexpr (sizeof(T) == 4) as_t2<T>(d.psi_t)[f] = xt;
+            const double a2 = y.x * y.x + y.y * y.y;
+            finite = finite && isfinite(a2);
+            e_part += a2;
+            if constexpr (sizeof(T) == 4) {
+              // photon monitor in FP32 (per-thread partial sums; FP64 across threads)
+              if (w0f != 0.0f) {
+                const int kk = (k <= (Gm::N >> 1)) ? k : k - Gm::N;
+                const float af = __int_as_float(0x4B400000 + kk) - 12582912.0f;  // kk as float, exact
+                p_part_f += __fdividef(xt.x * xt.x + xt.y * xt.y, fmaf(asf, af, w0f));
+              }
+            } else {
+              if (d.omega0_T0 != 0.0) p_part += a2 / (d.omega0_T0 + alpha);
             }
           }
-          d.psi_hat[row + k] = x;
-          const double a2 = x.x * x.x + x.y * x.y;
-          finite = finite && isfinite(a2);
-          e_part += a2;
-          if (d.omega0_T0 != 0.0) p_part += a2 / (d.omega0_T0 + alpha);
-          xt = from_d2<T>(x);
         } else {
           if constexpr (!kReadT) xt = from_d2<T>(ps[c]);
           else xt = pt[c];  // = psi_hat rounded to T
           const T cs = (T)cself;
           xt.x = fma(cs, nh.x, xt.x);
           xt.y = fma(cs, nh.y, xt.y);
+          if constexpr (NQ > 0) {
 #pragma unroll
-          for (int q = 0; q < NQ; ++q) {
-            if (q < nqr) {
-              const T cq = (T)s_cq[q];
-              xt.x = fma(cq, nj[c][q].x, xt.x);
-              xt.y = fma(cq, nj[c][q].y, xt.y);
+            for (int q = 0; q < NQ; ++q) {
+              xt.x = fma((T)cq[q], nj[c][q].x, xt.x);
+              xt.y = fma((T)cq[q], nj[c][q].y, xt.y);
             }
           }
         }
         V en;
         if (same_z) en = ei;
         else en = expi<T>(L * znext);
-        s[Gm::sidx(li)] = spec_in(cmul(xt, en));
+        w[c] = cmul(xt, en);
       }
-    }
-  };
-  // One body per kernel: every extra copy of this loop grows the kernel, and a larger
-  // kernel runs its transforms slower (measured: the forward transform ran ~50% slower
-  // with seven copies). The generic instantiation (stages of the order-6 and order-8
-  // tableaus) runs the same body with the count at run time (at most kFastQ stored terms,
-  // loads predicated), and an element-wise loop beyond that.
-  constexpr int kFastQ = 5;
-  if constexpr (BODY >= 0) {
-    constexpr int NQB = BODY >= kNuLastBody ? BODY - kNuLastBody : BODY;
-    body(std::integral_constant<int, NQB>{}, NQB);
-  } else if (nq <= kFastQ) {
-    body(std::integral_constant<int, kFastQ>{}, nq);
-  } else {
-#pragma unroll 2
-  for (int li = tid; li < Gm::NL; li += Gm::NTHR) {
-    const int k = Gm::freq_of(rank, li);
-    const double alpha = alpha_of(k, Gm::N, d.alpha_scale);
-    const double L = im_L(poly, d.n_beta, alpha);
-    // N_hat_i = i sgn(gamma) conj(E_i) FFT(sigma)   (src/MultimodePropagation_CPU.cpp:231-237)
-    const V xe = cmulc(s[Gm::sidx(li)], expi<T>(L * zi));
-    V nh;
-    nh.x = (T)(-d.sgn_gamma) * xe.y;
-    nh.y = (T)(d.sgn_gamma) * xe.x;
-    Nh[(size_t)i * mstride + row + k] = nh;
-    const double2 nhd = to_d2(nh);
-    double2 x = d.psi_hat[row + k];
-    if (last) {
-      // psi_{n+1} = psi_n + h sum_j b_j N_j  (src/MultimodePropagation_CPU.cpp:75-85), FP64
-      for (int j = 0; j < S; ++j) {
-        const double bj = kp.tab.b[j];
-        if (bj != 0.0) {
-          const double2 nj = (j == i) ? nhd : to_d2(Nh[(size_t)j * mstride + row + k]);
-          x.x = fma(bj * h, nj.x, x.x);
-          x.y = fma(bj * h, nj.y, x.y);
-        }
-      }
-      d.psi_hat[row + k] = x;
-      if constexpr (sizeof(T) == 4) psiT[row + k] = from_d2<T>(x);
-      const double a2 = x.x * x.x + x.y * x.y;
-      finite = finite && isfinite(a2);
-      e_part += a2;
-      if (d.omega0_T0 != 0.0) p_part += a2 / (d.omega0_T0 + alpha);
+    };
+    V w[Gm::RM];
+    fetch(0);
+#pragma unroll
+    for (int r = 0; r < Gm::RM; ++r) w[r] = x[Gm::pad(r)];
+    RegDFT<Gm::RM, false>::run(w);
+    if constexpr (CHK == Gm::RM) {
+      chunk(w, 0);
     } else {
-      for (int j = 0; j <= i; ++j) {
-        const double aij = kp.tab.a[i + 1][j];
-        if (aij != 0.0) {
-          const double2 nj = (j == i) ? nhd : to_d2(Nh[(size_t)j * mstride + row + k]);
-          x.x = fma(aij * h, nj.x, x.x);
-          x.y = fma(aij * h, nj.y, x.y);
-        }
+      // through the thread's own positions in shared memory: a loop with one body, whose
+      // registers hold one chunk
+#pragma unroll
+      for (int r = 0; r < Gm::RM; ++r) x[Gm::pad(r)] = w[r];
+#pragma unroll 1
+      for (int c0 = 0; c0 < Gm::RM; c0 += CHK) {
+        V wc[CHK];
+        if (c0 > 0) fetch(c0);
+#pragma unroll
+        for (int c = 0; c < CHK; ++c) wc[c] = x[Gm::pad(c0) + c];
+        chunk(wc, c0);
+#pragma unroll
+        for (int c = 0; c < CHK; ++c) x[Gm::pad(c0) + c] = wc[c];
       }
+#pragma unroll
+      for (int r = 0; r < Gm::RM; ++r) w[r] = x[Gm::pad(r)];
     }
-    s[Gm::sidx(li)] = spec_in(cmul(from_d2<T>(x), expi<T>(L * znext)));
-  }
-  }
+    RegDFT<Gm::RM, true>::run(w);
+#pragma unroll
+    for (int r = 0; r < Gm::RM; ++r) x[Gm::pad(r)] = w[r];
+  });
   p_part += (double)p_part_f;
   if (last) {
     // Block reduction of the monitors, then the last CTA of this solve advances the
-    // step. Done before the inverse transform, so none of it is live across that call;
-    // every CTA of the solve read the step counter at its start, and the next launch
-    // starts only after this one has finished.
+    // step. Done before the inverse passes, so none of it is live across them; every CTA of
+    // the solve has read the step counter, and the next launch's reads follow this launch.
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       e_part += __shfl_xor_sync(0xffffffffu, e_part, o);
@@ -799,23 +753,22 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
     if ((tid & 31) == 0) { red[0][tid >> 5] = e_part; red[1][tid >> 5] = p_part; }
     __syncthreads();
     if (tid == 0) {
-      const unsigned long long n = s_cnt[0], total = s_cnt[1];
       double es = 0.0, ps = 0.0;
       for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { es += red[0][w]; ps += red[1][w]; }
       if (!finite_all) atomicOr(d.status, kStatusNonFinite);
-      if (d.monitors && total < d.mon_cap) {
-        atomicAdd(&d.energy[total], es * d.energy_scale);
-        if (d.omega0_T0 != 0.0) atomicAdd(&d.photons[total], ps * d.photon_scale);
+      if (d.monitors && n_total < d.mon_cap) {
+        atomicAdd(&d.energy[n_total], es * d.energy_scale);
+        if (d.omega0_T0 != 0.0) atomicAdd(&d.photons[n_total], ps * d.photon_scale);
       }
       __threadfence();
       const unsigned prev = atomicAdd(d.done_ctr, 1u);
       if (prev == (unsigned)(d.M * Gm::C) - 1u) {
         *d.done_ctr = 0u;
-        *d.step = n + 1;
-        *d.total = total + 1;
-        if (d.drift_tol > 0.0 && d.monitors && total < d.mon_cap) {
+        *d.step = n_step + 1;
+        *d.total = n_total + 1;
+        if (d.drift_tol > 0.0 && d.monitors && n_total < d.mon_cap) {
           // every CTA's energy sum is in (their adds precede their counter increments)
-          const double en = __ldcg(&d.energy[total]), e0 = *d.drift_ref;
+          const double en = __ldcg(&d.energy[n_total]), e0 = *d.drift_ref;
           if (e0 == 0.0) *d.drift_ref = en;
           else if (!(fabs(en - e0) <= d.drift_tol * e0)) atomicOr(d.status, kStatusDrift);
         }
@@ -823,97 +776,122 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
       }
     }
   }
-  V* U = as_t2<T>(d.U);
+  rows_inv<Gm>(sr, tw, u);
+  row_last_inv<Gm>(v, s, tw, rank);
+  V* U = as_t2<T>(d.U) + row + i0;
   const T inv = (T)d.inv_nt;
-  if constexpr (Gm::C == 1) {
-    // inverse transform as conj(FFT(conj(x))): the spectrum was stored conjugated, so
-    // this kernel carries the forward transform's code only (a smaller kernel runs its
-    // transforms faster)
-    forward<T, LOGN, XC>(s, sq, kp.tw);
-#pragma unroll 8
-    for (int u = tid; u < Gm::NL; u += Gm::NTHR) U[(size_t)p * Gm::N + u] = cscale(cconj(s[pad(u)]), inv);
-  } else {
-    inverse<T, LOGN, XC>(s, sq, kp.tw);
-#pragma unroll 8
-    for (int w = tid; w < Gm::NL; w += Gm::NTHR)
-      U[(size_t)p * Gm::N + Gm::time_of_w(rank, w)] = cscale(s[Gm::sidx(Gm::local_of_w(w))], inv);
-  }
+#pragma unroll
+  for (int r = 0; r < Gm::E; ++r) U[r * Gm::B] = cscale(v[r], inv);
+  row_leave<Gm>();
 }
 
 // ---- k_result: phi_p = IFFT(exp(L_p z) psi_hat_p) / conversion_factor -> io (FP64) --------
+// psi_hat lies in the order of the solve's own kernels (kp.lay).
 template <typename T, int LOGN, int XC>
 __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_BLOCKS) k_result(const KParams kp) {
   using Gm = Geo<T, LOGN, XC>;
   using V = c2<T>;
-  MMP_ROW_SMEM();
+  MMP_ROW_SETUP();
   __shared__ double poly[kMaxBeta];
   __shared__ SolveDesc sdesc;
-  stage_desc(&sdesc, kp.descs + blockIdx.y);
-  const V* sq = load_twiddles<T, LOGN, XC>(smem_raw, kp.tw);
+  const SolveDesc* gd = kp.descs + blockIdx.y;
+  const int p = blockIdx.x / Gm::C;
+  if (p >= __ldg(&gd->M)) return;  // uniform over the cluster
+  stage_desc(&sdesc, gd);
+  stage_poly(poly, gd, p);
   __syncthreads();
   const SolveDesc& d = sdesc;
-  const int p = blockIdx.x / Gm::C;
-  if (p >= d.M) return;  // uniform over the cluster
-  const int rank = cluster_rank<Gm>();
-  const int tid = threadIdx.x;
-  load_poly(poly, d, p);
+  const V* tw = static_cast<const V*>(kp.tw);
   const unsigned long long n = __ldcg(d.step);
   const double z = (double)n * d.dz;
   const size_t row = (size_t)p * Gm::N;
-#pragma unroll 2
-  for (int li = tid; li < Gm::NL; li += Gm::NTHR) {
-    const int k = Gm::freq_of(rank, li);
-    const double th = im_L(poly, d.n_beta, alpha_of(k, Gm::N, d.alpha_scale)) * z;
-    s[Gm::sidx(li)] = cmul(from_d2<T>(d.psi_hat[row + k]), expi<T>(th));
+  rows_last<Gm>(sr, u, [&](int b, V* x) {
+    const int k0 = Gm::freq0(k1, b);
+    V w[Gm::RM];
+#pragma unroll
+    for (int r = 0; r < Gm::RM; ++r) w[r] = from_d2<T>(__ldcg(d.psi_hat + row + spec_pos(kp.lay, k0 + r * Gm::KSTR)));
+#pragma unroll
+    for (int r = 0; r < Gm::RM; ++r) {
+      const double th = im_L(poly, d.n_beta, alpha_of(k0 + r * Gm::KSTR, Gm::N, d.alpha_scale)) * z;
+      w[r] = cmul(w[r], expi<T>(th));
+    }
+    RegDFT<Gm::RM, true>::run(w);
+#pragma unroll
+    for (int r = 0; r < Gm::RM; ++r) x[Gm::pad(r)] = w[r];
+  });
+  rows_inv<Gm>(sr, tw, u);
+  V v[Gm::E];
+  row_last_inv<Gm>(v, s, tw, rank);
+  double2* io = d.io + row + i0;
+#pragma unroll
+  for (int r = 0; r < Gm::E; ++r) {
+    const double2 y = to_d2(v[r]);
+    io[r * Gm::B] = make_double2(y.x * d.result_scale, y.y * d.result_scale);
   }
-  inverse<T, LOGN, XC>(s, sq, kp.tw);
-#pragma unroll 8
-  for (int w = tid; w < Gm::NL; w += Gm::NTHR) {
-    const double2 r = to_d2(s[Gm::sidx(Gm::local_of_w(w))]);
-    d.io[row + Gm::time_of_w(rank, w)] = make_double2(r.x * d.result_scale, r.y * d.result_scale);
-  }
+  row_leave<Gm>();
 }
 
 // ---- k_dft: rows of FP64 samples -> transform in precision T -> rows of FP64 -------------
-// Forward (INV=false): out = scale * FFT(in). Inverse: out = scale * sum_k in[k] e^{+...}.
+// Forward (INV=false): out = scale * FFT(in), stored in order `lay`. Inverse (natural order
+// in): out = scale * sum_k in[k] e^{+...}. in may be out: a row is read whole before a
+// barrier after which it is written.
 struct DftArgs {
   const double2* in;
   double2* out;
   int rows;
   int pad_;
   double scale;
-  TwTables tw;
+  const void* tw;
+  SpecLayout lay;
 };
 
 template <typename T, int LOGN, int XC, bool INV>
 __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_BLOCKS) k_dft(const DftArgs a) {
   using Gm = Geo<T, LOGN, XC>;
   using V = c2<T>;
-  MMP_ROW_SMEM();
-  const int r = blockIdx.x / Gm::C;
-  if (r >= a.rows) return;
-  const int rank = cluster_rank<Gm>();
-  const int tid = threadIdx.x;
-  const V* sq = load_twiddles<T, LOGN, XC>(smem_raw, a.tw);
-  const size_t row = (size_t)r * Gm::N;
+  MMP_ROW_SETUP();
+  const int p = blockIdx.x / Gm::C;
+  if (p >= a.rows) return;
+  const V* tw = static_cast<const V*>(a.tw);
+  const size_t row = (size_t)p * Gm::N;
+  V v[Gm::E];
   if constexpr (!INV) {
-#pragma unroll 8
-    for (int w = tid; w < Gm::NL; w += Gm::NTHR) s[Gm::sidx(Gm::local_of_w(w))] = from_d2<T>(a.in[row + Gm::time_of_w(rank, w)]);
-    forward<T, LOGN, XC>(s, sq, a.tw);
-#pragma unroll 8
-    for (int li = tid; li < Gm::NL; li += Gm::NTHR) {
-      const double2 x = to_d2(s[Gm::sidx(li)]);
-      a.out[row + Gm::freq_of(rank, li)] = make_double2(x.x * a.scale, x.y * a.scale);
-    }
+    row_enter<Gm>();
+#pragma unroll
+    for (int r = 0; r < Gm::E; ++r) v[r] = from_d2<T>(__ldcg(a.in + row + i0 + r * Gm::B));
+    row_first<Gm>(v, s, tw, rank);
+    rows_fwd<Gm>(sr, tw, u);
+    rows_last<Gm>(sr, u, [&](int b, V* x) {
+      const int k0 = Gm::freq0(k1, b);
+      V w[Gm::RM];
+#pragma unroll
+      for (int r = 0; r < Gm::RM; ++r) w[r] = x[Gm::pad(r)];
+      RegDFT<Gm::RM, false>::run(w);
+#pragma unroll
+      for (int r = 0; r < Gm::RM; ++r) {
+        const double2 y = to_d2(w[r]);
+        a.out[row + spec_pos(a.lay, k0 + r * Gm::KSTR)] = make_double2(y.x * a.scale, y.y * a.scale);
+      }
+    });
+    // no peer's shared memory is touched after row_first
   } else {
-#pragma unroll 8
-    for (int li = tid; li < Gm::NL; li += Gm::NTHR) s[Gm::sidx(li)] = from_d2<T>(a.in[row + Gm::freq_of(rank, li)]);
-    inverse<T, LOGN, XC>(s, sq, a.tw);
-#pragma unroll 8
-    for (int w = tid; w < Gm::NL; w += Gm::NTHR) {
-      const double2 x = to_d2(s[Gm::sidx(Gm::local_of_w(w))]);
-      a.out[row + Gm::time_of_w(rank, w)] = make_double2(x.x * a.scale, x.y * a.scale);
+    rows_last<Gm>(sr, u, [&](int b, V* x) {
+      const int k0 = Gm::freq0(k1, b);
+      V w[Gm::RM];
+#pragma unroll
+      for (int r = 0; r < Gm::RM; ++r) w[r] = from_d2<T>(__ldcg(a.in + row + k0 + r * Gm::KSTR));
+      RegDFT<Gm::RM, true>::run(w);
+#pragma unroll
+      for (int r = 0; r < Gm::RM; ++r) x[Gm::pad(r)] = w[r];
+    });
+    rows_inv<Gm>(sr, tw, u);
+    row_last_inv<Gm>(v, s, tw, rank);
+#pragma unroll
+    for (int r = 0; r < Gm::E; ++r) {
+      const double2 y = to_d2(v[r]);
+      a.out[row + i0 + r * Gm::B] = make_double2(y.x * a.scale, y.y * a.scale);
     }
+    row_leave<Gm>();
   }
 }
 
@@ -1120,13 +1098,15 @@ __global__ void __launch_bounds__(256) k_raman_agg(const SolveDesc* __restrict__
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   V* sU = reinterpret_cast<V*>(smem_raw);
   V* sp = sU + (size_t)d.M * TT;  // lambda^j, j < TT
-  {  // the U tile and the powers of lambda as 16-byte asynchronous copies, before the step check
+  {  // the powers of lambda and the U tile as 16-byte asynchronous copies, before the step check
     const V* U = as_t2<T>(d.U);
     const int per_row = TT * (int)sizeof(V) / 16;
-    for (int idx = threadIdx.x; idx < (d.M + 1) * per_row; idx += blockDim.x) {
+    for (int c = threadIdx.x; c < per_row; c += blockDim.x)
+      cp_async16(reinterpret_cast<char*>(sp) + 16 * c, static_cast<const char*>(d.raman_pow) + 16 * c);
+    for (int idx = threadIdx.x; idx < d.M * per_row; idx += blockDim.x) {
       const int r = idx / per_row, c = idx - r * per_row;
-      const V* src = r < d.M ? U + (size_t)r * nt + t0 : as_t2<T>(d.raman_pow);
-      cp_async16(reinterpret_cast<char*>(sU + (size_t)r * TT) + 16 * c, reinterpret_cast<const char*>(src) + 16 * c);
+      cp_async16(reinterpret_cast<char*>(sU + (size_t)r * TT) + 16 * c,
+                 reinterpret_cast<const char*>(U + (size_t)r * nt + t0) + 16 * c);
     }
     cp_async_commit();
   }
@@ -1174,13 +1154,13 @@ __global__ void __launch_bounds__(32) k_raman_carry(const SolveDesc* __restrict_
   using V = c2<T>;
   const SolveDesc& d = descs[blockIdx.y];
   const int q = blockIdx.x;
-  if (q >= d.P || d.M == 0 || __ldcg(d.step) >= d.step_limit) return;
   const int lane = threadIdx.x;
   const int ntiles = nt / TT;
   const int per = (ntiles + 31) / 32;  // tiles per lane
   const int first = min(lane * per, ntiles), last = min(first + per, ntiles);
   double2 lamT = d.iir_lambda;  // lambda^TT (TT a power of two)
   for (int s = 1; s < TT; s <<= 1) lamT = cmul(lamT, lamT);
+  if (q >= d.P || d.M == 0 || __ldcg(d.step) >= d.step_limit) return;
   V* tiles = as_t2<T>(d.raman_tiles) + (size_t)q * ntiles * 2;
   Affine mine = affine_identity();
   for (int i = first; i < last; ++i) {
@@ -1274,23 +1254,9 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
   const int raman = raman_mode;
   const int P = d.P;                          // pair fields formed in this tile
   const int Pl = raman == 1 ? P : 0;          // pair rows loaded (Raman convolutions)
-  // The tile's rows are requested first, before the step check and the term staging
   const V* U = as_t2<T>(d.U);
   const V* R = as_t2<T>(d.W);
   const unsigned row_bytes = (unsigned)(TT * sizeof(V));
-  if (threadIdx.x == 0) {
-    mbar_init(&bar, 1);
-    mbar_arrive_expect_tx(&bar, (unsigned)(M + Pl) * row_bytes);
-  }
-  __syncthreads();
-  for (int r = threadIdx.x; r < M + Pl; r += blockDim.x) {
-    const V* src = (r < M) ? U + (size_t)r * nt + t0 : R + (size_t)(r - M) * nt + t0;
-    bulk_g2s(sU + (size_t)r * TT, src, row_bytes, &bar);
-  }
-  if (__ldcg(d.step) >= d.step_limit) {  // finished solve: the copies land before the CTA leaves
-    mbar_wait(&bar, 0, kMaxWaitPolls);
-    return;
-  }
   const T kerr = (T)d.one_minus_fR;
   V* sW = sU + (size_t)M * TT;
   const int n_terms = d.term_off[M];
@@ -1301,7 +1267,6 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
   V* sC = sW + (size_t)P * TT;
   // dense form: per warp, two chunks of kDenseChunk coefficient rows (cp.async double buffer)
   T* sA = reinterpret_cast<T*>(sC + (raman == 2 ? 2 * (size_t)P : 0));
-  if (raman == 2) stage_tile_carries<T>(sC, d, P, nt / TT, blockIdx.x);
   const size_t dense_elems = DENSE ? (size_t)(blockDim.x >> 5) * 2 * kDenseChunk * 2 * kDenseMaxModes : 0;
   ST* st = reinterpret_cast<ST*>(sA + dense_elems);
   if (stage_terms) {
@@ -1314,6 +1279,15 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
       st[j] = s;
     }
   }
+  if (threadIdx.x == 0) mbar_init(&bar, 1);
+  if (__ldcg(d.step) >= d.step_limit) return;  // finished solve (nothing is in flight yet)
+  if (threadIdx.x == 0) mbar_arrive_expect_tx(&bar, (unsigned)(M + Pl) * row_bytes);
+  __syncthreads();
+  for (int r = threadIdx.x; r < M + Pl; r += blockDim.x) {
+    const V* src = (r < M) ? U + (size_t)r * nt + t0 : R + (size_t)(r - M) * nt + t0;
+    bulk_g2s(sU + (size_t)r * TT, src, row_bytes, &bar);
+  }
+  if (raman == 2) stage_tile_carries<T>(sC, d, P, nt / TT, blockIdx.x);
   // every thread polls with a bound; the barrier makes the outcome CTA-uniform and
   // also publishes the staged terms
   const bool landed = mbar_wait(&bar, 0, d.tile_wait_polls);
@@ -1475,22 +1449,10 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2)) k_contract_pc(c
   if (t0 >= nt || d.M == 0) return;  // empty slot
   const int M = d.M, P = d.P;
   const unsigned row_bytes = (unsigned)(TT * sizeof(V));
-  if (threadIdx.x == 0) {
-    mbar_init(&bar, 1);
-    mbar_arrive_expect_tx(&bar, (unsigned)M * row_bytes);
-  }
-  __syncthreads();
-  for (int r = threadIdx.x; r < M; r += blockDim.x)
-    bulk_g2s(sU + (size_t)r * TT, as_t2<T>(d.U) + (size_t)r * nt + t0, row_bytes, &bar);
-  if (__ldcg(d.step) >= d.step_limit) {  // finished solve: the copies land before the CTA leaves
-    mbar_wait(&bar, 0, kMaxWaitPolls);
-    return;
-  }
   V* sW = sU + (size_t)M * TT;                             // [pc][TT], pair positions swizzled
   ST* st = reinterpret_cast<ST*>(sW + (size_t)pc * TT);   // every term, sorted by (p, pair field)
   const int n_terms = d.term_off[M];
   V* sC = reinterpret_cast<V*>(st + n_terms);               // states entering the tile, [P][2]
-  stage_tile_carries<T>(sC, d, P, nt / TT, blockIdx.x);
   for (int j = threadIdx.x; j < n_terms; j += blockDim.x) {
     const Term tm = d.terms[j];
     ST x;
@@ -1499,6 +1461,13 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2)) k_contract_pc(c
     x.q = (T)tm.q;
     st[j] = x;
   }
+  if (threadIdx.x == 0) mbar_init(&bar, 1);
+  if (__ldcg(d.step) >= d.step_limit) return;  // finished solve (nothing is in flight yet)
+  if (threadIdx.x == 0) mbar_arrive_expect_tx(&bar, (unsigned)M * row_bytes);
+  __syncthreads();
+  for (int r = threadIdx.x; r < M; r += blockDim.x)
+    bulk_g2s(sU + (size_t)r * TT, as_t2<T>(d.U) + (size_t)r * nt + t0, row_bytes, &bar);
+  stage_tile_carries<T>(sC, d, P, nt / TT, blockIdx.x);
   const bool landed = mbar_wait(&bar, 0, d.tile_wait_polls);
   if (!__syncthreads_and(landed ? 1 : 0)) {
     if (threadIdx.x == 0) atomicOr(d.status, kStatusTimeout);
@@ -1665,8 +1634,7 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TB;
-  if (t0 >= nt || d.M == 0) return;               // empty slot
-  if (__ldcg(d.step) >= d.step_limit) return;     // finished solve (nothing is in flight yet)
+  if (t0 >= nt || d.M == 0) return;  // empty slot
   const int M = d.M, P = d.P, nterm = d.sr_terms, rounds = d.sr_rounds;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // shared memory: U [2][M][RS], W [P][RS], group plan [rounds kSrGroups], merged terms
@@ -1685,6 +1653,7 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
     }
     for (int i = tid; i < rounds * kSrGroups; i += kSrThreads) sPlan[i] = d.sr_plan[i];
   }
+  if (__ldcg(d.step) >= d.step_limit) return;  // finished solve (nothing is in flight yet)
   // U staging: sample pair j of row r is item r J + j; a thread carries at most two
   const V* U = as_t2<T>(d.U);
   const int nu = M * J;
@@ -1983,14 +1952,11 @@ __global__ void __launch_bounds__(512, 1) k_contract_tc(const SolveDesc* __restr
       mbar_init(&bar_b[i], 1);
       mbar_init(&bar_m[i], 1);
     }
-    mbar_arrive_expect_tx(&bar_u, (unsigned)(M * TT * sizeof(V)));
   }
+  if (__ldcg(d.step) >= d.step_limit) return;  // finished solve (nothing is in flight yet)
+  if (tid == 0) mbar_arrive_expect_tx(&bar_u, (unsigned)(M * TT * sizeof(V)));
   __syncthreads();
   if (tid < M) bulk_g2s(sU + (size_t)tid * TT, as_t2<float>(d.U) + (size_t)tid * nt + t0, TT * sizeof(V), &bar_u);
-  if (__ldcg(d.step) >= d.step_limit) {  // finished solve: the copies land before the CTA leaves
-    mbar_wait(&bar_u, 0, kMaxWaitPolls);
-    return;
-  }
   if (raman_mode == 2) stage_tile_carries<float>(sC, d, P, nt / TT, blockIdx.x);
   if (warp == 0) {
     tc::alloc(&s_tmem, 512);
