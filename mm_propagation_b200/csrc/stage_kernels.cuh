@@ -185,6 +185,16 @@ __device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes) {
   }
 }
 
+// Programmatic dependent launch: the kernels of a step are launched to start while the one before
+// them still runs (solver.cu, launch). What does not depend on it (descriptors, polynomials,
+// terms: written only by copies, which order fully) is staged first; grid_sync_wait returns
+// once the earlier kernel is complete and its writes are visible. Every CTA passes it before it
+// reads a field or leaves, so that a kernel's completion implies that of all before it.
+// grid_release lets the next kernel start; it stands late, before a kernel's last stores, so that
+// the next one's waiting CTAs do not take SMs from kernels that could run.
+__device__ __forceinline__ void grid_sync_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Ampere-style asynchronous copies global -> shared (both addresses aligned to the size),
 // grouped and waited for per thread: the loads are in flight without holding registers.
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
@@ -268,12 +278,16 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
   MMP_ROW_SETUP();
   const SolveDesc* gd = kp.descs + blockIdx.y;
   const int q = blockIdx.x / Gm::C;
-  if (q >= __ldg(&gd->P)) return;  // uniform over the cluster
+  if (q >= __ldg(&gd->P)) {  // uniform over the cluster
+    grid_sync_wait();
+    return;
+  }
   const unsigned long long* step = ldg_ptr(&gd->step);
   const V* U = as_t2<T>(static_cast<const void*>(ldg_ptr(&gd->U))) + i0;
   const V* H = as_t2<T>(static_cast<const void*>(ldg_ptr(&gd->H)));
   V* W = as_t2<T>(ldg_ptr(&gd->W));
   const int2 lm = __ldg(ldg_ptr(&gd->pairs) + q);
+  grid_sync_wait();
   if (__ldcg(step) >= __ldg(&gd->step_limit)) return;  // uniform over the cluster
   row_enter<Gm>();
   const V* tw = static_cast<const V*>(kp.tw);
@@ -299,6 +313,7 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
     for (int r = 0; r < Gm::RM; ++r) x[Gm::pad(r)] = w[r];
   });
   rows_inv<Gm>(sr, tw, u);
+  grid_release();
   row_last_inv<Gm>(v, s, tw, rank);
   // R_q = (H_R conv V_q); the Kerr part (1 - fR) V_q is formed by the contraction from
   // the U tile it already holds
@@ -401,6 +416,7 @@ __global__ void __launch_bounds__(512) k_raman_scan(const SolveDesc* __restrict_
   __shared__ Affine seg_map[kMaxSeg];
   const SolveDesc& d = descs[blockIdx.y];
   const int q = blockIdx.x;
+  grid_sync_wait();
   if (q >= d.P || __ldcg(d.step) >= d.step_limit) return;  // uniform over the CTA
   const int tid = threadIdx.x;
   const int nthr = blockDim.x;                   // 32..512, a power of two
@@ -481,6 +497,7 @@ __global__ void __launch_bounds__(512) k_raman_scan(const SolveDesc* __restrict_
   double2 sa = cmul(row.ba, inv), sb = cmul(row.bb, inv);  // state entering segment 0
   const double2 kap = d.iir_kappa;
   const V kt = from_d2<T>(kap);
+  grid_release();
   // pass 2: outputs R = Im(kappa s), s = local + lambda^(k+1) C within each sub-chunk
   for (int g = 0; g < nseg; ++g) {
     if (nseg > 1) {
@@ -547,7 +564,10 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
   __shared__ SolveDesc sdesc;
   const SolveDesc* gd = kp.descs + blockIdx.y;
   const int p = blockIdx.x / Gm::C;
-  if (p >= __ldg(&gd->M)) return;  // also an empty slot (its descriptor is zero); uniform over the cluster
+  if (p >= __ldg(&gd->M)) {  // also an empty slot (its descriptor is zero); uniform over the cluster
+    grid_sync_wait();
+    return;
+  }
   const unsigned long long* stepp = ldg_ptr(&gd->step);
   const unsigned long long* totalp = ldg_ptr(&gd->total);
   const V* sg = as_t2<T>(static_cast<const void*>(ldg_ptr(&gd->sigma))) + (size_t)p * Gm::N + i0;
@@ -555,6 +575,7 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
   const double h = __ldg(&gd->dz);
   stage_desc(&sdesc, gd);
   stage_poly(poly, gd, p);
+  grid_sync_wait();
   const unsigned long long n_step = __ldcg(stepp), n_total = __ldcg(totalp);
   V v[Gm::E];
 #pragma unroll
@@ -777,6 +798,7 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
     }
   }
   rows_inv<Gm>(sr, tw, u);
+  grid_release();
   row_last_inv<Gm>(v, s, tw, rank);
   V* U = as_t2<T>(d.U) + row + i0;
   const T inv = (T)d.inv_nt;
@@ -1094,7 +1116,10 @@ __global__ void __launch_bounds__(256) k_raman_agg(const SolveDesc* __restrict__
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const SolveDesc& d = descs[blockIdx.y];
   const int tile = blockIdx.x, t0 = tile * TT;
-  if (t0 >= nt || d.M == 0) return;  // empty slot
+  if (t0 >= nt || d.M == 0) {  // empty slot
+    grid_sync_wait();
+    return;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   V* sU = reinterpret_cast<V*>(smem_raw);
   V* sp = sU + (size_t)d.M * TT;  // lambda^j, j < TT
@@ -1103,6 +1128,7 @@ __global__ void __launch_bounds__(256) k_raman_agg(const SolveDesc* __restrict__
     const int per_row = TT * (int)sizeof(V) / 16;
     for (int c = threadIdx.x; c < per_row; c += blockDim.x)
       cp_async16(reinterpret_cast<char*>(sp) + 16 * c, static_cast<const char*>(d.raman_pow) + 16 * c);
+    grid_sync_wait();
     for (int idx = threadIdx.x; idx < d.M * per_row; idx += blockDim.x) {
       const int r = idx / per_row, c = idx - r * per_row;
       cp_async16(reinterpret_cast<char*>(sU + (size_t)r * TT) + 16 * c,
@@ -1120,6 +1146,7 @@ __global__ void __launch_bounds__(256) k_raman_agg(const SolveDesc* __restrict__
   // lane + 32, ..., weighted from the table of powers, and the warp adds the lanes.
   cp_async_wait<0>();
   __syncthreads();
+  grid_release();
   const int ntiles = nt / TT;
   V* out = as_t2<T>(d.raman_tiles);
   for (int q = warp; q < d.P; q += nwarps) {
@@ -1160,6 +1187,8 @@ __global__ void __launch_bounds__(32) k_raman_carry(const SolveDesc* __restrict_
   const int first = min(lane * per, ntiles), last = min(first + per, ntiles);
   double2 lamT = d.iir_lambda;  // lambda^TT (TT a power of two)
   for (int s = 1; s < TT; s <<= 1) lamT = cmul(lamT, lamT);
+  grid_sync_wait();
+  grid_release();
   if (q >= d.P || d.M == 0 || __ldcg(d.step) >= d.step_limit) return;
   V* tiles = as_t2<T>(d.raman_tiles) + (size_t)q * ntiles * 2;
   Affine mine = affine_identity();
@@ -1249,7 +1278,10 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
   V* sU = reinterpret_cast<V*>(smem_raw);
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TT;
-  if (t0 >= nt || d.M == 0) return;  // empty slot
+  if (t0 >= nt || d.M == 0) {  // empty slot
+    grid_sync_wait();
+    return;
+  }
   const int M = d.M;
   const int raman = raman_mode;
   const int P = d.P;                          // pair fields formed in this tile
@@ -1269,6 +1301,7 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
   T* sA = reinterpret_cast<T*>(sC + (raman == 2 ? 2 * (size_t)P : 0));
   const size_t dense_elems = DENSE ? (size_t)(blockDim.x >> 5) * 2 * kDenseChunk * 2 * kDenseMaxModes : 0;
   ST* st = reinterpret_cast<ST*>(sA + dense_elems);
+  // the terms are staged while the kernel before this one still runs
   if (stage_terms) {
     for (int j = threadIdx.x; j < n_terms; j += blockDim.x) {
       const Term tm = d.terms[j];
@@ -1280,6 +1313,7 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
     }
   }
   if (threadIdx.x == 0) mbar_init(&bar, 1);
+  grid_sync_wait();
   if (__ldcg(d.step) >= d.step_limit) return;  // finished solve (nothing is in flight yet)
   if (threadIdx.x == 0) mbar_arrive_expect_tx(&bar, (unsigned)(M + Pl) * row_bytes);
   __syncthreads();
@@ -1323,6 +1357,7 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
       tile_pair_recurrence<T>(ts, sU, TT, d.pairs[q], sW + (size_t)q * TT, wmask, sC + 2 * q, kerr, lane);
   }
   __syncthreads();
+  grid_release();
   // 2. contraction
   V* sigma = as_t2<T>(d.sigma);
   if (DENSE == 1 || (DENSE == 2 && d.dense_q != nullptr)) {
@@ -1446,7 +1481,10 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2)) k_contract_pc(c
   V* sU = reinterpret_cast<V*>(smem_raw);  // [M][TT]
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TT;
-  if (t0 >= nt || d.M == 0) return;  // empty slot
+  if (t0 >= nt || d.M == 0) {  // empty slot
+    grid_sync_wait();
+    return;
+  }
   const int M = d.M, P = d.P;
   const unsigned row_bytes = (unsigned)(TT * sizeof(V));
   V* sW = sU + (size_t)M * TT;                             // [pc][TT], pair positions swizzled
@@ -1462,6 +1500,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2)) k_contract_pc(c
     st[j] = x;
   }
   if (threadIdx.x == 0) mbar_init(&bar, 1);
+  grid_sync_wait();
   if (__ldcg(d.step) >= d.step_limit) return;  // finished solve (nothing is in flight yet)
   if (threadIdx.x == 0) mbar_arrive_expect_tx(&bar, (unsigned)M * row_bytes);
   __syncthreads();
@@ -1523,6 +1562,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2)) k_contract_pc(c
     }
     __syncthreads();  // the chunk's fields are read before the next chunk overwrites them
   }
+  grid_release();
   V* sigma = as_t2<T>(d.sigma);
 #pragma unroll
   for (int i = 0; i < kPcItems; ++i) {
@@ -1634,7 +1674,10 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TB;
-  if (t0 >= nt || d.M == 0) return;  // empty slot
+  if (t0 >= nt || d.M == 0) {  // empty slot
+    grid_sync_wait();
+    return;
+  }
   const int M = d.M, P = d.P, nterm = d.sr_terms, rounds = d.sr_rounds;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // shared memory: U [2][M][RS], W [P][RS], group plan [rounds kSrGroups], merged terms
@@ -1653,6 +1696,7 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
     }
     for (int i = tid; i < rounds * kSrGroups; i += kSrThreads) sPlan[i] = d.sr_plan[i];
   }
+  grid_sync_wait();
   if (__ldcg(d.step) >= d.step_limit) return;  // finished solve (nothing is in flight yet)
   // U staging: sample pair j of row r is item r J + j; a thread carries at most two
   const V* U = as_t2<T>(d.U);
@@ -1715,6 +1759,7 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
   for (int sub = 0; sub < nsub; ++sub) {
     const int buf = sub & 1;
     if (sub + 1 < nsub) fetch(sub + 1);  // lands while this sub-block is worked on
+    else grid_release();
     const SP* uc = sU + (size_t)buf * M * RS;
     // phase A
 #pragma unroll
@@ -1814,6 +1859,7 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TB;
+  grid_sync_wait();
   if (t0 >= nt || d.M == 0) return;            // empty slot
   if (__ldcg(d.step) >= d.step_limit) return;  // finished solve
   const int M = d.M, P = d.P, tid = threadIdx.x;
@@ -1865,6 +1911,7 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
   for (int sub = 0; sub < nsub; ++sub) {
     const int buf = sub & 1;
     if (sub + 1 < nsub) fetch(sub + 1);
+    else grid_release();
     const SP* uc = sU + (size_t)buf * M * RS;
 #pragma unroll
     for (int i = 0; i < kSrPairsPerThread; ++i) {
@@ -1936,7 +1983,10 @@ __global__ void __launch_bounds__(512, 1) k_contract_tc(const SolveDesc* __restr
   __shared__ uint32_t s_tmem;
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TT;
-  if (t0 >= nt || d.M == 0) return;  // empty slot
+  if (t0 >= nt || d.M == 0) {  // empty slot
+    grid_sync_wait();
+    return;
+  }
   const int M = d.M, P = d.P, N = 16 * M;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   V* sU = reinterpret_cast<V*>(smem_raw);                        // [M][TT]
@@ -1953,6 +2003,7 @@ __global__ void __launch_bounds__(512, 1) k_contract_tc(const SolveDesc* __restr
       mbar_init(&bar_m[i], 1);
     }
   }
+  grid_sync_wait();
   if (__ldcg(d.step) >= d.step_limit) return;  // finished solve (nothing is in flight yet)
   if (tid == 0) mbar_arrive_expect_tx(&bar_u, (unsigned)(M * TT * sizeof(V)));
   __syncthreads();
@@ -2044,6 +2095,7 @@ __global__ void __launch_bounds__(512, 1) k_contract_tc(const SolveDesc* __restr
     }
     committed = c;
   }
+  grid_release();
   // the last chunk's MMAs complete after all earlier ones (in-order issue, one thread)
   if (ok && committed >= 0)
     ok = __syncthreads_and(mbar_wait(&bar_m[committed & 1], (committed >> 1) & 1, kMaxWaitPolls) ? 1 : 0);
