@@ -124,14 +124,17 @@ struct SolveDesc {
   // when the sampled h_R fits it; kappa = Delta_t T0 f_R c (1 - lambda^NT),
   // inv_one_minus = 1 / (1 - lambda^NT).
   int iir;
-  int pad2_;
+  // samples after which the recurrence has forgotten its state (|lambda|^iir_len below
+  // rounding): how far back a tile looks for the state entering it (tile_carry)
+  int iir_len;
   double2 iir_lambda;
   double2 iir_kappa;
   double2 iir_inv_one_minus;
   // [kRamanPow] (T complex): lambda^j, j < kRamanPow, computed once in FP64 (iir solves)
   const void* raman_pow;
-  // [P][NT/16][2] (T complex): per contraction tile and pair field, the recurrence's
-  // tile aggregate (k_raman_agg), then the state entering the tile (k_raman_carry)
+  // (T complex; room for tiles of 16 samples) per contraction tile and pair field, the recurrence's
+  // tile aggregate (k_raman_agg): [NT/TT][P][2], or [P][NT/TT][2] where k_raman_carry puts the
+  // state entering the tile in its place
   void* raman_tiles;
   // Dense form of the contraction (M <= kDenseMaxModes), T values [M][P][2 kDenseMaxModes]:
   // entry (p, q, k) sums Q over the terms of p with U_k and pair field q, entry

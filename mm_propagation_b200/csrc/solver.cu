@@ -152,6 +152,7 @@ void dev_free(void* p, cudaStream_t st = nullptr, bool pooled = false) {
 constexpr int kScanSmem = padded_len(128 * 1024 / 8) * 8;
 // Dynamic shared memory k_contract may take (the 227 KB per block, less its static part)
 constexpr size_t kContractSmemMax = 226 * 1024;
+constexpr int kMaxLook = 16;  // tiles the contraction looks back for a Raman state (choose_shape)
 constexpr int kSMs = 148;  // of a B200
 constexpr int kSmemSM = 228 * 1024;  // its shared memory
 
@@ -389,6 +390,7 @@ struct Member {
   int sr_rounds = 0;
   std::vector<double> poly;
   bool quirk = false;
+  double iir_decay = 0;   // -ln |lambda| of the Raman recurrence (h_R a damped sinusoid)
   bool dense_ok = false;  // the dense contraction form is built for this solve
   uint32_t flags = 0;
   // device
@@ -672,6 +674,7 @@ struct mmp_batch {
   uint32_t groups = 1;
   bool raman_iir = false;  // every solve's h_R is a damped sinusoid: pair fields by k_raman_scan
   bool raman_fused = false;  // ... and the recurrence runs inside the contraction tiles
+  bool lookback = false;     // ... which sum the states entering them themselves (no k_raman_carry)
   int dense = 0;  // contraction form: 0 term loop, 1 dense (k_contract<T, 1>), 2 per solve
   bool tc = false;  // dense form on the tensor cores (k_contract_tc)
   int pchunk = 0;   // > 0: pair fields per chunk of the pair-chunked contraction (k_contract_pc)
@@ -788,7 +791,7 @@ int launch_contract(mmp_batch* b, uint32_t first = 0, uint32_t count = ~0u, cuda
   if (count == 0) return MMP_OK;
   const SolveDesc* descs = b->d_descs + first;
   int nt = (int)b->nt, TT = b->TT, sterms = b->stage_terms;
-  int mode = !b->raman ? 0 : (b->raman_fused ? 2 : 1);
+  int mode = !b->raman ? 0 : (b->lookback ? 3 : b->raman_fused ? 2 : 1);
   void* args[] = {(void*)&descs, &nt, &TT, &sterms, &mode};
   dim3 grid((unsigned)(b->nt / b->TT), count, 1);
   const void* f32[] = {(const void*)&k_contract<float, 0>, (const void*)&k_contract<float, 1>,
@@ -804,7 +807,7 @@ int launch_contract(mmp_batch* b, uint32_t first = 0, uint32_t count = ~0u, cuda
   }
   if (b->pchunk) {
     int pc = b->pchunk;
-    void* pargs[] = {(void*)&descs, &nt, &TT, &pc};
+    void* pargs[] = {(void*)&descs, &nt, &TT, &pc, &mode};
     const void* fpc = b->fp64 ? (const void*)&k_contract_pc<double> : (const void*)&k_contract_pc<float>;
     CUDA_TRY(launch(fpc, grid, 256, (int)b->contract_smem, 1, st ? st : b->stream, pargs, true));
     return MMP_OK;
@@ -840,7 +843,8 @@ int launch_pairs(mmp_batch* b, const KernelSet& ks, int nsolves, int stage, cons
     const size_t t2 = b->fp64 ? sizeof(double2) : sizeof(float2);
     int TT = b->TT;
     const SolveDesc* dd = descs;
-    void* args[] = {(void*)&dd, &nt, &TT};
+    int by_tile = b->lookback ? 1 : 0;
+    void* args[] = {(void*)&dd, &nt, &TT, &by_tile};  // k_raman_carry takes the first three
     if (b->sr) {  // one thread per pair field through the tile (k_contract_sr's tiles)
       const int smem = (int)(2 * (size_t)b->Mmax * (kSrSub / 2 + 1) * 2 * t2);
       const void* fa = b->fp64 ? (const void*)&k_raman_agg_sr<double> : (const void*)&k_raman_agg_sr<float>;
@@ -851,6 +855,7 @@ int launch_pairs(mmp_batch* b, const KernelSet& ks, int nsolves, int stage, cons
       const void* fa = b->fp64 ? (const void*)&k_raman_agg<double> : (const void*)&k_raman_agg<float>;
       CUDA_TRY(launch(fa, dim3((unsigned)(nt / TT), (unsigned)nsolves, 1), 256, smem, 1, st ? st : b->stream, args, true));
     }
+    if (b->lookback) return MMP_OK;
     const void* fc = b->fp64 ? (const void*)&k_raman_carry<double> : (const void*)&k_raman_carry<float>;
     CUDA_TRY(launch(fc, dim3((unsigned)b->Pmax, (unsigned)nsolves, 1), 32, 0, 1, st ? st : b->stream, args, true));
     return MMP_OK;
@@ -1219,6 +1224,13 @@ bool fit_damped_sinusoid(const double* h, uint32_t n, std::complex<double>& lam,
   return true;
 }
 
+// Samples after which the Raman recurrence has forgotten its state: |lambda|^n below 1e-11
+// (FP32) or 1e-20 (FP64), four decades under the rounding of what it is added to.
+int iir_len(double decay, bool fp64) {
+  const double n = (fp64 ? 46.0 : 25.3) / std::max(decay, 1e-9);
+  return n < 1e9 ? (int)std::ceil(n) : 1000000000;
+}
+
 // Host setup, device state and uploads for slot idx from params p; leaves the solve
 // at z = 0 with its initial fields transformed. One cudaMalloc for all of it.
 int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
@@ -1314,6 +1326,8 @@ int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
       const std::complex<double> kap = (s.delta_t * s.T0 * s.fR) * c * (1.0 - lamN);
       const std::complex<double> inv = 1.0 / (1.0 - lamN);
       d.iir = 1;
+      s.iir_decay = -std::log(std::abs(lam));
+      d.iir_len = iir_len(s.iir_decay, b->fp64);
       d.iir_lambda = make_double2(lam.real(), lam.imag());
       d.iir_kappa = make_double2(kap.real(), kap.imag());
       d.iir_inv_one_minus = make_double2(inv.real(), inv.imag());
@@ -1421,6 +1435,7 @@ struct ShapeStats {
   int Mmax = 0, Mmin = 1 << 30, Pmax = 0, Pall = 0;
   size_t max_terms = 0, max_sr_terms = 0;
   bool iir = true, all_dense = true, any_dense = false;
+  double min_decay = 1e300;  // slowest Raman recurrence (where all have one: iir)
   uint32_t span = 0;
 };
 
@@ -1429,10 +1444,12 @@ struct SolveCounts {
   int M = 0;
   size_t pairs = 0, terms = 0, sr_terms = 0;
   bool iir = false, dense_ok = false;
+  double iir_decay = 0;
 };
 
 void add_stats(ShapeStats& st, const mmp_batch* b, const SolveCounts& c, uint32_t span) {
   st.iir = st.iir && c.iir;
+  st.min_decay = std::min(st.min_decay, c.iir_decay);
   st.all_dense = st.all_dense && c.dense_ok;
   st.any_dense = st.any_dense || c.dense_ok;
   st.span = std::max(st.span, span);
@@ -1451,6 +1468,7 @@ SolveCounts member_counts(const Member& s) {
   c.terms = s.terms.size();
   c.sr_terms = s.sr_kq.size();
   c.iir = s.desc.iir != 0;
+  c.iir_decay = s.iir_decay;
   c.dense_ok = s.dense_ok;
   return c;
 }
@@ -1466,7 +1484,7 @@ ShapeStats batch_stats(const mmp_batch* b) {
 // memory they take, chosen from its statistics alone.
 struct Shape {
   int Mmax = 0, Pmax = 0, TT = 32, dense = 0, pchunk = 0, stage_terms = 0;
-  bool tc = false, sr = false, fused = false, iir = false;
+  bool tc = false, sr = false, fused = false, iir = false, lookback = false;
   size_t smem = 0;
   uint32_t span = 0;
 };
@@ -1474,7 +1492,7 @@ struct Shape {
 // Shapes that run the same kernels with the same tiles on a solve (so give it the same bits).
 bool same_kernels(const Shape& x, const Shape& y) {
   return x.TT == y.TT && x.dense == y.dense && x.pchunk == y.pchunk && x.stage_terms == y.stage_terms &&
-         x.tc == y.tc && x.sr == y.sr && x.fused == y.fused && x.iir == y.iir;
+         x.tc == y.tc && x.sr == y.sr && x.fused == y.fused && x.iir == y.iir && x.lookback == y.lookback;
 }
 
 Shape choose_shape(const mmp_batch* b, const ShapeStats& st) {
@@ -1577,6 +1595,11 @@ Shape choose_shape(const mmp_batch* b, const ShapeStats& st) {
       smem = (need + 15) & ~(size_t)15;
     }
   }
+  // The tiles sum the states entering them from the aggregates before them where that takes few
+  // of them (kMaxLook), instead of a k_raman_carry launch. MMP_LOOKBACK=0 keeps the launch.
+  bool lookback = fused && std::min((int)b->nt / TT, (iir_len(st.min_decay, b->fp64) - 1) / TT + 1) <= kMaxLook;
+  if (const char* env = std::getenv("MMP_LOOKBACK"))
+    if (std::atoi(env) == 0) lookback = false;
   const int stage_terms = sr ? 0 : (pchunk ? 1 : (dense != 1 && !tc && smem + max_terms * staged <= 200 * 1024 ? 1 : 0));
   if (stage_terms && !pchunk) smem += max_terms * staged;
   Shape sh;
@@ -1590,6 +1613,7 @@ Shape choose_shape(const mmp_batch* b, const ShapeStats& st) {
   sh.sr = sr;
   sh.fused = fused;
   sh.iir = iir;
+  sh.lookback = lookback;
   sh.smem = smem;
   sh.span = span;
   return sh;
@@ -1611,6 +1635,7 @@ SolveCounts solve_counts(const mmp_params* p) {
   if (p->raman && p->raman_response) {
     std::complex<double> lam, cc;
     c.iir = fit_damped_sinusoid(p->raman_response, p->nt, lam, cc);
+    if (c.iir) c.iir_decay = -std::log(std::abs(lam));
   }
   c.dense_ok = dense_wanted(nullptr, m);
   return c;
@@ -1648,14 +1673,15 @@ bool batch_shape(mmp_batch* b) {
   const bool changed = resplit || sh.Mmax != b->Mmax || sh.Pmax != b->Pmax || sh.TT != b->TT || sh.smem != b->contract_smem ||
                        sh.stage_terms != b->stage_terms || sh.span != b->span || sh.iir != b->raman_iir ||
                        sh.fused != b->raman_fused || sh.dense != b->dense || sh.tc != b->tc ||
-                       sh.pchunk != b->pchunk || sh.sr != b->sr;
+                       sh.pchunk != b->pchunk || sh.sr != b->sr || sh.lookback != b->lookback;
   b->dense = sh.dense;
   b->tc = sh.tc;
   b->pchunk = sh.pchunk;
   b->sr = sh.sr;
   b->raman_iir = sh.iir;
   b->raman_fused = sh.fused;
-  b->kernels_per_step = b->tab.s * ((b->raman ? (sh.fused ? 2 : 1) : 0) + 2);
+  b->lookback = sh.lookback;
+  b->kernels_per_step = b->tab.s * ((b->raman ? (sh.fused && !sh.lookback ? 2 : 1) : 0) + 2);
   b->span = sh.span;
   b->Mmax = sh.Mmax;
   b->Pmax = sh.Pmax;

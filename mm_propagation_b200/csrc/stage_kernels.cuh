@@ -1020,13 +1020,52 @@ template <typename T> struct TileScan {
 // distinct banks per quarter warp; mask 0 is the plain layout.
 __device__ __forceinline__ int wsw(int h, int mask) { return h ^ ((h >> 3) & mask); }
 
-// The states entering tile `tile` for pair fields 0..P-1 (k_raman_carry's output) into
-// shared memory, [q][Re V, Im V]; published by the caller's next barrier.
+// The state entering tile `tile` for idx = 2 q (Re V of pair field q) or 2 q + 1 (Im V).
+// look = 0: k_raman_carry has left it in the aggregates' place. Else it is summed here from the
+// aggregates of the `look` tiles before (around the period),
+//   C = sum_{i=1..look} lambda^(TT (i-1)) A_{tile-i}     [times 1 / (1 - lambda^NT) over a whole row],
+// in FP64: what lies further back is below rounding. Measured on a B200 against a launch of
+// k_raman_carry per stage (microseconds a step): 6 modes of 16384 98 -> 91, 2 of 4096 in FP64
+// 65 -> 59, 1 of 2048 48 -> 44 (RK4, one solve); 3 solves of 10 x 32768 261 -> 257; 8 of the
+// 28-mode order-6 solves 6450 -> 6394.
+// The aggregates lie [tile][q][2] for that, and [q][tile][2] where k_raman_carry scans them.
 template <typename T>
-__device__ __forceinline__ void stage_tile_carries(c2<T>* sC, const SolveDesc& d, int P, int ntiles, int tile) {
-  const c2<T>* tiles = as_t2<T>(d.raman_tiles);
-  for (int i = threadIdx.x; i < 2 * P; i += blockDim.x)
-    sC[i] = tiles[((size_t)(i >> 1) * ntiles + tile) * 2 + (i & 1)];
+__device__ __forceinline__ c2<T> tile_carry(const SolveDesc& d, int ntiles, int tile, int idx, int look,
+                                            double2 lamT) {
+  using V = c2<T>;
+  const V* tiles = as_t2<T>(static_cast<const void*>(d.raman_tiles));
+  if (look == 0) return __ldcg(tiles + ((size_t)(idx >> 1) * ntiles + tile) * 2 + (idx & 1));
+  const size_t P2 = 2 * (size_t)d.P;
+  tiles += idx;
+  double2 c = make_double2(0.0, 0.0);
+  for (int i0 = look; i0 > 0; i0 -= 4) {  // the farthest first, four loads in flight
+    V a[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (i0 - e > 0) a[e] = __ldcg(tiles + (size_t)((tile - (i0 - e) + ntiles) & (ntiles - 1)) * P2);
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (i0 - e > 0) c = cadd(cmul(lamT, c), to_d2(a[e]));
+  }
+  if (look == ntiles) c = cmul(c, d.iir_inv_one_minus);
+  return from_d2<T>(c);
+}
+__device__ __forceinline__ double2 lambda_tile(const SolveDesc& d, int TT) {  // lambda^TT (TT a power of two)
+  double2 l = d.iir_lambda;
+  for (int s = 1; s < TT; s <<= 1) l = cmul(l, l);
+  return l;
+}
+// Tiles a solve looks back: all of a short row's.
+__device__ __forceinline__ int tile_look(const SolveDesc& d, int ntiles, int TT, int raman_mode) {
+  return raman_mode == 3 ? min((d.iir_len + TT - 1) / TT, ntiles) : 0;
+}
+
+// The states entering tile `tile` for pair fields 0..P-1 into shared memory, [q][Re V, Im V];
+// published by the caller's next barrier.
+template <typename T>
+__device__ __forceinline__ void stage_tile_carries(c2<T>* sC, const SolveDesc& d, int P, int ntiles, int tile,
+                                                   int look, double2 lamT) {
+  for (int i = threadIdx.x; i < 2 * P; i += blockDim.x) sC[i] = tile_carry<T>(d, ntiles, tile, i, look, lamT);
 }
 
 // The recurrence through one pair field of a contraction tile, by one warp (TT = 32 c
@@ -1111,7 +1150,7 @@ __device__ __forceinline__ void tile_pair_recurrence(const TileScan<T>& ts, cons
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_raman_agg(const SolveDesc* __restrict__ descs, int nt, int TT) {
+__global__ void __launch_bounds__(256) k_raman_agg(const SolveDesc* __restrict__ descs, int nt, int TT, int by_tile) {
   using V = c2<T>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const SolveDesc& d = descs[blockIdx.y];
@@ -1147,8 +1186,8 @@ __global__ void __launch_bounds__(256) k_raman_agg(const SolveDesc* __restrict__
   cp_async_wait<0>();
   __syncthreads();
   grid_release();
-  const int ntiles = nt / TT;
-  V* out = as_t2<T>(d.raman_tiles);
+  V* out = as_t2<T>(d.raman_tiles) + (size_t)tile * (by_tile ? 2 * d.P : 2);
+  const size_t sq = by_tile ? 2 : 2 * (size_t)(nt / TT);
   for (int q = warp; q < d.P; q += nwarps) {
     const int2 lm = d.pairs[q];
     V sa = mk<T>(0, 0), sb = mk<T>(0, 0);
@@ -1168,10 +1207,7 @@ __global__ void __launch_bounds__(256) k_raman_agg(const SolveDesc* __restrict__
       sb.x += __shfl_xor_sync(0xffffffffu, sb.x, o);
       sb.y += __shfl_xor_sync(0xffffffffu, sb.y, o);
     }
-    if (lane == 0) {
-      out[((size_t)q * ntiles + tile) * 2] = sa;
-      out[((size_t)q * ntiles + tile) * 2 + 1] = sb;
-    }
+    if (lane == 0) st2<T>(out + q * sq, sa, sb);
   }
 }
 
@@ -1185,8 +1221,7 @@ __global__ void __launch_bounds__(32) k_raman_carry(const SolveDesc* __restrict_
   const int ntiles = nt / TT;
   const int per = (ntiles + 31) / 32;  // tiles per lane
   const int first = min(lane * per, ntiles), last = min(first + per, ntiles);
-  double2 lamT = d.iir_lambda;  // lambda^TT (TT a power of two)
-  for (int s = 1; s < TT; s <<= 1) lamT = cmul(lamT, lamT);
+  const double2 lamT = lambda_tile(d, TT);
   grid_sync_wait();
   grid_release();
   if (q >= d.P || d.M == 0 || __ldcg(d.step) >= d.step_limit) return;
@@ -1260,7 +1295,8 @@ template <typename T, int DENSE> constexpr int contract_min_blocks() {
 }
 
 // raman_mode: 0 Raman off; 1 the convolutions R arrive as rows (k_pair / k_raman_scan);
-// 2 the recurrence runs through the tile here from the carries of k_raman_carry.
+// 2 the recurrence runs through the tile here from the carries of k_raman_carry; 3 from carries
+// the tile sums itself from the aggregates before it (tile_carry; no k_raman_carry).
 // DENSE = 1: the contraction in its dense form (SolveDesc::dense_q, M <= 16, TT >= 64);
 // DENSE = 2: per solve, the dense form where dense_q is set and the term loop elsewhere
 // (a batch that mixes both; each solve runs the same arithmetic as on its own):
@@ -1293,12 +1329,14 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
   V* sW = sU + (size_t)M * TT;
   const int n_terms = d.term_off[M];
   // pair-field rows: swizzled (wsw) when the recurrence runs here, else plain
-  const int wmask = raman == 2 ? max(TT >> 6, 1) - 1 : 0;
-  // raman_mode 2: the states entering this tile per pair field (Re V, Im V), staged while
+  const int wmask = raman >= 2 ? max(TT >> 6, 1) - 1 : 0;
+  // raman_mode 2, 3: the states entering this tile per pair field (Re V, Im V), staged while
   // the tile lands
   V* sC = sW + (size_t)P * TT;
+  const int ntiles = nt / TT, look = tile_look(d, ntiles, TT, raman);
+  const double2 lamT = look ? lambda_tile(d, TT) : make_double2(0.0, 0.0);
   // dense form: per warp, two chunks of kDenseChunk coefficient rows (cp.async double buffer)
-  T* sA = reinterpret_cast<T*>(sC + (raman == 2 ? 2 * (size_t)P : 0));
+  T* sA = reinterpret_cast<T*>(sC + (raman >= 2 ? 2 * (size_t)P : 0));
   const size_t dense_elems = DENSE ? (size_t)(blockDim.x >> 5) * 2 * kDenseChunk * 2 * kDenseMaxModes : 0;
   ST* st = reinterpret_cast<ST*>(sA + dense_elems);
   // the terms are staged while the kernel before this one still runs
@@ -1321,7 +1359,7 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
     const V* src = (r < M) ? U + (size_t)r * nt + t0 : R + (size_t)(r - M) * nt + t0;
     bulk_g2s(sU + (size_t)r * TT, src, row_bytes, &bar);
   }
-  if (raman == 2) stage_tile_carries<T>(sC, d, P, nt / TT, blockIdx.x);
+  if (raman >= 2) stage_tile_carries<T>(sC, d, P, ntiles, blockIdx.x, look, lamT);
   // every thread polls with a bound; the barrier makes the outcome CTA-uniform and
   // also publishes the staged terms
   const bool landed = mbar_wait(&bar, 0, d.tile_wait_polls);
@@ -1333,7 +1371,7 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
   }
   const int H = TT >> 1;  // sample pairs per row
   // 1. pair fields
-  if (raman != 2) {  // two samples per thread
+  if (raman < 2) {  // two samples per thread
     for (int idx = threadIdx.x; idx < P * H; idx += blockDim.x) {
       const int q = idx / H, tt = 2 * (idx - q * H);
       const int2 lm = d.pairs[q];
@@ -1473,7 +1511,7 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
 constexpr int kPcItems = 4;
 template <typename T>
 __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2)) k_contract_pc(const SolveDesc* __restrict__ descs,
-                                                                              int nt, int TT, int pc) {
+                                                                              int nt, int TT, int pc, int raman_mode) {
   using V = c2<T>;
   using ST = StagedTerm<T>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1506,7 +1544,10 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2)) k_contract_pc(c
   __syncthreads();
   for (int r = threadIdx.x; r < M; r += blockDim.x)
     bulk_g2s(sU + (size_t)r * TT, as_t2<T>(d.U) + (size_t)r * nt + t0, row_bytes, &bar);
-  stage_tile_carries<T>(sC, d, P, nt / TT, blockIdx.x);
+  {
+    const int look = tile_look(d, nt / TT, TT, raman_mode);
+    stage_tile_carries<T>(sC, d, P, nt / TT, blockIdx.x, look, lambda_tile(d, TT));
+  }
   const bool landed = mbar_wait(&bar, 0, d.tile_wait_polls);
   if (!__syncthreads_and(landed ? 1 : 0)) {
     if (threadIdx.x == 0) atomicOr(d.status, kStatusTimeout);
@@ -1661,7 +1702,8 @@ template <typename V> __device__ __forceinline__ V shfl_down_c(V v, int d) {
   return v;
 }
 
-// raman_mode: 0 Raman off, 2 the recurrence from the tile carries of k_raman_carry (tiles of TB)
+// raman_mode: 0 Raman off, 2 the recurrence from the tile carries of k_raman_carry (tiles of TB), 3 from
+// carries summed here (tile_carry)
 template <typename T>
 __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
     k_contract_sr(const SolveDesc* __restrict__ descs, int nt, int TB, int raman_mode) {
@@ -1696,6 +1738,7 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
     }
     for (int i = tid; i < rounds * kSrGroups; i += kSrThreads) sPlan[i] = d.sr_plan[i];
   }
+  const double2 lamT = raman_mode == 3 ? lambda_tile(d, TB) : make_double2(0.0, 0.0);
   grid_sync_wait();
   if (__ldcg(d.step) >= d.step_limit) return;  // finished solve (nothing is in flight yet)
   // U staging: sample pair j of row r is item r J + j; a thread carries at most two
@@ -1728,7 +1771,7 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
   // sr = (Re S_a, Re S_b), si = (Im S_a, Im S_b) (S_a for Re V, S_b for Im V)
   int pl[kSrPairsPerThread], pm[kSrPairsPerThread];
   V sr[kSrPairsPerThread], si[kSrPairsPerThread];
-  const int ntiles = nt / TB;
+  const int ntiles = nt / TB, look = tile_look(d, ntiles, TB, raman_mode);
 #pragma unroll
   for (int i = 0; i < kSrPairsPerThread; ++i) {
     const int q = tid + i * kSrThreads;
@@ -1738,9 +1781,9 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
       const int2 lm = d.pairs[q];
       pl[i] = lm.x;
       pm[i] = lm.y;
-      if (raman_mode == 2) {
-        const V* tiles = as_t2<T>(d.raman_tiles) + ((size_t)q * ntiles + blockIdx.x) * 2;
-        const V ca = tiles[0], cb = tiles[1];
+      if (raman_mode >= 2) {
+        const V ca = tile_carry<T>(d, ntiles, blockIdx.x, 2 * q, look, lamT);
+        const V cb = tile_carry<T>(d, ntiles, blockIdx.x, 2 * q + 1, look, lamT);
         sr[i] = mk<T>(ca.x, cb.x);
         si[i] = mk<T>(ca.y, cb.y);
       }
@@ -1779,7 +1822,7 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
             const V ue = e ? mk<T>(a.re.y, a.im.y) : mk<T>(a.re.x, a.im.x);
             const V me = e ? mk<T>(b.re.y, b.im.y) : mk<T>(b.re.x, b.im.x);
             const V x = cmulc(ue, me);  // V = U_l conj(U_m): (Re V, Im V)
-            if (raman_mode == 2) {
+            if (raman_mode >= 2) {
               // S <- lambda S + x for both recurrences, then W = (1 - f_R) V + Im(kappa S)
               const V t = pk_mul(li2, Sr);
               Sr = pk_fma(lr2, Sr, pk_fma(nli2, Si, x));
@@ -1851,7 +1894,7 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
 // k_raman_carry turns the aggregates into the states entering the tiles.
 template <typename T>
 __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
-    k_raman_agg_sr(const SolveDesc* __restrict__ descs, int nt, int TB) {
+    k_raman_agg_sr(const SolveDesc* __restrict__ descs, int nt, int TB, int by_tile) {
   using V = c2<T>;
   using SP = SrPair<T>;
   constexpr int J = kSrSub / 2;
@@ -1939,14 +1982,13 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
     if (sub + 1 < nsub) park(buf ^ 1);
     __syncthreads();
   }
-  const int ntiles = nt / TB;
-  V* out = as_t2<T>(d.raman_tiles);
+  V* out = as_t2<T>(d.raman_tiles) + (size_t)blockIdx.x * (by_tile ? 2 * P : 2);
+  const size_t sq = by_tile ? 2 : 2 * (size_t)(nt / TB);
 #pragma unroll
   for (int i = 0; i < kSrPairsPerThread; ++i) {
     const int q = tid + i * kSrThreads;
     if (q < P) {
-      out[((size_t)q * ntiles + blockIdx.x) * 2] = mk<T>(sr[i].x, si[i].x);      // Re V recurrence
-      out[((size_t)q * ntiles + blockIdx.x) * 2 + 1] = mk<T>(sr[i].y, si[i].y);  // Im V recurrence
+      st2<T>(out + q * sq, mk<T>(sr[i].x, si[i].x), mk<T>(sr[i].y, si[i].y));  // Re V, Im V recurrences
     }
   }
 }
@@ -1962,7 +2004,7 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
 // and every product is formed as hi hi + hi lo + lo hi with FP32 accumulation: relative
 // error about 2^-21 (plain TF32 would leave 2^-11).
 // Per chunk c the 16 warps build the chunk's pair fields W, one field each (the Raman
-// recurrence through the tile, raman_mode 2, or V = U_l conj(U_m), raman_mode 0), and each
+// recurrence through the tile, raman_mode 2 or 3, or V = U_l conj(U_m), raman_mode 0), and each
 // lane writes its 4 consecutive samples, split into TF32 hi and lo, straight into the A
 // operands (buffer c % 2) in the MN-major TF32 layout (samples contiguous: the 4 samples of
 // one field are one 16-byte chunk per matrix); one thread issues the chunk's 12 MMAs and
@@ -2008,7 +2050,8 @@ __global__ void __launch_bounds__(512, 1) k_contract_tc(const SolveDesc* __restr
   if (tid == 0) mbar_arrive_expect_tx(&bar_u, (unsigned)(M * TT * sizeof(V)));
   __syncthreads();
   if (tid < M) bulk_g2s(sU + (size_t)tid * TT, as_t2<float>(d.U) + (size_t)tid * nt + t0, TT * sizeof(V), &bar_u);
-  if (raman_mode == 2) stage_tile_carries<float>(sC, d, P, nt / TT, blockIdx.x);
+  if (raman_mode >= 2)
+    stage_tile_carries<float>(sC, d, P, nt / TT, blockIdx.x, tile_look(d, nt / TT, TT, raman_mode), lambda_tile(d, TT));
   if (warp == 0) {
     tc::alloc(&s_tmem, 512);
     tc::relinquish();
@@ -2020,7 +2063,7 @@ __global__ void __launch_bounds__(512, 1) k_contract_tc(const SolveDesc* __restr
   tc::fence_after_sync();
   const uint32_t tmem = s_tmem;
   TileScan<float> ts;
-  if (raman_mode == 2) ts.init(d, TT >> 5, lane);
+  if (raman_mode >= 2) ts.init(d, TT >> 5, lane);
   const float kerr = (float)d.one_minus_fR;
   const int nch = (P + KC - 1) / KC;
   const unsigned bbytes = (unsigned)(4 * KC * N * sizeof(float));
@@ -2061,7 +2104,7 @@ __global__ void __launch_bounds__(512, 1) k_contract_tc(const SolveDesc* __restr
       if (q >= P) {  // past the last field: zeros (the buffers start uninitialised)
         const V z[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
         put(z);
-      } else if (raman_mode == 2) {
+      } else if (raman_mode >= 2) {
         tile_pair_recurrence_to<float, true>(ts, sU, TT, d.pairs[q], nullptr, WMASK, sC + 2 * q, kerr, lane, put);
       } else {
         const int2 lm = d.pairs[q];
