@@ -128,6 +128,7 @@ struct SolveDesc {
   // rounding): how far back a tile looks for the state entering it (tile_carry)
   int iir_len;
   double2 iir_lambda;
+  double2 iir_lam64, iir_lam128, iir_lam256;  // lambda^64, ^128, ^256: the tiles' lambda^TT
   double2 iir_kappa;
   double2 iir_inv_one_minus;
   // [kRamanPow] (T complex): lambda^j, j < kRamanPow, computed once in FP64 (iir solves)
@@ -152,12 +153,14 @@ struct SolveDesc {
   // The contraction's terms merged per (p, k, pair field q) for k_contract_sr: a term
   // reading W_q and one reading conj(W_q) with the same k add up to
   //   U_k (a Re W_q + i b Im W_q),  a = Q1 + Q2, b = Q1 - Q2,
-  // sorted by p; sr_coef holds (a, b) in T, sr_kq = q | k << 16. sr_plan assigns the modes'
+  // sorted by p, then k; sr_coef holds (a, b) in T, sr_kq = q | k << 16, sr_off [M + 1] where
+  // each p's begin (k_contract_sp reads the same terms). sr_plan assigns the modes'
   // term ranges to the kernel's groups of eight lanes, sr_rounds rounds of kSrGroups groups:
   // (p, first term, end, role), role 0 a whole mode, 1 and 2 the lower and upper halves of a
   // split one (the upper half hands its sums to the lower), 3 an empty group.
   const void* sr_coef;
   const unsigned* sr_kq;
+  const int* sr_off;
   const int4* sr_plan;
   int sr_terms;
   int sr_rounds;

@@ -224,9 +224,9 @@ int ensure_device(int dev, DeviceRes** out) {
           if (f)
             CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(ks.smem, kSmemSM / 2)));
       }
-  const void* contract_fns[] = {(const void*)&k_contract<float, 0>,  (const void*)&k_contract<float, 1>,
-                                (const void*)&k_contract<float, 2>,  (const void*)&k_contract<double, 0>,
-                                (const void*)&k_contract<double, 1>, (const void*)&k_contract<double, 2>};
+  const void* contract_fns[] = {(const void*)&k_contract<float, 0>,   (const void*)&k_contract<float, 1>,
+                                (const void*)&k_contract<double, 0>,  (const void*)&k_contract<double, 1>,
+                                (const void*)&k_contract_sp<float>, (const void*)&k_contract_sp<double>};
   for (const void* f : contract_fns)
     CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kContractSmemMax));
   CUDA_TRY(cudaFuncSetAttribute((const void*)&k_contract_pc<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -675,7 +675,9 @@ struct mmp_batch {
   bool raman_iir = false;  // every solve's h_R is a damped sinusoid: pair fields by k_raman_scan
   bool raman_fused = false;  // ... and the recurrence runs inside the contraction tiles
   bool lookback = false;     // ... which sum the states entering them themselves (no k_raman_carry)
-  int dense = 0;  // contraction form: 0 term loop, 1 dense (k_contract<T, 1>), 2 per solve
+  int dense = 0;  // contraction form: 0 sparse, 1 dense (k_contract<T, 1>), 2 per solve (a launch of each)
+  bool sp = false;   // the sparse form runs k_contract_sp (else k_contract<T, 0>)
+  size_t sp_smem = 0;
   bool tc = false;  // dense form on the tensor cores (k_contract_tc)
   int pchunk = 0;   // > 0: pair fields per chunk of the pair-chunked contraction (k_contract_pc)
   bool sr = false;  // serial-recurrence contraction in sub-blocks (k_contract_sr)
@@ -792,12 +794,9 @@ int launch_contract(mmp_batch* b, uint32_t first = 0, uint32_t count = ~0u, cuda
   const SolveDesc* descs = b->d_descs + first;
   int nt = (int)b->nt, TT = b->TT, sterms = b->stage_terms;
   int mode = !b->raman ? 0 : (b->lookback ? 3 : b->raman_fused ? 2 : 1);
-  void* args[] = {(void*)&descs, &nt, &TT, &sterms, &mode};
+  int mixed = b->dense == 2;
+  void* args[] = {(void*)&descs, &nt, &TT, &sterms, &mode, &mixed};
   dim3 grid((unsigned)(b->nt / b->TT), count, 1);
-  const void* f32[] = {(const void*)&k_contract<float, 0>, (const void*)&k_contract<float, 1>,
-                       (const void*)&k_contract<float, 2>};
-  const void* f64[] = {(const void*)&k_contract<double, 0>, (const void*)&k_contract<double, 1>,
-                       (const void*)&k_contract<double, 2>};
   if (b->sr) {
     int tb = b->TT;
     void* sargs[] = {(void*)&descs, &nt, &tb, &mode};
@@ -817,8 +816,20 @@ int launch_contract(mmp_batch* b, uint32_t first = 0, uint32_t count = ~0u, cuda
     CUDA_TRY(launch((const void*)&k_contract_tc<float>, grid, 512, (int)b->contract_smem, 1, st ? st : b->stream, targs, true));
     return MMP_OK;
   }
-  const void* fn = b->fp64 ? f64[b->dense] : f32[b->dense];
-  CUDA_TRY(launch(fn, grid, 256, (int)b->contract_smem, 1, st ? st : b->stream, args, true));
+  if (b->dense != 1) {  // the sparse solves
+    if (b->sp) {
+      void* spargs[] = {(void*)&descs, &nt, &TT, &mode, &mixed};
+      const void* fsp = b->fp64 ? (const void*)&k_contract_sp<double> : (const void*)&k_contract_sp<float>;
+      CUDA_TRY(launch(fsp, grid, 256, (int)b->sp_smem, 1, st ? st : b->stream, spargs, true));
+    } else {
+      const void* f0 = b->fp64 ? (const void*)&k_contract<double, 0> : (const void*)&k_contract<float, 0>;
+      CUDA_TRY(launch(f0, grid, 256, (int)b->contract_smem, 1, st ? st : b->stream, args, true));
+    }
+  }
+  if (b->dense) {
+    const void* f1 = b->fp64 ? (const void*)&k_contract<double, 1> : (const void*)&k_contract<float, 1>;
+    CUDA_TRY(launch(f1, grid, 256, (int)b->contract_smem, 1, st ? st : b->stream, args, true));
+  }
   return MMP_OK;
 }
 
@@ -851,7 +862,7 @@ int launch_pairs(mmp_batch* b, const KernelSet& ks, int nsolves, int stage, cons
       CUDA_TRY(launch(fa, dim3((unsigned)(nt / TT), (unsigned)nsolves, 1), kSrThreads, smem, 1,
                       st ? st : b->stream, args, true));
     } else {
-      const int smem = (int)(((size_t)b->Mmax * TT + TT) * t2);  // U tile and the weight table
+      const int smem = (int)((size_t)b->Mmax * TT * t2);  // U tile
       const void* fa = b->fp64 ? (const void*)&k_raman_agg<double> : (const void*)&k_raman_agg<float>;
       CUDA_TRY(launch(fa, dim3((unsigned)(nt / TT), (unsigned)nsolves, 1), 256, smem, 1, st ? st : b->stream, args, true));
     }
@@ -1187,6 +1198,7 @@ size_t member_bytes(const mmp_batch* b, const Member& s) {
   off = align_up(off + std::max<size_t>(s.sr_kq.size(), 1) * 16);                // merged coefficients
   off = align_up(off + std::max<size_t>(s.sr_kq.size(), 1) * sizeof(unsigned));  // their k | q << 16
   off = align_up(off + s.sr_plan.size() * sizeof(int4));                         // group plan
+  off = align_up(off + (M + 1) * sizeof(int));                                   // merged terms per p
   off = align_up(off + kCounterWords * sizeof(unsigned long long));
   return off;
 }
@@ -1264,6 +1276,7 @@ int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
   const size_t o_src = off; off = align_up(off + std::max<size_t>(nsr, 1) * 16);
   const size_t o_skq = off; off = align_up(off + std::max<size_t>(nsr, 1) * sizeof(unsigned));
   const size_t o_splan = off; off = align_up(off + s.sr_plan.size() * sizeof(int4));
+  const size_t o_soff = off; off = align_up(off + (M + 1) * sizeof(int));
   const size_t o_cnt = off; off = align_up(off + kCounterWords * sizeof(unsigned long long));
   cudaError_t e = dev_malloc(&s.block, off, b->mempool, b->stream);
   if (e != cudaSuccess) {
@@ -1306,6 +1319,7 @@ int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
   d.sr_coef = T2ptr(s.block, o_src);
   d.sr_kq = (const unsigned*)T2ptr(s.block, o_skq);
   d.sr_plan = (const int4*)T2ptr(s.block, o_splan);
+  d.sr_off = (const int*)T2ptr(s.block, o_soff);
   d.sr_terms = (int)nsr;
   d.sr_rounds = s.sr_rounds;
   s.counters = (unsigned long long*)T2ptr(s.block, o_cnt);
@@ -1329,6 +1343,13 @@ int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
       s.iir_decay = -std::log(std::abs(lam));
       d.iir_len = iir_len(s.iir_decay, b->fp64);
       d.iir_lambda = make_double2(lam.real(), lam.imag());
+      std::complex<double> l2 = lam;
+      for (int e = 2; e <= 256; e <<= 1) {
+        l2 *= l2;
+        if (e == 64) d.iir_lam64 = make_double2(l2.real(), l2.imag());
+        if (e == 128) d.iir_lam128 = make_double2(l2.real(), l2.imag());
+        if (e == 256) d.iir_lam256 = make_double2(l2.real(), l2.imag());
+      }
       d.iir_kappa = make_double2(kap.real(), kap.imag());
       d.iir_inv_one_minus = make_double2(inv.real(), inv.imag());
       // lambda^j, j < kRamanPow, by binary powering in FP64 (the tile aggregates' weights)
@@ -1367,6 +1388,8 @@ int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
       CUDA_TRY(cudaMemcpyAsync((void*)d.sr_kq, s.sr_kq.data(), nsr * sizeof(unsigned), cudaMemcpyHostToDevice,
                                b->stream));
     }
+    CUDA_TRY(cudaMemcpyAsync((void*)d.sr_off, s.sr_off.data(), (M + 1) * sizeof(int), cudaMemcpyHostToDevice,
+                             b->stream));
     CUDA_TRY(cudaMemcpyAsync((void*)d.sr_plan, s.sr_plan.data(), s.sr_plan.size() * sizeof(int4),
                              cudaMemcpyHostToDevice, b->stream));
     CUDA_TRY(cudaStreamSynchronize(b->stream));  // the staging vectors are host temporaries
@@ -1484,15 +1507,16 @@ ShapeStats batch_stats(const mmp_batch* b) {
 // memory they take, chosen from its statistics alone.
 struct Shape {
   int Mmax = 0, Pmax = 0, TT = 32, dense = 0, pchunk = 0, stage_terms = 0;
-  bool tc = false, sr = false, fused = false, iir = false, lookback = false;
-  size_t smem = 0;
+  bool tc = false, sr = false, sp = false, fused = false, iir = false, lookback = false;
+  size_t smem = 0, sp_smem = 0;
   uint32_t span = 0;
 };
 
 // Shapes that run the same kernels with the same tiles on a solve (so give it the same bits).
 bool same_kernels(const Shape& x, const Shape& y) {
   return x.TT == y.TT && x.dense == y.dense && x.pchunk == y.pchunk && x.stage_terms == y.stage_terms &&
-         x.tc == y.tc && x.sr == y.sr && x.fused == y.fused && x.iir == y.iir && x.lookback == y.lookback;
+         x.tc == y.tc && x.sr == y.sr && x.fused == y.fused && x.iir == y.iir && x.lookback == y.lookback &&
+         x.sp == y.sp;
 }
 
 Shape choose_shape(const mmp_batch* b, const ShapeStats& st) {
@@ -1600,7 +1624,13 @@ Shape choose_shape(const mmp_batch* b, const ShapeStats& st) {
   bool lookback = fused && std::min((int)b->nt / TT, (iir_len(st.min_decay, b->fp64) - 1) / TT + 1) <= kMaxLook;
   if (const char* env = std::getenv("MMP_LOOKBACK"))
     if (std::atoi(env) == 0) lookback = false;
-  const int stage_terms = sr ? 0 : (pchunk ? 1 : (dense != 1 && !tc && smem + max_terms * staged <= 200 * 1024 ? 1 : 0));
+  // sparse solves in tiles of 64 samples or more: k_contract_sp, where its merged terms fit
+  // beside the tile. MMP_CONTRACT_SP=0 keeps the term loop over the unmerged ones.
+  const size_t sp_smem = ((size_t)rows * TT + 2 * (size_t)Pmax + 2 * max_sr_terms) * t2;
+  bool sp = !tc && !sr && !pchunk && dense != 1 && TT >= 64 && sp_smem <= 200 * 1024;
+  if (const char* env = std::getenv("MMP_CONTRACT_SP"))
+    if (std::atoi(env) == 0) sp = false;
+  const int stage_terms = sr || (sp && !dense) ? 0 : (pchunk ? 1 : (dense != 1 && !tc && smem + max_terms * staged <= 200 * 1024 ? 1 : 0));
   if (stage_terms && !pchunk) smem += max_terms * staged;
   Shape sh;
   sh.Mmax = Mmax;
@@ -1614,6 +1644,8 @@ Shape choose_shape(const mmp_batch* b, const ShapeStats& st) {
   sh.fused = fused;
   sh.iir = iir;
   sh.lookback = lookback;
+  sh.sp = sp;
+  sh.sp_smem = sp_smem;
   sh.smem = smem;
   sh.span = span;
   return sh;
@@ -1673,7 +1705,8 @@ bool batch_shape(mmp_batch* b) {
   const bool changed = resplit || sh.Mmax != b->Mmax || sh.Pmax != b->Pmax || sh.TT != b->TT || sh.smem != b->contract_smem ||
                        sh.stage_terms != b->stage_terms || sh.span != b->span || sh.iir != b->raman_iir ||
                        sh.fused != b->raman_fused || sh.dense != b->dense || sh.tc != b->tc ||
-                       sh.pchunk != b->pchunk || sh.sr != b->sr || sh.lookback != b->lookback;
+                       sh.pchunk != b->pchunk || sh.sr != b->sr || sh.lookback != b->lookback || sh.sp != b->sp ||
+                       sh.sp_smem != b->sp_smem;
   b->dense = sh.dense;
   b->tc = sh.tc;
   b->pchunk = sh.pchunk;
@@ -1681,7 +1714,9 @@ bool batch_shape(mmp_batch* b) {
   b->raman_iir = sh.iir;
   b->raman_fused = sh.fused;
   b->lookback = sh.lookback;
-  b->kernels_per_step = b->tab.s * ((b->raman ? (sh.fused && !sh.lookback ? 2 : 1) : 0) + 2);
+  b->sp = sh.sp;
+  b->sp_smem = sh.sp_smem;
+  b->kernels_per_step = b->tab.s * ((b->raman ? (sh.fused && !sh.lookback ? 2 : 1) : 0) + 2 + (sh.dense == 2 ? 1 : 0));
   b->span = sh.span;
   b->Mmax = sh.Mmax;
   b->Pmax = sh.Pmax;

@@ -226,6 +226,14 @@ __device__ __forceinline__ double2 ld_stream(const double2* p) { return __ldcg(p
   V* sr = s + lrow * Gm::RS;                                          \
   const int i0 = rank * Gm::NTHR + tid;
 
+// Packed two-lane FMA and product (FP32: one instruction; each lane rounds as the scalar one does).
+__device__ __forceinline__ float2 pk_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 pk_mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ double2 pk_fma(double2 a, double2 b, double2 c) {
+  return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
+}
+__device__ __forceinline__ double2 pk_mul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
+
 // ---- k_prime: U for stage 0 from psi_hat --------------------------------------------------
 template <typename T, int LOGN, int XC>
 __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_BLOCKS) k_prime(const KParams kp) {
@@ -1050,10 +1058,8 @@ __device__ __forceinline__ c2<T> tile_carry(const SolveDesc& d, int ntiles, int 
   if (look == ntiles) c = cmul(c, d.iir_inv_one_minus);
   return from_d2<T>(c);
 }
-__device__ __forceinline__ double2 lambda_tile(const SolveDesc& d, int TT) {  // lambda^TT (TT a power of two)
-  double2 l = d.iir_lambda;
-  for (int s = 1; s < TT; s <<= 1) l = cmul(l, l);
-  return l;
+__device__ __forceinline__ double2 lambda_tile(const SolveDesc& d, int TT) {  // lambda^TT, TT = 64, 128, 256
+  return TT == 256 ? d.iir_lam256 : TT == 128 ? d.iir_lam128 : d.iir_lam64;
 }
 // Tiles a solve looks back: all of a short row's.
 __device__ __forceinline__ int tile_look(const SolveDesc& d, int ntiles, int TT, int raman_mode) {
@@ -1149,8 +1155,16 @@ __device__ __forceinline__ void tile_pair_recurrence(const TileScan<T>& ts, cons
   });
 }
 
+// k_raman_agg: the recurrence's aggregate over a tile from a zero start, for every pair field, as
+// a weighted sum,
+//   S_end = sum_t lambda^(TT-1-t) x_t   (x = Re or Im of U_l conj(U_m)),
+// so it needs no sequential pass. A warp takes a field at a time: each lane sums its sample pairs
+// (2h, 2h + 1), h = lane, lane + 32, ..., with the weights it keeps in registers, and the lanes'
+// four sums are added by halving (each exchange hands over half of what a lane holds: 6
+// shuffles for the four). What bounds it: the latency of the tile's copy, then issue. Measured
+// on a B200, 32 solves of 6 x 16384, against weights read per field and 20 shuffles: 21 -> 18 us.
 template <typename T>
-__global__ void __launch_bounds__(256) k_raman_agg(const SolveDesc* __restrict__ descs, int nt, int TT, int by_tile) {
+__global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 5 : 3)) k_raman_agg(const SolveDesc* __restrict__ descs, int nt, int TT, int by_tile) {
   using V = c2<T>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const SolveDesc& d = descs[blockIdx.y];
@@ -1160,18 +1174,24 @@ __global__ void __launch_bounds__(256) k_raman_agg(const SolveDesc* __restrict__
     return;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  V* sU = reinterpret_cast<V*>(smem_raw);
-  V* sp = sU + (size_t)d.M * TT;  // lambda^j, j < TT
-  {  // the powers of lambda and the U tile as 16-byte asynchronous copies, before the step check
-    const V* U = as_t2<T>(d.U);
-    const int per_row = TT * (int)sizeof(V) / 16;
-    for (int c = threadIdx.x; c < per_row; c += blockDim.x)
-      cp_async16(reinterpret_cast<char*>(sp) + 16 * c, static_cast<const char*>(d.raman_pow) + 16 * c);
-    grid_sync_wait();
-    for (int idx = threadIdx.x; idx < d.M * per_row; idx += blockDim.x) {
-      const int r = idx / per_row, c = idx - r * per_row;
-      cp_async16(reinterpret_cast<char*>(sU + (size_t)r * TT) + 16 * c,
-                 reinterpret_cast<const char*>(U + (size_t)r * nt + t0) + 16 * c);
+  const int M = d.M, P = d.P;
+  V* sU = reinterpret_cast<V*>(smem_raw);  // [M][TT]
+  const V* U = as_t2<T>(d.U) + t0;
+  const int2* pairs = d.pairs;
+  V w0[4], w1[4];  // the weights of the lane's pairs
+  {
+    const V* pw = static_cast<const V*>(d.raman_pow) + TT - 2;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)  // lambda^(TT-2-2h) for sample 2h + 1, lambda^(TT-1-2h) for 2h
+      if (j < (TT >> 6)) ld2<T>(pw - 2 * (lane + 32 * j), w1[j], w0[j]);
+  }
+  grid_sync_wait();
+  {  // the U tile as 16-byte asynchronous copies, before the step check
+    constexpr int PER = 16 / (int)sizeof(V);  // samples a copy
+    const int per_row = TT / PER, sh = 31 - __clz(per_row);
+    for (int idx = threadIdx.x; idx < M * per_row; idx += blockDim.x) {
+      const int r = idx >> sh, c = idx & (per_row - 1);
+      cp_async16(sU + (size_t)r * TT + c * PER, U + (size_t)r * nt + c * PER);
     }
     cp_async_commit();
   }
@@ -1179,35 +1199,36 @@ __global__ void __launch_bounds__(256) k_raman_agg(const SolveDesc* __restrict__
     cp_async_wait<0>();
     return;
   }
-  // The aggregate over the tile from a zero start is a weighted sum,
-  //   S_end = sum_t lambda^(TT-1-t) x_t   (x = Re or Im of U_l conj(U_m)),
-  // so it needs no sequential pass: each lane sums sample pairs (2h, 2h + 1), h = lane,
-  // lane + 32, ..., weighted from the table of powers, and the warp adds the lanes.
   cp_async_wait<0>();
   __syncthreads();
   grid_release();
-  V* out = as_t2<T>(d.raman_tiles) + (size_t)tile * (by_tile ? 2 * d.P : 2);
-  const size_t sq = by_tile ? 2 : 2 * (size_t)(nt / TT);
-  for (int q = warp; q < d.P; q += nwarps) {
-    const int2 lm = d.pairs[q];
-    V sa = mk<T>(0, 0), sb = mk<T>(0, 0);
-    for (int h = lane; h < (TT >> 1); h += 32) {
-      V ul0, ul1, um0, um1, wb, wa;
-      ld2<T>(sU + lm.x * TT + 2 * h, ul0, ul1);
-      ld2<T>(sU + lm.y * TT + 2 * h, um0, um1);
-      ld2<T>(sp + TT - 2 - 2 * h, wb, wa);  // lambda^(TT-2-2h) for sample 2h+1, lambda^(TT-1-2h) for 2h
-      const V x0 = cmulc(ul0, um0), x1 = cmulc(ul1, um1);
-      sa = mk<T>(fma(wa.x, x0.x, fma(wb.x, x1.x, sa.x)), fma(wa.y, x0.x, fma(wb.y, x1.x, sa.y)));
-      sb = mk<T>(fma(wa.x, x0.y, fma(wb.x, x1.y, sb.x)), fma(wa.y, x0.y, fma(wb.y, x1.y, sb.y)));
-    }
+  T* out = static_cast<T*>(d.raman_tiles) + (size_t)tile * (by_tile ? 4 * P : 4);
+  const size_t sq = by_tile ? 4 : 4 * (size_t)(nt / TT);
+  for (int q = warp; q < P; q += nwarps) {
+    const int2 lm = __ldg(pairs + q);
+    const V* ul = sU + lm.x * TT + 2 * lane;
+    const V* um = sU + lm.y * TT + 2 * lane;
+    V sr = mk<T>(0, 0), si = mk<T>(0, 0);  // Re and Im of the sums for (Re V, Im V)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sa.x += __shfl_xor_sync(0xffffffffu, sa.x, o);
-      sa.y += __shfl_xor_sync(0xffffffffu, sa.y, o);
-      sb.x += __shfl_xor_sync(0xffffffffu, sb.x, o);
-      sb.y += __shfl_xor_sync(0xffffffffu, sb.y, o);
+    for (int j = 0; j < 4; ++j) {
+      if (j < (TT >> 6)) {
+        V ul0, ul1, um0, um1;
+        ld2<T>(ul + 64 * j, ul0, ul1);
+        ld2<T>(um + 64 * j, um0, um1);
+        const V x0 = cmulc(ul0, um0), x1 = cmulc(ul1, um1);
+        sr = pk_fma(mk<T>(w0[j].x, w0[j].x), x0, pk_fma(mk<T>(w1[j].x, w1[j].x), x1, sr));
+        si = pk_fma(mk<T>(w0[j].y, w0[j].y), x0, pk_fma(mk<T>(w1[j].y, w1[j].y), x1, si));
+      }
     }
-    if (lane == 0) st2<T>(out + q * sq, sa, sb);
+    // lanes 0-15 add up the sums for Re V, lanes 16-31 those for Im V, then real and imaginary
+    // parts part at bit 3
+    const bool up = (lane & 16) != 0, up2 = (lane & 8) != 0;
+    T a = (up ? sr.y : sr.x) + __shfl_xor_sync(0xffffffffu, up ? sr.x : sr.y, 16);
+    T b = (up ? si.y : si.x) + __shfl_xor_sync(0xffffffffu, up ? si.x : si.y, 16);
+    T v = (up2 ? b : a) + __shfl_xor_sync(0xffffffffu, up2 ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((lane & 7) == 0) out[q * sq + (lane >> 3)] = v;
   }
 }
 
@@ -1297,16 +1318,16 @@ template <typename T, int DENSE> constexpr int contract_min_blocks() {
 // raman_mode: 0 Raman off; 1 the convolutions R arrive as rows (k_pair / k_raman_scan);
 // 2 the recurrence runs through the tile here from the carries of k_raman_carry; 3 from carries
 // the tile sums itself from the aggregates before it (tile_carry; no k_raman_carry).
-// DENSE = 1: the contraction in its dense form (SolveDesc::dense_q, M <= 16, TT >= 64);
-// DENSE = 2: per solve, the dense form where dense_q is set and the term loop elsewhere
-// (a batch that mixes both; each solve runs the same arithmetic as on its own):
+// DENSE = 0: the term loop (tiles under 64 samples, or too many terms to stage: k_contract_sp
+// takes the rest). DENSE = 1: the contraction in its dense form (SolveDesc::dense_q, M <= 16, TT >= 64):
 //   T_pk(t) = sum_q A_re[p][q][k] Re W_q(t) + i sum_q A_im[p][q][k] Im W_q(t),
 //   sigma_p(t) = sum_k U_k(t) T_pk(t),
 // one warp per (p, 64 samples), each lane two samples with all k in registers: a
 // register-blocked matrix product instead of one complex triple product per term.
+// mixed: the batch holds solves of both forms; each kernel skips the other's.
 template <typename T, int DENSE>
 __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_contract(const SolveDesc* __restrict__ descs, int nt, int TT,
-                                                  int stage_terms, int raman_mode) {
+                                                  int stage_terms, int raman_mode, int mixed) {
   using V = c2<T>;
   using ST = StagedTerm<T>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1314,7 +1335,7 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
   V* sU = reinterpret_cast<V*>(smem_raw);
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TT;
-  if (t0 >= nt || d.M == 0) {  // empty slot
+  if (t0 >= nt || d.M == 0 || (mixed && (d.dense_q != nullptr) != (DENSE == 1))) {  // empty slot, other form
     grid_sync_wait();
     return;
   }
@@ -1398,7 +1419,7 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
   grid_release();
   // 2. contraction
   V* sigma = as_t2<T>(d.sigma);
-  if (DENSE == 1 || (DENSE == 2 && d.dense_q != nullptr)) {
+  if constexpr (DENSE == 1) {
     constexpr int K = kDenseMaxModes;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     constexpr int ROW = 2 * K;                       // values per coefficient row (p, q)
@@ -1643,13 +1664,6 @@ constexpr int kSrSub = 16;
 constexpr int kSrThreads = 256;
 constexpr int kSrPairsPerThread = 2;  // pair fields per thread: P <= 512
 constexpr int kSrMaxModes = 64;       // staging: M * kSrSub / 2 <= 2 kSrThreads
-
-__device__ __forceinline__ float2 pk_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 pk_mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ double2 pk_fma(double2 a, double2 b, double2 c) {
-  return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
-}
-__device__ __forceinline__ double2 pk_mul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
 
 // A sample pair (t, t + 1) of one row: re = (Re t, Re t+1), im = (Im t, Im t+1).
 template <typename T> struct SrPair {
@@ -1990,6 +2004,238 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
     if (q < P) {
       st2<T>(out + q * sq, mk<T>(sr[i].x, si[i].x), mk<T>(sr[i].y, si[i].y));  // Re V, Im V recurrences
     }
+  }
+}
+
+// ---- k_contract_sp: the sparse contraction of tiles of 64 to 256 samples -------------------
+// All pair fields of the tile at once in shared memory, as k_contract, with the arithmetic of
+// k_contract_sr: packed two-lane FMAs (FP32) and merged terms. Samples lie in pairs
+// (Re t, Re t+1, Im t, Im t+1), pair h of a row at wsw(h), so that a warp's 32 consecutive
+// pairs and lane L's own g = TT/64 pairs g L .. g L + g - 1 are both conflict-free.
+//   1. the U tile lands (bulk copies, bounded wait) and is put in that form, each warp its own
+//      32 pairs in place;
+//   2. one warp per pair field: each lane forms V of its c = TT/32 samples, runs the recurrence
+//      through them from zero, the lanes' ends are scanned, and the lane runs it again from the
+//      state entering it, now with W = (1 - f_R) V + Im(kappa S) as output. The recurrences of
+//      Re V and Im V are the two lanes of one packed chain. (Raman off, or R from rows: W
+//      pointwise.)
+//   3. one warp per (p, 32 pairs): sigma = sum over p's merged terms of U_k (a Re W + i b Im W),
+//      terms as one record (a, b, positions of row k and row q), U_k read when k changes.
+// What bounds it: issue (62% of cycles on 28 warps), then the latency of the tile. Measured on a
+// B200 against the scalar term loop over unmerged terms (k_contract<T, 0>), a launch: 32 solves
+// of 6 x 16384 (21 pair fields) 56 -> 44 us, 38.2 -> 27.8 million warp instructions; 128 of
+// 2 x 4096 29 -> 24 us; a step of one 6 x 8192 FP64 solve 112 -> 96 us.
+template <typename T> struct LaneScan {
+  using V = c2<T>;
+  V lr2, li2, nli2, kr2, ki2;  // lambda and kappa, each component in both lanes
+  V lvl[5];                    // lambda^(c 2^j), zero for the lanes a level does not reach
+  V lane_pow;                  // lambda^(c lane)
+  int c;
+  __device__ __forceinline__ void init(const SolveDesc& d, int c_, int lane) {
+    c = c_;
+    const T lr = (T)d.iir_lambda.x, li = (T)d.iir_lambda.y;
+    lr2 = mk<T>(lr, lr);
+    li2 = mk<T>(li, li);
+    nli2 = mk<T>(-li, -li);
+    kr2 = mk<T>((T)d.iir_kappa.x, (T)d.iir_kappa.x);
+    ki2 = mk<T>((T)d.iir_kappa.y, (T)d.iir_kappa.y);
+    const V* pw = static_cast<const V*>(d.raman_pow);  // lambda^j, j < 256, from FP64
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+      const V l = __ldg(pw + (c << j));
+      lvl[j] = lane >= (1 << j) ? l : mk<T>(0, 0);
+    }
+    lane_pow = __ldg(pw + c * lane);
+  }
+  // S <- lambda S + x, S = (re, im), lanes Re V and Im V
+  __device__ __forceinline__ void step(V& re, V& im, V x) const {
+    const V t = pk_mul(li2, re);
+    re = pk_fma(lr2, re, pk_fma(nli2, im, x));
+    im = pk_fma(lr2, im, t);
+  }
+};
+
+template <typename T>
+__global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
+    k_contract_sp(const SolveDesc* __restrict__ descs, int nt, int TT, int raman_mode, int mixed) {
+  using V = c2<T>;
+  using SP = SrPair<T>;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ __align__(8) unsigned long long bar;
+  const SolveDesc& d = descs[blockIdx.y];
+  const int t0 = blockIdx.x * TT;
+  if (t0 >= nt || d.M == 0 || (mixed && d.dense_q != nullptr)) {  // empty slot, or the dense form's
+    grid_sync_wait();
+    return;
+  }
+  const int M = d.M, P = d.P, nterm = d.sr_terms;
+  const int H = TT >> 1, wmask = (TT >> 6) - 1;  // pairs per row
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  SP* sU = reinterpret_cast<SP*>(smem_raw);      // [M][H]
+  SP* sW = sU + (size_t)M * H;                   // [P][H]
+  SrRec<T>* sRec = reinterpret_cast<SrRec<T>*>(sW + (size_t)P * H);
+  V* sC = reinterpret_cast<V*>(sRec + nterm);    // states entering the tile, [P][2]
+  // staged while the kernel before this one still runs: the terms, with k and q as row positions
+  {
+    const V* cf = static_cast<const V*>(d.sr_coef);
+    for (int i = tid; i < nterm; i += blockDim.x) {
+      const unsigned kq = d.sr_kq[i];
+      SrRec<T> r = {};
+      r.ab = cf[i];
+      r.kq = (kq & 0xffffu) * H | ((kq >> 16) * H) << 16;
+      sRec[i] = r;
+    }
+  }
+  const int ntiles = nt / TT, look = tile_look(d, ntiles, TT, raman_mode);
+  const double2 lamT = look ? lambda_tile(d, TT) : make_double2(0.0, 0.0);
+  const T kerr = (T)d.one_minus_fR;
+  LaneScan<T> ts;
+  if (raman_mode >= 2) ts.init(d, TT >> 5, lane);
+  if (tid == 0) mbar_init(&bar, 1);
+  const int Pl = raman_mode == 1 ? P : 0;      // rows of R loaded
+  const unsigned row_bytes = (unsigned)(TT * sizeof(V));
+  if (tid == 0) mbar_arrive_expect_tx(&bar, (unsigned)(M + Pl) * row_bytes);
+  __syncthreads();
+  grid_sync_wait();
+  for (int r = tid; r < M + Pl; r += blockDim.x) {
+    const V* src = r < M ? as_t2<T>(d.U) + (size_t)r * nt + t0 : as_t2<T>(d.W) + (size_t)(r - M) * nt + t0;
+    bulk_g2s(sU + (size_t)r * H, src, row_bytes, &bar);
+  }
+  if (__ldcg(d.step) >= d.step_limit) {  // finished solve: the copies land before the CTA leaves
+    mbar_wait(&bar, 0, kMaxWaitPolls);
+    return;
+  }
+  if (raman_mode >= 2) stage_tile_carries<T>(sC, d, P, ntiles, blockIdx.x, look, lamT);
+  const bool landed = mbar_wait(&bar, 0, d.tile_wait_polls);
+  if (!__syncthreads_and(landed ? 1 : 0)) {
+    if (tid == 0) atomicOr(d.status, kStatusTimeout);
+    // give the copies a second bounded chance to land before the CTA leaves
+    mbar_wait(&bar, 0, kMaxWaitPolls);
+    return;
+  }
+  // 1. U in pairs of real and imaginary parts (rows of H = 32, 64 or 128 pairs: a warp stays in one)
+  for (int i = tid; i < M * H; i += blockDim.x) {
+    const int h = i & (H - 1);
+    SP* row = sU + (i - h);
+    V u0, u1;
+    ld2<T>(reinterpret_cast<const V*>(row + h), u0, u1);
+    __syncwarp();
+    st_pair<T>(row + wsw(h, wmask), mk<T>(u0.x, u1.x), mk<T>(u0.y, u1.y));
+  }
+  __syncthreads();
+  // V of one pair of samples
+  auto pair_product = [](const SP& a, const SP& b, V& vre, V& vim) {
+    vre = pk_fma(a.re, b.re, pk_mul(a.im, b.im));
+    vim = pk_fma(a.im, b.re, pk_mul(mk<T>(-a.re.x, -a.re.y), b.im));
+  };
+  // 2. pair fields
+  if (raman_mode >= 2) {
+    const int g = ts.c >> 1;
+    for (int q = warp; q < P; q += nwarps) {
+      const int2 lm = __ldg(d.pairs + q);
+      const SP* ul = sU + lm.x * H;
+      const SP* um = sU + lm.y * H;
+      SP* wq = sW + (size_t)q * H;
+      V x[8];  // (Re V, Im V) of the lane's samples
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (j < g) {
+          const int at = wsw(g * lane + j, wmask);
+          V vre, vim;
+          pair_product(ld_pair<T>(ul + at), ld_pair<T>(um + at), vre, vim);
+          x[2 * j] = mk<T>(vre.x, vim.x);
+          x[2 * j + 1] = mk<T>(vre.y, vim.y);
+        }
+      }
+      V sr = x[0], si = mk<T>(0, 0);  // the lane's end from a zero start
+#pragma unroll
+      for (int k = 1; k < 8; ++k)
+        if (k < ts.c) ts.step(sr, si, x[k]);
+      // inclusive scan over the lanes: S_L = lambda^c S_{L-1} + end_L
+#pragma unroll
+      for (int j = 0; j < 5; ++j) {
+        const int o = 1 << j;
+        V pr, pi;
+        pr.x = __shfl_up_sync(0xffffffffu, sr.x, o);
+        pr.y = __shfl_up_sync(0xffffffffu, sr.y, o);
+        pi.x = __shfl_up_sync(0xffffffffu, si.x, o);
+        pi.y = __shfl_up_sync(0xffffffffu, si.y, o);
+        const V l = ts.lvl[j];
+        sr = mk<T>(fma(l.x, pr.x, fma(-l.y, pi.x, sr.x)), fma(l.x, pr.y, fma(-l.y, pi.y, sr.y)));
+        si = mk<T>(fma(l.x, pi.x, fma(l.y, pr.x, si.x)), fma(l.x, pi.y, fma(l.y, pr.y, si.y)));
+      }
+      // the state entering the lane: the lanes before it, and the tile's
+      V er, ei;
+      er.x = __shfl_up_sync(0xffffffffu, sr.x, 1);
+      er.y = __shfl_up_sync(0xffffffffu, sr.y, 1);
+      ei.x = __shfl_up_sync(0xffffffffu, si.x, 1);
+      ei.y = __shfl_up_sync(0xffffffffu, si.y, 1);
+      if (lane == 0) er = ei = mk<T>(0, 0);
+      V ca, cb;
+      ld2<T>(sC + 2 * q, ca, cb);
+      const V l = ts.lane_pow;
+      sr = mk<T>(fma(l.x, ca.x, fma(-l.y, ca.y, er.x)), fma(l.x, cb.x, fma(-l.y, cb.y, er.y)));
+      si = mk<T>(fma(l.x, ca.y, fma(l.y, ca.x, ei.x)), fma(l.x, cb.y, fma(l.y, cb.x, ei.y)));
+      const V kerr2 = mk<T>(kerr, kerr);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (j < g) {
+          V w[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            ts.step(sr, si, x[2 * j + e]);
+            w[e] = pk_fma(kerr2, x[2 * j + e], pk_fma(ts.kr2, si, pk_mul(ts.ki2, sr)));
+          }
+          st_pair<T>(wq + wsw(g * lane + j, wmask), mk<T>(w[0].x, w[1].x), mk<T>(w[0].y, w[1].y));
+        }
+      }
+    }
+  } else {
+    for (int i = tid; i < P * H; i += blockDim.x) {
+      const int h = i & (H - 1), at = wsw(h, wmask);
+      const int2 lm = __ldg(d.pairs + i / H);
+      SP* row = sW + (i - h);
+      V vre, vim;
+      pair_product(ld_pair<T>(sU + lm.x * H + at), ld_pair<T>(sU + lm.y * H + at), vre, vim);
+      if (raman_mode == 1) {  // W = (1 - f_R) V + R, R in place as it landed
+        V r0, r1;
+        ld2<T>(reinterpret_cast<const V*>(row + h), r0, r1);
+        vre = pk_fma(mk<T>(kerr, kerr), vre, mk<T>(r0.x, r1.x));
+        vim = pk_fma(mk<T>(kerr, kerr), vim, mk<T>(r0.y, r1.y));
+        __syncwarp();
+      }
+      st_pair<T>(row + at, vre, vim);
+    }
+  }
+  __syncthreads();
+  grid_release();
+  // 3. contraction
+  V* sigma = as_t2<T>(d.sigma);
+  for (int item = warp; item < M * (H >> 5); item += nwarps) {
+    const int p = item / (H >> 5), h = (item - p * (H >> 5)) * 32 + lane, at = wsw(h, wmask);
+    const SP* uc = sU + at;
+    const SP* wc = sW + at;
+    const int n1 = __ldg(d.sr_off + p + 1);
+    V a1 = mk<T>(0, 0), a2 = a1, a3 = a1, a4 = a1;
+    SP u = {};
+    unsigned kprev = ~0u;
+#pragma unroll 2
+    for (int n = __ldg(d.sr_off + p); n < n1; ++n) {
+      V c;
+      unsigned kq;
+      ld_rec<T>(sRec + n, c, kq);
+      if ((kq >> 16) != kprev) {
+        kprev = kq >> 16;
+        u = ld_pair<T>(uc + kprev);
+      }
+      const SP w = ld_pair<T>(wc + (kq & 0xffffu));
+      const V xr = pk_mul(mk<T>(c.x, c.x), w.re), xi = pk_mul(mk<T>(c.y, c.y), w.im);  // a Re W, b Im W
+      a1 = pk_fma(u.re, xr, a1);
+      a2 = pk_fma(u.im, xi, a2);
+      a3 = pk_fma(u.re, xi, a3);
+      a4 = pk_fma(u.im, xr, a4);
+    }
+    st2<T>(sigma + (size_t)p * nt + t0 + 2 * h, mk<T>(a1.x - a2.x, a3.x + a4.x), mk<T>(a1.y - a2.y, a3.y + a4.y));
   }
 }
 
