@@ -173,10 +173,11 @@ constexpr int kDenseMaxModes = 16;
 constexpr int kRamanPow = 256;
 constexpr int kDenseChunk = 16;
 // Tensor-core form of the dense contraction: samples per tile (the MMA's M), pair fields
-// per K chunk, and the fewest modes a solve needs for it (from 6 modes, 21 pair fields,
+// per K chunk (one MMA step), chunks in flight, and the fewest modes a solve needs for it (from 6 modes, 21 pair fields,
 // on; below that the register-blocked form costs less than a tile's MMA pipeline).
 constexpr int kTcTile = 128;
-constexpr int kTcChunk = 16;
+constexpr int kTcChunk = 8;
+constexpr int kTcStages = 4;
 constexpr int kTcMinModes = 6;
 
 // RK tableau passed by value to the stage kernels (identical for a batch).

@@ -813,7 +813,7 @@ int launch_contract(mmp_batch* b, uint32_t first = 0, uint32_t count = ~0u, cuda
   }
   if (b->tc) {
     void* targs[] = {(void*)&descs, &nt, &mode};
-    CUDA_TRY(launch((const void*)&k_contract_tc<float>, grid, 512, (int)b->contract_smem, 1, st ? st : b->stream, targs, true));
+    CUDA_TRY(launch((const void*)&k_contract_tc<float>, grid, kTcThreads, (int)b->contract_smem, 1, st ? st : b->stream, targs, true));
     return MMP_OK;
   }
   if (b->dense != 1) {  // the sparse solves
@@ -1562,8 +1562,8 @@ Shape choose_shape(const mmp_batch* b, const ShapeStats& st) {
     fused = b->raman;
     dense = 1;
     smem = ((size_t)Mmax * TT + (b->raman ? 2 * (size_t)Pmax : 0)) * sizeof(float2) +
-           2 * 4 * (size_t)kTcChunk * (TT + 16 * (size_t)Mmax) * sizeof(float) +  // two operand buffers
-           1024;                                                                  // their alignment
+           kTcStages * 4 * (size_t)kTcChunk * (TT + 16 * (size_t)Mmax) * sizeof(float) +  // operand stages
+           1024;                                                                          // their alignment
   } else if (dense) {
     smem += 8 * 2 * (size_t)kDenseChunk * 2 * kDenseMaxModes * (t2 / 2);  // staged coefficient rows
   }

@@ -2053,6 +2053,34 @@ template <typename T> struct LaneScan {
     re = pk_fma(lr2, re, pk_fma(nli2, im, x));
     im = pk_fma(lr2, im, t);
   }
+  // (re, im): the lane's end from a zero start -> the state entering the lane, from the ends
+  // of the lanes before it (inclusive scan S_L = lambda^c S_{L-1} + end_L, handed up by one) and
+  // the state entering the tile, carry = (Re V's, Im V's)
+  __device__ __forceinline__ void enter(V& re, V& im, int lane, const V* carry) const {
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+      const int o = 1 << j;
+      V pr, pi;
+      pr.x = __shfl_up_sync(0xffffffffu, re.x, o);
+      pr.y = __shfl_up_sync(0xffffffffu, re.y, o);
+      pi.x = __shfl_up_sync(0xffffffffu, im.x, o);
+      pi.y = __shfl_up_sync(0xffffffffu, im.y, o);
+      const V l = lvl[j];
+      re = mk<T>(fma(l.x, pr.x, fma(-l.y, pi.x, re.x)), fma(l.x, pr.y, fma(-l.y, pi.y, re.y)));
+      im = mk<T>(fma(l.x, pi.x, fma(l.y, pr.x, im.x)), fma(l.x, pi.y, fma(l.y, pr.y, im.y)));
+    }
+    V er, ei;
+    er.x = __shfl_up_sync(0xffffffffu, re.x, 1);
+    er.y = __shfl_up_sync(0xffffffffu, re.y, 1);
+    ei.x = __shfl_up_sync(0xffffffffu, im.x, 1);
+    ei.y = __shfl_up_sync(0xffffffffu, im.y, 1);
+    if (lane == 0) er = ei = mk<T>(0, 0);
+    V ca, cb;
+    ld2<T>(carry, ca, cb);
+    const V l = lane_pow;
+    re = mk<T>(fma(l.x, ca.x, fma(-l.y, ca.y, er.x)), fma(l.x, cb.x, fma(-l.y, cb.y, er.y)));
+    im = mk<T>(fma(l.x, ca.y, fma(l.y, ca.x, ei.x)), fma(l.x, cb.y, fma(l.y, cb.x, ei.y)));
+  }
 };
 
 template <typename T>
@@ -2151,31 +2179,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
 #pragma unroll
       for (int k = 1; k < 8; ++k)
         if (k < ts.c) ts.step(sr, si, x[k]);
-      // inclusive scan over the lanes: S_L = lambda^c S_{L-1} + end_L
-#pragma unroll
-      for (int j = 0; j < 5; ++j) {
-        const int o = 1 << j;
-        V pr, pi;
-        pr.x = __shfl_up_sync(0xffffffffu, sr.x, o);
-        pr.y = __shfl_up_sync(0xffffffffu, sr.y, o);
-        pi.x = __shfl_up_sync(0xffffffffu, si.x, o);
-        pi.y = __shfl_up_sync(0xffffffffu, si.y, o);
-        const V l = ts.lvl[j];
-        sr = mk<T>(fma(l.x, pr.x, fma(-l.y, pi.x, sr.x)), fma(l.x, pr.y, fma(-l.y, pi.y, sr.y)));
-        si = mk<T>(fma(l.x, pi.x, fma(l.y, pr.x, si.x)), fma(l.x, pi.y, fma(l.y, pr.y, si.y)));
-      }
-      // the state entering the lane: the lanes before it, and the tile's
-      V er, ei;
-      er.x = __shfl_up_sync(0xffffffffu, sr.x, 1);
-      er.y = __shfl_up_sync(0xffffffffu, sr.y, 1);
-      ei.x = __shfl_up_sync(0xffffffffu, si.x, 1);
-      ei.y = __shfl_up_sync(0xffffffffu, si.y, 1);
-      if (lane == 0) er = ei = mk<T>(0, 0);
-      V ca, cb;
-      ld2<T>(sC + 2 * q, ca, cb);
-      const V l = ts.lane_pow;
-      sr = mk<T>(fma(l.x, ca.x, fma(-l.y, ca.y, er.x)), fma(l.x, cb.x, fma(-l.y, cb.y, er.y)));
-      si = mk<T>(fma(l.x, ca.y, fma(l.y, ca.x, ei.x)), fma(l.x, cb.y, fma(l.y, cb.x, ei.y)));
+      ts.enter(sr, si, lane, sC + 2 * q);  // the state entering the lane
       const V kerr2 = mk<T>(kerr, kerr);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -2246,29 +2250,52 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
 // followed by sigma_p(t) = sum_k U_k(t) (T_re + i T_im) (the k_contract<T, 1> arithmetic).
 // The products are tcgen05 TF32 MMAs: M = 128 samples (TMEM lane = sample), N = 16 M
 // columns (p, k) per product (Re in TMEM columns [0, N), Im in [256, 256 + N)), K = the pair
-// fields in chunks of kTcChunk = 16. Both operands are split x = hi + lo into TF32 parts
+// fields in chunks of kTcChunk = 8. Both operands are split x = hi + lo into TF32 parts
 // and every product is formed as hi hi + hi lo + lo hi with FP32 accumulation: relative
 // error about 2^-21 (plain TF32 would leave 2^-11).
-// Per chunk c the 16 warps build the chunk's pair fields W, one field each (the Raman
-// recurrence through the tile, raman_mode 2 or 3, or V = U_l conj(U_m), raman_mode 0), and each
-// lane writes its 4 consecutive samples, split into TF32 hi and lo, straight into the A
-// operands (buffer c % 2) in the MN-major TF32 layout (samples contiguous: the 4 samples of
-// one field are one 16-byte chunk per matrix); one thread issues the chunk's 12 MMAs and
-// commits them to an mbarrier; the chunk's split coefficients (SolveDesc::dense_tc, K-major)
-// arrive by one bulk copy issued when the chunk starts. The MMAs of chunk c run while the
-// warps build chunk c + 1. Every wait is bounded: on a timeout the CTA flags kStatusTimeout,
-// waits once more for its MMAs and frees its TMEM.
+// Warps 0-15 build the pair fields, one field of every other chunk each: V of the lane's 4 consecutive
+// samples, the Raman recurrence through them (raman_mode 2 or 3; the packed chain and lane scan of
+// k_contract_sp), and W split into TF32 hi and lo straight into the A operands (stage c % 4) in the
+// MN-major TF32 layout (samples contiguous: 4 samples of a field are one 16-byte chunk per
+// matrix). Warp 16 drives: it copies the chunk's split coefficients (SolveDesc::dense_tc,
+// K-major) up to four ahead, and when the fields and the coefficients are in, issues the chunk's
+// 6 MMAs and commits them to the mbarrier that frees the stage. No barrier of the whole CTA stands
+// between the chunks: builders run up to four chunks ahead of the tensor core. Every wait is
+// bounded; when one gives up, a flag ends the others' waits, the CTA reports kStatusTimeout, waits
+// once more for what is in flight and frees its TMEM.
+// What bounds it: shared-memory bandwidth (a chunk's MMAs read 70 KB, its operands are written
+// with 46 KB: 15.6 thousand of a CTA's 31 thousand cycles), then the CTA's start and end (7
+// thousand). Measured on a B200, 16 solves of 15 x 8192, a launch, against two 16-field buffers
+// between barriers of the whole CTA and scalar recurrences: 183 -> 141 us, 64 -> 44 million warp
+// instructions (24 builder warps instead of 16: 143).
+constexpr int kTcBuilders = 2;  // chunks built at a time, by eight warps each
+constexpr int kTcThreads = 32 * (8 * kTcBuilders + 1);
+
+// mbar_wait that also gives up once *stop is set (by another warp whose wait ran out)
+__device__ __forceinline__ bool mbar_wait_or(unsigned long long* bar, unsigned parity, volatile int* stop) {
+  for (unsigned it = 0; it < kMaxWaitPolls; it += 64) {
+    if (mbar_wait(bar, parity, 64)) return true;
+    if (*stop) return false;
+  }
+  *stop = 1;
+  return false;
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
 template <typename T>
-__global__ void __launch_bounds__(512, 1) k_contract_tc(const SolveDesc* __restrict__ descs, int nt, int raman_mode) {
+__global__ void __launch_bounds__(kTcThreads, 1) k_contract_tc(const SolveDesc* __restrict__ descs, int nt, int raman_mode) {
   static_assert(sizeof(T) == 4, "TF32 operands come from FP32 solves");
   using V = float2;
-  constexpr int TT = kTcTile, KC = kTcChunk, WMASK = TT / 64 - 1;
+  constexpr int TT = kTcTile, KC = kTcChunk, NS = kTcStages, BW = kTcBuilders * KC;  // builder warps
   // A operand (MN-major TF32 layout): 32-sample atoms 512 bytes apart, 4-field groups 2048
-  static_assert(TT == 128 && KC % 8 == 0, "one MMA covers the tile's 128 samples");
+  static_assert(TT == 128 && KC == 8 && kTcThreads == 32 * (BW + 1), "one MMA covers the tile's 128 samples");
   constexpr uint32_t A_LBO = 512, A_SBO = 2048;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ __align__(8) unsigned long long bar_u, bar_b[2], bar_m[2];
+  __shared__ __align__(8) unsigned long long bar_u, bar_a[NS], bar_b[NS], bar_m[NS];
   __shared__ uint32_t s_tmem;
+  __shared__ volatile int s_stop;
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TT;
   if (t0 >= nt || d.M == 0) {  // empty slot
@@ -2276,150 +2303,179 @@ __global__ void __launch_bounds__(512, 1) k_contract_tc(const SolveDesc* __restr
     return;
   }
   const int M = d.M, P = d.P, N = 16 * M;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   V* sU = reinterpret_cast<V*>(smem_raw);                        // [M][TT]
-  // [2][4][KC * TT] MN-major operands, on the next 1024-byte boundary (the swizzle pattern's
+  // [NS][4][KC * TT] MN-major operands, on the next 1024-byte boundary (the swizzle pattern's
   // alignment; the launch reserves the slack)
   unsigned char* after_u = reinterpret_cast<unsigned char*>(sU + (size_t)M * TT);
   float* sA = reinterpret_cast<float*>(after_u + ((1024u - (tc::smem_u32(after_u) & 1023u)) & 1023u));
-  float* sB = sA + 2 * 4 * KC * TT;                              // [2][4][KC/4][N][4]
-  V* sC = reinterpret_cast<V*>(sB + 2 * 4 * KC * N);              // states entering the tile, [P][2]
+  float* sB = sA + NS * 4 * KC * TT;                             // [NS][4][KC/4][N][4]
+  V* sC = reinterpret_cast<V*>(sB + NS * 4 * KC * N);             // states entering the tile, [P][2]
+  const int nch = (P + KC - 1) / KC;
+  const unsigned bbytes = (unsigned)(4 * KC * N * sizeof(float));
+  LaneScan<float> ts;
+  if (raman_mode >= 2) ts.init(d, TT >> 5, lane);
   if (tid == 0) {
+    s_stop = 0;
     mbar_init(&bar_u, 1);
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < NS; ++i) {
+      mbar_init(&bar_a[i], KC);
       mbar_init(&bar_b[i], 1);
       mbar_init(&bar_m[i], 1);
     }
+    mbar_arrive_expect_tx(&bar_u, (unsigned)(M * TT * sizeof(V)));
   }
-  grid_sync_wait();
-  if (__ldcg(d.step) >= d.step_limit) return;  // finished solve (nothing is in flight yet)
-  if (tid == 0) mbar_arrive_expect_tx(&bar_u, (unsigned)(M * TT * sizeof(V)));
   __syncthreads();
+  int b_issued = 0, committed = 0;  // driver: chunks whose copy was issued, whose MMAs were committed
+  const bool driver = warp == BW && lane == 0;
+  auto copy_b = [&](int c) {
+    mbar_arrive_expect_tx(&bar_b[c % NS], bbytes);
+    bulk_g2s(sB + (size_t)(c % NS) * 4 * KC * N, d.dense_tc + (size_t)c * 4 * KC * N, bbytes, &bar_b[c % NS]);
+    b_issued = c + 1;
+  };
+  auto drain_b = [&]() {  // the coefficient copies in flight have landed
+    for (int c = b_issued > NS ? b_issued - NS : 0; c < b_issued; ++c)
+      mbar_wait(&bar_b[c % NS], (c / NS) & 1, kMaxWaitPolls);
+  };
+  if (driver)  // the first chunks' coefficients, while the kernel before this one still runs
+    for (int c = 0; c < NS && c < nch; ++c) copy_b(c);
+  grid_sync_wait();
   if (tid < M) bulk_g2s(sU + (size_t)tid * TT, as_t2<float>(d.U) + (size_t)tid * nt + t0, TT * sizeof(V), &bar_u);
+  if (__ldcg(d.step) >= d.step_limit) {  // finished solve: the copies land before the CTA leaves
+    mbar_wait(&bar_u, 0, kMaxWaitPolls);
+    if (driver) drain_b();
+    return;
+  }
   if (raman_mode >= 2)
     stage_tile_carries<float>(sC, d, P, nt / TT, blockIdx.x, tile_look(d, nt / TT, TT, raman_mode), lambda_tile(d, TT));
-  if (warp == 0) {
+  if (warp == BW) {
     tc::alloc(&s_tmem, 512);
     tc::relinquish();
   }
   tc::fence_before_sync();
   bool ok = __syncthreads_and(mbar_wait(&bar_u, 0, d.tile_wait_polls) ? 1 : 0);
   const bool u_landed = ok;
-  int b_issued = -1;  // last chunk whose coefficient copy was issued
   tc::fence_after_sync();
   const uint32_t tmem = s_tmem;
-  TileScan<float> ts;
-  if (raman_mode >= 2) ts.init(d, TT >> 5, lane);
-  const float kerr = (float)d.one_minus_fR;
-  const int nch = (P + KC - 1) / KC;
-  const unsigned bbytes = (unsigned)(4 * KC * N * sizeof(float));
-  const uint32_t idesc = tc::idesc_tf32(TT, N, true);
-  int committed = -1;  // last chunk whose MMAs were committed
-  for (int c = 0; c < nch && ok; ++c) {
-    const int buf = c & 1;
-    float* A = sA + (size_t)buf * 4 * KC * TT;
-    float* B = sB + (size_t)buf * 4 * KC * N;
-    if (c >= 2) {  // chunk c - 2's MMAs read this buffer pair: wait for them
-      ok = __syncthreads_and(mbar_wait(&bar_m[buf], ((c - 2) >> 1) & 1, kMaxWaitPolls) ? 1 : 0);
-      if (!ok) break;
-      tc::fence_after_sync();
-    }
-    if (tid == 0) {
-      mbar_arrive_expect_tx(&bar_b[buf], bbytes);
-      bulk_g2s(B, d.dense_tc + (size_t)c * 4 * KC * N, bbytes, &bar_b[buf]);
-    }
-    b_issued = c;
-    for (int j = warp; j < KC; j += nwarps) {  // pair field q = c KC + j, one warp each
-      const int q = c * KC + j;
-      // lane L's samples 4L .. 4L + 3 of field j: one 16-byte chunk of each operand matrix
-      float* a0 = A + tc::mn_tf32_offset(4 * lane, j, A_LBO, A_SBO) / 4;
-      auto put = [&](const V* x) {
-        float rh[4], rl[4], ih[4], il[4];
+  if (ok && warp < BW) {
+    const float kerr = (float)d.one_minus_fR;
+    const int f = warp & (KC - 1);  // this warp's field of every other chunk
+    for (int c = warp / KC; c < nch; c += kTcBuilders) {
+      const int buf = c % NS, q = c * KC + f;
+      // chunk c - NS's MMAs read this buffer pair
+      if (c >= NS && !mbar_wait_or(&bar_m[buf], ((c / NS) - 1) & 1, &s_stop)) break;
+      // lane L's samples 4L .. 4L + 3 of the field: one 16-byte chunk of each operand matrix
+      float* a0 = sA + (size_t)buf * 4 * KC * TT + tc::mn_tf32_offset(4 * lane, f, A_LBO, A_SBO) / 4;
+      V x[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      if (q < P) {  // past the last field: zeros
+        const int2 lm = __ldg(d.pairs + q);
+        V a[4], b[4];
+        const V* ul = sU + lm.x * TT + 4 * lane;
+        const V* um = sU + lm.y * TT + 4 * lane;
+        ld2<float>(ul, a[0], a[1]);
+        ld2<float>(ul + 2, a[2], a[3]);
+        ld2<float>(um, b[0], b[1]);
+        ld2<float>(um + 2, b[2], b[3]);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          rh[e] = tc::tf32_hi(x[e].x);
-          rl[e] = x[e].x - rh[e];
-          ih[e] = tc::tf32_hi(x[e].y);
-          il[e] = x[e].y - ih[e];
+        for (int e = 0; e < 4; ++e) x[e] = cmulc(a[e], b[e]);
+        if (raman_mode >= 2) {
+          V sr = x[0], si = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int e = 1; e < 4; ++e) ts.step(sr, si, x[e]);
+          ts.enter(sr, si, lane, sC + 2 * q);
+          const V kerr2 = make_float2(kerr, kerr);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            ts.step(sr, si, x[e]);
+            x[e] = pk_fma(kerr2, x[e], pk_fma(ts.kr2, si, pk_mul(ts.ki2, sr)));
+          }
         }
-        *reinterpret_cast<float4*>(a0) = make_float4(rh[0], rh[1], rh[2], rh[3]);
-        *reinterpret_cast<float4*>(a0 + KC * TT) = make_float4(rl[0], rl[1], rl[2], rl[3]);
-        *reinterpret_cast<float4*>(a0 + 2 * KC * TT) = make_float4(ih[0], ih[1], ih[2], ih[3]);
-        *reinterpret_cast<float4*>(a0 + 3 * KC * TT) = make_float4(il[0], il[1], il[2], il[3]);
-      };
-      if (q >= P) {  // past the last field: zeros (the buffers start uninitialised)
-        const V z[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-        put(z);
-      } else if (raman_mode >= 2) {
-        tile_pair_recurrence_to<float, true>(ts, sU, TT, d.pairs[q], nullptr, WMASK, sC + 2 * q, kerr, lane, put);
-      } else {
-        const int2 lm = d.pairs[q];
-        V x[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) x[e] = cmulc(sU[lm.x * TT + 4 * lane + e], sU[lm.y * TT + 4 * lane + e]);
-        put(x);
       }
+      float rh[4], rl[4], ih[4], il[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        rh[e] = tc::tf32_hi(x[e].x);
+        rl[e] = x[e].x - rh[e];
+        ih[e] = tc::tf32_hi(x[e].y);
+        il[e] = x[e].y - ih[e];
+      }
+      *reinterpret_cast<float4*>(a0) = make_float4(rh[0], rh[1], rh[2], rh[3]);
+      *reinterpret_cast<float4*>(a0 + KC * TT) = make_float4(rl[0], rl[1], rl[2], rl[3]);
+      *reinterpret_cast<float4*>(a0 + 2 * KC * TT) = make_float4(ih[0], ih[1], ih[2], ih[3]);
+      *reinterpret_cast<float4*>(a0 + 3 * KC * TT) = make_float4(il[0], il[1], il[2], il[3]);
+      tc::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_a[buf]);
     }
-    tc::fence_proxy_async();
-    // the chunk's coefficients have landed and every thread's operand writes are done
-    ok = __syncthreads_and(mbar_wait(&bar_b[buf], (c >> 1) & 1, kMaxWaitPolls) ? 1 : 0);
-    if (!ok) break;
-    b_issued = -1;  // landed
-    tc::fence_after_sync();
-    if (tid == 0) {
+  } else if (ok && driver) {
+    const uint32_t idesc = tc::idesc_tf32(TT, N, true);
+    for (int c = 0; c < nch; ++c) {
+      const int buf = c % NS;
+      const unsigned par = (c / NS) & 1;
+      if (!mbar_wait_or(&bar_b[buf], par, &s_stop) || !mbar_wait_or(&bar_a[buf], par, &s_stop)) break;
+      tc::fence_after_sync();
+      const float* A = sA + (size_t)buf * 4 * KC * TT;
+      const float* B = sB + (size_t)buf * 4 * KC * N;
       // Re: (A Re hi, B Re hi), (Re hi, Re lo), (Re lo, Re hi); Im likewise
       constexpr int ta[3] = {0, 0, 1}, tb[3] = {0, 1, 0};
 #pragma unroll
       for (int part = 0; part < 2; ++part)
 #pragma unroll
         for (int term = 0; term < 3; ++term)
-#pragma unroll
-          for (int ks = 0; ks < KC / 8; ++ks) {
-            const float* a = A + (size_t)(2 * part + ta[term]) * KC * TT + ks * 2 * A_SBO / 4;
-            const float* b = B + (size_t)(2 * part + tb[term]) * KC * N + ks * 2 * N * 4;
-            tc::mma_tf32(tmem + 256u * part, tc::desc_mn_tf32(a, A_LBO, A_SBO), tc::desc_kmajor(b, N * 16, 128),
-                         idesc, (c > 0 || term > 0 || ks > 0) ? 1u : 0u);
-          }
+        {
+          const float* a = A + (size_t)(2 * part + ta[term]) * KC * TT;
+          const float* b = B + (size_t)(2 * part + tb[term]) * KC * N;
+          tc::mma_tf32(tmem + 256u * part, tc::desc_mn_tf32(a, A_LBO, A_SBO), tc::desc_kmajor(b, N * 16, 128),
+                       idesc, (c > 0 || term > 0) ? 1u : 0u);
+        }
       tc::commit(&bar_m[buf]);
+      committed = c + 1;
+      if (c >= 1 && c - 1 + NS < nch) {  // once chunk c - 1 is done, its coefficients may be replaced
+        if (!mbar_wait_or(&bar_m[(c - 1) % NS], ((c - 1) / NS) & 1, &s_stop)) break;
+        copy_b(c - 1 + NS);
+      }
     }
-    committed = c;
+    // the last chunk's MMAs complete after all earlier ones (in-order issue, one thread)
+    if (committed == nch && nch > 0) mbar_wait_or(&bar_m[(nch - 1) % NS], ((nch - 1) / NS) & 1, &s_stop);
   }
   grid_release();
-  // the last chunk's MMAs complete after all earlier ones (in-order issue, one thread)
-  if (ok && committed >= 0)
-    ok = __syncthreads_and(mbar_wait(&bar_m[committed & 1], (committed >> 1) & 1, kMaxWaitPolls) ? 1 : 0);
+  ok = __syncthreads_and(ok && !s_stop ? 1 : 0);
   tc::fence_after_sync();
   if (ok) {
     // sigma_p(t) = sum_k U_k(t) (T_re + i T_im): warp w reads TMEM lanes 32 (w % 4) .. + 31
-    const int quad = warp & 3, t = quad * 32 + lane;
-    const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16);
-    V* sigma = as_t2<float>(d.sigma);
-    for (int p = warp >> 2; p < M; p += nwarps >> 2) {
-      float re[16], im[16];
-      tc::ld16(tl + 16u * p, re);
-      tc::ld16(tl + 256u + 16u * p, im);
-      float sx = 0.f, sy = 0.f;
+    if (warp < BW) {
+      const int quad = warp & 3, t = quad * 32 + lane;
+      const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16);
+      V* sigma = as_t2<float>(d.sigma);
+      for (int p = warp >> 2; p < M; p += BW >> 2) {
+        float re[16], im[16];
+        tc::ld16(tl + 16u * p, re);
+        tc::ld16(tl + 256u + 16u * p, im);
+        float sx = 0.f, sy = 0.f;
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        if (k < M) {
-          const V u = sU[k * TT + t];
-          sx = fmaf(u.x, re[k], fmaf(-u.y, im[k], sx));
-          sy = fmaf(u.x, im[k], fmaf(u.y, re[k], sy));
+        for (int k = 0; k < 16; ++k) {
+          if (k < M) {
+            const V u = sU[k * TT + t];
+            sx = fmaf(u.x, re[k], fmaf(-u.y, im[k], sx));
+            sy = fmaf(u.x, im[k], fmaf(u.y, re[k], sy));
+          }
         }
+        sigma[(size_t)p * nt + t0 + t] = make_float2(sx, sy);
       }
-      sigma[(size_t)p * nt + t0 + t] = make_float2(sx, sy);
     }
   } else {
     if (tid == 0) atomicOr(d.status, kStatusTimeout);
     // nothing may still be writing this CTA's shared memory or TMEM when it leaves: the
     // tile and coefficient copies in flight, the MMAs in flight (each waited for once more)
     if (!u_landed) mbar_wait(&bar_u, 0, kMaxWaitPolls);
-    if (b_issued >= 0) mbar_wait(&bar_b[b_issued & 1], (b_issued >> 1) & 1, kMaxWaitPolls);
-    if (committed >= 0) mbar_wait(&bar_m[committed & 1], (committed >> 1) & 1, kMaxWaitPolls);
+    if (driver) {
+      drain_b();
+      if (committed > 0) mbar_wait(&bar_m[(committed - 1) % NS], ((committed - 1) / NS) & 1, kMaxWaitPolls);
+    }
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::dealloc(tmem, 512);
+  if (warp == BW) tc::dealloc(tmem, 512);
 }
 
 // FP64 rows -> T rows (used for the Raman spectrum)
