@@ -75,6 +75,16 @@ struct Term {
 };
 static_assert(sizeof(Term) == 16, "Term layout");
 
+// The REAL form of the Raman and contraction kernels. A coupling symmetric in (l, m), as every
+// physical one is, reads a pair field only as W_lm + W_ml = 2 Re W_lm (and Im W_ll is 0): every merged
+// term's b is 0 (up to rounding, host_setup). Raman's convolution is real, so Re W needs Re V alone, and two pair fields 2 s
+// and 2 s + 1 share one slot s: x_s = Re V_{2s} + i Re V_{2s+1} goes through the same recurrence or
+// transform as one complex V_q, for half the work, and comes out as W_{2s} + i W_{2s+1}. In
+// the general form slot q holds V_q. Per-slot data (tile aggregates, carries, R rows) have the
+// same shape in both. The form is a solve's own (SolveDesc::real); a batch that holds both
+// launches one kernel for each, which skips the other's solves.
+template <bool REAL> __host__ __device__ constexpr int slot_count(int P) { return REAL ? (P + 1) >> 1 : P; }
+
 // Everything a kernel needs about one solve. Lives in device memory (an array
 // of these per batch); kernels index it with blockIdx.y.
 struct SolveDesc {
@@ -82,6 +92,8 @@ struct SolveDesc {
   int P;            // distinct pair fields (l <= m) formed on the device
   int n_beta;       // polynomial coefficients per mode
   int raman;        // 1: Raman on (contraction adds R = h_R (*) V to (1-fR) V)
+  int real;         // 1: the Raman and contraction kernels run this solve in the REAL form
+  int pad1_;
   double alpha_scale;   // 2*pi / t_final
   double dz;            // h (dimensionless)
   double sgn_gamma;     // +1 / -1
@@ -103,6 +115,8 @@ struct SolveDesc {
   const void* H;        // [NT] scaled Raman spectrum (T2) or null
   double2* io;          // [M][NT] FP64 staging for upload / result
   const int2* pairs;    // [P] (l, m)
+  // [(P + 1) / 2] (l, m) of pair fields 2 s and 2 s + 1, for the REAL form
+  const int4* rpairs;
   const Term* terms;    // sorted by p
   const int* term_off;  // [M+1]
   unsigned long long* step;   // steps since the last z reset

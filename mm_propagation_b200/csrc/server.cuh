@@ -145,8 +145,8 @@ int admit(mmp_server* sv, Request* r, int pi, uint32_t slot) {
     s.desc.step_limit = r->p.n_steps;  // this solve stops at its own step count
     rc = upload_desc(b);
   }
+  if (rc == MMP_OK) rc = batch_shape(b);
   if (rc == MMP_OK) {
-    batch_shape(b);
     rc = launch_row_kernel(b, b->ks, b->ks.prime, (int)s.M, 1, 0, b->d_descs + slot);
   }
   if (rc) {

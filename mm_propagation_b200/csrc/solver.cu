@@ -156,6 +156,33 @@ constexpr int kMaxLook = 16;  // tiles the contraction looks back for a Raman st
 constexpr int kSMs = 148;  // of a B200
 constexpr int kSmemSM = 228 * 1024;  // its shared memory
 
+// Kernels by precision and form (REAL: common.cuh).
+template <typename F> const void* fn_ptr(F f) { return (const void*)f; }
+const void* contract_fn(bool fp64, int dense, bool real) {
+  if (!dense) return fp64 ? fn_ptr(&k_contract<double, 0, false>) : fn_ptr(&k_contract<float, 0, false>);
+  if (real) return fp64 ? fn_ptr(&k_contract<double, 1, true>) : fn_ptr(&k_contract<float, 1, true>);
+  return fp64 ? fn_ptr(&k_contract<double, 1, false>) : fn_ptr(&k_contract<float, 1, false>);
+}
+const void* sp_fn(bool fp64, bool real) {
+  if (real) return fp64 ? fn_ptr(&k_contract_sp<double, true>) : fn_ptr(&k_contract_sp<float, true>);
+  return fp64 ? fn_ptr(&k_contract_sp<double, false>) : fn_ptr(&k_contract_sp<float, false>);
+}
+const void* sr_fn(bool fp64, bool real) {
+  if (real) return fp64 ? fn_ptr(&k_contract_sr<double, true>) : fn_ptr(&k_contract_sr<float, true>);
+  return fp64 ? fn_ptr(&k_contract_sr<double, false>) : fn_ptr(&k_contract_sr<float, false>);
+}
+const void* agg_sr_fn(bool fp64, bool real) {
+  if (real) return fp64 ? fn_ptr(&k_raman_agg_sr<double, true>) : fn_ptr(&k_raman_agg_sr<float, true>);
+  return fp64 ? fn_ptr(&k_raman_agg_sr<double, false>) : fn_ptr(&k_raman_agg_sr<float, false>);
+}
+const void* agg_fn(bool fp64, bool real) {
+  if (real) return fp64 ? fn_ptr(&k_raman_agg<double, true>) : fn_ptr(&k_raman_agg<float, true>);
+  return fp64 ? fn_ptr(&k_raman_agg<double, false>) : fn_ptr(&k_raman_agg<float, false>);
+}
+const void* tc_fn(bool real) {
+  return real ? fn_ptr(&k_contract_tc<float, true>) : fn_ptr(&k_contract_tc<float, false>);
+}
+
 // ---- per-device resources: twiddle tables, kernel attributes ------------------------------
 struct DeviceRes {
   bool ready = false;
@@ -217,36 +244,33 @@ int ensure_device(int dev, DeviceRes** out) {
     for (int L = kMinLogN; L <= kMaxLogN; ++L)
       for (int xc = 0; xc <= max_split(fp64 != 0, L); ++xc) {
         KernelSet ks = kernels_for(fp64, L, xc);
-        std::vector<const void*> fns = {ks.prime, ks.pair, ks.nu, ks.result, ks.dft_fwd, ks.dft_inv};
+        std::vector<const void*> fns = {ks.prime, ks.pair, ks.pair_real, ks.nu, ks.result, ks.dft_fwd, ks.dft_inv};
         for (const void* f : ks.nu_mid) fns.push_back(f);
         for (const void* f : ks.nu_last) fns.push_back(f);
         for (const void* f : fns)
           if (f)
             CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(ks.smem, kSmemSM / 2)));
       }
-  const void* contract_fns[] = {(const void*)&k_contract<float, 0>,   (const void*)&k_contract<float, 1>,
-                                (const void*)&k_contract<double, 0>,  (const void*)&k_contract<double, 1>,
-                                (const void*)&k_contract_sp<float>, (const void*)&k_contract_sp<double>};
-  for (const void* f : contract_fns)
-    CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kContractSmemMax));
-  CUDA_TRY(cudaFuncSetAttribute((const void*)&k_contract_pc<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                110 * 1024));
-  CUDA_TRY(cudaFuncSetAttribute((const void*)&k_contract_pc<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                110 * 1024));
-  CUDA_TRY(cudaFuncSetAttribute((const void*)&k_contract_tc<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                227 * 1024 - 256));
-  CUDA_TRY(cudaFuncSetAttribute((const void*)&k_contract_sr<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                227 * 1024));
-  CUDA_TRY(cudaFuncSetAttribute((const void*)&k_contract_sr<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                227 * 1024));
+  struct Attr { const void* f; int smem; };
+  const int most = 227 * 1024, contract = (int)kContractSmemMax;
+  const Attr attrs[] = {
+      {contract_fn(false, 0, false), contract}, {contract_fn(true, 0, false), contract},
+      {contract_fn(false, 1, false), contract}, {contract_fn(true, 1, false), contract},
+      {contract_fn(false, 1, true), contract},  {contract_fn(true, 1, true), contract},
+      {sp_fn(false, false), contract},          {sp_fn(false, true), contract},
+      {sp_fn(true, false), contract},           {sp_fn(true, true), contract},
+      {sr_fn(false, false), most},              {sr_fn(false, true), most},
+      {sr_fn(true, false), most},               {sr_fn(true, true), most},
+      {tc_fn(false), most - 256},               {tc_fn(true), most - 256},
+      {agg_fn(false, false), 200 * 1024},       {agg_fn(false, true), 200 * 1024},
+      {agg_fn(true, false), 200 * 1024},        {agg_fn(true, true), 200 * 1024},
+      {(const void*)&k_contract_pc<float>, 110 * 1024}, {(const void*)&k_contract_pc<double>, 110 * 1024}};
+  for (const Attr& a : attrs)
+    CUDA_TRY(cudaFuncSetAttribute(a.f, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smem));
   CUDA_TRY(cudaFuncSetAttribute((const void*)&k_raman_scan<float>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmem));
   CUDA_TRY(cudaFuncSetAttribute((const void*)&k_raman_scan<double>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmem));
-  CUDA_TRY(cudaFuncSetAttribute((const void*)&k_raman_agg<float>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  CUDA_TRY(cudaFuncSetAttribute((const void*)&k_raman_agg<double>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   r.ready = true;
   *out = &r;
   return MMP_OK;
@@ -390,6 +414,10 @@ struct Member {
   int sr_rounds = 0;
   std::vector<double> poly;
   bool quirk = false;
+  bool symmetric = false; // every merged term's b is 0 (up to rounding)
+  bool real_ok = false;   // the REAL form serves (common.cuh) and pays (real_pays)
+  std::vector<int4> rpairs;  // (l, m) of pair fields 2 s and 2 s + 1
+  int dense_form = -1;    // form the dense coefficients on the device have: 0 general, 1 REAL (-1: none yet)
   double iir_decay = 0;   // -ln |lambda| of the Raman recurrence (h_R a damped sinusoid)
   bool dense_ok = false;  // the dense contraction form is built for this solve
   uint32_t flags = 0;
@@ -644,6 +672,21 @@ void host_setup(const mmp_params* p, Member& s) {
   }
   s.sr_off[M] = (int)s.sr_kq.size();
   sr_make_plan(s);
+  // Symmetric in (l, m) up to rounding: b within the rounding of the two Q_tilde it is the
+  // difference of (FP64), or four decades under that of FP32 coefficients next to max |Q_tilde| = 1
+  // (a symmetrisation that sums in another order for each entry leaves about 1e-16).
+  const bool fp64 = (p->flags & MMP_F_FP64) != 0;
+  s.symmetric = !s.pairs.empty();
+  for (size_t j = 0; j < s.sr_kq.size() && s.symmetric; ++j) {
+    const int2 lm = s.pairs[s.sr_kq[j] & 0xffffu];
+    const double a = std::fabs(s.sr_ab[2 * j]), b = std::fabs(s.sr_ab[2 * j + 1]);
+    s.symmetric = lm.x == lm.y || b <= (fp64 ? 0x1p-52 * a : 1e-12);
+  }
+  s.rpairs.clear();
+  for (size_t q = 0; q < s.pairs.size(); q += 2) {
+    const int2 a = s.pairs[q], b = q + 1 < s.pairs.size() ? s.pairs[q + 1] : a;  // an odd last field twice
+    s.rpairs.push_back(make_int4(a.x, a.y, b.x, b.y));
+  }
 }
 
 size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -688,6 +731,9 @@ struct mmp_batch {
   std::vector<cudaEvent_t> branch_ev;
   cudaEvent_t fork_ev = nullptr;
   int Mmax = 0, Pmax = 0;
+  bool real = false;  // solves whose coupling allows it run in the REAL form (common.cuh)
+  bool forms[2] = {}; // some solve runs in the general, in the REAL form
+  int slots = 0;      // most slots of a solve (Raman on)
   int TT = 32;
   int stage_terms = 0;
   size_t contract_smem = 0;
@@ -787,50 +833,46 @@ int launch_row_kernel(mmp_batch* b, const KernelSet& ks, const void* fn, int row
   return MMP_OK;
 }
 
-// contraction over solves [first, first + count) (default: every slot)
+// contraction over solves [first, first + count) (default: every slot): one launch, or one for
+// each form among the solves (dense or sparse, general or REAL), which skips the others
 int launch_contract(mmp_batch* b, uint32_t first = 0, uint32_t count = ~0u, cudaStream_t st = nullptr) {
   if (count == ~0u) count = b->span;
   if (count == 0) return MMP_OK;
+  if (!st) st = b->stream;
   const SolveDesc* descs = b->d_descs + first;
-  int nt = (int)b->nt, TT = b->TT, sterms = b->stage_terms;
-  int mode = !b->raman ? 0 : (b->lookback ? 3 : b->raman_fused ? 2 : 1);
-  int mixed = b->dense == 2;
-  void* args[] = {(void*)&descs, &nt, &TT, &sterms, &mode, &mixed};
-  dim3 grid((unsigned)(b->nt / b->TT), count, 1);
-  if (b->sr) {
-    int tb = b->TT;
-    void* sargs[] = {(void*)&descs, &nt, &tb, &mode};
-    const void* fsr = b->fp64 ? (const void*)&k_contract_sr<double> : (const void*)&k_contract_sr<float>;
-    CUDA_TRY(launch(fsr, grid, kSrThreads, (int)b->contract_smem, 1, st ? st : b->stream, sargs, true));
-    return MMP_OK;
-  }
-  if (b->pchunk) {
-    int pc = b->pchunk;
-    void* pargs[] = {(void*)&descs, &nt, &TT, &pc, &mode};
-    const void* fpc = b->fp64 ? (const void*)&k_contract_pc<double> : (const void*)&k_contract_pc<float>;
-    CUDA_TRY(launch(fpc, grid, 256, (int)b->contract_smem, 1, st ? st : b->stream, pargs, true));
-    return MMP_OK;
-  }
-  if (b->tc) {
-    void* targs[] = {(void*)&descs, &nt, &mode};
-    CUDA_TRY(launch((const void*)&k_contract_tc<float>, grid, kTcThreads, (int)b->contract_smem, 1, st ? st : b->stream, targs, true));
-    return MMP_OK;
-  }
-  if (b->dense != 1) {  // the sparse solves
-    if (b->sp) {
-      void* spargs[] = {(void*)&descs, &nt, &TT, &mode, &mixed};
-      const void* fsp = b->fp64 ? (const void*)&k_contract_sp<double> : (const void*)&k_contract_sp<float>;
-      CUDA_TRY(launch(fsp, grid, 256, (int)b->sp_smem, 1, st ? st : b->stream, spargs, true));
+  int nt = (int)b->nt, TT = b->TT, sterms = b->stage_terms, pc = b->pchunk;
+  int mode = !b->raman ? 0 : (b->lookback ? 3 : b->raman_fused ? 2 : 1), mixed = b->dense == 2;
+  const dim3 grid((unsigned)(b->nt / b->TT), count, 1);
+  const int smem = (int)b->contract_smem;
+  for (int real = 0; real < 2; ++real) {
+    if (!b->forms[real]) continue;
+    void* args[] = {(void*)&descs, &nt, &TT, &sterms, &mode, &mixed};
+    void* margs[] = {(void*)&descs, &nt, &TT, &mode, &mixed};
+    if (b->sr) {
+      CUDA_TRY(launch(sr_fn(b->fp64, real), grid, kSrThreads, smem, 1, st, margs, true));
+    } else if (b->pchunk) {
+      void* pargs[] = {(void*)&descs, &nt, &TT, &pc, &mode};
+      const void* fpc = b->fp64 ? (const void*)&k_contract_pc<double> : (const void*)&k_contract_pc<float>;
+      CUDA_TRY(launch(fpc, grid, 256, smem, 1, st, pargs, true));
+    } else if (b->tc) {
+      void* targs[] = {(void*)&descs, &nt, &mode};
+      CUDA_TRY(launch(tc_fn(real), grid, real ? tc_threads<true>() : tc_threads<false>(), smem, 1, st, targs, true));
     } else {
-      const void* f0 = b->fp64 ? (const void*)&k_contract<double, 0> : (const void*)&k_contract<float, 0>;
-      CUDA_TRY(launch(f0, grid, 256, (int)b->contract_smem, 1, st ? st : b->stream, args, true));
+      if (b->dense != 1 && b->sp) CUDA_TRY(launch(sp_fn(b->fp64, real), grid, 256, (int)b->sp_smem, 1, st, margs, true));
+      if (b->dense != 1 && !b->sp) CUDA_TRY(launch(contract_fn(b->fp64, 0, false), grid, 256, smem, 1, st, args, true));
+      if (b->dense) CUDA_TRY(launch(contract_fn(b->fp64, 1, real), grid, 256, smem, 1, st, args, true));
     }
   }
-  if (b->dense) {
-    const void* f1 = b->fp64 ? (const void*)&k_contract<double, 1> : (const void*)&k_contract<float, 1>;
-    CUDA_TRY(launch(f1, grid, 256, (int)b->contract_smem, 1, st ? st : b->stream, args, true));
-  }
   return MMP_OK;
+}
+
+// Kernels of one RK step of one group.
+int step_kernels(const mmp_batch* b) {
+  const int forms = (int)b->forms[0] + (int)b->forms[1];
+  int n = 1 + forms * ((b->sr || b->pchunk || b->tc || b->dense != 2) ? 1 : 2);
+  if (b->raman && b->Pmax > 0)
+    n += b->raman_iir && !b->raman_fused ? 1 : forms + (b->raman_fused && !b->lookback ? 1 : 0);
+  return b->tab.s * n;
 }
 
 // The k_nu instantiation for stage i: the body built for its count of stored N_hat_j, or the
@@ -848,38 +890,39 @@ const void* nu_kernel(const KernelSet& ks, const Tableau& tab, int i) {
 int launch_pairs(mmp_batch* b, const KernelSet& ks, int nsolves, int stage, const SolveDesc* descs,
                  cudaStream_t st = nullptr) {
   if (!(b->raman && b->Pmax > 0) || nsolves <= 0) return MMP_OK;
-  if (!b->raman_iir) return launch_row_kernel(b, ks, ks.pair, b->Pmax, nsolves, stage, descs, st, true);
-  int nt = (int)b->nt;
-  if (b->raman_fused) {
-    const size_t t2 = b->fp64 ? sizeof(double2) : sizeof(float2);
-    int TT = b->TT;
-    const SolveDesc* dd = descs;
-    int by_tile = b->lookback ? 1 : 0;
-    void* args[] = {(void*)&dd, &nt, &TT, &by_tile};  // k_raman_carry takes the first three
-    if (b->sr) {  // one thread per pair field through the tile (k_contract_sr's tiles)
-      const int smem = (int)(2 * (size_t)b->Mmax * (kSrSub / 2 + 1) * 2 * t2);
-      const void* fa = b->fp64 ? (const void*)&k_raman_agg_sr<double> : (const void*)&k_raman_agg_sr<float>;
-      CUDA_TRY(launch(fa, dim3((unsigned)(nt / TT), (unsigned)nsolves, 1), kSrThreads, smem, 1,
-                      st ? st : b->stream, args, true));
-    } else {
-      const int smem = (int)((size_t)b->Mmax * TT * t2);  // U tile
-      const void* fa = b->fp64 ? (const void*)&k_raman_agg<double> : (const void*)&k_raman_agg<float>;
-      CUDA_TRY(launch(fa, dim3((unsigned)(nt / TT), (unsigned)nsolves, 1), 256, smem, 1, st ? st : b->stream, args, true));
+  int nt = (int)b->nt, TT = b->TT, by_tile = b->lookback ? 1 : 0;
+  const size_t t2 = b->fp64 ? sizeof(double2) : sizeof(float2);
+  const SolveDesc* dd = descs;
+  if (!st) st = b->stream;
+  if (!b->raman_iir || b->raman_fused) {
+    for (int real = 0; real < 2; ++real) {  // a launch for each form among the solves
+      if (!b->forms[real]) continue;
+      void* args[] = {(void*)&dd, &nt, &TT, &by_tile};
+      const dim3 grid((unsigned)(nt / TT), (unsigned)nsolves, 1);
+      if (!b->raman_iir) {
+        int rc = launch_row_kernel(b, ks, real ? ks.pair_real : ks.pair, b->slots, nsolves, stage, descs, st, true);
+        if (rc) return rc;
+      } else if (b->sr) {  // one thread per slot through the tile (k_contract_sr's tiles)
+        const int smem = (int)(2 * (size_t)b->Mmax * (kSrSub / 2 + 1) * 2 * t2);
+        CUDA_TRY(launch(agg_sr_fn(b->fp64, real), grid, kSrThreads, smem, 1, st, args, true));
+      } else {
+        const int smem = (int)((size_t)b->Mmax * TT * t2);  // U tile
+        CUDA_TRY(launch(agg_fn(b->fp64, real), grid, 256, smem, 1, st, args, true));
+      }
     }
-    if (b->lookback) return MMP_OK;
+    if (!b->raman_iir || b->lookback) return MMP_OK;
+    void* cargs[] = {(void*)&dd, &nt, &TT};
     const void* fc = b->fp64 ? (const void*)&k_raman_carry<double> : (const void*)&k_raman_carry<float>;
-    CUDA_TRY(launch(fc, dim3((unsigned)b->Pmax, (unsigned)nsolves, 1), 32, 0, 1, st ? st : b->stream, args, true));
+    CUDA_TRY(launch(fc, dim3((unsigned)b->slots, (unsigned)nsolves, 1), 32, 0, 1, st, cargs, true));
     return MMP_OK;
   }
   // segments of at most 128 KB of V staged in shared memory
-  const size_t t2 = b->fp64 ? sizeof(double2) : sizeof(float2);
   int seg = std::min(nt, (int)((128 * 1024) / t2));
   const int thr = std::max(32, std::min(512, seg / 8));
   const int smem = padded_len(seg) * (int)t2;
-  const SolveDesc* dd = descs;
   void* args[] = {(void*)&dd, &nt, &seg};
   const void* fn = b->fp64 ? (const void*)&k_raman_scan<double> : (const void*)&k_raman_scan<float>;
-  CUDA_TRY(launch(fn, dim3((unsigned)b->Pmax, (unsigned)nsolves, 1), thr, smem, 1, st ? st : b->stream, args, true));
+  CUDA_TRY(launch(fn, dim3((unsigned)b->Pmax, (unsigned)nsolves, 1), thr, smem, 1, st, args, true));
   return MMP_OK;
 }
 
@@ -1103,7 +1146,6 @@ int batch_open(mmp_batch* b, const mmp_params* p0, const Tableau& tab0) {
   b->ks = kernels_for(b->fp64 ? 1 : 0, b->logn, std::max(b->xc_req, 0));
   b->ks64 = kernels_for(1, b->logn);
   if (!b->ks.prime || !b->ks64.prime) return fail(MMP_ENOTSUP, "no kernels built for this nt");
-  b->kernels_per_step = b->tab.s * ((b->raman ? 1 : 0) + 2);
   CUDA_TRY(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
   CUDA_TRY(dev_malloc((void**)&b->d_descs, (size_t)b->capacity * sizeof(SolveDesc) + 16));
   b->d_flag = reinterpret_cast<int*>(b->d_descs + b->capacity);
@@ -1133,22 +1175,59 @@ float tf32_round(float x) {
   std::memcpy(&x, &u, 4);
   return x;
 }
-std::vector<float> tc_operand(const std::vector<double>& A, int M, int P) {
+// REAL form (A[p][slot][2 K]): [hi, lo] of the one real product, field q = 2 slot + component.
+std::vector<float> tc_operand(const std::vector<double>& A, int M, int P, bool real) {
   constexpr int K = kDenseMaxModes, KC = kTcChunk;
-  const int N = 16 * M, nch = (P + KC - 1) / KC;
-  std::vector<float> B(tc_floats(M, P), 0.0f);
-  for (int c = 0; c < nch; ++c)
-    for (int m = 0; m < 4; ++m)
-      for (int jq = 0; jq < KC / 4; ++jq)
-        for (int n = 0; n < N; ++n)
-          for (int i = 0; i < 4; ++i) {
-            const int q = c * KC + 4 * jq + i, p = n / 16, k = n % 16;
-            if (q >= P || k >= M) continue;
-            const double x = A[((size_t)p * P + q) * 2 * K + (m < 2 ? 0 : K) + k];
-            const float hi = tf32_round((float)x);
-            B[((((size_t)c * 4 + m) * (KC / 4) + jq) * N + n) * 4 + i] = (m & 1) ? (float)(x - (double)hi) : hi;
-          }
+  const int N = 16 * M, nch = (P + KC - 1) / KC, mats = real ? 2 : 4;
+  const int S = real ? slot_count<true>(P) : P;
+  std::vector<float> B((size_t)nch * mats * KC * N, 0.0f);
+  for (int q = 0; q < P; ++q)
+    for (int m = 0; m < mats; ++m)
+      for (int p = 0; p < M; ++p) {
+        const double* a = real ? &A[((size_t)p * S + q / 2) * 2 * K + (q & 1) * K] : &A[((size_t)p * S + q) * 2 * K + (m < 2 ? 0 : K)];
+        float* o = &B[((((size_t)(q / KC) * mats + m) * (KC / 4) + q % KC / 4) * N + 16 * p) * 4 + q % 4];
+        for (int k = 0; k < M; ++k) {
+          const float hi = tf32_round((float)a[k]);
+          o[4 * k] = (m & 1) ? (float)(a[k] - (double)hi) : hi;
+        }
+      }
   return B;
+}
+
+// The dense coefficients of member s on the device in the form the batch runs.
+int upload_dense(mmp_batch* b, Member& s) {
+  const int form = s.desc.real;
+  if (!s.dense_ok || s.dense_form == form) return MMP_OK;
+  // general: A[p][q][k] += Q, A[p][q][16 + k] += Q or -Q (terms that read conj of pair field q);
+  // REAL: A[p][slot][16 c + k] += Q, q = 2 slot + c
+  constexpr int K = kDenseMaxModes;
+  const size_t M = s.M, P = s.pairs.size(), S = form ? s.rpairs.size() : P;
+  std::vector<double> A(M * S * 2 * K, 0.0);
+  for (uint32_t p = 0; p < M; ++p)
+    for (int j = s.term_off[p]; j < s.term_off[p + 1]; ++j) {
+      const Term& t = s.terms[j];
+      const size_t q = t.pc & 0x7fff;
+      if (form) {
+        A[(p * S + q / 2) * 2 * K + (q & 1) * K + t.k] += t.q;
+      } else {
+        A[(p * S + q) * 2 * K + t.k] += t.q;
+        A[(p * S + q) * 2 * K + K + t.k] += (t.pc & 0x8000) ? -t.q : t.q;
+      }
+    }
+  const size_t n = A.size();
+  if (b->fp64) {
+    CUDA_TRY(cudaMemcpyAsync((void*)s.desc.dense_q, A.data(), n * sizeof(double), cudaMemcpyHostToDevice, b->stream));
+    CUDA_TRY(cudaStreamSynchronize(b->stream));  // A is a host temporary
+  } else {
+    std::vector<float> Af(A.begin(), A.end());
+    CUDA_TRY(cudaMemcpyAsync((void*)s.desc.dense_q, Af.data(), n * sizeof(float), cudaMemcpyHostToDevice, b->stream));
+    const std::vector<float> B = tc_operand(A, (int)M, (int)P, form != 0);
+    CUDA_TRY(cudaMemcpyAsync((void*)s.desc.dense_tc, B.data(), B.size() * sizeof(float), cudaMemcpyHostToDevice,
+                             b->stream));
+    CUDA_TRY(cudaStreamSynchronize(b->stream));  // Af and B are host temporaries
+  }
+  s.dense_form = form;
+  return MMP_OK;
 }
 
 // Build the dense contraction form for this solve? Per sample, the register-blocked
@@ -1199,6 +1278,7 @@ size_t member_bytes(const mmp_batch* b, const Member& s) {
   off = align_up(off + std::max<size_t>(s.sr_kq.size(), 1) * sizeof(unsigned));  // their k | q << 16
   off = align_up(off + s.sr_plan.size() * sizeof(int4));                         // group plan
   off = align_up(off + (M + 1) * sizeof(int));                                   // merged terms per p
+  off = align_up(off + std::max<size_t>(s.rpairs.size(), 1) * sizeof(int4));     // slots of the REAL form
   off = align_up(off + kCounterWords * sizeof(unsigned long long));
   return off;
 }
@@ -1243,6 +1323,15 @@ int iir_len(double decay, bool fp64) {
   return n < 1e9 ? (int)std::ceil(n) : 1000000000;
 }
 
+// Does the REAL form pay? With up to 8 pair fields, one to a warp of the contraction, halving them
+// saves no pass over them (128 solves of 2 x 4096: 158 against 154 us a step); a Raman convolution
+// by transforms always has fewer rows.
+bool real_pays(size_t pairs, bool raman, const mmp_params* p) {
+  if (pairs > 8) return true;
+  std::complex<double> lam, c;
+  return raman && pairs > 1 && !fit_damped_sinusoid(p->raman_response, p->nt, lam, c);
+}
+
 // Host setup, device state and uploads for slot idx from params p; leaves the solve
 // at z = 0 with its initial fields transformed. One cudaMalloc for all of it.
 int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
@@ -1277,6 +1366,7 @@ int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
   const size_t o_skq = off; off = align_up(off + std::max<size_t>(nsr, 1) * sizeof(unsigned));
   const size_t o_splan = off; off = align_up(off + s.sr_plan.size() * sizeof(int4));
   const size_t o_soff = off; off = align_up(off + (M + 1) * sizeof(int));
+  const size_t o_rp4 = off; off = align_up(off + std::max<size_t>(s.rpairs.size(), 1) * sizeof(int4));
   const size_t o_cnt = off; off = align_up(off + kCounterWords * sizeof(unsigned long long));
   cudaError_t e = dev_malloc(&s.block, off, b->mempool, b->stream);
   if (e != cudaSuccess) {
@@ -1291,6 +1381,8 @@ int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
   d.P = (int)P;
   d.n_beta = (int)s.n_beta;
   d.raman = b->raman ? 1 : 0;
+  s.real_ok = s.symmetric && real_pays(s.pairs.size(), b->raman, p);
+  d.real = s.real_ok ? 1 : 0;  // batch_shape turns it off where the kernels chosen have no such form
   d.alpha_scale = 2 * M_PI / s.t_final;
   d.dz = s.delta_z;
   d.sgn_gamma = s.sgn_gamma;
@@ -1320,6 +1412,7 @@ int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
   d.sr_kq = (const unsigned*)T2ptr(s.block, o_skq);
   d.sr_plan = (const int4*)T2ptr(s.block, o_splan);
   d.sr_off = (const int*)T2ptr(s.block, o_soff);
+  d.rpairs = (const int4*)T2ptr(s.block, o_rp4);
   d.sr_terms = (int)nsr;
   d.sr_rounds = s.sr_rounds;
   s.counters = (unsigned long long*)T2ptr(s.block, o_cnt);
@@ -1388,36 +1481,13 @@ int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
       CUDA_TRY(cudaMemcpyAsync((void*)d.sr_kq, s.sr_kq.data(), nsr * sizeof(unsigned), cudaMemcpyHostToDevice,
                                b->stream));
     }
+    if (P) CUDA_TRY(cudaMemcpyAsync((void*)d.rpairs, s.rpairs.data(), s.rpairs.size() * sizeof(int4),
+                                    cudaMemcpyHostToDevice, b->stream));
     CUDA_TRY(cudaMemcpyAsync((void*)d.sr_off, s.sr_off.data(), (M + 1) * sizeof(int), cudaMemcpyHostToDevice,
                              b->stream));
     CUDA_TRY(cudaMemcpyAsync((void*)d.sr_plan, s.sr_plan.data(), s.sr_plan.size() * sizeof(int4),
                              cudaMemcpyHostToDevice, b->stream));
     CUDA_TRY(cudaStreamSynchronize(b->stream));  // the staging vectors are host temporaries
-  }
-  if (s.dense_ok) {
-    // A[p][q][k] += Q, A[p][q][16 + k] += Q or -Q (terms that read conj of pair field q)
-    constexpr int K = kDenseMaxModes;
-    std::vector<double> A((size_t)M * P * 2 * K, 0.0);
-    for (uint32_t p = 0; p < M; ++p)
-      for (int j = s.term_off[p]; j < s.term_off[p + 1]; ++j) {
-        const Term& t = s.terms[j];
-        const size_t q = t.pc & 0x7fff;
-        const double v = t.q;
-        A[((size_t)p * P + q) * 2 * K + t.k] += v;
-        A[((size_t)p * P + q) * 2 * K + K + t.k] += (t.pc & 0x8000) ? -v : v;
-      }
-    const size_t n = A.size();
-    if (b->fp64) {
-      CUDA_TRY(cudaMemcpyAsync((void*)d.dense_q, A.data(), n * sizeof(double), cudaMemcpyHostToDevice, b->stream));
-      CUDA_TRY(cudaStreamSynchronize(b->stream));  // A is a host temporary
-    } else {
-      std::vector<float> Af(A.begin(), A.end());
-      CUDA_TRY(cudaMemcpyAsync((void*)d.dense_q, Af.data(), n * sizeof(float), cudaMemcpyHostToDevice, b->stream));
-      const std::vector<float> B = tc_operand(A, (int)M, (int)P);
-      CUDA_TRY(cudaMemcpyAsync((void*)d.dense_tc, B.data(), B.size() * sizeof(float), cudaMemcpyHostToDevice,
-                               b->stream));
-      CUDA_TRY(cudaStreamSynchronize(b->stream));  // Af and B are host temporaries
-    }
   }
   if (b->raman) {
     // Raman spectrum: H = FFT(h_R) * dt * T0 * fR / NT  (src/MultimodePropagation_CPU.cpp:170-176, :241-251)
@@ -1458,6 +1528,8 @@ struct ShapeStats {
   int Mmax = 0, Mmin = 1 << 30, Pmax = 0, Pall = 0;
   size_t max_terms = 0, max_sr_terms = 0;
   bool iir = true, all_dense = true, any_dense = false;
+  int Smax = 0, Sall = 0;    // as Pmax and Pall, in slots (half the pair fields where real_ok)
+  bool any_real = false, all_real = true;
   double min_decay = 1e300;  // slowest Raman recurrence (where all have one: iir)
   uint32_t span = 0;
 };
@@ -1466,7 +1538,7 @@ struct ShapeStats {
 struct SolveCounts {
   int M = 0;
   size_t pairs = 0, terms = 0, sr_terms = 0;
-  bool iir = false, dense_ok = false;
+  bool iir = false, dense_ok = false, real_ok = false;
   double iir_decay = 0;
 };
 
@@ -1474,6 +1546,11 @@ void add_stats(ShapeStats& st, const mmp_batch* b, const SolveCounts& c, uint32_
   st.iir = st.iir && c.iir;
   st.min_decay = std::min(st.min_decay, c.iir_decay);
   st.all_dense = st.all_dense && c.dense_ok;
+  st.any_real = st.any_real || c.real_ok;
+  st.all_real = st.all_real && c.real_ok;
+  const int slots = c.real_ok ? slot_count<true>((int)c.pairs) : (int)c.pairs;
+  st.Smax = std::max(st.Smax, b->raman ? slots : 0);
+  st.Sall = std::max(st.Sall, slots);
   st.any_dense = st.any_dense || c.dense_ok;
   st.span = std::max(st.span, span);
   st.Mmax = std::max(st.Mmax, c.M);
@@ -1492,6 +1569,7 @@ SolveCounts member_counts(const Member& s) {
   c.sr_terms = s.sr_kq.size();
   c.iir = s.desc.iir != 0;
   c.iir_decay = s.iir_decay;
+  c.real_ok = s.real_ok;
   c.dense_ok = s.dense_ok;
   return c;
 }
@@ -1507,7 +1585,8 @@ ShapeStats batch_stats(const mmp_batch* b) {
 // memory they take, chosen from its statistics alone.
 struct Shape {
   int Mmax = 0, Pmax = 0, TT = 32, dense = 0, pchunk = 0, stage_terms = 0;
-  bool tc = false, sr = false, sp = false, fused = false, iir = false, lookback = false;
+  bool tc = false, sr = false, sp = false, fused = false, iir = false, lookback = false, real = false;
+  int slots = 0;
   size_t smem = 0, sp_smem = 0;
   uint32_t span = 0;
 };
@@ -1516,12 +1595,17 @@ struct Shape {
 bool same_kernels(const Shape& x, const Shape& y) {
   return x.TT == y.TT && x.dense == y.dense && x.pchunk == y.pchunk && x.stage_terms == y.stage_terms &&
          x.tc == y.tc && x.sr == y.sr && x.fused == y.fused && x.iir == y.iir && x.lookback == y.lookback &&
-         x.sp == y.sp;
+         x.sp == y.sp && x.real == y.real;
 }
 
-Shape choose_shape(const mmp_batch* b, const ShapeStats& st) {
+Shape choose_shape(const mmp_batch* b, const ShapeStats& st, bool try_real = true) {
   const size_t t2 = b->fp64 ? sizeof(double2) : sizeof(float2);
-  const int Mmax = st.Mmax, Pmax = st.Pmax, Pall = st.Pall, Mmin = st.Mmin;
+  // The REAL form for the solves whose coupling allows it, where the kernels chosen below have it
+  // (else chosen again without). MMP_REAL_PAIRS=0 keeps the general form.
+  bool real = try_real && st.any_real && st.span > 0;
+  if (const char* env = std::getenv("MMP_REAL_PAIRS"))
+    if (std::atoi(env) == 0) real = false;
+  const int Mmax = st.Mmax, Pmax = real ? st.Smax : st.Pmax, Pall = real ? st.Sall : st.Pall, Mmin = st.Mmin;
   const uint32_t span = st.span;
   const size_t max_terms = st.max_terms, max_sr_terms = st.max_sr_terms;
   bool iir = b->raman && st.iir;
@@ -1562,7 +1646,7 @@ Shape choose_shape(const mmp_batch* b, const ShapeStats& st) {
     fused = b->raman;
     dense = 1;
     smem = ((size_t)Mmax * TT + (b->raman ? 2 * (size_t)Pmax : 0)) * sizeof(float2) +
-           kTcStages * 4 * (size_t)kTcChunk * (TT + 16 * (size_t)Mmax) * sizeof(float) +  // operand stages
+           kTcStages * (real && st.all_real ? 2 : 4) * (size_t)kTcChunk * (TT + 16 * (size_t)Mmax) * sizeof(float) +  // operand stages
            1024;                                                                          // their alignment
   } else if (dense) {
     smem += 8 * 2 * (size_t)kDenseChunk * 2 * kDenseMaxModes * (t2 / 2);  // staged coefficient rows
@@ -1598,9 +1682,9 @@ Shape choose_shape(const mmp_batch* b, const ShapeStats& st) {
   // recurrence fused): the serial-recurrence contraction in sub-blocks of kSrSub samples
   // (k_contract_sr, tiles of up to 256 samples) when its shared memory fits, in place of the
   // pair-chunked one. MMP_CONTRACT_SR=0 keeps the latter.
-  bool sr = false;
+  bool sr = false, tall = false;
   {
-    const bool tall = (size_t)rows * 64 * t2 > 100 * 1024;
+    tall = (size_t)(Mmax + st.Pall) * 64 * t2 > 100 * 1024;  // in the general form
     bool ok = tall && span > 0 && !any_dense && Mmax <= kSrMaxModes &&
               Pall <= kSrPairsPerThread * kSrThreads && (!b->raman || iir) && (int)b->nt >= kSrSub * 4;
     if (const char* env = std::getenv("MMP_CONTRACT_SR"))
@@ -1630,11 +1714,16 @@ Shape choose_shape(const mmp_batch* b, const ShapeStats& st) {
   bool sp = !tc && !sr && !pchunk && dense != 1 && TT >= 64 && sp_smem <= 200 * 1024;
   if (const char* env = std::getenv("MMP_CONTRACT_SP"))
     if (std::atoi(env) == 0) sp = false;
+  if (real && (!(tc || sr || sp || dense == 1) || (dense == 2 && !sp) || (tall && !sr) ||
+               (b->raman && !fused && (iir || dense))))  // k_raman_scan, and R rows for the dense form
+    return choose_shape(b, st, false);
   const int stage_terms = sr || (sp && !dense) ? 0 : (pchunk ? 1 : (dense != 1 && !tc && smem + max_terms * staged <= 200 * 1024 ? 1 : 0));
   if (stage_terms && !pchunk) smem += max_terms * staged;
   Shape sh;
   sh.Mmax = Mmax;
-  sh.Pmax = Pmax;
+  sh.Pmax = st.Pmax;
+  sh.slots = Pmax;
+  sh.real = real;
   sh.TT = TT;
   sh.dense = dense;
   sh.pchunk = pchunk;
@@ -1670,6 +1759,7 @@ SolveCounts solve_counts(const mmp_params* p) {
     if (c.iir) c.iir_decay = -std::log(std::abs(lam));
   }
   c.dense_ok = dense_wanted(nullptr, m);
+  c.real_ok = m.symmetric && real_pays(m.pairs.size(), p->raman != 0, p);
   return c;
 }
 
@@ -1697,7 +1787,8 @@ int row_split(bool fp64, int logn, int rows) {
   return xc;
 }
 
-bool batch_shape(mmp_batch* b) {
+// Take the shape the batch's solves lead to (a captured graph of another is dropped).
+int batch_shape(mmp_batch* b) {
   const Shape sh = choose_shape(b, batch_stats(b));
   const int xc = b->xc_req >= 0 ? b->xc_req : row_split(b->fp64, b->logn, sh.Mmax * (int)sh.span);
   const bool resplit = xc != b->ks.xc;
@@ -1706,7 +1797,7 @@ bool batch_shape(mmp_batch* b) {
                        sh.stage_terms != b->stage_terms || sh.span != b->span || sh.iir != b->raman_iir ||
                        sh.fused != b->raman_fused || sh.dense != b->dense || sh.tc != b->tc ||
                        sh.pchunk != b->pchunk || sh.sr != b->sr || sh.lookback != b->lookback || sh.sp != b->sp ||
-                       sh.sp_smem != b->sp_smem;
+                       sh.sp_smem != b->sp_smem || sh.real != b->real || sh.slots != b->slots;
   b->dense = sh.dense;
   b->tc = sh.tc;
   b->pchunk = sh.pchunk;
@@ -1715,20 +1806,35 @@ bool batch_shape(mmp_batch* b) {
   b->raman_fused = sh.fused;
   b->lookback = sh.lookback;
   b->sp = sh.sp;
+  b->real = sh.real;
+  b->slots = sh.slots;
   b->sp_smem = sh.sp_smem;
-  b->kernels_per_step = b->tab.s * ((b->raman ? (sh.fused && !sh.lookback ? 2 : 1) : 0) + 2 + (sh.dense == 2 ? 1 : 0));
+  const bool had[2] = {b->forms[0], b->forms[1]};
+  b->forms[0] = b->forms[1] = false;
   b->span = sh.span;
   b->Mmax = sh.Mmax;
   b->Pmax = sh.Pmax;
   b->TT = sh.TT;
   b->contract_smem = sh.smem;
   b->stage_terms = sh.stage_terms;
-  if (changed && b->graph) {
+  bool redo = false;
+  for (size_t i = 0; i < b->members.size(); ++i) {
+    if (!b->active[i]) continue;
+    Member& s = b->members[i];
+    const int form = b->real && s.real_ok ? 1 : 0;
+    redo = redo || s.desc.real != form;
+    s.desc.real = form;
+    b->forms[form] = true;
+    if (int rc = upload_dense(b, s)) return rc;
+  }
+  const bool forms_changed = had[0] != b->forms[0] || had[1] != b->forms[1];
+  if ((changed || forms_changed) && b->graph) {
     cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
     b->graph_steps = 0;
   }
-  return changed;
+  b->kernels_per_step = step_kernels(b);
+  return redo ? upload_desc(b) : MMP_OK;
 }
 
 // ---- autotuner -------------------------------------------------------------------------
@@ -1817,10 +1923,12 @@ int autotune(mmp_batch* b, const mmp_params* const* params) {
     if (*env) tiles = {std::atoi(env)};
   if (const char* env = std::getenv("MMP_GROUPS"))
     if (*env) gs = {std::max(1, std::atoi(env))};
+  int rc = MMP_OK;
   auto apply = [&](const TuneChoice& c) {
     b->xc_req = c.xc;
     b->tile_req = c.tile;
-    batch_shape(b);
+    const int e = batch_shape(b);
+    if (rc == MMP_OK) rc = e;
     b->groups = (uint32_t)c.groups;
   };
   TuneChoice c;
@@ -1830,11 +1938,11 @@ int autotune(mmp_batch* b, const mmp_params* const* params) {
   b->tuned = 0;
   if (b->span < 2 || (xcs.size() == 1 && tiles.size() == 1 && gs.size() == 1)) {
     apply(c);
-    return MMP_OK;
+    return rc;
   }
   std::vector<int> key = {b->device, b->fp64 ? 1 : 0, b->logn, b->tab.s, b->Mmax, b->Pmax,
                           (int)b->span, b->raman ? 1 : 0, b->tc ? 1 : 0, b->sr ? 1 : 0,
-                          b->pchunk ? 1 : 0, b->dense, -1};
+                          b->pchunk ? 1 : 0, b->dense, (b->forms[0] ? 1 : 0) + (b->forms[1] ? 2 : 0), -1};
   for (const std::vector<int>* v : {&xcs, &tiles, &gs}) {
     key.insert(key.end(), v->begin(), v->end());
     key.push_back(-1);
@@ -1845,11 +1953,10 @@ int autotune(mmp_batch* b, const mmp_params* const* params) {
     if (it != g_tune_cache.end()) {
       apply(it->second);
       b->tuned = 1;
-      return MMP_OK;
+      return rc;
     }
   }
   const uint64_t counted = g_launches.load();
-  int rc = MMP_OK;
   auto sweep = [&](int TuneChoice::*field, const std::vector<int>& vals) {
     if (vals.size() < 2 || rc) return;
     float best = 0.f;
@@ -1859,7 +1966,7 @@ int autotune(mmp_batch* b, const mmp_params* const* params) {
       t.*field = vals[i];
       apply(t);
       float ms = 0.f;
-      rc = time_steps(b, 3, &ms);
+      if (rc == MMP_OK) rc = time_steps(b, 3, &ms);
       if (rc == MMP_OK && (i == 0 || ms < best)) {
         best = ms;
         pick = vals[i];
@@ -1903,10 +2010,8 @@ int create_batch(const mmp_params* const* params, uint32_t n, mmp_batch** out) {
     if (!same_shape(b, params[i]))
       rc = fail(MMP_EINVAL, "batch members must share nt, precision, raman and the RK tableau");
   for (uint32_t i = 0; i < n && rc == MMP_OK; ++i) rc = member_init(b, i, params[i]);
-  if (rc == MMP_OK) {
-    batch_shape(b);
-    rc = autotune(b, params);
-  }
+  if (rc == MMP_OK) rc = batch_shape(b);
+  if (rc == MMP_OK) rc = autotune(b, params);
   if (rc == MMP_OK) {
     cudaError_t e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) rc = fail(MMP_ECUDA, cudaGetErrorString(e));

@@ -234,6 +234,21 @@ __device__ __forceinline__ double2 pk_fma(double2 a, double2 b, double2 c) {
 }
 __device__ __forceinline__ double2 pk_mul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
 
+// The U rows a slot reads, and its value from their samples (common.cuh: V_q, or the
+// real parts of two fields).
+template <bool REAL> __device__ __forceinline__ int4 slot_rows(const SolveDesc& d, int s) {
+  if constexpr (REAL) return __ldg(d.rpairs + s);
+  const int2 lm = __ldg(d.pairs + s);
+  return make_int4(lm.x, lm.y, 0, 0);
+}
+template <bool REAL, typename V> __device__ __forceinline__ V slot_value(V l0, V m0, V l1, V m1) {
+  if constexpr (!REAL) return cmulc(l0, m0);
+  V r;
+  r.x = fma(l0.x, m0.x, l0.y * m0.y);
+  r.y = fma(l1.x, m1.x, l1.y * m1.y);
+  return r;
+}
+
 // ---- k_prime: U for stage 0 from psi_hat --------------------------------------------------
 template <typename T, int LOGN, int XC>
 __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_BLOCKS) k_prime(const KParams kp) {
@@ -279,14 +294,15 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
 }
 
 // ---- k_pair: R_q = IFFT(FFT(V_q) * H), V_q = U_l conj(U_m) -------------------------------
-template <typename T, int LOGN, int XC>
+// One slot per row; the REAL form stores R's two fields as two real rows.
+template <typename T, int LOGN, int XC, bool REAL>
 __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_BLOCKS) k_pair(const KParams kp) {
   using Gm = Geo<T, LOGN, XC>;
   using V = c2<T>;
   MMP_ROW_SETUP();
   const SolveDesc* gd = kp.descs + blockIdx.y;
   const int q = blockIdx.x / Gm::C;
-  if (q >= __ldg(&gd->P)) {  // uniform over the cluster
+  if (q >= slot_count<REAL>(__ldg(&gd->P)) || __ldg(&gd->real) != REAL) {  // other form; uniform over the cluster
     grid_sync_wait();
     return;
   }
@@ -294,7 +310,7 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
   const V* U = as_t2<T>(static_cast<const void*>(ldg_ptr(&gd->U))) + i0;
   const V* H = as_t2<T>(static_cast<const void*>(ldg_ptr(&gd->H)));
   V* W = as_t2<T>(ldg_ptr(&gd->W));
-  const int2 lm = __ldg(ldg_ptr(&gd->pairs) + q);
+  const int4 lm = slot_rows<REAL>(*gd, q);
   grid_sync_wait();
   if (__ldcg(step) >= __ldg(&gd->step_limit)) return;  // uniform over the cluster
   row_enter<Gm>();
@@ -303,8 +319,13 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
   {
     const V* Ul = U + (size_t)lm.x * Gm::N;
     const V* Um = U + (size_t)lm.y * Gm::N;
+    const V* Ul1 = U + (size_t)lm.z * Gm::N;
+    const V* Um1 = U + (size_t)lm.w * Gm::N;
 #pragma unroll
-    for (int r = 0; r < Gm::E; ++r) v[r] = cmulc(ld_stream(Ul + r * Gm::B), ld_stream(Um + r * Gm::B));
+    for (int r = 0; r < Gm::E; ++r) {
+      const V l1 = REAL ? ld_stream(Ul1 + r * Gm::B) : V(), m1 = REAL ? ld_stream(Um1 + r * Gm::B) : V();
+      v[r] = slot_value<REAL>(ld_stream(Ul + r * Gm::B), ld_stream(Um + r * Gm::B), l1, m1);
+    }
   }
   row_first<Gm>(v, s, tw, rank);
   rows_fwd<Gm>(sr, tw, u);
@@ -325,9 +346,18 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
   row_last_inv<Gm>(v, s, tw, rank);
   // R_q = (H_R conv V_q); the Kerr part (1 - fR) V_q is formed by the contraction from
   // the U tile it already holds
-  V* R = W + (size_t)q * Gm::N + i0;
+  if constexpr (REAL) {
+    T* R = reinterpret_cast<T*>(W) + (size_t)(2 * q) * Gm::N + i0;
 #pragma unroll
-  for (int r = 0; r < Gm::E; ++r) R[r * Gm::B] = v[r];
+    for (int r = 0; r < Gm::E; ++r) {
+      R[r * Gm::B] = v[r].x;
+      R[Gm::N + r * Gm::B] = v[r].y;
+    }
+  } else {
+    V* R = W + (size_t)q * Gm::N + i0;
+#pragma unroll
+    for (int r = 0; r < Gm::E; ++r) R[r * Gm::B] = v[r];
+  }
   row_leave<Gm>();
 }
 
@@ -1028,7 +1058,7 @@ template <typename T> struct TileScan {
 // distinct banks per quarter warp; mask 0 is the plain layout.
 __device__ __forceinline__ int wsw(int h, int mask) { return h ^ ((h >> 3) & mask); }
 
-// The state entering tile `tile` for idx = 2 q (Re V of pair field q) or 2 q + 1 (Im V).
+// The state entering tile `tile` for idx = 2 s (real part of slot s) or 2 s + 1 (imaginary part).
 // look = 0: k_raman_carry has left it in the aggregates' place. Else it is summed here from the
 // aggregates of the `look` tiles before (around the period),
 //   C = sum_{i=1..look} lambda^(TT (i-1)) A_{tile-i}     [times 1 / (1 - lambda^NT) over a whole row],
@@ -1038,12 +1068,12 @@ __device__ __forceinline__ int wsw(int h, int mask) { return h ^ ((h >> 3) & mas
 // 28-mode order-6 solves 6450 -> 6394.
 // The aggregates lie [tile][q][2] for that, and [q][tile][2] where k_raman_carry scans them.
 template <typename T>
-__device__ __forceinline__ c2<T> tile_carry(const SolveDesc& d, int ntiles, int tile, int idx, int look,
+__device__ __forceinline__ c2<T> tile_carry(const SolveDesc& d, int slots, int ntiles, int tile, int idx, int look,
                                             double2 lamT) {
   using V = c2<T>;
   const V* tiles = as_t2<T>(static_cast<const void*>(d.raman_tiles));
   if (look == 0) return __ldcg(tiles + ((size_t)(idx >> 1) * ntiles + tile) * 2 + (idx & 1));
-  const size_t P2 = 2 * (size_t)d.P;
+  const size_t P2 = 2 * (size_t)slots;
   tiles += idx;
   double2 c = make_double2(0.0, 0.0);
   for (int i0 = look; i0 > 0; i0 -= 4) {  // the farthest first, four loads in flight
@@ -1066,52 +1096,41 @@ __device__ __forceinline__ int tile_look(const SolveDesc& d, int ntiles, int TT,
   return raman_mode == 3 ? min((d.iir_len + TT - 1) / TT, ntiles) : 0;
 }
 
-// The states entering tile `tile` for pair fields 0..P-1 into shared memory, [q][Re V, Im V];
-// published by the caller's next barrier.
+// The states entering tile `tile` for every slot into shared memory, [s][2]; published by the
+// caller's next barrier.
 template <typename T>
-__device__ __forceinline__ void stage_tile_carries(c2<T>* sC, const SolveDesc& d, int P, int ntiles, int tile,
+__device__ __forceinline__ void stage_tile_carries(c2<T>* sC, const SolveDesc& d, int slots, int ntiles, int tile,
                                                    int look, double2 lamT) {
-  for (int i = threadIdx.x; i < 2 * P; i += blockDim.x) sC[i] = tile_carry<T>(d, ntiles, tile, i, look, lamT);
+  for (int i = threadIdx.x; i < 2 * slots; i += blockDim.x) sC[i] = tile_carry<T>(d, slots, ntiles, tile, i, look, lamT);
 }
 
 // The recurrence through one pair field of a contraction tile, by one warp (TT = 32 c
 // samples, 64 <= TT <= 256): V = U_l conj(U_m) is written coalesced to row (pair positions
 // swizzled by wmask), each lane takes its c samples into registers, the lanes' aggregates
 // are scanned, every lane runs the recurrence from the state entering it (carry[0..1]: the
-// states entering the tile for Re V and Im V) and hands W = (1 - f_R) V + R for its samples
-// c lane .. c lane + c - 1 to fin(x) (tile_pair_recurrence: back into row, in place). With
-// DIRECT each lane forms V for its own samples straight from U (row unused).
-template <typename T, bool DIRECT = false, typename Fin>
-__device__ __forceinline__ void tile_pair_recurrence_to(const TileScan<T>& ts, const c2<T>* sU, int TT, int2 lm,
-                                                        c2<T>* row, int wmask, const c2<T>* carry, T kerr,
-                                                        int lane, Fin&& fin) {
+// states entering the tile for Re V and Im V) and writes W = (1 - f_R) V + R for its samples
+// c lane .. c lane + c - 1 back into row, in place. One slot (REAL: two pair fields).
+template <typename T, bool REAL>
+__device__ __forceinline__ void tile_pair_recurrence(const TileScan<T>& ts, const c2<T>* sU, int TT, int4 lm,
+                                                     c2<T>* row, int wmask, const c2<T>* carry, T kerr, int lane) {
   using V = c2<T>;
   const int H = TT >> 1, c = ts.c, g = c >> 1;
   V x[8];
-  if constexpr (!DIRECT) {
-    // V = U_l conj(U_m), coalesced over the sample pairs, then each lane's own samples
-    for (int h = lane; h < H; h += 32) {
-      V ul0, ul1, um0, um1;
-      ld2<T>(sU + lm.x * TT + 2 * h, ul0, ul1);
-      ld2<T>(sU + lm.y * TT + 2 * h, um0, um1);
-      st2<T>(row + 2 * wsw(h, wmask), cmulc(ul0, um0), cmulc(ul1, um1));
+  // V = U_l conj(U_m), coalesced over the sample pairs, then each lane's own samples
+  for (int h = lane; h < H; h += 32) {
+    V ul0, ul1, um0, um1, vl0 = {}, vl1 = {}, vm0 = {}, vm1 = {};
+    ld2<T>(sU + lm.x * TT + 2 * h, ul0, ul1);
+    ld2<T>(sU + lm.y * TT + 2 * h, um0, um1);
+    if constexpr (REAL) {
+      ld2<T>(sU + lm.z * TT + 2 * h, vl0, vl1);
+      ld2<T>(sU + lm.w * TT + 2 * h, vm0, vm1);
     }
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (j < g) ld2<T>(row + 2 * wsw(g * lane + j, wmask), x[2 * j], x[2 * j + 1]);
-  } else {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (j < g) {
-        V ul0, ul1, um0, um1;
-        ld2<T>(sU + lm.x * TT + 2 * (g * lane + j), ul0, ul1);
-        ld2<T>(sU + lm.y * TT + 2 * (g * lane + j), um0, um1);
-        x[2 * j] = cmulc(ul0, um0);
-        x[2 * j + 1] = cmulc(ul1, um1);
-      }
-    }
+    st2<T>(row + 2 * wsw(h, wmask), slot_value<REAL>(ul0, um0, vl0, vm0), slot_value<REAL>(ul1, um1, vl1, vm1));
   }
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (j < g) ld2<T>(row + 2 * wsw(g * lane + j, wmask), x[2 * j], x[2 * j + 1]);
   // this lane's aggregate from a zero start: sum_k lambda^(c-1-k) x_k, x_k = Re or Im V
   V la = mk<T>(0, 0), lb = mk<T>(0, 0);
 #pragma unroll
@@ -1141,21 +1160,12 @@ __device__ __forceinline__ void tile_pair_recurrence_to(const TileScan<T>& ts, c
                    fma(kerr, x[k].y, fma(ts.kt.x, sb.y, ts.kt.y * sb.x)));
     }
   }
-  fin(x);
-}
-template <typename T>
-__device__ __forceinline__ void tile_pair_recurrence(const TileScan<T>& ts, const c2<T>* sU, int TT, int2 lm,
-                                                     c2<T>* row, int wmask, const c2<T>* carry, T kerr,
-                                                     int lane) {
-  const int g = ts.c >> 1;
-  tile_pair_recurrence_to<T>(ts, sU, TT, lm, row, wmask, carry, kerr, lane, [&](const c2<T>* x) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (j < g) st2<T>(row + 2 * wsw(g * lane + j, wmask), x[2 * j], x[2 * j + 1]);
-  });
+  for (int j = 0; j < 4; ++j)
+    if (j < g) st2<T>(row + 2 * wsw(g * lane + j, wmask), x[2 * j], x[2 * j + 1]);
 }
 
-// k_raman_agg: the recurrence's aggregate over a tile from a zero start, for every pair field, as
+// k_raman_agg: the recurrence's aggregate over a tile from a zero start, for every slot, as
 // a weighted sum,
 //   S_end = sum_t lambda^(TT-1-t) x_t   (x = Re or Im of U_l conj(U_m)),
 // so it needs no sequential pass. A warp takes a field at a time: each lane sums its sample pairs
@@ -1163,21 +1173,20 @@ __device__ __forceinline__ void tile_pair_recurrence(const TileScan<T>& ts, cons
 // four sums are added by halving (each exchange hands over half of what a lane holds: 6
 // shuffles for the four). What bounds it: the latency of the tile's copy, then issue. Measured
 // on a B200, 32 solves of 6 x 16384, against weights read per field and 20 shuffles: 21 -> 18 us.
-template <typename T>
+template <typename T, bool REAL>
 __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 5 : 3)) k_raman_agg(const SolveDesc* __restrict__ descs, int nt, int TT, int by_tile) {
   using V = c2<T>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const SolveDesc& d = descs[blockIdx.y];
   const int tile = blockIdx.x, t0 = tile * TT;
-  if (t0 >= nt || d.M == 0) {  // empty slot
+  if (t0 >= nt || d.M == 0 || d.real != REAL) {  // empty slot, other form
     grid_sync_wait();
     return;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int M = d.M, P = d.P;
+  const int M = d.M, P = slot_count<REAL>(d.P);
   V* sU = reinterpret_cast<V*>(smem_raw);  // [M][TT]
   const V* U = as_t2<T>(d.U) + t0;
-  const int2* pairs = d.pairs;
   V w0[4], w1[4];  // the weights of the lane's pairs
   {
     const V* pw = static_cast<const V*>(d.raman_pow) + TT - 2;
@@ -1205,17 +1214,23 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 5 : 3)) k_raman_agg(con
   T* out = static_cast<T*>(d.raman_tiles) + (size_t)tile * (by_tile ? 4 * P : 4);
   const size_t sq = by_tile ? 4 : 4 * (size_t)(nt / TT);
   for (int q = warp; q < P; q += nwarps) {
-    const int2 lm = __ldg(pairs + q);
+    const int4 lm = slot_rows<REAL>(d, q);
     const V* ul = sU + lm.x * TT + 2 * lane;
     const V* um = sU + lm.y * TT + 2 * lane;
+    const V* vl = sU + lm.z * TT + 2 * lane;
+    const V* vm = sU + lm.w * TT + 2 * lane;
     V sr = mk<T>(0, 0), si = mk<T>(0, 0);  // Re and Im of the sums for (Re V, Im V)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if (j < (TT >> 6)) {
-        V ul0, ul1, um0, um1;
+        V ul0, ul1, um0, um1, vl0 = {}, vl1 = {}, vm0 = {}, vm1 = {};
         ld2<T>(ul + 64 * j, ul0, ul1);
         ld2<T>(um + 64 * j, um0, um1);
-        const V x0 = cmulc(ul0, um0), x1 = cmulc(ul1, um1);
+        if constexpr (REAL) {
+          ld2<T>(vl + 64 * j, vl0, vl1);
+          ld2<T>(vm + 64 * j, vm0, vm1);
+        }
+        const V x0 = slot_value<REAL>(ul0, um0, vl0, vm0), x1 = slot_value<REAL>(ul1, um1, vl1, vm1);
         sr = pk_fma(mk<T>(w0[j].x, w0[j].x), x0, pk_fma(mk<T>(w1[j].x, w1[j].x), x1, sr));
         si = pk_fma(mk<T>(w0[j].y, w0[j].y), x0, pk_fma(mk<T>(w1[j].y, w1[j].y), x1, si));
       }
@@ -1245,7 +1260,7 @@ __global__ void __launch_bounds__(32) k_raman_carry(const SolveDesc* __restrict_
   const double2 lamT = lambda_tile(d, TT);
   grid_sync_wait();
   grid_release();
-  if (q >= d.P || d.M == 0 || __ldcg(d.step) >= d.step_limit) return;
+  if (q >= (d.real ? slot_count<true>(d.P) : d.P) || d.M == 0 || __ldcg(d.step) >= d.step_limit) return;
   V* tiles = as_t2<T>(d.raman_tiles) + (size_t)q * ntiles * 2;
   Affine mine = affine_identity();
   for (int i = first; i < last; ++i) {
@@ -1325,7 +1340,7 @@ template <typename T, int DENSE> constexpr int contract_min_blocks() {
 // one warp per (p, 64 samples), each lane two samples with all k in registers: a
 // register-blocked matrix product instead of one complex triple product per term.
 // mixed: the batch holds solves of both forms; each kernel skips the other's.
-template <typename T, int DENSE>
+template <typename T, int DENSE, bool REAL>
 __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_contract(const SolveDesc* __restrict__ descs, int nt, int TT,
                                                   int stage_terms, int raman_mode, int mixed) {
   using V = c2<T>;
@@ -1335,13 +1350,14 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
   V* sU = reinterpret_cast<V*>(smem_raw);
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TT;
-  if (t0 >= nt || d.M == 0 || (mixed && (d.dense_q != nullptr) != (DENSE == 1))) {  // empty slot, other form
+  if (t0 >= nt || d.M == 0 || d.real != REAL || (mixed && (d.dense_q != nullptr) != (DENSE == 1))) {  // empty slot, other form
     grid_sync_wait();
     return;
   }
   const int M = d.M;
   const int raman = raman_mode;
-  const int P = d.P;                          // pair fields formed in this tile
+  static_assert(DENSE == 1 || !REAL, "the term loop reads complex pair fields");
+  const int P = slot_count<REAL>(d.P);        // slots formed in this tile
   const int Pl = raman == 1 ? P : 0;          // pair rows loaded (Raman convolutions)
   const V* U = as_t2<T>(d.U);
   const V* R = as_t2<T>(d.W);
@@ -1395,11 +1411,15 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
   if (raman < 2) {  // two samples per thread
     for (int idx = threadIdx.x; idx < P * H; idx += blockDim.x) {
       const int q = idx / H, tt = 2 * (idx - q * H);
-      const int2 lm = d.pairs[q];
-      V ul0, ul1, um0, um1;
+      const int4 lm = slot_rows<REAL>(d, q);
+      V ul0, ul1, um0, um1, vl0 = {}, vl1 = {}, vm0 = {}, vm1 = {};
       ld2<T>(sU + lm.x * TT + tt, ul0, ul1);
       ld2<T>(sU + lm.y * TT + tt, um0, um1);
-      V w0 = cmulc(ul0, um0), w1 = cmulc(ul1, um1);
+      if constexpr (REAL) {
+        ld2<T>(sU + lm.z * TT + tt, vl0, vl1);
+        ld2<T>(sU + lm.w * TT + tt, vm0, vm1);
+      }
+      V w0 = slot_value<REAL>(ul0, um0, vl0, vm0), w1 = slot_value<REAL>(ul1, um1, vl1, vm1);
       if (raman) {
         V r0, r1;
         ld2<T>(sW + q * TT + tt, r0, r1);
@@ -1413,7 +1433,7 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
     TileScan<T> ts;
     ts.init(d, TT >> 5, lane);
     for (int q = warp; q < P; q += nwarps)
-      tile_pair_recurrence<T>(ts, sU, TT, d.pairs[q], sW + (size_t)q * TT, wmask, sC + 2 * q, kerr, lane);
+      tile_pair_recurrence<T, REAL>(ts, sU, TT, slot_rows<REAL>(d, q), sW + (size_t)q * TT, wmask, sC + 2 * q, kerr, lane);
   }
   __syncthreads();
   grid_release();
@@ -1468,8 +1488,13 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
           for (int k = 0; k < K; ++k) {
             re0[k] = fma(ar[k], w0.x, re0[k]);
             re1[k] = fma(ar[k], w1.x, re1[k]);
-            im0[k] = fma(ai[k], w0.y, im0[k]);
-            im1[k] = fma(ai[k], w1.y, im1[k]);
+            if constexpr (REAL) {  // the slot's second field
+              re0[k] = fma(ai[k], w0.y, re0[k]);
+              re1[k] = fma(ai[k], w1.y, re1[k]);
+            } else {
+              im0[k] = fma(ai[k], w0.y, im0[k]);
+              im1[k] = fma(ai[k], w1.y, im1[k]);
+            }
           }
         }
         __syncwarp();  // reads of buffer c & 1 done before chunk c + 2 is staged into it
@@ -1480,10 +1505,17 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
         if (k < M) {
           V u0, u1;
           ld2<T>(sU + k * TT + tt, u0, u1);
-          sx0 = fma(u0.x, re0[k], fma(-u0.y, im0[k], sx0));
-          sy0 = fma(u0.x, im0[k], fma(u0.y, re0[k], sy0));
-          sx1 = fma(u1.x, re1[k], fma(-u1.y, im1[k], sx1));
-          sy1 = fma(u1.x, im1[k], fma(u1.y, re1[k], sy1));
+          if constexpr (REAL) {
+            sx0 = fma(u0.x, re0[k], sx0);
+            sy0 = fma(u0.y, re0[k], sy0);
+            sx1 = fma(u1.x, re1[k], sx1);
+            sy1 = fma(u1.y, re1[k], sy1);
+          } else {
+            sx0 = fma(u0.x, re0[k], fma(-u0.y, im0[k], sx0));
+            sy0 = fma(u0.x, im0[k], fma(u0.y, re0[k], sy0));
+            sx1 = fma(u1.x, re1[k], fma(-u1.y, im1[k], sx1));
+            sy1 = fma(u1.x, im1[k], fma(u1.y, re1[k], sy1));
+          }
         }
       }
       st2<T>(sigma + (size_t)p * nt + t0 + tt, mk<T>(sx0, sy0), mk<T>(sx1, sy1));
@@ -1594,7 +1626,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2)) k_contract_pc(c
   for (int c0 = 0; c0 < P; c0 += pc) {
     const int c1 = min(P, c0 + pc);
     for (int q = c0 + warp; q < c1; q += nwarps)
-      tile_pair_recurrence<T>(ts, sU, TT, d.pairs[q], sW + (size_t)(q - c0) * TT, wmask, sC + 2 * q, kerr, lane);
+      tile_pair_recurrence<T, false>(ts, sU, TT, slot_rows<false>(d, q), sW + (size_t)(q - c0) * TT, wmask, sC + 2 * q, kerr, lane);
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < kPcItems; ++i) {
@@ -1718,7 +1750,7 @@ template <typename V> __device__ __forceinline__ V shfl_down_c(V v, int d) {
 
 // raman_mode: 0 Raman off, 2 the recurrence from the tile carries of k_raman_carry (tiles of TB), 3 from
 // carries summed here (tile_carry)
-template <typename T>
+template <typename T, bool REAL>
 __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
     k_contract_sr(const SolveDesc* __restrict__ descs, int nt, int TB, int raman_mode) {
   using V = c2<T>;
@@ -1730,16 +1762,19 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TB;
-  if (t0 >= nt || d.M == 0) {  // empty slot
+  if (t0 >= nt || d.M == 0 || d.real != REAL) {  // empty slot, other form
     grid_sync_wait();
     return;
   }
-  const int M = d.M, P = d.P, nterm = d.sr_terms, rounds = d.sr_rounds;
+  const int M = d.M, P = slot_count<REAL>(d.P), nterm = d.sr_terms, rounds = d.sr_rounds;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // shared memory: U [2][M][RS], W [P][RS], group plan [rounds kSrGroups], merged terms
-  // [nterm] (coefficients and q | k << 16)
+  // shared memory: U [2][M][RS], W [P][RS] (REAL: two planes [P][RS] of sample pairs, the slots'
+  // first and second fields, so that a quarter warp's rows stay on different banks), group
+  // plan [rounds kSrGroups], merged terms [nterm] (coefficients and q | k << 16)
   SP* sU = reinterpret_cast<SP*>(smem_raw);
   SP* sW = sU + 2 * (size_t)M * RS;
+  V* sW0 = reinterpret_cast<V*>(sW);
+  V* sW1 = sW0 + (size_t)P * RS;
   int4* sPlan = reinterpret_cast<int4*>(sW + (size_t)P * RS);
   SrRec<T>* sRec = reinterpret_cast<SrRec<T>*>(sPlan + rounds * kSrGroups);
   {
@@ -1748,6 +1783,10 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
       SrRec<T> r = {};
       r.ab = gCf[i];
       r.kq = d.sr_kq[i];
+      if constexpr (REAL) {  // the pair field's plane and row as one position
+        const unsigned q = r.kq & 0xffffu;
+        r.kq = (r.kq & 0xffff0000u) | ((q & 1u) * P + (q >> 1)) * RS;
+      }
       sRec[i] = r;
     }
     for (int i = tid; i < rounds * kSrGroups; i += kSrThreads) sPlan[i] = d.sr_plan[i];
@@ -1783,21 +1822,19 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
   };
   // phase A: this thread's pair fields and their recurrence states, packed as
   // sr = (Re S_a, Re S_b), si = (Im S_a, Im S_b) (S_a for Re V, S_b for Im V)
-  int pl[kSrPairsPerThread], pm[kSrPairsPerThread];
+  int4 lm[kSrPairsPerThread];
   V sr[kSrPairsPerThread], si[kSrPairsPerThread];
   const int ntiles = nt / TB, look = tile_look(d, ntiles, TB, raman_mode);
 #pragma unroll
   for (int i = 0; i < kSrPairsPerThread; ++i) {
     const int q = tid + i * kSrThreads;
-    pl[i] = pm[i] = 0;
+    lm[i] = make_int4(0, 0, 0, 0);
     sr[i] = si[i] = mk<T>(0, 0);
     if (q < P) {
-      const int2 lm = d.pairs[q];
-      pl[i] = lm.x;
-      pm[i] = lm.y;
+      lm[i] = slot_rows<REAL>(d, q);
       if (raman_mode >= 2) {
-        const V ca = tile_carry<T>(d, ntiles, blockIdx.x, 2 * q, look, lamT);
-        const V cb = tile_carry<T>(d, ntiles, blockIdx.x, 2 * q + 1, look, lamT);
+        const V ca = tile_carry<T>(d, P, ntiles, blockIdx.x, 2 * q, look, lamT);
+        const V cb = tile_carry<T>(d, P, ntiles, blockIdx.x, 2 * q + 1, look, lamT);
         sr[i] = mk<T>(ca.x, cb.x);
         si[i] = mk<T>(ca.y, cb.y);
       }
@@ -1823,19 +1860,32 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
     for (int i = 0; i < kSrPairsPerThread; ++i) {
       const int q = tid + i * kSrThreads;
       if (q < P) {
-        const SP* ul = uc + pl[i] * RS;
-        const SP* um = uc + pm[i] * RS;
+        const SP* ul = uc + lm[i].x * RS;
+        const SP* um = uc + lm[i].y * RS;
+        const SP* vl = uc + lm[i].z * RS;
+        const SP* vm = uc + lm[i].w * RS;
         SP* wq = sW + (size_t)q * RS;
         V Sr = sr[i], Si = si[i];
 #pragma unroll
         for (int j = 0; j < J; ++j) {
           const SP a = ld_pair<T>(ul + j), b = ld_pair<T>(um + j);
+          V v0 = {}, v1 = {};  // REAL: Re V of the two fields, both samples
+          if constexpr (REAL) {
+            const SP a1 = ld_pair<T>(vl + j), b1 = ld_pair<T>(vm + j);
+            v0 = pk_fma(a.re, b.re, pk_mul(a.im, b.im));
+            v1 = pk_fma(a1.re, b1.re, pk_mul(a1.im, b1.im));
+          }
           V w[2];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const V ue = e ? mk<T>(a.re.y, a.im.y) : mk<T>(a.re.x, a.im.x);
-            const V me = e ? mk<T>(b.re.y, b.im.y) : mk<T>(b.re.x, b.im.x);
-            const V x = cmulc(ue, me);  // V = U_l conj(U_m): (Re V, Im V)
+            V x;  // V = U_l conj(U_m): (Re V, Im V), or the slot's two Re V
+            if constexpr (REAL) {
+              x = e ? mk<T>(v0.y, v1.y) : mk<T>(v0.x, v1.x);
+            } else {
+              const V ue = e ? mk<T>(a.re.y, a.im.y) : mk<T>(a.re.x, a.im.x);
+              const V me = e ? mk<T>(b.re.y, b.im.y) : mk<T>(b.re.x, b.im.x);
+              x = cmulc(ue, me);
+            }
             if (raman_mode >= 2) {
               // S <- lambda S + x for both recurrences, then W = (1 - f_R) V + Im(kappa S)
               const V t = pk_mul(li2, Sr);
@@ -1846,7 +1896,12 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
               w[e] = x;
             }
           }
-          st_pair<T>(wq + j, mk<T>(w[0].x, w[1].x), mk<T>(w[0].y, w[1].y));
+          if constexpr (REAL) {
+            sW0[(size_t)q * RS + j] = mk<T>(w[0].x, w[1].x);
+            sW1[(size_t)q * RS + j] = mk<T>(w[0].y, w[1].y);
+          } else {
+            st_pair<T>(wq + j, mk<T>(w[0].x, w[1].x), mk<T>(w[0].y, w[1].y));
+          }
         }
         sr[i] = Sr;
         si[i] = Si;
@@ -1875,15 +1930,26 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
             u = ld_pair<T>(uc + k * RS + j);
             kprev = k;
           }
-          const SP w = ld_pair<T>(sW + (kq & 0xffffu) * RS + j);
-          const V xr = pk_mul(mk<T>(c.x, c.x), w.re), xi = pk_mul(mk<T>(c.y, c.y), w.im);  // X
-          a1 = pk_fma(u.re, xr, a1);
-          a2 = pk_fma(u.im, xi, a2);
-          a3 = pk_fma(u.re, xi, a3);
-          a4 = pk_fma(u.im, xr, a4);
+          if constexpr (REAL) {
+            const V xr = pk_mul(mk<T>(c.x, c.x), sW0[(kq & 0xffffu) + j]);  // X = a Re W
+            a1 = pk_fma(u.re, xr, a1);
+            a4 = pk_fma(u.im, xr, a4);
+          } else {
+            const SP w = ld_pair<T>(sW + (kq & 0xffffu) * RS + j);
+            const V xr = pk_mul(mk<T>(c.x, c.x), w.re), xi = pk_mul(mk<T>(c.y, c.y), w.im);  // X
+            a1 = pk_fma(u.re, xr, a1);
+            a2 = pk_fma(u.im, xi, a2);
+            a3 = pk_fma(u.re, xi, a3);
+            a4 = pk_fma(u.im, xr, a4);
+          }
         }
         // the upper half of a split mode (the next group, 8 lanes up) adds into the lower half
-        const V b1 = shfl_down_c(a1, 8), b2 = shfl_down_c(a2, 8), b3 = shfl_down_c(a3, 8), b4 = shfl_down_c(a4, 8);
+        const V b1 = shfl_down_c(a1, 8), b4 = shfl_down_c(a4, 8);
+        V b2 = {}, b3 = {};
+        if constexpr (!REAL) {
+          b2 = shfl_down_c(a2, 8);
+          b3 = shfl_down_c(a3, 8);
+        }
         if (pl.w == 1) {
           a1 = cadd(a1, b1);
           a2 = cadd(a2, b2);
@@ -1906,7 +1972,7 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
 // S <- lambda S + x sample after sample (the arithmetic of k_contract_sr's phase A without
 // the output), U arriving in sub-blocks of kSrSub samples through the same double buffer.
 // k_raman_carry turns the aggregates into the states entering the tiles.
-template <typename T>
+template <typename T, bool REAL>
 __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
     k_raman_agg_sr(const SolveDesc* __restrict__ descs, int nt, int TB, int by_tile) {
   using V = c2<T>;
@@ -1917,9 +1983,9 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TB;
   grid_sync_wait();
-  if (t0 >= nt || d.M == 0) return;            // empty slot
+  if (t0 >= nt || d.M == 0 || d.real != REAL) return;  // empty slot, other form
   if (__ldcg(d.step) >= d.step_limit) return;  // finished solve
-  const int M = d.M, P = d.P, tid = threadIdx.x;
+  const int M = d.M, P = slot_count<REAL>(d.P), tid = threadIdx.x;
   SP* sU = reinterpret_cast<SP*>(smem_raw);  // [2][M][RS]
   const V* U = as_t2<T>(d.U);
   const int nu = M * J;
@@ -1946,18 +2012,14 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
       }
     }
   };
-  int pl[kSrPairsPerThread], pm[kSrPairsPerThread];
+  int4 lm[kSrPairsPerThread];
   V sr[kSrPairsPerThread], si[kSrPairsPerThread];
 #pragma unroll
   for (int i = 0; i < kSrPairsPerThread; ++i) {
     const int q = tid + i * kSrThreads;
-    pl[i] = pm[i] = 0;
+    lm[i] = make_int4(0, 0, 0, 0);
     sr[i] = si[i] = mk<T>(0, 0);
-    if (q < P) {
-      const int2 lm = d.pairs[q];
-      pl[i] = lm.x;
-      pm[i] = lm.y;
-    }
+    if (q < P) lm[i] = slot_rows<REAL>(d, q);
   }
   const T lr = (T)d.iir_lambda.x, li = (T)d.iir_lambda.y;
   const V lr2 = mk<T>(lr, lr), li2 = mk<T>(li, li), nli2 = mk<T>(-li, -li);
@@ -1973,16 +2035,27 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
 #pragma unroll
     for (int i = 0; i < kSrPairsPerThread; ++i) {
       if (tid + i * kSrThreads < P) {
-        const SP* ul = uc + pl[i] * RS;
-        const SP* um = uc + pm[i] * RS;
+        const SP* ul = uc + lm[i].x * RS;
+        const SP* um = uc + lm[i].y * RS;
+        const SP* vl = uc + lm[i].z * RS;
+        const SP* vm = uc + lm[i].w * RS;
         V Sr = sr[i], Si = si[i];
 #pragma unroll
         for (int j = 0; j < J; ++j) {
           const SP a = ld_pair<T>(ul + j), b = ld_pair<T>(um + j);
+          V v0 = {}, v1 = {};
+          if constexpr (REAL) {
+            const SP a1 = ld_pair<T>(vl + j), b1 = ld_pair<T>(vm + j);
+            v0 = pk_fma(a.re, b.re, pk_mul(a.im, b.im));
+            v1 = pk_fma(a1.re, b1.re, pk_mul(a1.im, b1.im));
+          }
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const V x = cmulc(e ? mk<T>(a.re.y, a.im.y) : mk<T>(a.re.x, a.im.x),
-                              e ? mk<T>(b.re.y, b.im.y) : mk<T>(b.re.x, b.im.x));
+            V x;
+            if constexpr (REAL) x = e ? mk<T>(v0.y, v1.y) : mk<T>(v0.x, v1.x);
+            else
+              x = cmulc(e ? mk<T>(a.re.y, a.im.y) : mk<T>(a.re.x, a.im.x),
+                        e ? mk<T>(b.re.y, b.im.y) : mk<T>(b.re.x, b.im.x));
             const V t = pk_mul(li2, Sr);
             Sr = pk_fma(lr2, Sr, pk_fma(nli2, Si, x));
             Si = pk_fma(lr2, Si, t);
@@ -2083,7 +2156,13 @@ template <typename T> struct LaneScan {
   }
 };
 
-template <typename T>
+// REAL form: rows of W are real, one per pair field (TT values of T): pair h at rs(h), which spreads
+// a lane's own 16-byte chunks (four samples in FP32, two in FP64) over the banks.
+template <typename T> __device__ __forceinline__ int rs(int h, int wmask) {
+  return sizeof(T) == 8 ? wsw(h, wmask) : h ^ (wmask == 3 ? ((h >> 4) & 1) << 1 : 0);
+}
+
+template <typename T, bool REAL>
 __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
     k_contract_sp(const SolveDesc* __restrict__ descs, int nt, int TT, int raman_mode, int mixed) {
   using V = c2<T>;
@@ -2092,15 +2171,16 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
   __shared__ __align__(8) unsigned long long bar;
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TT;
-  if (t0 >= nt || d.M == 0 || (mixed && d.dense_q != nullptr)) {  // empty slot, or the dense form's
+  if (t0 >= nt || d.M == 0 || d.real != REAL || (mixed && d.dense_q != nullptr)) {  // empty slot, other form
     grid_sync_wait();
     return;
   }
-  const int M = d.M, P = d.P, nterm = d.sr_terms;
+  const int M = d.M, P = slot_count<REAL>(d.P), nterm = d.sr_terms;
   const int H = TT >> 1, wmask = (TT >> 6) - 1;  // pairs per row
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   SP* sU = reinterpret_cast<SP*>(smem_raw);      // [M][H]
-  SP* sW = sU + (size_t)M * H;                   // [P][H]
+  SP* sW = sU + (size_t)M * H;                   // [P][H] (REAL: [2 P][H] real pairs)
+  V* sR = reinterpret_cast<V*>(sW);
   SrRec<T>* sRec = reinterpret_cast<SrRec<T>*>(sW + (size_t)P * H);
   V* sC = reinterpret_cast<V*>(sRec + nterm);    // states entering the tile, [P][2]
   // staged while the kernel before this one still runs: the terms, with k and q as row positions
@@ -2110,7 +2190,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
       const unsigned kq = d.sr_kq[i];
       SrRec<T> r = {};
       r.ab = cf[i];
-      r.kq = (kq & 0xffffu) * H | ((kq >> 16) * H) << 16;
+      r.kq = (kq & 0xffffu) * H | ((kq >> 16) * H) << 16;  // a row of W is H pairs in both forms
       sRec[i] = r;
     }
   }
@@ -2120,15 +2200,16 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
   LaneScan<T> ts;
   if (raman_mode >= 2) ts.init(d, TT >> 5, lane);
   if (tid == 0) mbar_init(&bar, 1);
-  const int Pl = raman_mode == 1 ? P : 0;      // rows of R loaded
-  const unsigned row_bytes = (unsigned)(TT * sizeof(V));
-  if (tid == 0) mbar_arrive_expect_tx(&bar, (unsigned)(M + Pl) * row_bytes);
+  const int Pl = raman_mode == 1 ? (REAL ? 2 * P : P) : 0;  // rows of R loaded
+  const unsigned row_bytes = (unsigned)(TT * sizeof(V)), r_bytes = REAL ? row_bytes / 2 : row_bytes;
+  if (tid == 0) mbar_arrive_expect_tx(&bar, (unsigned)M * row_bytes + (unsigned)Pl * r_bytes);
   __syncthreads();
   grid_sync_wait();
-  for (int r = tid; r < M + Pl; r += blockDim.x) {
-    const V* src = r < M ? as_t2<T>(d.U) + (size_t)r * nt + t0 : as_t2<T>(d.W) + (size_t)(r - M) * nt + t0;
-    bulk_g2s(sU + (size_t)r * H, src, row_bytes, &bar);
-  }
+  for (int r = tid; r < M; r += blockDim.x)
+    bulk_g2s(sU + (size_t)r * H, as_t2<T>(d.U) + (size_t)r * nt + t0, row_bytes, &bar);
+  for (int r = tid; r < Pl; r += blockDim.x)
+    bulk_g2s(reinterpret_cast<char*>(sW) + (size_t)r * r_bytes,
+             static_cast<const char*>(d.W) + ((size_t)r * nt + t0) * (r_bytes / TT), r_bytes, &bar);
   if (__ldcg(d.step) >= d.step_limit) {  // finished solve: the copies land before the CTA leaves
     mbar_wait(&bar, 0, kMaxWaitPolls);
     return;
@@ -2156,21 +2237,27 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
     vre = pk_fma(a.re, b.re, pk_mul(a.im, b.im));
     vim = pk_fma(a.im, b.re, pk_mul(mk<T>(-a.re.x, -a.re.y), b.im));
   };
+  auto real_product = [](const SP& a, const SP& b) { return pk_fma(a.re, b.re, pk_mul(a.im, b.im)); };
   // 2. pair fields
   if (raman_mode >= 2) {
     const int g = ts.c >> 1;
     for (int q = warp; q < P; q += nwarps) {
-      const int2 lm = __ldg(d.pairs + q);
+      const int4 lm = slot_rows<REAL>(d, q);
       const SP* ul = sU + lm.x * H;
       const SP* um = sU + lm.y * H;
       SP* wq = sW + (size_t)q * H;
-      V x[8];  // (Re V, Im V) of the lane's samples
+      V x[8];  // (Re V, Im V) of the lane's samples, or the slot's two Re V
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         if (j < g) {
           const int at = wsw(g * lane + j, wmask);
           V vre, vim;
-          pair_product(ld_pair<T>(ul + at), ld_pair<T>(um + at), vre, vim);
+          if constexpr (REAL) {
+            vre = real_product(ld_pair<T>(ul + at), ld_pair<T>(um + at));
+            vim = real_product(ld_pair<T>(sU + lm.z * H + at), ld_pair<T>(sU + lm.w * H + at));
+          } else {
+            pair_product(ld_pair<T>(ul + at), ld_pair<T>(um + at), vre, vim);
+          }
           x[2 * j] = mk<T>(vre.x, vim.x);
           x[2 * j + 1] = mk<T>(vre.y, vim.y);
         }
@@ -2182,24 +2269,63 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
       ts.enter(sr, si, lane, sC + 2 * q);  // the state entering the lane
       const V kerr2 = mk<T>(kerr, kerr);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (j < g) {
-          V w[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            ts.step(sr, si, x[2 * j + e]);
-            w[e] = pk_fma(kerr2, x[2 * j + e], pk_fma(ts.kr2, si, pk_mul(ts.ki2, sr)));
-          }
-          st_pair<T>(wq + wsw(g * lane + j, wmask), mk<T>(w[0].x, w[1].x), mk<T>(w[0].y, w[1].y));
+      for (int k = 0; k < 8; ++k) {
+        if (k < ts.c) {
+          ts.step(sr, si, x[k]);
+          x[k] = pk_fma(kerr2, x[k], pk_fma(ts.kr2, si, pk_mul(ts.ki2, sr)));
         }
+      }
+      if constexpr (REAL) {
+        V* w0 = sR + (size_t)(2 * q) * H;
+        V* w1 = w0 + H;
+        if (sizeof(T) == 4 && g > 1) {  // four samples of a field per 16 bytes
+#pragma unroll
+          for (int j = 0; j < 4; j += 2) {
+            if (j < g) {
+              const int at = rs<T>(g * lane + j, wmask);
+              st2<T>(w0 + at, mk<T>(x[2 * j].x, x[2 * j + 1].x), mk<T>(x[2 * j + 2].x, x[2 * j + 3].x));
+              st2<T>(w1 + at, mk<T>(x[2 * j].y, x[2 * j + 1].y), mk<T>(x[2 * j + 2].y, x[2 * j + 3].y));
+            }
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (j < g) {
+              const int at = rs<T>(g * lane + j, wmask);
+              w0[at] = mk<T>(x[2 * j].x, x[2 * j + 1].x);
+              w1[at] = mk<T>(x[2 * j].y, x[2 * j + 1].y);
+            }
+          }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j < g)
+            st_pair<T>(wq + wsw(g * lane + j, wmask), mk<T>(x[2 * j].x, x[2 * j + 1].x),
+                       mk<T>(x[2 * j].y, x[2 * j + 1].y));
       }
     }
   } else {
     for (int i = tid; i < P * H; i += blockDim.x) {
       const int h = i & (H - 1), at = wsw(h, wmask);
-      const int2 lm = __ldg(d.pairs + i / H);
-      SP* row = sW + (i - h);
+      const int4 lm = slot_rows<REAL>(d, i / H);
       V vre, vim;
+      if constexpr (REAL) {
+        vre = real_product(ld_pair<T>(sU + lm.x * H + at), ld_pair<T>(sU + lm.y * H + at));
+        vim = real_product(ld_pair<T>(sU + lm.z * H + at), ld_pair<T>(sU + lm.w * H + at));
+        V* w0 = sR + 2 * (size_t)(i - h);
+        V* w1 = w0 + H;
+        if (raman_mode == 1) {  // W = (1 - f_R) V + R, R in place as it landed
+          const V r0 = w0[h], r1 = w1[h];
+          vre = pk_fma(mk<T>(kerr, kerr), vre, r0);
+          vim = pk_fma(mk<T>(kerr, kerr), vim, r1);
+          __syncwarp();
+        }
+        w0[rs<T>(h, wmask)] = vre;
+        w1[rs<T>(h, wmask)] = vim;
+        continue;
+      }
+      SP* row = sW + (i - h);
       pair_product(ld_pair<T>(sU + lm.x * H + at), ld_pair<T>(sU + lm.y * H + at), vre, vim);
       if (raman_mode == 1) {  // W = (1 - f_R) V + R, R in place as it landed
         V r0, r1;
@@ -2219,6 +2345,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
     const int p = item / (H >> 5), h = (item - p * (H >> 5)) * 32 + lane, at = wsw(h, wmask);
     const SP* uc = sU + at;
     const SP* wc = sW + at;
+    const V* rc = sR + rs<T>(h, wmask);
     const int n1 = __ldg(d.sr_off + p + 1);
     V a1 = mk<T>(0, 0), a2 = a1, a3 = a1, a4 = a1;
     SP u = {};
@@ -2232,12 +2359,18 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
         kprev = kq >> 16;
         u = ld_pair<T>(uc + kprev);
       }
-      const SP w = ld_pair<T>(wc + (kq & 0xffffu));
-      const V xr = pk_mul(mk<T>(c.x, c.x), w.re), xi = pk_mul(mk<T>(c.y, c.y), w.im);  // a Re W, b Im W
-      a1 = pk_fma(u.re, xr, a1);
-      a2 = pk_fma(u.im, xi, a2);
-      a3 = pk_fma(u.re, xi, a3);
-      a4 = pk_fma(u.im, xr, a4);
+      if constexpr (REAL) {
+        const V xr = pk_mul(mk<T>(c.x, c.x), rc[kq & 0xffffu]);  // a Re W
+        a1 = pk_fma(u.re, xr, a1);
+        a4 = pk_fma(u.im, xr, a4);
+      } else {
+        const SP w = ld_pair<T>(wc + (kq & 0xffffu));
+        const V xr = pk_mul(mk<T>(c.x, c.x), w.re), xi = pk_mul(mk<T>(c.y, c.y), w.im);  // a Re W, b Im W
+        a1 = pk_fma(u.re, xr, a1);
+        a2 = pk_fma(u.im, xi, a2);
+        a3 = pk_fma(u.re, xi, a3);
+        a4 = pk_fma(u.im, xr, a4);
+      }
     }
     st2<T>(sigma + (size_t)p * nt + t0 + 2 * h, mk<T>(a1.x - a2.x, a3.x + a4.x), mk<T>(a1.y - a2.y, a3.y + a4.y));
   }
@@ -2268,8 +2401,8 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
 // thousand). Measured on a B200, 16 solves of 15 x 8192, a launch, against two 16-field buffers
 // between barriers of the whole CTA and scalar recurrences: 183 -> 141 us, 64 -> 44 million warp
 // instructions (24 builder warps instead of 16: 143).
-constexpr int kTcBuilders = 2;  // chunks built at a time, by eight warps each
-constexpr int kTcThreads = 32 * (8 * kTcBuilders + 1);
+constexpr int kTcBuilders = 2;  // chunks built at a time, a warp per slot
+template <bool REAL> constexpr int tc_threads() { return 32 * (slot_count<REAL>(kTcChunk) * kTcBuilders + 1); }
 
 // mbar_wait that also gives up once *stop is set (by another warp whose wait ran out)
 __device__ __forceinline__ bool mbar_wait_or(unsigned long long* bar, unsigned parity, volatile int* stop) {
@@ -2284,13 +2417,18 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kTcThreads, 1) k_contract_tc(const SolveDesc* __restrict__ descs, int nt, int raman_mode) {
+template <typename T, bool REAL>
+__global__ void __launch_bounds__(tc_threads<REAL>(), REAL ? 2 : 1) k_contract_tc(const SolveDesc* __restrict__ descs, int nt, int raman_mode) {
   static_assert(sizeof(T) == 4, "TF32 operands come from FP32 solves");
   using V = float2;
-  constexpr int TT = kTcTile, KC = kTcChunk, NS = kTcStages, BW = kTcBuilders * KC;  // builder warps
+  constexpr int TT = kTcTile, KC = kTcChunk, NS = kTcStages;
+  constexpr int SC = slot_count<REAL>(KC);      // slots per chunk
+  constexpr int BW = kTcBuilders * SC;          // builder warps
+  constexpr int PARTS = REAL ? 1 : 2;           // products: Re, Im
+  constexpr int MATS = 2 * PARTS;               // operand matrices: hi and lo of each
+  constexpr uint32_t COLS = 256 * PARTS;        // TMEM columns
   // A operand (MN-major TF32 layout): 32-sample atoms 512 bytes apart, 4-field groups 2048
-  static_assert(TT == 128 && KC == 8 && kTcThreads == 32 * (BW + 1), "one MMA covers the tile's 128 samples");
+  static_assert(TT == 128 && KC == 8, "one MMA covers the tile's 128 samples and a chunk");
   constexpr uint32_t A_LBO = 512, A_SBO = 2048;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long bar_u, bar_a[NS], bar_b[NS], bar_m[NS];
@@ -2298,28 +2436,28 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_contract_tc(const SolveDesc* 
   __shared__ volatile int s_stop;
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TT;
-  if (t0 >= nt || d.M == 0) {  // empty slot
+  if (t0 >= nt || d.M == 0 || d.real != REAL) {  // empty slot, other form
     grid_sync_wait();
     return;
   }
-  const int M = d.M, P = d.P, N = 16 * M;
+  const int M = d.M, P = d.P, PS = slot_count<REAL>(P), N = 16 * M;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   V* sU = reinterpret_cast<V*>(smem_raw);                        // [M][TT]
-  // [NS][4][KC * TT] MN-major operands, on the next 1024-byte boundary (the swizzle pattern's
+  // [NS][MATS][KC * TT] MN-major operands, on the next 1024-byte boundary (the swizzle pattern's
   // alignment; the launch reserves the slack)
   unsigned char* after_u = reinterpret_cast<unsigned char*>(sU + (size_t)M * TT);
   float* sA = reinterpret_cast<float*>(after_u + ((1024u - (tc::smem_u32(after_u) & 1023u)) & 1023u));
-  float* sB = sA + NS * 4 * KC * TT;                             // [NS][4][KC/4][N][4]
-  V* sC = reinterpret_cast<V*>(sB + NS * 4 * KC * N);             // states entering the tile, [P][2]
+  float* sB = sA + NS * MATS * KC * TT;                          // [NS][MATS][KC/4][N][4]
+  V* sC = reinterpret_cast<V*>(sB + NS * MATS * KC * N);          // states entering the tile, [PS][2]
   const int nch = (P + KC - 1) / KC;
-  const unsigned bbytes = (unsigned)(4 * KC * N * sizeof(float));
+  const unsigned bbytes = (unsigned)(MATS * KC * N * sizeof(float));
   LaneScan<float> ts;
   if (raman_mode >= 2) ts.init(d, TT >> 5, lane);
   if (tid == 0) {
     s_stop = 0;
     mbar_init(&bar_u, 1);
     for (int i = 0; i < NS; ++i) {
-      mbar_init(&bar_a[i], KC);
+      mbar_init(&bar_a[i], SC);
       mbar_init(&bar_b[i], 1);
       mbar_init(&bar_m[i], 1);
     }
@@ -2330,7 +2468,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_contract_tc(const SolveDesc* 
   const bool driver = warp == BW && lane == 0;
   auto copy_b = [&](int c) {
     mbar_arrive_expect_tx(&bar_b[c % NS], bbytes);
-    bulk_g2s(sB + (size_t)(c % NS) * 4 * KC * N, d.dense_tc + (size_t)c * 4 * KC * N, bbytes, &bar_b[c % NS]);
+    bulk_g2s(sB + (size_t)(c % NS) * MATS * KC * N, d.dense_tc + (size_t)c * MATS * KC * N, bbytes, &bar_b[c % NS]);
     b_issued = c + 1;
   };
   auto drain_b = [&]() {  // the coefficient copies in flight have landed
@@ -2347,9 +2485,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_contract_tc(const SolveDesc* 
     return;
   }
   if (raman_mode >= 2)
-    stage_tile_carries<float>(sC, d, P, nt / TT, blockIdx.x, tile_look(d, nt / TT, TT, raman_mode), lambda_tile(d, TT));
+    stage_tile_carries<float>(sC, d, PS, nt / TT, blockIdx.x, tile_look(d, nt / TT, TT, raman_mode), lambda_tile(d, TT));
   if (warp == BW) {
-    tc::alloc(&s_tmem, 512);
+    tc::alloc(&s_tmem, COLS);
     tc::relinquish();
   }
   tc::fence_before_sync();
@@ -2359,25 +2497,36 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_contract_tc(const SolveDesc* 
   const uint32_t tmem = s_tmem;
   if (ok && warp < BW) {
     const float kerr = (float)d.one_minus_fR;
-    const int f = warp & (KC - 1);  // this warp's field of every other chunk
-    for (int c = warp / KC; c < nch; c += kTcBuilders) {
-      const int buf = c % NS, q = c * KC + f;
+    const int f = warp % SC;  // this warp's slot of every other chunk
+    for (int c = warp / SC; c < nch; c += kTcBuilders) {
+      const int buf = c % NS, q = c * SC + f;
       // chunk c - NS's MMAs read this buffer pair
       if (c >= NS && !mbar_wait_or(&bar_m[buf], ((c / NS) - 1) & 1, &s_stop)) break;
-      // lane L's samples 4L .. 4L + 3 of the field: one 16-byte chunk of each operand matrix
-      float* a0 = sA + (size_t)buf * 4 * KC * TT + tc::mn_tf32_offset(4 * lane, f, A_LBO, A_SBO) / 4;
+      // lane L's samples 4L .. 4L + 3 of a field: one 16-byte chunk of each operand matrix; the
+      // slot's second component goes to the Im matrices, or (REAL) is the next field
+      float* a0 = sA + (size_t)buf * MATS * KC * TT + tc::mn_tf32_offset(4 * lane, REAL ? 2 * f : f, A_LBO, A_SBO) / 4;
+      float* a1 = REAL ? sA + (size_t)buf * MATS * KC * TT + tc::mn_tf32_offset(4 * lane, 2 * f + 1, A_LBO, A_SBO) / 4
+                       : a0 + 2 * KC * TT;
       V x[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-      if (q < P) {  // past the last field: zeros
-        const int2 lm = __ldg(d.pairs + q);
-        V a[4], b[4];
+      if (q < PS) {  // past the last slot: zeros
+        const int4 lm = slot_rows<REAL>(d, q);
+        V a[4], b[4], a2[4] = {}, b2[4] = {};
         const V* ul = sU + lm.x * TT + 4 * lane;
         const V* um = sU + lm.y * TT + 4 * lane;
         ld2<float>(ul, a[0], a[1]);
         ld2<float>(ul + 2, a[2], a[3]);
         ld2<float>(um, b[0], b[1]);
         ld2<float>(um + 2, b[2], b[3]);
+        if constexpr (REAL) {
+          const V* vl = sU + lm.z * TT + 4 * lane;
+          const V* vm = sU + lm.w * TT + 4 * lane;
+          ld2<float>(vl, a2[0], a2[1]);
+          ld2<float>(vl + 2, a2[2], a2[3]);
+          ld2<float>(vm, b2[0], b2[1]);
+          ld2<float>(vm + 2, b2[2], b2[3]);
+        }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) x[e] = cmulc(a[e], b[e]);
+        for (int e = 0; e < 4; ++e) x[e] = slot_value<REAL>(a[e], b[e], a2[e], b2[e]);
         if (raman_mode >= 2) {
           V sr = x[0], si = make_float2(0.f, 0.f);
 #pragma unroll
@@ -2401,8 +2550,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_contract_tc(const SolveDesc* 
       }
       *reinterpret_cast<float4*>(a0) = make_float4(rh[0], rh[1], rh[2], rh[3]);
       *reinterpret_cast<float4*>(a0 + KC * TT) = make_float4(rl[0], rl[1], rl[2], rl[3]);
-      *reinterpret_cast<float4*>(a0 + 2 * KC * TT) = make_float4(ih[0], ih[1], ih[2], ih[3]);
-      *reinterpret_cast<float4*>(a0 + 3 * KC * TT) = make_float4(il[0], il[1], il[2], il[3]);
+      *reinterpret_cast<float4*>(a1) = make_float4(ih[0], ih[1], ih[2], ih[3]);
+      *reinterpret_cast<float4*>(a1 + KC * TT) = make_float4(il[0], il[1], il[2], il[3]);
       tc::fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_a[buf]);
@@ -2414,12 +2563,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_contract_tc(const SolveDesc* 
       const unsigned par = (c / NS) & 1;
       if (!mbar_wait_or(&bar_b[buf], par, &s_stop) || !mbar_wait_or(&bar_a[buf], par, &s_stop)) break;
       tc::fence_after_sync();
-      const float* A = sA + (size_t)buf * 4 * KC * TT;
-      const float* B = sB + (size_t)buf * 4 * KC * N;
+      const float* A = sA + (size_t)buf * MATS * KC * TT;
+      const float* B = sB + (size_t)buf * MATS * KC * N;
       // Re: (A Re hi, B Re hi), (Re hi, Re lo), (Re lo, Re hi); Im likewise
       constexpr int ta[3] = {0, 0, 1}, tb[3] = {0, 1, 0};
 #pragma unroll
-      for (int part = 0; part < 2; ++part)
+      for (int part = 0; part < PARTS; ++part)
 #pragma unroll
         for (int term = 0; term < 3; ++term)
         {
@@ -2450,14 +2599,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_contract_tc(const SolveDesc* 
       for (int p = warp >> 2; p < M; p += BW >> 2) {
         float re[16], im[16];
         tc::ld16(tl + 16u * p, re);
-        tc::ld16(tl + 256u + 16u * p, im);
+        if constexpr (!REAL) tc::ld16(tl + 256u + 16u * p, im);
         float sx = 0.f, sy = 0.f;
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
           if (k < M) {
             const V u = sU[k * TT + t];
-            sx = fmaf(u.x, re[k], fmaf(-u.y, im[k], sx));
-            sy = fmaf(u.x, im[k], fmaf(u.y, re[k], sy));
+            if constexpr (REAL) {
+              sx = fmaf(u.x, re[k], sx);
+              sy = fmaf(u.y, re[k], sy);
+            } else {
+              sx = fmaf(u.x, re[k], fmaf(-u.y, im[k], sx));
+              sy = fmaf(u.x, im[k], fmaf(u.y, re[k], sy));
+            }
           }
         }
         sigma[(size_t)p * nt + t0 + t] = make_float2(sx, sy);
@@ -2475,7 +2629,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_contract_tc(const SolveDesc* 
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == BW) tc::dealloc(tmem, 512);
+  if (warp == BW) tc::dealloc(tmem, COLS);
 }
 
 // FP64 rows -> T rows (used for the Raman spectrum)
