@@ -171,6 +171,12 @@ const void* sr_fn(bool fp64, bool real) {
   if (real) return fp64 ? fn_ptr(&k_contract_sr<double, true>) : fn_ptr(&k_contract_sr<float, true>);
   return fp64 ? fn_ptr(&k_contract_sr<double, false>) : fn_ptr(&k_contract_sr<float, false>);
 }
+// k_contract_sr's shared memory: M rows, `slots` slots, `groups` plan entries, `terms` merged terms
+size_t sr_bytes(bool fp64, bool real, size_t M, size_t slots, size_t groups, size_t terms) {
+  if (real)
+    return fp64 ? SrLayout<double, true>::bytes(M, slots, groups, terms) : SrLayout<float, true>::bytes(M, slots, groups, terms);
+  return fp64 ? SrLayout<double, false>::bytes(M, slots, groups, terms) : SrLayout<float, false>::bytes(M, slots, groups, terms);
+}
 const void* agg_sr_fn(bool fp64, bool real) {
   if (real) return fp64 ? fn_ptr(&k_raman_agg_sr<double, true>) : fn_ptr(&k_raman_agg_sr<float, true>);
   return fp64 ? fn_ptr(&k_raman_agg_sr<double, false>) : fn_ptr(&k_raman_agg_sr<float, false>);
@@ -1691,16 +1697,16 @@ Shape choose_shape(const mmp_batch* b, const ShapeStats& st, bool try_real = tru
       if (std::atoi(env) == 0) ok = false;
     if (const char* env = std::getenv("MMP_RAMAN_FUSED"))
       if (std::atoi(env) == 0 && b->raman) ok = false;
-    const size_t sp = 2 * t2;  // one sample pair of one row
-    const size_t rs = kSrSub / 2 + 1;
-    const size_t plan = (size_t)((Mmax + kSrGroups - 1) / kSrGroups) * kSrGroups * sizeof(int4);
-    const size_t need = (2 * (size_t)Mmax + (size_t)Pall) * rs * sp + plan + max_sr_terms * 2 * t2;  // SrRec
+    const size_t groups = (size_t)((Mmax + kSrGroups - 1) / kSrGroups) * kSrGroups;
+    size_t need = 0;
+    if (!real || !st.all_real) need = sr_bytes(b->fp64, false, Mmax, Pall, groups, max_sr_terms);
+    if (real) need = std::max(need, sr_bytes(b->fp64, true, Mmax, Pall, groups, max_sr_terms));
     if (ok && need <= 227 * 1024) {
       sr = true;
       pchunk = 0;
       TT = std::min(tile_req >= 64 ? std::min(tile_req, 256) : 256, (int)b->nt);
       fused = b->raman;
-      smem = (need + 15) & ~(size_t)15;
+      smem = need;
     }
   }
   // The tiles sum the states entering them from the aggregates before them where that takes few

@@ -1669,24 +1669,30 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2)) k_contract_pc(c
 
 // ---- k_contract_sr: the term loop with the Raman recurrence run serially per pair field --
 // For tall tiles (more pair fields than k_contract holds in a tile). A CTA owns TB
-// consecutive samples of one solve and walks them in sub-blocks of kSrSub = 16 samples:
+// consecutive samples of one solve and walks them in sub-blocks of kSrSub = 16 samples
+// (SrLayout: two at a time in the FP32 REAL form):
 //   staging  U of the next sub-block is loaded from global memory while this one is
-//            worked on, into a double buffer in which each sample pair (t, t + 1) of a
+//            worked on; in shared memory each sample pair (t, t + 1) of a
 //            row is stored as (Re t, Re t+1, Im t, Im t+1);
 //   phase A  each thread owns one or two pair fields q = (l, m) for the whole tile and runs
 //            the Raman recurrence S = lambda S + x (x = Re V and Im V, V = U_l conj(U_m))
-//            sample after sample from the state entering the tile (k_raman_carry); the
-//            state stays in registers from one sub-block to the next, and
+//            sample after sample from the state entering the tile; the state stays in registers from one sub-block to the next, and
 //            W_q = (1 - f_R) V + Im(kappa S) for the sub-block goes to shared memory
-//            (Raman off: W_q = V);
+//            (Raman off: W_q = V). REAL form: a slot's two fields are the two lanes, and
+//            only their Re W is formed;
 //   phase B  sigma_p(t) = sum over p's merged terms of U_k (a Re W_q + i b Im W_q)
-//            (SolveDesc::sr_coef), eight lanes (one per sample pair) per group; a plan
+//            (SolveDesc::sr_coef), eight lanes per group, each with one sample pair (FP32
+//            REAL: two); a plan
 //            made on the host (SolveDesc::sr_plan) gives each group a mode, or half of a
 //            mode with many terms (the two halves sit in one warp and are added by a
 //            shuffle), so the longest group's term loop is about half as long as the
 //            heaviest mode's; groups of similar length share a warp.
-// Per term a lane reads U_k and W_q (16 bytes each for its two samples) and the 8-byte
-// coefficient from shared memory, whose bandwidth bounds the kernel.
+// Shared memory bounds it: per term a lane reads W_q (16 bytes) and the term's record, and U_k
+// when k changes; per sub-block a slot reads two rows of U (REAL: four). Measured on a B200 at
+// 28 x 65536, 203 slots, 1060 merged terms, 8 solves, a launch: 519 us in the general form; REAL
+// form, which halves the phase-A chains and the FMAs of a term, 420 us; with four samples a
+// lane (half the W loads and records a sample; one U buffer keeps three CTAs an SM) 378 us, the
+// shared-memory pipe busy 75% of the time, issue 49%.
 // Compared with the warp-per-field scan, a sample costs one step of each recurrence and no
 // scan levels. FP32 solves use the packed two-lane FMA (fma.rn.f32x2): phase A packs the
 // two recurrences (Re V and Im V share lambda), phase B the two samples of a pair; each
@@ -1748,6 +1754,40 @@ template <typename V> __device__ __forceinline__ V shfl_down_c(V v, int d) {
   return v;
 }
 
+// Shared-memory layout of k_contract_sr. General form and FP64: sub-blocks of
+// kSrSub samples, U double-buffered, a lane of phase B takes one sample pair. FP32 REAL form:
+// two sub-blocks at a time; a lane takes four samples, so that a term costs it 16 bytes of W and
+// an 8-byte record.
+template <typename T, bool REAL> struct SrLayout {
+  static constexpr bool WIDE = REAL && sizeof(T) == 4;
+  static constexpr int S = WIDE ? 2 * kSrSub : kSrSub;  // samples at a time
+  static constexpr int J = S / 2;                       // sample pairs
+  static constexpr int NI = (kSrMaxModes * J + kSrThreads - 1) / kSrThreads;  // staged pairs a thread
+  static constexpr int BUF = WIDE ? 1 : 2;
+  // Row strides: consecutive rows start 16 bytes apart mod 128, so that a quarter warp's rows
+  // fall on different banks. U in sample pairs, a field's Re W (REAL) in pairs of reals.
+  static constexpr int RS = J + 1;
+  static constexpr int WS = WIDE ? J + 2 : J + 1;
+  static constexpr int SLOT_BYTES = REAL ? 2 * WS * (int)sizeof(c2<T>) : RS * (int)sizeof(SrPair<T>);
+  // where pair j of a U row lies: WIDE has a lane's two pairs 8 positions apart, so that eight
+  // lanes read 128 consecutive bytes
+  static __host__ __device__ constexpr int pos(int j) { return WIDE ? (j >> 1) + (j & 1) * (J / 2) : j; }
+  struct Narrow {
+    float ab;
+    unsigned kq;
+  };
+  using Rec = std::conditional_t<WIDE, Narrow, SrRec<T>>;
+  static __device__ __forceinline__ auto coef(c2<T> ab) {
+    if constexpr (WIDE) return ab.x;
+    else return ab;
+  }
+  static size_t bytes(size_t M, size_t slots, size_t groups, size_t terms) {
+    const size_t n = BUF * M * RS * sizeof(SrPair<T>) + slots * SLOT_BYTES + groups * sizeof(int4) + terms * sizeof(Rec);
+    return (n + 15) & ~(size_t)15;
+  }
+};
+static_assert(sizeof(SrLayout<float, true>::Rec) == 8, "one term in 8 bytes");
+
 // raman_mode: 0 Raman off, 2 the recurrence from the tile carries of k_raman_carry (tiles of TB), 3 from
 // carries summed here (tile_carry)
 template <typename T, bool REAL>
@@ -1755,10 +1795,10 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
     k_contract_sr(const SolveDesc* __restrict__ descs, int nt, int TB, int raman_mode) {
   using V = c2<T>;
   using SP = SrPair<T>;
-  using CF = c2<T>;              // merged coefficient (a, b)
-  constexpr int J = kSrSub / 2;  // sample pairs per sub-block
-  constexpr int RS = J + 1;      // row stride in sample pairs: consecutive rows start 16 bytes apart
-                                 // mod 128, so a quarter warp's rows fall on different banks
+  using CF = c2<T>;  // merged coefficient (a, b)
+  using L = SrLayout<T, REAL>;
+  constexpr bool WIDE = L::WIDE;
+  constexpr int J = L::J, RS = L::RS, NI = L::NI;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const SolveDesc& d = descs[blockIdx.y];
   const int t0 = blockIdx.x * TB;
@@ -1768,24 +1808,25 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
   }
   const int M = d.M, P = slot_count<REAL>(d.P), nterm = d.sr_terms, rounds = d.sr_rounds;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // shared memory: U [2][M][RS], W [P][RS] (REAL: two planes [P][RS] of sample pairs, the slots'
+  // shared memory: U [BUF][M][RS], W [P][RS] (REAL: two planes [P][WS] of sample pairs, the slots'
   // first and second fields, so that a quarter warp's rows stay on different banks), group
-  // plan [rounds kSrGroups], merged terms [nterm] (coefficients and q | k << 16)
+  // plan [rounds kSrGroups], merged terms [nterm] (coefficients and row positions)
   SP* sU = reinterpret_cast<SP*>(smem_raw);
-  SP* sW = sU + 2 * (size_t)M * RS;
+  SP* sW = sU + (size_t)L::BUF * M * RS;
   V* sW0 = reinterpret_cast<V*>(sW);
-  V* sW1 = sW0 + (size_t)P * RS;
-  int4* sPlan = reinterpret_cast<int4*>(sW + (size_t)P * RS);
-  SrRec<T>* sRec = reinterpret_cast<SrRec<T>*>(sPlan + rounds * kSrGroups);
+  V* sW1 = sW0 + (size_t)P * L::WS;
+  int4* sPlan = reinterpret_cast<int4*>(reinterpret_cast<unsigned char*>(sW) + (size_t)P * L::SLOT_BYTES);
+  using Rec = typename L::Rec;
+  Rec* sRec = reinterpret_cast<Rec*>(sPlan + rounds * kSrGroups);
   {
     const CF* gCf = static_cast<const CF*>(d.sr_coef);
     for (int i = tid; i < nterm; i += kSrThreads) {
-      SrRec<T> r = {};
-      r.ab = gCf[i];
+      Rec r = {};
+      r.ab = L::coef(gCf[i]);
       r.kq = d.sr_kq[i];
       if constexpr (REAL) {  // the pair field's plane and row as one position
         const unsigned q = r.kq & 0xffffu;
-        r.kq = (r.kq & 0xffff0000u) | ((q & 1u) * P + (q >> 1)) * RS;
+        r.kq = (r.kq >> 16) * (WIDE ? RS << 16 : 1 << 16) | ((q & 1u) * P + (q >> 1)) * L::WS;
       }
       sRec[i] = r;
     }
@@ -1794,14 +1835,14 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
   const double2 lamT = raman_mode == 3 ? lambda_tile(d, TB) : make_double2(0.0, 0.0);
   grid_sync_wait();
   if (__ldcg(d.step) >= d.step_limit) return;  // finished solve (nothing is in flight yet)
-  // U staging: sample pair j of row r is item r J + j; a thread carries at most two
+  // U staging: sample pair j of row r is item r J + j; a thread carries at most NI
   const V* U = as_t2<T>(d.U);
   const int nu = M * J;
-  V pre[2][2];
+  V pre[NI][2];
   auto fetch = [&](int sub) {
-    const int ts = t0 + sub * kSrSub;
+    const int ts = t0 + sub * L::S;
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < NI; ++r) {
       const int idx = tid + r * kSrThreads;
       if (idx < nu) {
         const int row = idx / J, j = idx - row * J;
@@ -1811,11 +1852,11 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
   };
   auto park = [&](int buf) {
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < NI; ++r) {
       const int idx = tid + r * kSrThreads;
       if (idx < nu) {
         const int row = idx / J, j = idx - row * J;
-        st_pair<T>(sU + ((size_t)buf * M + row) * RS + j, mk<T>(pre[r][0].x, pre[r][1].x),
+        st_pair<T>(sU + ((size_t)buf * M + row) * RS + L::pos(j), mk<T>(pre[r][0].x, pre[r][1].x),
                    mk<T>(pre[r][0].y, pre[r][1].y));
       }
     }
@@ -1846,14 +1887,14 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
   const T kerr = (T)d.one_minus_fR;
   const V kerr2 = mk<T>(kerr, kerr);
   V* sigma = as_t2<T>(d.sigma);
-  const int nsub = TB / kSrSub;
+  const int nsub = TB / L::S;
   fetch(0);
   park(0);
   __syncthreads();  // U of sub-block 0, the terms
   for (int sub = 0; sub < nsub; ++sub) {
-    const int buf = sub & 1;
-    if (sub + 1 < nsub) fetch(sub + 1);  // lands while this sub-block is worked on
-    else grid_release();
+    const int buf = WIDE ? 0 : sub & 1;
+    if (sub + 1 == nsub) grid_release();
+    else if (!WIDE) fetch(sub + 1);  // lands while this sub-block is worked on
     const SP* uc = sU + (size_t)buf * M * RS;
     // phase A
 #pragma unroll
@@ -1866,8 +1907,8 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
         const SP* vm = uc + lm[i].w * RS;
         SP* wq = sW + (size_t)q * RS;
         V Sr = sr[i], Si = si[i];
-#pragma unroll
-        for (int j = 0; j < J; ++j) {
+        // pair j of the slot: W of its two samples, by fields (REAL) or by parts
+        auto pair_w = [&](int j, V (&w)[2]) {
           const SP a = ld_pair<T>(ul + j), b = ld_pair<T>(um + j);
           V v0 = {}, v1 = {};  // REAL: Re V of the two fields, both samples
           if constexpr (REAL) {
@@ -1875,7 +1916,6 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
             v0 = pk_fma(a.re, b.re, pk_mul(a.im, b.im));
             v1 = pk_fma(a1.re, b1.re, pk_mul(a1.im, b1.im));
           }
-          V w[2];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             V x;  // V = U_l conj(U_m): (Re V, Im V), or the slot's two Re V
@@ -1896,11 +1936,29 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
               w[e] = x;
             }
           }
-          if constexpr (REAL) {
-            sW0[(size_t)q * RS + j] = mk<T>(w[0].x, w[1].x);
-            sW1[(size_t)q * RS + j] = mk<T>(w[0].y, w[1].y);
-          } else {
-            st_pair<T>(wq + j, mk<T>(w[0].x, w[1].x), mk<T>(w[0].y, w[1].y));
+        };
+        if constexpr (WIDE) {
+          float4* w0 = reinterpret_cast<float4*>(sW0 + (size_t)q * L::WS);
+          float4* w1 = reinterpret_cast<float4*>(sW1 + (size_t)q * L::WS);
+#pragma unroll 4
+          for (int h = 0; h < J / 2; ++h) {  // pairs 2h, 2h + 1
+            V w[2], y[2];
+            pair_w(L::pos(2 * h), w);
+            pair_w(L::pos(2 * h + 1), y);
+            w0[h] = make_float4(w[0].x, w[1].x, y[0].x, y[1].x);
+            w1[h] = make_float4(w[0].y, w[1].y, y[0].y, y[1].y);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < J; ++j) {
+            V w[2];
+            pair_w(j, w);
+            if constexpr (REAL) {
+              sW0[(size_t)q * L::WS + j] = mk<T>(w[0].x, w[1].x);
+              sW1[(size_t)q * L::WS + j] = mk<T>(w[0].y, w[1].y);
+            } else {
+              st_pair<T>(wq + j, mk<T>(w[0].x, w[1].x), mk<T>(w[0].y, w[1].y));
+            }
           }
         }
         sr[i] = Sr;
@@ -1908,60 +1966,100 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
       }
     }
     __syncthreads();  // W of this sub-block is complete
+    if (WIDE && sub + 1 < nsub) fetch(sub + 1);  // lands during phase B
     // phase B
     {
       const int j = lane & 7;
-      const int ts = t0 + sub * kSrSub;
+      const int ts = t0 + sub * L::S;
       for (int r = 0; r < rounds; ++r) {
         const int4 pl = sPlan[r * kSrGroups + warp * 4 + (lane >> 3)];  // p, first term, end, role
-        // sigma = U X summed over the terms: Re = a1 - a2, Im = a3 + a4 with a1 = sum Re U Re X,
-        // a2 = sum Im U Im X, a3 = sum Re U Im X, a4 = sum Im U Re X (packed over the pair)
-        V a1 = mk<T>(0, 0), a2 = a1, a3 = a1, a4 = a1;
-        // a mode's terms are sorted by k: U_k is read again only when k changes
-        SP u = {};
-        int kprev = -1;
+        if constexpr (WIDE) {
+          // sigma = U X summed over the terms, X = a Re W: Re and Im of the lane's pairs 2j, 2j + 1
+          V ra = mk<T>(0, 0), rb = ra, ia = ra, ib = ra;
+          SP u = {}, v = {};
+          int kprev = -1;
 #pragma unroll 2
-        for (int n = pl.y; n < pl.z; ++n) {
-          CF c;
-          unsigned kq;
-          ld_rec<T>(sRec + n, c, kq);
-          const int k = (int)(kq >> 16);
-          if (k != kprev) {
-            u = ld_pair<T>(uc + k * RS + j);
-            kprev = k;
+          for (int n = pl.y; n < pl.z; ++n) {
+            const Rec c = sRec[n];
+            const int k = (int)(c.kq >> 16);
+            if (k != kprev) {  // a mode's terms are sorted by k
+              u = ld_pair<T>(uc + k + j);
+              v = ld_pair<T>(uc + k + j + 8);
+              kprev = k;
+            }
+            const float4 w = *reinterpret_cast<const float4*>(sW0 + (c.kq & 0xffffu) + 2 * j);
+            const V c2 = mk<T>(c.ab, c.ab);
+            const V xa = pk_mul(c2, mk<T>(w.x, w.y)), xb = pk_mul(c2, mk<T>(w.z, w.w));
+            ra = pk_fma(u.re, xa, ra);
+            ia = pk_fma(u.im, xa, ia);
+            rb = pk_fma(v.re, xb, rb);
+            ib = pk_fma(v.im, xb, ib);
           }
-          if constexpr (REAL) {
-            const V xr = pk_mul(mk<T>(c.x, c.x), sW0[(kq & 0xffffu) + j]);  // X = a Re W
-            a1 = pk_fma(u.re, xr, a1);
-            a4 = pk_fma(u.im, xr, a4);
-          } else {
-            const SP w = ld_pair<T>(sW + (kq & 0xffffu) * RS + j);
-            const V xr = pk_mul(mk<T>(c.x, c.x), w.re), xi = pk_mul(mk<T>(c.y, c.y), w.im);  // X
-            a1 = pk_fma(u.re, xr, a1);
-            a2 = pk_fma(u.im, xi, a2);
-            a3 = pk_fma(u.re, xi, a3);
-            a4 = pk_fma(u.im, xr, a4);
+          // the upper half of a split mode (the next group, 8 lanes up) adds into the lower half
+          const V ra2 = shfl_down_c(ra, 8), ia2 = shfl_down_c(ia, 8);
+          const V rb2 = shfl_down_c(rb, 8), ib2 = shfl_down_c(ib, 8);
+          if (pl.w == 1) {
+            ra = cadd(ra, ra2);
+            ia = cadd(ia, ia2);
+            rb = cadd(rb, rb2);
+            ib = cadd(ib, ib2);
           }
+          if (pl.w <= 1) {
+            V* out = sigma + (size_t)pl.x * nt + ts + 4 * j;
+            st2<T>(out, mk<T>(ra.x, ia.x), mk<T>(ra.y, ia.y));
+            st2<T>(out + 2, mk<T>(rb.x, ib.x), mk<T>(rb.y, ib.y));
+          }
+        } else {
+          // sigma = U X summed over the terms: Re = a1 - a2, Im = a3 + a4 with a1 = sum Re U Re X,
+          // a2 = sum Im U Im X, a3 = sum Re U Im X, a4 = sum Im U Re X (packed over the pair)
+          V a1 = mk<T>(0, 0), a2 = a1, a3 = a1, a4 = a1;
+          // a mode's terms are sorted by k: U_k is read again only when k changes
+          SP u = {};
+          int kprev = -1;
+#pragma unroll 2
+          for (int n = pl.y; n < pl.z; ++n) {
+            CF c;
+            unsigned kq;
+            ld_rec<T>(sRec + n, c, kq);
+            const int k = (int)(kq >> 16);
+            if (k != kprev) {
+              u = ld_pair<T>(uc + k * RS + j);
+              kprev = k;
+            }
+            if constexpr (REAL) {
+              const V xr = pk_mul(mk<T>(c.x, c.x), sW0[(kq & 0xffffu) + j]);  // X = a Re W
+              a1 = pk_fma(u.re, xr, a1);
+              a4 = pk_fma(u.im, xr, a4);
+            } else {
+              const SP w = ld_pair<T>(sW + (kq & 0xffffu) * RS + j);
+              const V xr = pk_mul(mk<T>(c.x, c.x), w.re), xi = pk_mul(mk<T>(c.y, c.y), w.im);  // X
+              a1 = pk_fma(u.re, xr, a1);
+              a2 = pk_fma(u.im, xi, a2);
+              a3 = pk_fma(u.re, xi, a3);
+              a4 = pk_fma(u.im, xr, a4);
+            }
+          }
+          // the upper half of a split mode (the next group, 8 lanes up) adds into the lower half
+          const V b1 = shfl_down_c(a1, 8), b4 = shfl_down_c(a4, 8);
+          V b2 = {}, b3 = {};
+          if constexpr (!REAL) {
+            b2 = shfl_down_c(a2, 8);
+            b3 = shfl_down_c(a3, 8);
+          }
+          if (pl.w == 1) {
+            a1 = cadd(a1, b1);
+            a2 = cadd(a2, b2);
+            a3 = cadd(a3, b3);
+            a4 = cadd(a4, b4);
+          }
+          if (pl.w <= 1)
+            st2<T>(sigma + (size_t)pl.x * nt + ts + 2 * j, mk<T>(a1.x - a2.x, a3.x + a4.x), mk<T>(a1.y - a2.y, a3.y + a4.y));
         }
-        // the upper half of a split mode (the next group, 8 lanes up) adds into the lower half
-        const V b1 = shfl_down_c(a1, 8), b4 = shfl_down_c(a4, 8);
-        V b2 = {}, b3 = {};
-        if constexpr (!REAL) {
-          b2 = shfl_down_c(a2, 8);
-          b3 = shfl_down_c(a3, 8);
-        }
-        if (pl.w == 1) {
-          a1 = cadd(a1, b1);
-          a2 = cadd(a2, b2);
-          a3 = cadd(a3, b3);
-          a4 = cadd(a4, b4);
-        }
-        if (pl.w <= 1)
-          st2<T>(sigma + (size_t)pl.x * nt + ts + 2 * j, mk<T>(a1.x - a2.x, a3.x + a4.x), mk<T>(a1.y - a2.y, a3.y + a4.y));
       }
     }
-    // buffer buf ^ 1 was last read in the previous sub-block, which ended at a barrier
-    if (sub + 1 < nsub) park(buf ^ 1);
+    if constexpr (WIDE) __syncthreads();  // the one U buffer is free
+    // else buffer buf ^ 1 was last read in the previous sub-block, which ended at a barrier
+    if (sub + 1 < nsub) park(WIDE ? 0 : buf ^ 1);
     __syncthreads();  // W is free again; the next U is in place
   }
 }

@@ -96,3 +96,17 @@ def test_mixed_batch_gives_the_bits_of_each_alone(mmp, monkeypatch, form, M, nnz
         b.propagate(base.n_steps)
         for i, ref in enumerate(alone):
             assert np.array_equal(b.result(i), ref), i
+
+
+@pytest.mark.parametrize("M,nnz,nt,tile,raman", [(22, 1200, 64, 64, True), (23, 1200, 256, 64, True), (64, 1500, 128, 128, True),
+                                                 (22, 1200, 256, 128, False)])
+def test_tall_tiles_of_two_sub_blocks_and_up(mmp, monkeypatch, M, nnz, nt, tile, raman):
+    """The FP32 tall form takes 32 samples at a time: its shortest tiles, its most rows of U, odd slot counts."""
+    prob = W.small_case(seed=40 + M, M=M, nt=nt, n_steps=2, raman=raman, nnz_target=nnz, physical_order=True, peak_w=20.0)
+    monkeypatch.setenv("MMP_CONTRACT_TILE", str(tile))
+    out, info = _solve(mmp, prob)
+    assert info["contract_sub_block"] > 0 and info["contract_tile"] == tile
+    monkeypatch.setenv("MMP_REAL_PAIRS", "0")
+    ref, _ = _solve(mmp, prob)
+    assert mo.rel_l2_per_mode(out, ref).max() < 1e-6
+    assert mo.rel_l2_per_mode(out, mo.solve(prob)).max() < 1e-5
