@@ -121,6 +121,26 @@ __global__ void __launch_bounds__(256) k_check_finite(const double2* __restrict_
   if (__syncthreads_or(bad) && threadIdx.x == 0) *flag = 1;
 }
 
+// One CTA over a batch's solves: back to z = 0 (a call of propagate that is not a continuation),
+// and the OR of their status words. One launch each instead of a memset and a synchronous copy a
+// solve, which took 128 solves of 2 x 4096 about 1.5 ms a pass.
+__global__ void __launch_bounds__(256) k_restart(const SolveDesc* __restrict__ descs, int span) {
+  for (int i = threadIdx.x; i < span; i += blockDim.x)
+    if (descs[i].M) *descs[i].step = 0;
+}
+__global__ void __launch_bounds__(256) k_status(const SolveDesc* __restrict__ descs, int span, int* out) {
+  int bad = 0;
+  for (int i = threadIdx.x; i < span; i += blockDim.x)
+    if (descs[i].M) bad |= __ldcg(descs[i].status);
+  bad = (int)__reduce_or_sync(0xffffffffu, (unsigned)bad);
+  __shared__ int all;
+  if (threadIdx.x == 0) all = 0;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) atomicOr(&all, bad);
+  __syncthreads();
+  if (threadIdx.x == 0) *out = all;
+}
+
 // ---- device allocations: every one goes through dev_malloc / dev_free ------------------
 // Failure injection for tests (mmp_debug_fail_alloc): after `g_fail_after` more
 // successful allocations the next one fails as cudaErrorMemoryAllocation (-1: never).
@@ -714,7 +734,9 @@ struct mmp_batch {
   std::vector<Member> members;
   std::vector<uint8_t> active;
   SolveDesc* d_descs = nullptr;
-  int* d_flag = nullptr;  // set_fields' non-finite-input flag (in the d_descs allocation)
+  // Mapped host words that kernels write and the host reads after a stream synchronisation:
+  // [0] set_fields' non-finite-input flag, [1] the OR of the solves' status words
+  volatile int* words = nullptr;
   uint32_t span = 0;  // slots the kernels are launched over: highest active slot + 1
   // Served pools take solve state from a stream-ordered pool (no device-wide
   // synchronisation when a solve is admitted or retired); null: cudaMalloc/cudaFree.
@@ -1007,15 +1029,18 @@ int build_graph(mmp_batch* b, int steps) {
   return MMP_OK;
 }
 
-int check_status(mmp_batch* b) {
+// Waits for the batch's stream and reads its solves' status.
+int sync_status(mmp_batch* b) {
   int bad = 0;
-  for (auto& s : b->members) {
-    if (!s.block) continue;  // empty slot
-    int st = 0;
-    CUDA_TRY(cudaMemcpy(&st, (char*)s.counters + 3 * sizeof(unsigned long long), sizeof(int),
-                        cudaMemcpyDeviceToHost));
-    bad |= st;
+  if (b->span) {
+    b->words[1] = 0;
+    const SolveDesc* descs = b->d_descs;
+    int span = (int)b->span, *out = (int*)b->words + 1;
+    void* args[] = {(void*)&descs, &span, &out};
+    CUDA_TRY(launch((const void*)&k_status, dim3(1, 1, 1), 256, 0, 1, b->stream, args));
   }
+  CUDA_TRY(cudaStreamSynchronize(b->stream));
+  if (b->span) bad = b->words[1];
   if (bad & kStatusTimeout) return fail(MMP_ETIMEOUT, "a device-side bounded wait gave up");
   if (bad & kStatusNonFinite) return fail(MMP_ENONFINITE, "the field became NaN/Inf during propagation");
   if (bad & kStatusDrift)
@@ -1027,12 +1052,25 @@ int batch_propagate_async(mmp_batch* b, uint32_t nz) {
   if (!b) return fail(MMP_EINVAL, "NULL batch");
   mmp_detail::Range range("mmp.propagate");
   CUDA_TRY(cudaSetDevice(b->device));
+  uint32_t restarts = 0, used = 0;
+  for (auto& s : b->members) {
+    if (!s.block) continue;  // empty slot
+    ++used;
+    if (!(s.flags & MMP_F_CONTINUOUS)) ++restarts;
+  }
+  if (restarts == used && used > 1) {
+    const SolveDesc* descs = b->d_descs;
+    int span = (int)b->span;
+    void* args[] = {(void*)&descs, &span};
+    CUDA_TRY(launch((const void*)&k_restart, dim3(1, 1, 1), 256, 0, 1, b->stream, args));
+  }
   for (auto& s : b->members) {
     if (!s.block) continue;  // empty slot
     const bool continuous = (s.flags & MMP_F_CONTINUOUS) != 0;
     if (!continuous) {
       // initLawsonRK: z = 0 (src/MultimodePropagation.cpp:158-163)
-      CUDA_TRY(cudaMemsetAsync(s.counters, 0, sizeof(unsigned long long), b->stream));
+      if (restarts != used || used == 1)
+        CUDA_TRY(cudaMemsetAsync(s.counters, 0, sizeof(unsigned long long), b->stream));
       s.step_host = 0;
     }
     if (!(s.flags & MMP_F_NO_MONITORS)) {
@@ -1069,8 +1107,7 @@ int batch_propagate_async(mmp_batch* b, uint32_t nz) {
 int batch_sync(mmp_batch* b) {
   mmp_detail::Range range("mmp.synchronize");
   CUDA_TRY(cudaSetDevice(b->device));
-  CUDA_TRY(cudaStreamSynchronize(b->stream));
-  return check_status(b);
+  return sync_status(b);
 }
 
 int member_result(mmp_batch* b, uint32_t idx, double* out) {
@@ -1095,16 +1132,15 @@ int member_set_fields(mmp_batch* b, uint32_t idx, const double* phi0) {
   CUDA_TRY(cudaMemcpyAsync(s.desc.io, phi0, bytes, cudaMemcpyHostToDevice, b->stream));
   {
     // the fields are checked on the device copy, before anything of the solve changes
-    CUDA_TRY(cudaMemsetAsync(b->d_flag, 0, sizeof(int), b->stream));
     const double2* io = s.desc.io;
     size_t n = (size_t)s.M * s.nt;
-    int* flag = b->d_flag;
+    int* flag = (int*)b->words;
+    b->words[0] = 0;
     void* args[] = {(void*)&io, &n, &flag};
-    CUDA_TRY(launch((const void*)&k_check_finite, dim3(1184, 1, 1), 256, 0, 1, b->stream, args));
-    int bad = 0;
-    CUDA_TRY(cudaMemcpyAsync(&bad, b->d_flag, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
+    const unsigned grid = (unsigned)std::min<size_t>(1184, (n + 1023) / 1024);
+    CUDA_TRY(launch((const void*)&k_check_finite, dim3(grid, 1, 1), 256, 0, 1, b->stream, args));
     CUDA_TRY(cudaStreamSynchronize(b->stream));
-    if (bad) return fail(MMP_EINVAL, "initial fields not finite");
+    if (b->words[0]) return fail(MMP_EINVAL, "initial fields not finite");
   }
   // psi_hat = FFT(cf * phi0)   (src/MultimodePropagation.cpp:59-63 in the frequency domain)
   DftArgs a;
@@ -1115,20 +1151,11 @@ int member_set_fields(mmp_batch* b, uint32_t idx, const double* phi0) {
   a.scale = s.cf;
   a.tw = b->dev->tw[1][b->logn];
   a.lay = spec_layout(b->logn);
+  a.out_t = b->fp64 ? nullptr : (float2*)s.desc.psi_t;  // psi_hat rounded to T
+  a.restart = s.counters;  // z = 0, status, and the drift check's reference energy
   void* args[] = {&a};
   CUDA_TRY(launch(b->ks64.dft_fwd, dim3((unsigned)(s.M * b->ks64.C), 1, 1), b->ks64.nthr, b->ks64.smem,
                   b->ks64.C, b->stream, args));
-  if (!b->fp64) {  // psi_hat rounded to T
-    const double2* src = s.desc.psi_hat;
-    float2* dst = (float2*)s.desc.psi_t;
-    size_t n = (size_t)s.M * s.nt;
-    void* cargs[] = {(void*)&src, &dst, &n};
-    CUDA_TRY(launch((const void*)&k_to_t2<float>, dim3(1184, 1, 1), 256, 0, 1, b->stream, cargs));
-  }
-  CUDA_TRY(cudaMemsetAsync(s.counters, 0, sizeof(unsigned long long), b->stream));  // z = 0
-  CUDA_TRY(cudaMemsetAsync((char*)s.counters + 3 * sizeof(unsigned long long), 0, sizeof(int), b->stream));
-  // the drift check's reference energy: the first step's energy from these fields on
-  CUDA_TRY(cudaMemsetAsync((char*)s.counters + 4 * sizeof(unsigned long long), 0, sizeof(double), b->stream));
   s.step_host = 0;
   return MMP_OK;
 }
@@ -1153,8 +1180,8 @@ int batch_open(mmp_batch* b, const mmp_params* p0, const Tableau& tab0) {
   b->ks64 = kernels_for(1, b->logn);
   if (!b->ks.prime || !b->ks64.prime) return fail(MMP_ENOTSUP, "no kernels built for this nt");
   CUDA_TRY(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
-  CUDA_TRY(dev_malloc((void**)&b->d_descs, (size_t)b->capacity * sizeof(SolveDesc) + 16));
-  b->d_flag = reinterpret_cast<int*>(b->d_descs + b->capacity);
+  CUDA_TRY(dev_malloc((void**)&b->d_descs, (size_t)b->capacity * sizeof(SolveDesc)));
+  CUDA_TRY(cudaHostAlloc((void**)&b->words, 2 * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
   return MMP_OK;
 }
 
@@ -2139,7 +2166,7 @@ int mmp_batch_propagate_timed(mmp_batch* b, uint32_t nz, uint32_t repeats, doubl
   if (rc) return rc;
   if (e != cudaSuccess) return fail(MMP_ECUDA, cudaGetErrorString(e));
   *ms = f;
-  return check_status(b);
+  return sync_status(b);
 }
 
 int mmp_batch_profile(mmp_batch* b, uint32_t nz, double* ms_per_launch, uint32_t* launches) {
@@ -2209,6 +2236,7 @@ void mmp_batch_destroy(mmp_batch* b) {
   for (cudaEvent_t e : b->branch_ev) cudaEventDestroy(e);
   if (b->fork_ev) cudaEventDestroy(b->fork_ev);
   dev_free(b->d_descs);
+  if (b->words) cudaFreeHost((void*)b->words);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
 }

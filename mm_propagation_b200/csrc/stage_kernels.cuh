@@ -903,6 +903,10 @@ struct DftArgs {
   double scale;
   const void* tw;
   SpecLayout lay;
+  // forward, where not null: the spectrum in single precision too, and a solve's counters to
+  // clear (step, status, drift reference), so that new fields take one launch
+  float2* out_t;
+  unsigned long long* restart;
 };
 
 template <typename T, int LOGN, int XC, bool INV>
@@ -916,6 +920,11 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
   const size_t row = (size_t)p * Gm::N;
   V v[Gm::E];
   if constexpr (!INV) {
+    if (a.restart && blockIdx.x == 0 && threadIdx.x == 0) {
+      a.restart[0] = 0;
+      *reinterpret_cast<int*>(a.restart + 3) = 0;
+      a.restart[4] = 0;
+    }
     row_enter<Gm>();
 #pragma unroll
     for (int r = 0; r < Gm::E; ++r) v[r] = from_d2<T>(__ldcg(a.in + row + i0 + r * Gm::B));
@@ -929,8 +938,10 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
       RegDFT<Gm::RM, false>::run(w);
 #pragma unroll
       for (int r = 0; r < Gm::RM; ++r) {
-        const double2 y = to_d2(w[r]);
-        a.out[row + spec_pos(a.lay, k0 + r * Gm::KSTR)] = make_double2(y.x * a.scale, y.y * a.scale);
+        const double2 y = to_d2(w[r]), z = make_double2(y.x * a.scale, y.y * a.scale);
+        const size_t at = row + spec_pos(a.lay, k0 + r * Gm::KSTR);
+        a.out[at] = z;
+        if (a.out_t) a.out_t[at] = make_float2((float)z.x, (float)z.y);
       }
     });
     // no peer's shared memory is touched after row_first
