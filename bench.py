@@ -372,6 +372,12 @@ def read_ncu_traffic(kind: str, workload: str):
 
 
 # ---- CPU side: the reference's own solver in worker processes ------------------------------
+def reference_built() -> bool:
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import ref_lib
+    return ref_lib.available()
+
+
 def _ref_worker(q, spec):
     os.environ["OMP_NUM_THREADS"] = str(spec["threads"])
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
@@ -412,6 +418,8 @@ def run_reference_cpu(workload: str, n_members: int, steps: int, order: int, pea
 def reference_arm(args, dist):
     if dist.rank != 0:
         return None
+    if not reference_built():
+        return {"impl": "reference", "unavailable": "the reference's CPU solver is not built (its sources were not there)"}
     probe = make_problem(args.workload, 0, args.order, args.peak_w)
     steps = max(1, min(args.steps, {"grin6": 20, "grin2": 20, "dense15": 2}.get(args.workload, 1)))
     r = run_reference_cpu(args.workload, args.batch, steps, args.order, args.peak_w)
@@ -561,7 +569,7 @@ def ours_arm(args, dist):
     pc = bool(info.get("contract_pair_chunk", 0))
     sr = bool(info.get("contract_sub_block", 0))
     flops = stage_flops(probe, n_pairs, n_terms, raman_path, recurrence_in_contract=(raman_path == 2))
-    names = {"pair": ("k_pair", "k_raman_scan", "k_raman_agg+k_raman_carry")[raman_path],
+    names = {"pair": ("k_pair", "k_raman_scan", "k_raman_agg (and k_raman_carry where it runs)")[raman_path],
              "contract": ("k_contract_tc" if tc else "k_contract_sr" if sr else "k_contract_pc" if pc
                           else "k_contract"), "nu": "k_nu"}
     share = {k: prof[k]["ms_per_launch"] * prof[k]["launches"] for k in prof}
@@ -630,7 +638,7 @@ def ours_arm(args, dist):
     # the CPU baseline: the reference's solver on the host cores (rank 0, N=1 only), and
     # both precisions against its output after a few steps
     cpu = None
-    if dist.rank == 0 and dist.world == 1 and not args.no_accuracy:
+    if dist.rank == 0 and dist.world == 1 and not args.no_accuracy and reference_built():
         cs = args.cpu_steps
         keep = args.batch - 1
         r = run_reference_cpu(args.workload, args.batch, cs, args.order, args.peak_w, keep=keep)
