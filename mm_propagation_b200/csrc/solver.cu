@@ -218,6 +218,36 @@ struct DeviceRes {
 std::mutex g_dev_mu;
 std::map<int, DeviceRes> g_dev;
 
+// Mapped host words of the batches (mmp_batch::words), 64 bytes each. Allocating and freeing them a
+// batch took a solve's creation from 0.7 to 1.7-3.3 ms, so the first kWordSlots batches alive
+// share one allocation, kept for the process; further ones have their own.
+constexpr int kWordSlots = 256, kWordStride = 16;  // ints
+std::mutex g_words_mu;
+int* g_words = nullptr;
+std::vector<int> g_words_free;
+cudaError_t words_take(volatile int** out) {
+  std::lock_guard<std::mutex> lk(g_words_mu);
+  const unsigned how = cudaHostAllocPortable | cudaHostAllocMapped;
+  if (!g_words) {
+    int* block = nullptr;
+    const cudaError_t e = cudaHostAlloc((void**)&block, kWordSlots * kWordStride * sizeof(int), how);
+    if (e != cudaSuccess) return e;
+    for (int i = kWordSlots - 1; i >= 0; --i) g_words_free.push_back(i);
+    g_words = block;
+  }
+  if (g_words_free.empty()) return cudaHostAlloc((void**)out, kWordStride * sizeof(int), how);
+  *out = g_words + g_words_free.back() * kWordStride;
+  g_words_free.pop_back();
+  return cudaSuccess;
+}
+void words_give(volatile int* w) {  // no kernel that writes them is in flight
+  if (!w) return;
+  std::lock_guard<std::mutex> lk(g_words_mu);
+  const int* p = const_cast<const int*>(w);
+  if (p >= g_words && p < g_words + kWordSlots * kWordStride) g_words_free.push_back((int)(p - g_words) / kWordStride);
+  else cudaFreeHost((void*)p);
+}
+
 int ensure_device(int dev, DeviceRes** out) {
   std::lock_guard<std::mutex> lk(g_dev_mu);
   DeviceRes& r = g_dev[dev];
@@ -1181,7 +1211,7 @@ int batch_open(mmp_batch* b, const mmp_params* p0, const Tableau& tab0) {
   if (!b->ks.prime || !b->ks64.prime) return fail(MMP_ENOTSUP, "no kernels built for this nt");
   CUDA_TRY(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
   CUDA_TRY(dev_malloc((void**)&b->d_descs, (size_t)b->capacity * sizeof(SolveDesc)));
-  CUDA_TRY(cudaHostAlloc((void**)&b->words, 2 * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+  CUDA_TRY(words_take(&b->words));
   return MMP_OK;
 }
 
@@ -2236,7 +2266,7 @@ void mmp_batch_destroy(mmp_batch* b) {
   for (cudaEvent_t e : b->branch_ev) cudaEventDestroy(e);
   if (b->fork_ev) cudaEventDestroy(b->fork_ev);
   dev_free(b->d_descs);
-  if (b->words) cudaFreeHost((void*)b->words);
+  words_give(b->words);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
 }

@@ -52,3 +52,21 @@ def test_one_failing_solve_of_many_is_reported_until_it_gets_new_fields(mmp, whe
             assert np.isfinite(b.result(i)).all()
         b.set_fields(where, bad.initial_fields)
         b.propagate(2)  # clean again (these fields last two steps and not four)
+
+
+def test_more_solvers_alive_than_shared_words(mmp):
+    """Solvers share one block of mapped words (256 of them), further ones have their own; given back when closed."""
+    prob = W.small_case(seed=3, M=1, nt=64, n_steps=2, raman=False)
+    bad = np.full_like(prob.initial_fields, np.nan)
+    for _ in range(2):
+        solvers = [mmp.Solver(prob) for _ in range(260)]
+        out = []
+        for s in (solvers[0], solvers[255], solvers[259]):
+            with pytest.raises(mmp.MMPError):
+                s.set_fields(bad)
+            s.set_fields(prob.initial_fields)
+            s.propagate(2)
+            out.append(s.result())
+        for s in solvers:
+            s.close()
+        assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
