@@ -360,6 +360,16 @@ def read_measured_peaks():
     return 6650.0, "fallback"
 
 
+def symmetric_in_lm(prob) -> bool:
+    """Q_pklm = Q_pkml for every entry, to 1e-12 of the largest."""
+    q = {}
+    for e in prob.coupling:
+        key = (int(e["p"]), int(e["k"]), int(e["l"]), int(e["m"]))
+        q[key] = q.get(key, 0.0) + float(e["value"])
+    top = max(abs(v) for v in q.values())
+    return all(abs(v - q.get((p, k, m, l), 0.0)) <= 1e-12 * top for (p, k, l, m), v in q.items())
+
+
 def read_ncu_traffic(kind: str, workload: str):
     """dram bytes per launch from the committed ncu summary, scaled to this batch."""
     p = os.path.join(ROOT, "profiles", f"{kind}_{workload}.md")
@@ -571,6 +581,7 @@ def ours_arm(args, dist):
     flops = stage_flops(probe, n_pairs, n_terms, raman_path, recurrence_in_contract=(raman_path == 2))
     names = {"pair": ("k_pair", "k_raman_scan", "k_raman_agg (and k_raman_carry where it runs)")[raman_path],
              "contract": ("k_contract_tc" if tc else "k_contract_sr" if sr else "k_contract_pc" if pc
+                          else "k_contract_sp" if not info.get("dense_contraction") and info["contract_tile"] >= 64
                           else "k_contract"), "nu": "k_nu"}
     share = {k: prof[k]["ms_per_launch"] * prof[k]["launches"] for k in prof}
     tot = sum(share.values())
@@ -598,6 +609,8 @@ def ours_arm(args, dist):
         # and the useful GEMM work (8 M^4 NT per stage and solve) against the TF32 peak
         kc = kernels["contract"]
         tflops = tc_mma_flops(probe, n_pairs) * args.batch
+        if symmetric_in_lm(probe):  # the REAL form: one real product instead of two
+            tflops /= 2
         useful = 8.0 * probe.n_modes ** 4 * probe.nt * args.batch
         t = kc["ms_per_launch"] / 1e3
         t_tensor = tflops / (tpeak * 1e12)

@@ -9,20 +9,22 @@
 // to turn sigma into N_hat, instead of two of each.
 //
 // One RK stage i of step n is, with Raman on and h_R a damped sinusoid (every workload),
-// four launches; two with Raman off:
+// three launches; two with Raman off:
 //   k_raman_agg    per time tile:   the Raman recurrence's aggregate over the tile for
 //                                   every pair field V = U_l conj(U_m)
-//   k_raman_carry  per pair field:  tile aggregates -> the state entering each tile
-//   k_contract     per time tile:   R through the tile from that state, then
+//   k_contract_sp  per time tile:   the state entering the tile from the aggregates of the tiles
+//                                   before it (tile_carry; a response too long for that takes a
+//                                   k_raman_carry launch), R through the tile, then
 //                                   sigma_p = sum Q U_k [(1-fR) V_lm + R_lm] (all p)
-//                  (k_contract_pc for tiles with too many pair fields to hold at once,
-//                   k_contract_tc for dense Q on the tensor cores)
+//                  (k_contract_sr for tiles with too many pair fields to hold at once,
+//                   k_contract_tc for dense Q on the tensor cores, k_contract for short tiles and
+//                   the register-blocked dense form)
 //   k_nu           per mode p:      FFT(sigma_p) -> N_hat_i = i sgn(gamma) conj(E_i) *.,
 //                                   [last stage: psi_hat += h sum b_j N_hat_j, monitors],
 //                                   x_hat = psi_hat + h sum a_{i+1,j} N_hat_j,
 //                                   * E_{i+1} -> IFFT -> U for the next stage
 // Any other h_R takes k_pair (V -> FFT -> * H_R -> IFFT = R per pair field) instead of
-// the first two, and k_contract reads R as rows. k_prime makes U for stage 0 when a
+// the first, and the contraction reads R as rows. k_prime makes U for stage 0 when a
 // propagate call starts. E_i = exp(i Im L_p(w) z) is never stored: the phase
 // Im L_p(w) * (z_n + c_i h) is evaluated in FP64, reduced in FP64 and only then passed
 // to sin/cos in T.
@@ -2080,7 +2082,9 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
 // start, S_end = sum_t lambda^(TB-1-t) x_t (x = Re V, Im V, V = U_l conj(U_m)), run as
 // S <- lambda S + x sample after sample (the arithmetic of k_contract_sr's phase A without
 // the output), U arriving in sub-blocks of kSrSub samples through the same double buffer.
-// k_raman_carry turns the aggregates into the states entering the tiles.
+// The contraction's tiles (tile_carry), or k_raman_carry, make the states entering the tiles of them.
+// Shared-memory reads of U bound it (l1tex 88% busy): 8 solves of 28 x 65536 with 203 slots, 105 us a
+// launch; skipping the second row where a slot's two fields share a mode made it 134.
 template <typename T, bool REAL>
 __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
     k_raman_agg_sr(const SolveDesc* __restrict__ descs, int nt, int TB, int by_tile) {
@@ -2206,7 +2210,8 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
 // What bounds it: issue (62% of cycles on 28 warps), then the latency of the tile. Measured on a
 // B200 against the scalar term loop over unmerged terms (k_contract<T, 0>), a launch: 32 solves
 // of 6 x 16384 (21 pair fields) 56 -> 44 us, 38.2 -> 27.8 million warp instructions; 128 of
-// 2 x 4096 29 -> 24 us; a step of one 6 x 8192 FP64 solve 112 -> 96 us.
+// 2 x 4096 29 -> 24 us; a step of one 6 x 8192 FP64 solve 112 -> 96 us. REAL form (11 slots for
+// the 21 pair fields): 45 -> 41 us.
 template <typename T> struct LaneScan {
   using V = c2<T>;
   V lr2, li2, nli2, kr2, ki2;  // lambda and kappa, each component in both lanes
@@ -2509,7 +2514,8 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
 // with 46 KB: 15.6 thousand of a CTA's 31 thousand cycles), then the CTA's start and end (7
 // thousand). Measured on a B200, 16 solves of 15 x 8192, a launch, against two 16-field buffers
 // between barriers of the whole CTA and scalar recurrences: 183 -> 141 us, 64 -> 44 million warp
-// instructions (24 builder warps instead of 16: 143).
+// instructions (24 builder warps instead of 16: 143). REAL form (one product over all fields, half the
+// recurrences, operands and MMAs; two CTAs an SM): 76 us.
 constexpr int kTcBuilders = 2;  // chunks built at a time, a warp per slot
 template <bool REAL> constexpr int tc_threads() { return 32 * (slot_count<REAL>(kTcChunk) * kTcBuilders + 1); }
 
