@@ -117,8 +117,8 @@ typedef struct mmp_info {
   uint32_t contract_pair_chunk;             /* > 0: pair fields held per chunk by the contraction
                                                of tall tiles (Raman recurrence in the tiles) */
   uint32_t contract_sub_block;              /* > 0: the contraction of tall tiles runs the Raman
-                                               recurrence serially per pair field, in sub-blocks of
-                                               this many samples (merged terms) */
+                                               recurrence serially per pair field, in units of this
+                                               many samples (merged terms) */
   uint32_t contract_tile;                   /* samples per contraction tile (CTA) */
   uint32_t autotuned;                       /* 1: cluster_ctas, contract_tile and graph_branches
                                                were chosen by timing steps of this batch on
@@ -333,6 +333,11 @@ int mmp_debug_fail_alloc(int64_t after);
  * 2^24, far above any copy time); 0 makes that bounded wait give up at once, so the
  * propagate call reports MMP_ETIMEOUT (the copies still land before a CTA leaves). */
 int64_t mmp_debug_live_allocations(void);
+/* Which kernels member `index` of a batch runs (either pointer may be NULL): *merged_terms = 1
+ * when its contraction reads merged terms over tiles of 64 to 256 samples, 0 for the term loop
+ * and the dense, tensor-core and tall-tile forms; *real_pairs = 1 when only the real parts of
+ * its pair fields are formed (a coupling symmetric in (l, m)), 0 in the general form. */
+int mmp_debug_batch_form(mmp_batch* b, uint32_t index, uint32_t* merged_terms, uint32_t* real_pairs);
 
 #ifdef __cplusplus
 }

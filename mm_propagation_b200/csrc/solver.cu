@@ -2475,6 +2475,15 @@ int mmp_debug_fail_alloc(int64_t after) {
 
 int64_t mmp_debug_live_allocations(void) { return g_live.load(); }
 
+int mmp_debug_batch_form(mmp_batch* b, uint32_t index, uint32_t* merged_terms, uint32_t* real_pairs) {
+  if (!b || index >= b->members.size()) return fail(MMP_EINVAL, "bad form arguments");
+  const Member& s = b->members[index];
+  const bool dense = b->dense == 1 || (b->dense == 2 && s.dense_ok);
+  if (merged_terms) *merged_terms = b->sp && !dense ? 1 : 0;
+  if (real_pairs) *real_pairs = s.desc.real ? 1 : 0;
+  return MMP_OK;
+}
+
 }  // extern "C"
 
 // serving loop (mmp_server_*): slot pools built on the batch machinery above
