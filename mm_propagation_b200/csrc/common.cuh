@@ -79,13 +79,15 @@ static_assert(sizeof(Term) == 16, "Term layout");
 // physical one is, reads a pair field only as W_lm + W_ml = 2 Re W_lm (and Im W_ll is 0): every merged
 // term's b is 0 (up to rounding, host_setup). Raman's convolution is real, so Re W needs Re V
 // alone, and two pair fields 2 s and 2 s + 1 share one slot s: x_s = Re V_{2s} + i Re V_{2s+1} goes
-// through the same recurrence or
-// transform as one complex V_q, for half the work, and comes out as W_{2s} + i W_{2s+1}. In
-// the general form slot q holds V_q. Per-slot data (tile aggregates, carries, R rows) have the
-// same shape in both. The form is a solve's own (SolveDesc::real); a batch that holds both
-// launches one kernel for each, which skips the other's solves. Measured on a B200, a launch of the
-// contraction, general against REAL: dense 16 x 15 x 8192 141 -> 76 us, 8 x 28 x 65536 519 -> 420,
-// 32 x 6 x 16384 45 -> 41; k_pair has half the rows.
+// through the same recurrence as one complex V_q, for half the work, and comes out as
+// W_{2s} + i W_{2s+1}. The two parts of a recurrence never meet, so each field keeps its own rounding. A
+// complex transform would mix them (its rounding is relative to the stronger part: the mode
+// a weak field drives came out wrong by 6% next to one 1e8 times as strong), so solves whose
+// convolution runs by transforms keep the general form. In the general form slot q holds V_q. Per-slot
+// data (tile aggregates, carries) have the same shape in both. The form is a solve's own
+// (SolveDesc::real); a batch that holds both launches one kernel for each, which skips the other's
+// solves. Measured on a B200, a launch of the contraction, general against REAL: dense
+// 16 x 15 x 8192 141 -> 76 us, 8 x 28 x 65536 519 -> 420, 32 x 6 x 16384 45 -> 41.
 template <bool REAL> __host__ __device__ constexpr int slot_count(int P) { return REAL ? (P + 1) >> 1 : P; }
 
 // Everything a kernel needs about one solve. Lives in device memory (an array

@@ -22,8 +22,7 @@ KernelSet MMP_CAT4(make_kernels_, MMP_TAG, MMP_LOGN, MMP_XC)() {
   using Gm = Geo<T, L, X>;
   KernelSet k;
   k.prime = (const void*)&k_prime<T, L, X>;
-  k.pair = (const void*)&k_pair<T, L, X, false>;
-  k.pair_real = (const void*)&k_pair<T, L, X, true>;
+  k.pair = (const void*)&k_pair<T, L, X>;
   k.nu = (const void*)&k_nu<T, L, X, -1>;
   // specialised stage bodies: RK4's (0 and last-3), the order-6 and order-8 tableaus'
   // (intermediate 1..5, last 4)

@@ -9,7 +9,6 @@ namespace mmp {
 struct KernelSet {
   const void* prime = nullptr;
   const void* pair = nullptr;
-  const void* pair_real = nullptr;   // ... in the REAL form (common.cuh)
   const void* nu = nullptr;          // k_nu for any stage
   const void* nu_mid[6] = {};        // ... for intermediate stages reading n stored N_hat_j
   const void* nu_last[5] = {};       // ... for last stages reading n (null: not built)

@@ -300,7 +300,7 @@ int ensure_device(int dev, DeviceRes** out) {
     for (int L = kMinLogN; L <= kMaxLogN; ++L)
       for (int xc = 0; xc <= max_split(fp64 != 0, L); ++xc) {
         KernelSet ks = kernels_for(fp64, L, xc);
-        std::vector<const void*> fns = {ks.prime, ks.pair, ks.pair_real, ks.nu, ks.result, ks.dft_fwd, ks.dft_inv};
+        std::vector<const void*> fns = {ks.prime, ks.pair, ks.nu, ks.result, ks.dft_fwd, ks.dft_inv};
         for (const void* f : ks.nu_mid) fns.push_back(f);
         for (const void* f : ks.nu_last) fns.push_back(f);
         for (const void* f : fns)
@@ -929,7 +929,7 @@ int step_kernels(const mmp_batch* b) {
   const int forms = (int)b->forms[0] + (int)b->forms[1];
   int n = 1 + forms * ((b->sr || b->pchunk || b->tc || b->dense != 2) ? 1 : 2);
   if (b->raman && b->Pmax > 0)
-    n += b->raman_iir && !b->raman_fused ? 1 : forms + (b->raman_fused && !b->lookback ? 1 : 0);
+    n += b->raman_fused ? forms + (b->lookback ? 0 : 1) : 1;
   return b->tab.s * n;
 }
 
@@ -952,15 +952,13 @@ int launch_pairs(mmp_batch* b, const KernelSet& ks, int nsolves, int stage, cons
   const size_t t2 = b->fp64 ? sizeof(double2) : sizeof(float2);
   const SolveDesc* dd = descs;
   if (!st) st = b->stream;
-  if (!b->raman_iir || b->raman_fused) {
+  if (!b->raman_iir) return launch_row_kernel(b, ks, ks.pair, b->Pmax, nsolves, stage, descs, st, true);
+  if (b->raman_fused) {
     for (int real = 0; real < 2; ++real) {  // a launch for each form among the solves
       if (!b->forms[real]) continue;
       void* args[] = {(void*)&dd, &nt, &TT, &by_tile};
       const dim3 grid((unsigned)(nt / TT), (unsigned)nsolves, 1);
-      if (!b->raman_iir) {
-        int rc = launch_row_kernel(b, ks, real ? ks.pair_real : ks.pair, b->slots, nsolves, stage, descs, st, true);
-        if (rc) return rc;
-      } else if (b->sr) {  // one thread per slot through the tile (k_contract_sr's tiles)
+      if (b->sr) {  // one thread per slot through the tile (k_contract_sr's tiles)
         const int smem = (int)(2 * (size_t)b->Mmax * (kSrSub / 2 + 1) * 2 * t2);
         CUDA_TRY(launch(agg_sr_fn(b->fp64, real), grid, kSrThreads, smem, 1, st, args, true));
       } else {
@@ -968,7 +966,7 @@ int launch_pairs(mmp_batch* b, const KernelSet& ks, int nsolves, int stage, cons
         CUDA_TRY(launch(agg_fn(b->fp64, real), grid, 256, smem, 1, st, args, true));
       }
     }
-    if (!b->raman_iir || b->lookback) return MMP_OK;
+    if (b->lookback) return MMP_OK;
     void* cargs[] = {(void*)&dd, &nt, &TT};
     const void* fc = b->fp64 ? (const void*)&k_raman_carry<double> : (const void*)&k_raman_carry<float>;
     CUDA_TRY(launch(fc, dim3((unsigned)b->slots, (unsigned)nsolves, 1), 32, 0, 1, st, cargs, true));
@@ -1387,13 +1385,8 @@ int iir_len(double decay, bool fp64) {
 }
 
 // Does the REAL form pay? With up to 8 pair fields, one to a warp of the contraction, halving them
-// saves no pass over them (128 solves of 2 x 4096: 158 against 154 us a step); a Raman convolution
-// by transforms always has fewer rows.
-bool real_pays(size_t pairs, bool raman, const mmp_params* p) {
-  if (pairs > 8) return true;
-  std::complex<double> lam, c;
-  return raman && pairs > 1 && !fit_damped_sinusoid(p->raman_response, p->nt, lam, c);
-}
+// saves no pass over them (128 solves of 2 x 4096: 158 against 154 us a step).
+bool real_pays(size_t pairs) { return pairs > 8; }
 
 // Host setup, device state and uploads for slot idx from params p; leaves the solve
 // at z = 0 with its initial fields transformed. One cudaMalloc for all of it.
@@ -1444,7 +1437,7 @@ int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
   d.P = (int)P;
   d.n_beta = (int)s.n_beta;
   d.raman = b->raman ? 1 : 0;
-  s.real_ok = s.symmetric && real_pays(s.pairs.size(), b->raman, p);
+  s.real_ok = s.symmetric && real_pays(s.pairs.size());
   d.real = s.real_ok ? 1 : 0;  // batch_shape turns it off where the kernels chosen have no such form
   d.alpha_scale = 2 * M_PI / s.t_final;
   d.dz = s.delta_z;
@@ -1778,7 +1771,7 @@ Shape choose_shape(const mmp_batch* b, const ShapeStats& st, bool try_real = tru
   if (const char* env = std::getenv("MMP_CONTRACT_SP"))
     if (std::atoi(env) == 0) sp = false;
   if (real && (!(tc || sr || sp || dense == 1) || (dense == 2 && !sp) || (tall && !sr) ||
-               (b->raman && !fused && (iir || dense))))  // k_raman_scan, and R rows for the dense form
+               (b->raman && !fused)))  // R from rows: complex fields (common.cuh)
     return choose_shape(b, st, false);
   const int stage_terms = sr || (sp && !dense) ? 0 : (pchunk ? 1 : (dense != 1 && !tc && smem + max_terms * staged <= 200 * 1024 ? 1 : 0));
   if (stage_terms && !pchunk) smem += max_terms * staged;
@@ -1822,7 +1815,7 @@ SolveCounts solve_counts(const mmp_params* p) {
     if (c.iir) c.iir_decay = -std::log(std::abs(lam));
   }
   c.dense_ok = dense_wanted(nullptr, m);
-  c.real_ok = m.symmetric && real_pays(m.pairs.size(), p->raman != 0, p);
+  c.real_ok = m.symmetric && real_pays(m.pairs.size());
   return c;
 }
 

@@ -296,15 +296,15 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
 }
 
 // ---- k_pair: R_q = IFFT(FFT(V_q) * H), V_q = U_l conj(U_m) -------------------------------
-// One slot per row; the REAL form stores R's two fields as two real rows.
-template <typename T, int LOGN, int XC, bool REAL>
+// One pair field per row (common.cuh: why never two).
+template <typename T, int LOGN, int XC>
 __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_BLOCKS) k_pair(const KParams kp) {
   using Gm = Geo<T, LOGN, XC>;
   using V = c2<T>;
   MMP_ROW_SETUP();
   const SolveDesc* gd = kp.descs + blockIdx.y;
   const int q = blockIdx.x / Gm::C;
-  if (q >= slot_count<REAL>(__ldg(&gd->P)) || __ldg(&gd->real) != REAL) {  // other form; uniform over the cluster
+  if (q >= __ldg(&gd->P)) {  // uniform over the cluster
     grid_sync_wait();
     return;
   }
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
   const V* U = as_t2<T>(static_cast<const void*>(ldg_ptr(&gd->U))) + i0;
   const V* H = as_t2<T>(static_cast<const void*>(ldg_ptr(&gd->H)));
   V* W = as_t2<T>(ldg_ptr(&gd->W));
-  const int4 lm = slot_rows<REAL>(*gd, q);
+  const int4 lm = slot_rows<false>(*gd, q);
   grid_sync_wait();
   if (__ldcg(step) >= __ldg(&gd->step_limit)) return;  // uniform over the cluster
   row_enter<Gm>();
@@ -321,13 +321,8 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
   {
     const V* Ul = U + (size_t)lm.x * Gm::N;
     const V* Um = U + (size_t)lm.y * Gm::N;
-    const V* Ul1 = U + (size_t)lm.z * Gm::N;
-    const V* Um1 = U + (size_t)lm.w * Gm::N;
 #pragma unroll
-    for (int r = 0; r < Gm::E; ++r) {
-      const V l1 = REAL ? ld_stream(Ul1 + r * Gm::B) : V(), m1 = REAL ? ld_stream(Um1 + r * Gm::B) : V();
-      v[r] = slot_value<REAL>(ld_stream(Ul + r * Gm::B), ld_stream(Um + r * Gm::B), l1, m1);
-    }
+    for (int r = 0; r < Gm::E; ++r) v[r] = cmulc(ld_stream(Ul + r * Gm::B), ld_stream(Um + r * Gm::B));
   }
   row_first<Gm>(v, s, tw, rank);
   rows_fwd<Gm>(sr, tw, u);
@@ -348,18 +343,9 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
   row_last_inv<Gm>(v, s, tw, rank);
   // R_q = (H_R conv V_q); the Kerr part (1 - fR) V_q is formed by the contraction from
   // the U tile it already holds
-  if constexpr (REAL) {
-    T* R = reinterpret_cast<T*>(W) + (size_t)(2 * q) * Gm::N + i0;
+  V* R = W + (size_t)q * Gm::N + i0;
 #pragma unroll
-    for (int r = 0; r < Gm::E; ++r) {
-      R[r * Gm::B] = v[r].x;
-      R[Gm::N + r * Gm::B] = v[r].y;
-    }
-  } else {
-    V* R = W + (size_t)q * Gm::N + i0;
-#pragma unroll
-    for (int r = 0; r < Gm::E; ++r) R[r * Gm::B] = v[r];
-  }
+  for (int r = 0; r < Gm::E; ++r) R[r * Gm::B] = v[r];
   row_leave<Gm>();
 }
 
@@ -2314,16 +2300,15 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
   LaneScan<T> ts;
   if (raman_mode >= 2) ts.init(d, TT >> 5, lane);
   if (tid == 0) mbar_init(&bar, 1);
-  const int Pl = raman_mode == 1 ? (REAL ? 2 * P : P) : 0;  // rows of R loaded
-  const unsigned row_bytes = (unsigned)(TT * sizeof(V)), r_bytes = REAL ? row_bytes / 2 : row_bytes;
-  if (tid == 0) mbar_arrive_expect_tx(&bar, (unsigned)M * row_bytes + (unsigned)Pl * r_bytes);
+  const int Pl = !REAL && raman_mode == 1 ? P : 0;  // rows of R loaded (never in the REAL form)
+  const unsigned row_bytes = (unsigned)(TT * sizeof(V));
+  if (tid == 0) mbar_arrive_expect_tx(&bar, (unsigned)(M + Pl) * row_bytes);
   __syncthreads();
   grid_sync_wait();
   for (int r = tid; r < M; r += blockDim.x)
     bulk_g2s(sU + (size_t)r * H, as_t2<T>(d.U) + (size_t)r * nt + t0, row_bytes, &bar);
   for (int r = tid; r < Pl; r += blockDim.x)
-    bulk_g2s(reinterpret_cast<char*>(sW) + (size_t)r * r_bytes,
-             static_cast<const char*>(d.W) + ((size_t)r * nt + t0) * (r_bytes / TT), r_bytes, &bar);
+    bulk_g2s(sW + (size_t)r * H, as_t2<T>(d.W) + (size_t)r * nt + t0, row_bytes, &bar);
   if (__ldcg(d.step) >= d.step_limit) {  // finished solve: the copies land before the CTA leaves
     mbar_wait(&bar, 0, kMaxWaitPolls);
     return;
@@ -2428,15 +2413,8 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
         vre = real_product(ld_pair<T>(sU + lm.x * H + at), ld_pair<T>(sU + lm.y * H + at));
         vim = real_product(ld_pair<T>(sU + lm.z * H + at), ld_pair<T>(sU + lm.w * H + at));
         V* w0 = sR + 2 * (size_t)(i - h);
-        V* w1 = w0 + H;
-        if (raman_mode == 1) {  // W = (1 - f_R) V + R, R in place as it landed
-          const V r0 = w0[h], r1 = w1[h];
-          vre = pk_fma(mk<T>(kerr, kerr), vre, r0);
-          vim = pk_fma(mk<T>(kerr, kerr), vim, r1);
-          __syncwarp();
-        }
         w0[rs<T>(h, wmask)] = vre;
-        w1[rs<T>(h, wmask)] = vim;
+        w0[H + rs<T>(h, wmask)] = vim;
         continue;
       }
       SP* row = sW + (i - h);
