@@ -331,7 +331,9 @@ int mmp_debug_fail_alloc(int64_t after);
  * The environment variable MMP_TILE_WAIT_POLLS, read when a solve is created, sets how
  * many polls the contraction kernels give the first wait for their tile copy (default
  * 2^24, far above any copy time); 0 makes that bounded wait give up at once, so the
- * propagate call reports MMP_ETIMEOUT (the copies still land before a CTA leaves). */
+ * propagate call reports MMP_ETIMEOUT (the copies still land before a CTA leaves).
+ * MMP_STAGE_WAIT_POLLS does the same for the waits between the tensor-core contraction's
+ * builder warps and the thread that issues its matrix instructions. */
 int64_t mmp_debug_live_allocations(void);
 /* Which kernels member `index` of a batch runs (either pointer may be NULL): *merged_terms = 1
  * when its contraction reads merged terms over tiles of 64 to 256 samples, 0 for the term loop

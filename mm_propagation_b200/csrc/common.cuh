@@ -98,7 +98,7 @@ struct SolveDesc {
   int n_beta;       // polynomial coefficients per mode
   int raman;        // 1: Raman on (contraction adds R = h_R (*) V to (1-fR) V)
   int real;         // 1: the Raman and contraction kernels run this solve in the REAL form
-  int pad1_;
+  unsigned stage_wait_polls;  // polls of k_contract_tc's waits for an operand stage
   double alpha_scale;   // 2*pi / t_final
   double dz;            // h (dimensionless)
   double sgn_gamma;     // +1 / -1

@@ -1309,9 +1309,10 @@ constexpr int kCounterWords = 6;
 
 // Polls the contraction kernels give the first wait for their tile copy: far above any
 // copy time. MMP_TILE_WAIT_POLLS (read when a solve is created) lowers it, for tests that
-// make that bounded wait run out and check that the call reports MMP_ETIMEOUT.
-unsigned tile_wait_polls() {
-  if (const char* env = std::getenv("MMP_TILE_WAIT_POLLS"))
+// make that bounded wait run out and check that the call reports MMP_ETIMEOUT. MMP_STAGE_WAIT_POLLS
+// does the same for the tensor-core kernel's waits for its operand stages.
+unsigned wait_polls(const char* name) {
+  if (const char* env = std::getenv(name))
     if (*env) return (unsigned)std::strtoul(env, nullptr, 10);
   return kMaxWaitPolls;
 }
@@ -1481,7 +1482,8 @@ int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
   d.drift_tol = 0.0;
   d.monitors = (s.flags & MMP_F_NO_MONITORS) ? 0 : 1;
   d.step_limit = ~0ull;
-  d.tile_wait_polls = tile_wait_polls();
+  d.tile_wait_polls = wait_polls("MMP_TILE_WAIT_POLLS");
+  d.stage_wait_polls = wait_polls("MMP_STAGE_WAIT_POLLS");
   if (b->raman) {
     std::complex<double> lam, c;
     if (fit_damped_sinusoid(p->raman_response, (uint32_t)nt, lam, c)) {

@@ -2497,14 +2497,19 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : 2))
 constexpr int kTcBuilders = 2;  // chunks built at a time, a warp per slot
 template <bool REAL> constexpr int tc_threads() { return 32 * (slot_count<REAL>(kTcChunk) * kTcBuilders + 1); }
 
-// mbar_wait that also gives up once *stop is set (by another warp whose wait ran out)
-__device__ __forceinline__ bool mbar_wait_or(unsigned long long* bar, unsigned parity, volatile int* stop) {
-  for (unsigned it = 0; it < kMaxWaitPolls; it += 64) {
+// mbar_wait that also gives up once *stop is set (by another warp whose wait ran out). The answer is
+// a thread's own: two lanes may see the barrier complete and *stop set in either order.
+__device__ __forceinline__ bool mbar_wait_or(unsigned long long* bar, unsigned parity, volatile int* stop, unsigned polls) {
+  for (unsigned it = 0; it < polls; it += 64) {
     if (mbar_wait(bar, parity, 64)) return true;
     if (*stop) return false;
   }
   *stop = 1;
   return false;
+}
+// ... for a whole warp: one answer for its lanes, which meet again at full-mask shuffles
+__device__ __forceinline__ bool mbar_wait_or_warp(unsigned long long* bar, unsigned parity, volatile int* stop, unsigned polls) {
+  return __all_sync(0xffffffffu, mbar_wait_or(bar, parity, stop, polls));
 }
 __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
@@ -2544,6 +2549,7 @@ __global__ void __launch_bounds__(tc_threads<REAL>(), REAL ? 2 : 1) k_contract_t
   V* sC = reinterpret_cast<V*>(sB + NS * MATS * KC * N);          // states entering the tile, [PS][2]
   const int nch = (P + KC - 1) / KC;
   const unsigned bbytes = (unsigned)(MATS * KC * N * sizeof(float));
+  const unsigned polls = d.stage_wait_polls;
   LaneScan<float> ts;
   if (raman_mode >= 2) ts.init(d, TT >> 5, lane);
   if (tid == 0) {
@@ -2594,7 +2600,7 @@ __global__ void __launch_bounds__(tc_threads<REAL>(), REAL ? 2 : 1) k_contract_t
     for (int c = warp / SC; c < nch; c += kTcBuilders) {
       const int buf = c % NS, q = c * SC + f;
       // chunk c - NS's MMAs read this buffer pair
-      if (c >= NS && !mbar_wait_or(&bar_m[buf], ((c / NS) - 1) & 1, &s_stop)) break;
+      if (c >= NS && !mbar_wait_or_warp(&bar_m[buf], ((c / NS) - 1) & 1, &s_stop, polls)) break;
       // lane L's samples 4L .. 4L + 3 of a field: one 16-byte chunk of each operand matrix; the
       // slot's second component goes to the Im matrices, or (REAL) is the next field
       float* a0 = sA + (size_t)buf * MATS * KC * TT + tc::mn_tf32_offset(4 * lane, REAL ? 2 * f : f, A_LBO, A_SBO) / 4;
@@ -2654,7 +2660,7 @@ __global__ void __launch_bounds__(tc_threads<REAL>(), REAL ? 2 : 1) k_contract_t
     for (int c = 0; c < nch; ++c) {
       const int buf = c % NS;
       const unsigned par = (c / NS) & 1;
-      if (!mbar_wait_or(&bar_b[buf], par, &s_stop) || !mbar_wait_or(&bar_a[buf], par, &s_stop)) break;
+      if (!mbar_wait_or(&bar_b[buf], par, &s_stop, polls) || !mbar_wait_or(&bar_a[buf], par, &s_stop, polls)) break;
       tc::fence_after_sync();
       const float* A = sA + (size_t)buf * MATS * KC * TT;
       const float* B = sB + (size_t)buf * MATS * KC * N;
@@ -2673,12 +2679,12 @@ __global__ void __launch_bounds__(tc_threads<REAL>(), REAL ? 2 : 1) k_contract_t
       tc::commit(&bar_m[buf]);
       committed = c + 1;
       if (c >= 1 && c - 1 + NS < nch) {  // once chunk c - 1 is done, its coefficients may be replaced
-        if (!mbar_wait_or(&bar_m[(c - 1) % NS], ((c - 1) / NS) & 1, &s_stop)) break;
+        if (!mbar_wait_or(&bar_m[(c - 1) % NS], ((c - 1) / NS) & 1, &s_stop, polls)) break;
         copy_b(c - 1 + NS);
       }
     }
     // the last chunk's MMAs complete after all earlier ones (in-order issue, one thread)
-    if (committed == nch && nch > 0) mbar_wait_or(&bar_m[(nch - 1) % NS], ((nch - 1) / NS) & 1, &s_stop);
+    if (committed == nch && nch > 0) mbar_wait_or(&bar_m[(nch - 1) % NS], ((nch - 1) / NS) & 1, &s_stop, polls);
   }
   grid_release();
   ok = __syncthreads_and(ok && !s_stop ? 1 : 0);
