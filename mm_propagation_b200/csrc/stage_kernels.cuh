@@ -84,7 +84,8 @@ __device__ __forceinline__ double alpha_of(int k, int nt, double alpha_scale) {
 // series of sin and cos to x^9 and x^10 (truncation below 2e-9 on that interval),
 // evaluated by Horner in x^2 in FP32; the quadrant swaps and negates. Short, branch-free
 // code with no large-argument path (the argument is already small). FP64: the same reduction
-// and the series to x^17 and x^16 (truncation below 1e-19 and 2e-18).
+// (a finite theta beyond its range ends on the unit circle too) and the series to x^17 and x^16
+// (truncation below 1e-19 and 2.1e-18).
 template <typename T> __device__ __forceinline__ c2<T> expi(double theta) {
   if constexpr (sizeof(T) == 4) {
     constexpr double k2OverPi = 0.63661977236758134308;
@@ -112,7 +113,9 @@ template <typename T> __device__ __forceinline__ c2<T> expi(double theta) {
     constexpr double kRound = 6755399441055744.0;
     const double t = fma(theta, k2OverPi, kRound);
     const double n = t - kRound;
-    const double x = fma(-n, kHalfPiLo, fma(-n, kHalfPiHi, theta)), x2 = x * x;
+    double x = fma(-n, kHalfPiLo, fma(-n, kHalfPiHi, theta));
+    x = fabs(x) > 1.0 ? 0.0 : x;  // |theta| > 3.5e15, whose own spacing is 0.5 or more: some point of the circle
+    const double x2 = x * x;
     double sp = 1.0 / 355687428096000.0, cp = 1.0 / 20922789888000.0;  // 1/17!, 1/16!
     constexpr double sc[7] = {-1.0 / 1307674368000.0, 1.0 / 6227020800.0, -1.0 / 39916800.0, 1.0 / 362880.0,
                               -1.0 / 5040.0, 1.0 / 120.0, -1.0 / 6.0};
