@@ -1058,11 +1058,11 @@ int build_graph(mmp_batch* b, int steps) {
   return MMP_OK;
 }
 
-// Waits for the batch's stream and reads its solves' status.
+// Waits for the batch's stream and reads its solves' status. k_status writes the word whatever it
+// finds and the host never clears it, so that threads waiting on one batch all read a status.
 int sync_status(mmp_batch* b) {
   int bad = 0;
   if (b->span) {
-    b->words[1] = 0;
     const SolveDesc* descs = b->d_descs;
     int span = (int)b->span, *out = (int*)b->words + 1;
     void* args[] = {(void*)&descs, &span, &out};
