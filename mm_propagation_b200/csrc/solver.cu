@@ -14,6 +14,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -214,6 +215,7 @@ struct DeviceRes {
   bool ready = false;
   void* tw_mem = nullptr;
   const void* tw[2][kMaxLogN + 1] = {};  // [precision][log2 size]: twiddle tables (radix_plan.h)
+  std::set<const void*> prepared;        // kernels that have their shared-memory opt-in
 };
 std::mutex g_dev_mu;
 std::map<int, DeviceRes> g_dev;
@@ -295,42 +297,30 @@ int ensure_device(int dev, DeviceRes** out) {
     r.tw[0][L] = df + twiddle_offset(L);
   }
   r.tw_mem = mem;
-  // dynamic shared memory opt-in for every instantiated kernel
-  for (int fp64 = 0; fp64 < 2; ++fp64)
-    for (int L = kMinLogN; L <= kMaxLogN; ++L)
-      for (int xc = 0; xc <= max_split(fp64 != 0, L); ++xc) {
-        KernelSet ks = kernels_for(fp64, L, xc);
-        std::vector<const void*> fns = {ks.prime, ks.pair, ks.nu, ks.result, ks.dft_fwd, ks.dft_inv};
-        for (const void* f : ks.nu_mid) fns.push_back(f);
-        for (const void* f : ks.nu_last) fns.push_back(f);
-        for (const void* f : fns)
-          if (f)
-            CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(ks.smem, kSmemSM / 2)));
-      }
-  struct Attr { const void* f; int smem; };
-  const int most = 227 * 1024, contract = (int)kContractSmemMax;
-  const Attr attrs[] = {
-      {contract_fn(false, 0, false), contract}, {contract_fn(true, 0, false), contract},
-      {contract_fn(false, 1, false), contract}, {contract_fn(true, 1, false), contract},
-      {contract_fn(false, 1, true), contract},  {contract_fn(true, 1, true), contract},
-      {sp_fn(false, false), contract},          {sp_fn(false, true), contract},
-      {sp_fn(true, false), contract},           {sp_fn(true, true), contract},
-      {sr_fn(false, false), most},              {sr_fn(false, true), most},
-      {sr_fn(true, false), most},               {sr_fn(true, true), most},
-      {tc_fn(false), most - 256},               {tc_fn(true), most - 256},
-      {agg_fn(false, false), 200 * 1024},       {agg_fn(false, true), 200 * 1024},
-      {agg_fn(true, false), 200 * 1024},        {agg_fn(true, true), 200 * 1024},
-      {(const void*)&k_contract_pc<float>, 110 * 1024}, {(const void*)&k_contract_pc<double>, 110 * 1024}};
-  for (const Attr& a : attrs)
-    CUDA_TRY(cudaFuncSetAttribute(a.f, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smem));
-  CUDA_TRY(cudaFuncSetAttribute((const void*)&k_raman_scan<float>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmem));
-  CUDA_TRY(cudaFuncSetAttribute((const void*)&k_raman_scan<double>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmem));
   r.ready = true;
   *out = &r;
   return MMP_OK;
 }
+
+// A kernel and the most dynamic shared memory it is launched with.
+struct KernelUse {
+  const void* fn;
+  int smem;
+};
+// Load the kernels and opt them in to their shared memory, each once per device (the device current):
+// before any capture, and only what a batch runs: a process's first solver takes 12 ms (81 with all 310
+// instantiations loaded), the first of another kind 1 to 6 ms more than a later one.
+int prepare_kernels(DeviceRes* dev, const std::vector<KernelUse>& uses) {
+  std::lock_guard<std::mutex> lk(g_dev_mu);
+  for (const KernelUse& u : uses) {
+    if (!u.fn || dev->prepared.count(u.fn)) continue;
+    CUDA_TRY(cudaFuncSetAttribute(u.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, u.smem));
+    dev->prepared.insert(u.fn);
+  }
+  return MMP_OK;
+}
+// Row kernels may be launched with more than their own rows take (launch_row_kernel).
+int row_smem(const KernelSet& ks) { return std::max(ks.smem, kSmemSM / 2); }
 
 // overlap: a kernel of a step's chain, launched so that it may start while the one before it
 // in the stream still runs (it waits for that one itself, grid_sync_wait). Microseconds a step,
@@ -1208,6 +1198,8 @@ int batch_open(mmp_batch* b, const mmp_params* p0, const Tableau& tab0) {
   b->ks = kernels_for(b->fp64 ? 1 : 0, b->logn, std::max(b->xc_req, 0));
   b->ks64 = kernels_for(1, b->logn);
   if (!b->ks.prime || !b->ks64.prime) return fail(MMP_ENOTSUP, "no kernels built for this nt");
+  rc = prepare_kernels(res, {{b->ks64.dft_fwd, row_smem(b->ks64)}, {b->ks64.result, row_smem(b->ks64)}});
+  if (rc) return rc;
   CUDA_TRY(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
   CUDA_TRY(dev_malloc((void**)&b->d_descs, (size_t)b->capacity * sizeof(SolveDesc)));
   CUDA_TRY(words_take(&b->words));
@@ -1846,6 +1838,35 @@ int row_split(bool fp64, int logn, int rows) {
   return xc;
 }
 
+// The kernels of a step of the batch as it is shaped, and k_prime.
+std::vector<KernelUse> batch_kernels(const mmp_batch* b) {
+  const int row = row_smem(b->ks), contract = (int)kContractSmemMax, most = 227 * 1024;
+  std::vector<KernelUse> u = {{b->ks.prime, row}};
+  for (int i = 0; i < b->tab.s; ++i) u.push_back({nu_kernel(b->ks, b->tab, i), row});
+  const bool raman = b->raman && b->Pmax > 0;
+  if (raman && !b->raman_iir) u.push_back({b->ks.pair, row});
+  if (raman && b->raman_iir && !b->raman_fused)
+    u.push_back({b->fp64 ? fn_ptr(&k_raman_scan<double>) : fn_ptr(&k_raman_scan<float>), kScanSmem});
+  if (raman && b->raman_fused && !b->lookback)
+    u.push_back({b->fp64 ? fn_ptr(&k_raman_carry<double>) : fn_ptr(&k_raman_carry<float>), 0});
+  for (int real = 0; real < 2; ++real) {
+    if (!b->forms[real]) continue;
+    if (raman && b->raman_fused)
+      u.push_back(b->sr ? KernelUse{agg_sr_fn(b->fp64, real), 48 * 1024} : KernelUse{agg_fn(b->fp64, real), 200 * 1024});
+    if (b->sr) {
+      u.push_back({sr_fn(b->fp64, real), most});
+    } else if (b->pchunk) {
+      u.push_back({b->fp64 ? fn_ptr(&k_contract_pc<double>) : fn_ptr(&k_contract_pc<float>), 110 * 1024});
+    } else if (b->tc) {
+      u.push_back({tc_fn(real), most - 256});
+    } else {
+      if (b->dense != 1) u.push_back({b->sp ? sp_fn(b->fp64, real) : contract_fn(b->fp64, 0, false), contract});
+      if (b->dense) u.push_back({contract_fn(b->fp64, 1, real), contract});
+    }
+  }
+  return u;
+}
+
 // Take the shape the batch's solves lead to (a captured graph of another is dropped).
 int batch_shape(mmp_batch* b) {
   const Shape sh = choose_shape(b, batch_stats(b));
@@ -1893,6 +1914,7 @@ int batch_shape(mmp_batch* b) {
     b->graph_steps = 0;
   }
   b->kernels_per_step = step_kernels(b);
+  if (int rc = prepare_kernels(b->dev, batch_kernels(b))) return rc;
   return redo ? upload_desc(b) : MMP_OK;
 }
 
@@ -2412,6 +2434,8 @@ int mmp_dft(uint32_t n, uint32_t rows, int direction, int fp64, const double* in
   int rc = ensure_device(dev, &res);
   if (rc) return rc;
   KernelSet ks = kernels_for(fp64 ? 1 : 0, lg);
+  rc = prepare_kernels(res, {{direction < 0 ? ks.dft_fwd : ks.dft_inv, row_smem(ks)}});
+  if (rc) return rc;
   const size_t bytes = (size_t)rows * n * sizeof(double2);
   double2* d_in = nullptr;
   double2* d_out = nullptr;
