@@ -335,11 +335,13 @@ int mmp_debug_fail_alloc(int64_t after);
  * MMP_STAGE_WAIT_POLLS does the same for the waits between the tensor-core contraction's
  * builder warps and the thread that issues its matrix instructions. */
 int64_t mmp_debug_live_allocations(void);
-/* Which kernels member `index` of a batch runs (either pointer may be NULL): *merged_terms = 1
+/* Which kernels member `index` of a batch runs (any pointer may be NULL): *merged_terms = 1
  * when its contraction reads merged terms over tiles of 64 to 256 samples, 0 for the term loop
  * and the dense, tensor-core and tall-tile forms; *real_pairs = 1 when only the real parts of
- * its pair fields are formed (a coupling symmetric in (l, m)), 0 in the general form. */
-int mmp_debug_batch_form(mmp_batch* b, uint32_t index, uint32_t* merged_terms, uint32_t* real_pairs);
+ * its pair fields are formed (a coupling symmetric in (l, m)), 0 in the general form;
+ * *contract_smem = bytes of dynamic shared memory a CTA of its contraction is launched with. */
+int mmp_debug_batch_form(mmp_batch* b, uint32_t index, uint32_t* merged_terms, uint32_t* real_pairs,
+                         uint32_t* contract_smem);
 
 #ifdef __cplusplus
 }

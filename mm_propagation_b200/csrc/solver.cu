@@ -308,8 +308,8 @@ struct KernelUse {
   int smem;
 };
 // Load the kernels and opt them in to their shared memory, each once per device (the device current):
-// before any capture, and only what a batch runs: a process's first solver takes 12 ms (81 with all 310
-// instantiations loaded), the first of another kind 1 to 6 ms more than a later one.
+// before any capture, and only what a batch runs: a process's first solver takes 12 ms (81 with all
+// instantiations loaded, about 600), the first of another kind 1 to 6 ms more than a later one.
 int prepare_kernels(DeviceRes* dev, const std::vector<KernelUse>& uses) {
   std::lock_guard<std::mutex> lk(g_dev_mu);
   for (const KernelUse& u : uses) {
@@ -1702,8 +1702,8 @@ Shape choose_shape(const mmp_batch* b, const ShapeStats& st, bool try_real = tru
   } else if (dense) {
     smem += 8 * 2 * (size_t)kDenseChunk * 2 * kDenseMaxModes * (t2 / 2);  // staged coefficient rows
   }
-  // terms follow the tiles in shared memory, coefficient in T, when they fit (else they
-  // are read through L1 from the FP64 table); the dense form reads no terms
+  // the term loop's terms follow the tiles in shared memory, coefficient in T, when they fit (else they
+  // are read through L1 from the FP64 table); the dense form and k_contract_sp read none of these
   const size_t staged = b->fp64 ? sizeof(StagedTerm<double>) : sizeof(StagedTerm<float>);
   // Tall tiles (the U tile and every pair field do not fit at 64 samples or more): the
   // pair-chunked contraction keeps the recurrence in the tiles with only a chunk of pair
@@ -1768,7 +1768,7 @@ Shape choose_shape(const mmp_batch* b, const ShapeStats& st, bool try_real = tru
   if (real && (!(tc || sr || sp || dense == 1) || (dense == 2 && !sp) || (tall && !sr) ||
                (b->raman && !fused)))  // R from rows: complex fields (common.cuh)
     return choose_shape(b, st, false);
-  const int stage_terms = sr || (sp && !dense) ? 0 : (pchunk ? 1 : (dense != 1 && !tc && smem + max_terms * staged <= 200 * 1024 ? 1 : 0));
+  const int stage_terms = sr || sp ? 0 : (pchunk ? 1 : (dense != 1 && !tc && smem + max_terms * staged <= 200 * 1024 ? 1 : 0));
   if (stage_terms && !pchunk) smem += max_terms * staged;
   Shape sh;
   sh.Mmax = Mmax;
@@ -2495,12 +2495,14 @@ int mmp_debug_fail_alloc(int64_t after) {
 
 int64_t mmp_debug_live_allocations(void) { return g_live.load(); }
 
-int mmp_debug_batch_form(mmp_batch* b, uint32_t index, uint32_t* merged_terms, uint32_t* real_pairs) {
+int mmp_debug_batch_form(mmp_batch* b, uint32_t index, uint32_t* merged_terms, uint32_t* real_pairs,
+                         uint32_t* contract_smem) {
   if (!b || index >= b->members.size()) return fail(MMP_EINVAL, "bad form arguments");
   const Member& s = b->members[index];
   const bool dense = b->dense == 1 || (b->dense == 2 && s.dense_ok);
   if (merged_terms) *merged_terms = b->sp && !dense ? 1 : 0;
   if (real_pairs) *real_pairs = s.desc.real ? 1 : 0;
+  if (contract_smem) *contract_smem = (uint32_t)(b->sp && !dense ? b->sp_smem : b->contract_smem);
   return MMP_OK;
 }
 

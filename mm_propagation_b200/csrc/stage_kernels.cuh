@@ -1379,7 +1379,7 @@ __global__ void __launch_bounds__(256, (contract_min_blocks<T, DENSE>())) k_cont
   const size_t dense_elems = DENSE ? (size_t)(blockDim.x >> 5) * 2 * kDenseChunk * 2 * kDenseMaxModes : 0;
   ST* st = reinterpret_cast<ST*>(sA + dense_elems);
   // the terms are staged while the kernel before this one still runs
-  if (stage_terms) {
+  if (DENSE == 0 && stage_terms) {
     for (int j = threadIdx.x; j < n_terms; j += blockDim.x) {
       const Term tm = d.terms[j];
       ST s;

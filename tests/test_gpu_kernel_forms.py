@@ -10,16 +10,16 @@ from test_gpu_real_form import CASES, _prob, _skewed
 pytestmark = pytest.mark.gpu
 
 
-def forms(mmp, probs):
-    """(merged terms, real pair fields) of each member."""
+def forms(mmp, probs, smem=False):
+    """(merged terms, real pair fields[, shared memory of the contraction]) of each member."""
     lib = capi.load()
     with mmp.Batch(probs) as b:
         out = []
         for i in range(len(probs)):
-            sp, real = C.c_uint32(9), C.c_uint32(9)
-            assert lib.mmp_debug_batch_form(b._ptr, i, C.byref(sp), C.byref(real)) == capi.MMP_OK
-            out.append((sp.value, real.value))
-        assert lib.mmp_debug_batch_form(b._ptr, len(probs), None, None) == capi.MMP_EINVAL
+            v = [C.c_uint32(9) for _ in range(3)]
+            assert lib.mmp_debug_batch_form(b._ptr, i, *(C.byref(x) for x in v)) == capi.MMP_OK
+            out.append(tuple(x.value for x in v[:3 if smem else 2]))
+        assert lib.mmp_debug_batch_form(b._ptr, len(probs), None, None, None) == capi.MMP_EINVAL
         return out
 
 
@@ -61,3 +61,18 @@ def test_sparse_tiles_read_merged_terms(mmp, monkeypatch, M, nnz, nt, tile, fp64
     assert forms(mmp, [prob])[0][0] == 1
     monkeypatch.setenv("MMP_CONTRACT_SP", "0")
     assert forms(mmp, [prob])[0][0] == 0
+
+
+@pytest.mark.parametrize("fp64", [True, False])
+def test_sparse_neighbours_cost_a_dense_solve_nothing(mmp, monkeypatch, fp64):
+    """Beside solves whose contraction reads merged terms, the dense kernel holds no terms in shared memory."""
+    monkeypatch.setenv("MMP_CONTRACT_TILE", "64")
+    monkeypatch.setenv("MMP_TC", "0")
+    monkeypatch.setenv("MMP_REAL_PAIRS", "0")
+    dense = _prob("dense", 6, 0, 512)
+    sparse = W.small_case(seed=60, M=3, nt=512, n_steps=3)
+    dense, sparse = (p.replace(flags=capi.MMP_F_FP64 if fp64 else 0) for p in (dense, sparse))
+    alone = forms(mmp, [dense], smem=True)[0]
+    mixed = forms(mmp, [dense, sparse], smem=True)
+    assert alone[0] == mixed[0][0] == 0 and mixed[1][0] == 1
+    assert mixed[0][2] == alone[2]
