@@ -335,6 +335,8 @@ int mmp_debug_fail_alloc(int64_t after);
  * MMP_STAGE_WAIT_POLLS does the same for the waits between the tensor-core contraction's
  * builder warps and the thread that issues its matrix instructions. */
 int64_t mmp_debug_live_allocations(void);
+/* Batch shapes whose launch parameters this process has chosen by timing. */
+int64_t mmp_debug_tuned_shapes(void);
 /* Which kernels member `index` of a batch runs (any pointer may be NULL): *merged_terms = 1
  * when its contraction reads merged terms over tiles of 64 to 256 samples, 0 for the term loop
  * and the dense, tensor-core and tall-tile forms; *real_pairs = 1 when only the real parts of

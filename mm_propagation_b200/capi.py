@@ -156,6 +156,7 @@ SIGNATURES = {
     "mmp_batch_set_energy_drift_limit": (C.c_int, [C.c_void_p, C.c_uint32, C.c_double]),
     "mmp_debug_fail_alloc": (C.c_int, [C.c_int64]),
     "mmp_debug_live_allocations": (C.c_int64, []),
+    "mmp_debug_tuned_shapes": (C.c_int64, []),
     "mmp_debug_batch_form": (C.c_int, [C.c_void_p, C.c_uint32, C.POINTER(C.c_uint32), C.POINTER(C.c_uint32),
                                        C.POINTER(C.c_uint32)]),
 }

@@ -1930,8 +1930,8 @@ int batch_shape(mmp_batch* b) {
 //      chains per captured step.
 // The timed steps advance the solves; afterwards every member gets its initial fields
 // back at z = 0 with its counters cleared, as if nothing had run. The choice is cached
-// per shape (device, precision, NT, tableau size, largest M and P, batch size, Raman,
-// contraction form, candidate lists). Batches of one solve are not tuned: they keep the
+// per shape (device, precision, NT, tableau size, largest M and P, batch size, Raman and how its
+// convolution runs, contraction form, merged terms to the power of two, candidate lists). Batches of one solve are not tuned: they keep the
 // default parameters, the ones the serving loop's pools use, so that a served solve and
 // the same solve run alone give the same bits. MMP_ROW_SPLIT, MMP_CONTRACT_TILE and
 // MMP_GROUPS each fix one parameter instead.
@@ -2023,7 +2023,9 @@ int autotune(mmp_batch* b, const mmp_params* const* params) {
   }
   std::vector<int> key = {b->device, b->fp64 ? 1 : 0, b->logn, b->tab.s, b->Mmax, b->Pmax,
                           (int)b->span, b->raman ? 1 : 0, b->tc ? 1 : 0, b->sr ? 1 : 0,
-                          b->pchunk ? 1 : 0, b->dense, (b->forms[0] ? 1 : 0) + (b->forms[1] ? 2 : 0), -1};
+                          b->pchunk ? 1 : 0, b->dense, (b->forms[0] ? 1 : 0) + (b->forms[1] ? 2 : 0),
+                          b->raman_iir ? 1 : 0, b->raman_fused ? 1 : 0, b->lookback ? 1 : 0, b->sp ? 1 : 0,
+                          std::ilogb((double)std::max<size_t>(batch_stats(b).max_sr_terms, 1)), -1};
   for (const std::vector<int>* v : {&xcs, &tiles, &gs}) {
     key.insert(key.end(), v->begin(), v->end());
     key.push_back(-1);
@@ -2494,6 +2496,11 @@ int mmp_debug_fail_alloc(int64_t after) {
 }
 
 int64_t mmp_debug_live_allocations(void) { return g_live.load(); }
+
+int64_t mmp_debug_tuned_shapes(void) {
+  std::lock_guard<std::mutex> lk(g_tune_mu);
+  return (int64_t)g_tune_cache.size();
+}
 
 int mmp_debug_batch_form(mmp_batch* b, uint32_t index, uint32_t* merged_terms, uint32_t* real_pairs,
                          uint32_t* contract_smem) {
