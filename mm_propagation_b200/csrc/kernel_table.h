@@ -21,6 +21,7 @@ struct KernelSet {
   int logn = 0;
   int fp64 = 0;
   int xc = 0;     // rows split over 2^xc times the minimal number of CTAs
+  int resident = 0;  // rows resident at once with one CTA per SM (0: not asked)
 };
 
 // Row splits built for rows of 2^logn samples: xc = 0 .. max_split, clusters of 2^xc times the

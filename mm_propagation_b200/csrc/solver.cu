@@ -129,6 +129,8 @@ __global__ void __launch_bounds__(256) k_restart(const SolveDesc* __restrict__ d
   for (int i = threadIdx.x; i < span; i += blockDim.x)
     if (descs[i].M) *descs[i].step = 0;
 }
+// Never launched: the kernel of which the driver is asked how many clusters fit (clusters_resident)
+__global__ void __launch_bounds__(256) k_cluster_probe() {}
 __global__ void __launch_bounds__(256) k_status(const SolveDesc* __restrict__ descs, int span, int* out) {
   int bad = 0;
   for (int i = threadIdx.x; i < span; i += blockDim.x)
@@ -216,6 +218,7 @@ struct DeviceRes {
   void* tw_mem = nullptr;
   const void* tw[2][kMaxLogN + 1] = {};  // [precision][log2 size]: twiddle tables (radix_plan.h)
   std::set<const void*> prepared;        // kernels that have their shared-memory opt-in
+  int clusters[4] = {};  // clusters of 1, 2, 4, 8 CTAs resident at once, one CTA per SM
 };
 std::mutex g_dev_mu;
 std::map<int, DeviceRes> g_dev;
@@ -248,6 +251,27 @@ void words_give(volatile int* w) {  // no kernel that writes them is in flight
   const int* p = const_cast<const int*>(w);
   if (p >= g_words && p < g_words + kWordSlots * kWordStride) g_words_free.push_back((int)(p - g_words) / kWordStride);
   else cudaFreeHost((void*)p);
+}
+
+// Clusters of C CTAs that are resident at once with one CTA per SM: fewer than 148 / C, since a cluster
+// lies within one of the chip's groups of SMs (15 of 8 CTAs where 18 would fit by count, 33 of 4).
+int clusters_resident(int C) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3((unsigned)(C * kSMs));
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = kSmemSM / 2;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)C;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  const void* fn = (const void*)&k_cluster_probe;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSM / 2);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, fn, &cfg);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e == cudaSuccess && n > 0 ? std::min(n, kSMs / C) : kSMs / C;
 }
 
 int ensure_device(int dev, DeviceRes** out) {
@@ -297,6 +321,7 @@ int ensure_device(int dev, DeviceRes** out) {
     r.tw[0][L] = df + twiddle_offset(L);
   }
   r.tw_mem = mem;
+  for (int i = 0; i < 4; ++i) r.clusters[i] = clusters_resident(1 << i);
   r.ready = true;
   *out = &r;
   return MMP_OK;
@@ -867,9 +892,11 @@ int launch_row_kernel(mmp_batch* b, const KernelSet& ks, const void* fn, int row
   if (rows <= 0 || nsolves <= 0) return MMP_OK;
   // Where n CTAs per SM take the launch in one wave, an early start must not pack more of them
   // onto the SMs that the kernel before has left already: they ask for enough shared memory
-  // that n + 1 do not fit (12 rows of 16384 on 4 CTAs each: 123 -> 102 us a step).
+  // that n + 1 do not fit (12 rows of 16384 on 4 CTAs each: 123 -> 102 us a step), counted in rows
+  // that are resident together.
   int smem = ks.smem;
-  if (overlap) smem = std::max(smem, kSmemSM / ((rows * nsolves * ks.C + kSMs - 1) / kSMs + 1));
+  const int per_wave = ks.resident ? ks.resident : kSMs / ks.C;
+  if (overlap) smem = std::max(smem, kSmemSM / ((rows * nsolves + per_wave - 1) / per_wave + 1));
   KParams kp;
   std::memset(&kp, 0, sizeof(kp));
   kp.descs = descs;
@@ -1825,16 +1852,18 @@ bool joins_same_kernels(const mmp_batch* b, const SolveCounts& c) {
   return empty || same_kernels(choose_shape(b, batch_stats(b)), w);
 }
 
-// Row split for a launch of `rows` rows: the widest cluster that still leaves an SM to every
-// CTA. A transform's bits do not depend on it (fft.cuh), so it may follow what a served pool
+// Row split for a launch of `rows` rows: the widest cluster of which all are resident at once, one
+// CTA to an SM (clusters_resident). A transform's bits do not depend on it (fft.cuh), so it may follow what a served pool
 // holds. Measured, microseconds a step (RK4, one branch), C = 1 / 2 / 4 / 8: 6 rows of 16384
 // samples 157 / 133 / 118 / 111; 2 rows of 4096 in FP64 98 / 91 / 83 / 81; 27 rows of 8192
-// 116 / 107 / 102 / 103; 192 rows of 16384 499 / 485 / 495 / 541. A row of 2048 is quicker in
+// 116 / 107 / 102 / 103; 192 rows of 16384 499 / 485 / 495 / 541. Around the line, 8192 samples,
+// C = 1 / 2 / 4 / 8: 15 rows 120 / 112 / 107 / 105; 16 rows 127 / 120 / 115 / 148 (15 clusters of 8 fit, not 18);
+// 34 rows 298 / 288 / 325 / 320 (33 of 4 fit, not 37). A row of 2048 is quicker in
 // one CTA (64 against 73 / 71 for a single-mode solve): nothing shorter than 4096 is split.
-int row_split(bool fp64, int logn, int rows) {
+int row_split(const DeviceRes* dev, bool fp64, int logn, int rows) {
   int xc = 0;
   const int c0 = kernels_for(fp64 ? 1 : 0, logn).C;
-  while (logn >= 12 && xc < max_split(fp64, logn) && rows * c0 * (2 << xc) <= kSMs) ++xc;
+  while (logn >= 12 && xc < max_split(fp64, logn) && rows <= dev->clusters[ilog2_exact(c0 << (xc + 1))]) ++xc;
   return xc;
 }
 
@@ -1870,9 +1899,10 @@ std::vector<KernelUse> batch_kernels(const mmp_batch* b) {
 // Take the shape the batch's solves lead to (a captured graph of another is dropped).
 int batch_shape(mmp_batch* b) {
   const Shape sh = choose_shape(b, batch_stats(b));
-  const int xc = b->xc_req >= 0 ? b->xc_req : row_split(b->fp64, b->logn, sh.Mmax * (int)sh.span);
+  const int xc = b->xc_req >= 0 ? b->xc_req : row_split(b->dev, b->fp64, b->logn, sh.Mmax * (int)sh.span);
   const bool resplit = xc != b->ks.xc;
   if (resplit) b->ks = kernels_for(b->fp64 ? 1 : 0, b->logn, xc);
+  b->ks.resident = b->dev->clusters[ilog2_exact((uint32_t)b->ks.C)];
   const bool changed = resplit || sh.Mmax != b->Mmax || sh.Pmax != b->Pmax || sh.TT != b->TT || sh.smem != b->contract_smem ||
                        sh.stage_terms != b->stage_terms || sh.span != b->span || sh.iir != b->raman_iir ||
                        sh.fused != b->raman_fused || sh.dense != b->dense || sh.tc != b->tc ||
