@@ -12,7 +12,7 @@
 //   last pass    leaves X[k_1 + A k_2] in registers, where the caller works on it.
 // The inverse runs the same steps backwards with conjugate twiddles, from registers to
 // registers: x[i + B r] ends in the thread that stores it. A spectrum is never put in natural
-// order: it is stored in the order of the last pass (SpecLayout, radix_plan.h).
+// order: it is stored in the order of the last pass (radix_plan.h).
 //
 // With C > 1 the CTA of rank c takes i in [c B/C, (c+1) B/C) in the first pass and keeps the
 // sub-rows [c A/C, (c+1) A/C): the first pass's outputs go to their owners through
@@ -208,19 +208,6 @@ template <typename T, int LOGN_, int XC_ = 0> struct Geo {
   __device__ __forceinline__ static int freq0(int k1, int b) { return k1 + (digits(b) << LOGA); }
   __device__ __forceinline__ static int spec0(int k1, int b) { return (k1 << LOGB) + b; }
 };
-
-// Where frequency k of a spectrum in storage order `l` lies (kernels that meet another
-// geometry's order; the stage kernels step through their own).
-__device__ __forceinline__ int spec_pos(const SpecLayout& l, int k) {
-  if (l.n == 0) return k;
-  const int k1 = k & ((1 << l.loga) - 1);
-  int rest = k >> l.loga, b = 0;
-  for (int p = 0; p + 1 < l.n; ++p) {
-    b = (b << l.r[p]) | (rest & ((1 << l.r[p]) - 1));
-    rest >>= l.r[p];
-  }
-  return (k1 << l.logb) + (rest << (l.logb - l.r[l.n - 1])) + b;
-}
 
 template <bool CONJ, typename V> __device__ __forceinline__ V twiddle(V v, V w) {
   return CONJ ? cmulc(v, w) : cmul(v, w);

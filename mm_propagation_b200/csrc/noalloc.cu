@@ -156,6 +156,7 @@ int mmp_dft_noalloc(uint32_t n, uint32_t rows, int direction, int fp64, const do
     a.rows = (int)rows;
     a.scale = direction < 0 ? 1.0 : 1.0 / (double)n;
     a.tw = r->tw[fp64 ? 1 : 0][lg];
+    a.natural = 1;
     void* args[] = {&a};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows * (unsigned)ks.C, 1, 1);

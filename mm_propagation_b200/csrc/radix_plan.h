@@ -64,17 +64,7 @@ constexpr size_t kTwiddles = twiddle_offset(kMaxLogN + 1);
 //   k = k_1 + A (q_1 + R_1 (q_2 + R_2 (...)))
 // of a transform is left in sub-row k_1, butterfly b = (q_1, ..., q_{m-1}) (q_1 most
 // significant), output q_m of the last pass; it is stored at k_1 B + q_m (B / R_m) + b, so
-// that the lanes of a warp (consecutive b) touch consecutive samples. n = 0: natural order.
-struct SpecLayout {
-  int n;  // row passes (0: natural)
-  int loga, logb;
-  int r[kMaxPasses];  // log2 of the row passes' radices
-};
-constexpr SpecLayout spec_layout(int logn) {
-  const RadixPlan p = radix_plan(logn);
-  SpecLayout s{p.n - 1, p.r[0], logn - p.r[0], {}};
-  for (int i = 1; i < p.n; ++i) s.r[i - 1] = p.r[i];
-  return s;
-}
+// that the lanes of a warp (consecutive b) touch consecutive samples. The order is the same for
+// both precisions and every row split (Geo::spec0).
 
 }  // namespace mmp

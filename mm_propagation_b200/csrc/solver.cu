@@ -902,7 +902,6 @@ int launch_row_kernel(mmp_batch* b, const KernelSet& ks, const void* fn, int row
   kp.descs = descs;
   kp.tw = b->dev->tw[ks.fp64][ks.logn];
   kp.st = stage_args(b->tab, stage);
-  kp.lay = spec_layout(b->logn);
   void* args[] = {&kp};
   dim3 grid((unsigned)(rows * ks.C), (unsigned)nsolves, 1);
   CUDA_TRY(launch(fn, grid, ks.nthr, smem, ks.C, st ? st : b->stream, args, overlap));
@@ -1196,7 +1195,6 @@ int member_set_fields(mmp_batch* b, uint32_t idx, const double* phi0) {
   a.rows = (int)s.M;
   a.scale = s.cf;
   a.tw = b->dev->tw[1][b->logn];
-  a.lay = spec_layout(b->logn);
   a.out_t = b->fp64 ? nullptr : (float2*)s.desc.psi_t;  // psi_hat rounded to T
   a.restart = s.counters;  // z = 0, status, and the drift check's reference energy
   void* args[] = {&a};
@@ -1582,7 +1580,6 @@ int member_init(mmp_batch* b, uint32_t idx, const mmp_params* p) {
     a.rows = 1;
     a.scale = s.delta_t * s.T0 * s.fR / (double)nt;
     a.tw = b->dev->tw[1][b->logn];
-    a.lay = spec_layout(b->logn);
     void* args[] = {&a};
     CUDA_TRY(launch(b->ks64.dft_fwd, dim3((unsigned)b->ks64.C, 1, 1), b->ks64.nthr, b->ks64.smem, b->ks64.C, b->stream, args));
     const void* conv = b->fp64 ? (const void*)&k_to_t2<double> : (const void*)&k_to_t2<float>;
@@ -2484,6 +2481,7 @@ int mmp_dft(uint32_t n, uint32_t rows, int direction, int fp64, const double* in
     a.rows = (int)rows;
     a.scale = direction < 0 ? 1.0 : 1.0 / (double)n;
     a.tw = res->tw[fp64 ? 1 : 0][lg];
+    a.natural = 1;
     void* args[] = {&a};
     e = launch(direction < 0 ? ks.dft_fwd : ks.dft_inv, dim3(rows * (unsigned)ks.C, 1, 1), ks.nthr,
                ks.smem, ks.C, st, args);

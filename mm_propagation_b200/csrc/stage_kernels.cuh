@@ -55,7 +55,6 @@ struct KParams {
   const SolveDesc* descs;
   const void* tw;    // twiddle table of the kernel's precision and size (radix_plan.h)
   StageArgs st;
-  SpecLayout lay;    // psi_hat's storage order (kernels of another geometry)
 };
 
 // Im L_p(alpha) by Horner over the per-mode polynomial (FP64).
@@ -837,7 +836,7 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
 }
 
 // ---- k_result: phi_p = IFFT(exp(L_p z) psi_hat_p) / conversion_factor -> io (FP64) --------
-// psi_hat lies in the order of the solve's own kernels (kp.lay).
+// In FP64 whatever the solve's precision: psi_hat's order is the same.
 template <typename T, int LOGN, int XC>
 __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_BLOCKS) k_result(const KParams kp) {
   using Gm = Geo<T, LOGN, XC>;
@@ -857,10 +856,11 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
   const double z = (double)n * d.dz;
   const size_t row = (size_t)p * Gm::N;
   rows_last<Gm>(sr, u, [&](int b, V* x) {
+    const double2* ps = d.psi_hat + row + Gm::spec0(k1, b);
     const int k0 = Gm::freq0(k1, b);
     V w[Gm::RM];
 #pragma unroll
-    for (int r = 0; r < Gm::RM; ++r) w[r] = from_d2<T>(__ldcg(d.psi_hat + row + spec_pos(kp.lay, k0 + r * Gm::KSTR)));
+    for (int r = 0; r < Gm::RM; ++r) w[r] = from_d2<T>(__ldcg(ps + r * Gm::SSTR));
 #pragma unroll
     for (int r = 0; r < Gm::RM; ++r) {
       const double th = im_L(poly, d.n_beta, alpha_of(k0 + r * Gm::KSTR, Gm::N, d.alpha_scale)) * z;
@@ -883,17 +883,16 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
 }
 
 // ---- k_dft: rows of FP64 samples -> transform in precision T -> rows of FP64 -------------
-// Forward (INV=false): out = scale * FFT(in), stored in order `lay`. Inverse (natural order
+// Forward (INV=false): out = scale * FFT(in), in a solve's order or (natural) by frequency. Inverse (natural order
 // in): out = scale * sum_k in[k] e^{+...}. in may be out: a row is read whole before a
 // barrier after which it is written.
 struct DftArgs {
   const double2* in;
   double2* out;
   int rows;
-  int pad_;
+  int natural;
   double scale;
   const void* tw;
-  SpecLayout lay;
   // forward, where not null: the spectrum in single precision too, and a solve's counters to
   // clear (step, status, drift reference), so that new fields take one launch
   float2* out_t;
@@ -922,7 +921,7 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
     row_first<Gm>(v, s, tw, rank);
     rows_fwd<Gm>(sr, tw, u);
     rows_last<Gm>(sr, u, [&](int b, V* x) {
-      const int k0 = Gm::freq0(k1, b);
+      const int at0 = a.natural ? Gm::freq0(k1, b) : Gm::spec0(k1, b), step = a.natural ? Gm::KSTR : Gm::SSTR;
       V w[Gm::RM];
 #pragma unroll
       for (int r = 0; r < Gm::RM; ++r) w[r] = x[Gm::pad(r)];
@@ -930,7 +929,7 @@ __global__ void __launch_bounds__(Geo<T, LOGN, XC>::NTHR, Geo<T, LOGN, XC>::MIN_
 #pragma unroll
       for (int r = 0; r < Gm::RM; ++r) {
         const double2 y = to_d2(w[r]), z = make_double2(y.x * a.scale, y.y * a.scale);
-        const size_t at = row + spec_pos(a.lay, k0 + r * Gm::KSTR);
+        const size_t at = row + at0 + r * step;
         a.out[at] = z;
         if (a.out_t) a.out_t[at] = make_float2((float)z.x, (float)z.y);
       }

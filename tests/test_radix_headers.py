@@ -1,5 +1,5 @@
 """The numpy restatement of the row transform (test_row_transform) and the build's list of kernel sets
-hold the library's own numbers: the radix plans, row splits, storage order and twiddle tables of
+hold the library's own numbers: the radix plans, row splits and twiddle tables of
 radix_plan.h and kernel_table.h, printed by a host program compiled from them."""
 import os
 import re
@@ -18,11 +18,8 @@ using namespace mmp;
 int main() {
   for (int L = kMinLogN; L <= kMaxLogN; ++L) {
     const RadixPlan p = radix_plan(L);
-    const SpecLayout s = spec_layout(L);
-    std::printf("%d %d %d %zu %zu %d %d %d", L, max_split(false, L), max_split(true, L), twiddle_entries(L),
-                twiddle_offset(L), s.n, s.loga, s.logb);
+    std::printf("%d %d %d %zu %zu", L, max_split(false, L), max_split(true, L), twiddle_entries(L), twiddle_offset(L));
     for (int i = 0; i < p.n; ++i) std::printf(" %d", p.r[i]);
-    for (int i = 0; i < s.n; ++i) std::printf(" %d", s.r[i]);
     std::printf("\\n");
   }
 }
@@ -43,7 +40,7 @@ def test_plans_and_splits_are_the_headers(tmp_path):
             left.append(left[-1] - x)
         entries = sum(1 << x for x in left[:len(r) - 1])  # every pass but the last
         assert left[-1] == 0
-        assert v == [L, max_split(0, L), max_split(1, L), entries, offset, len(r) - 1, r[0], L - r[0], *r, *r[1:]]
+        assert v == [L, max_split(0, L), max_split(1, L), entries, offset, *r]
         assert build._max_split(False, L) == max_split(0, L) and build._max_split(True, L) == max_split(1, L)
         offset += entries
 
