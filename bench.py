@@ -277,7 +277,13 @@ def stage_bytes(prob, tab_s, a, b, bt, pairs, raman_path):
     return {"pair": pair, "contract": contract, "nu": nu / tab_s}
 
 
-def stage_flops(prob, pairs, n_terms, raman_path, recurrence_in_contract=False):
+def merged_terms(prob) -> int:
+    """Terms of the contraction once those with the same p, k and unordered (l, m) are one."""
+    return len({(int(e["p"]), int(e["k"]), min(int(e["l"]), int(e["m"])), max(int(e["l"]), int(e["m"])))
+                for e in prob.coupling if e["value"] != 0})
+
+
+def stage_flops(prob, pairs, n_terms, raman_path, recurrence_in_contract=False, merged=None, real=False):
     """Algorithmic FP32 flops per launch for each kernel kind, one solve, on the
     per-sample model of the hot path: 5 N log2 N per complex transform; the Raman
     recurrence 24 flops per sample and pair field (pair product, two complex first-order
@@ -286,7 +292,10 @@ def stage_flops(prob, pairs, n_terms, raman_path, recurrence_in_contract=False):
     about 70 per sample for k_nu's phase factors and stage combination. When the
     contraction kernel runs the recurrence through its own tiles (k_contract, k_contract_sr)
     the recurrence's flops are its own; the pair kernel then only forms the tile
-    aggregates (the same 24 per sample and pair field)."""
+    aggregates (the same 24 per sample and pair field). `merged` (a count) is the contraction over
+    merged terms: one complex product of U_k with (a Re W, b Im W), 10 flops a term; `real` the
+    form for couplings symmetric in (l, m), where only Re W is formed: 5 a term, 12 a pair field's
+    recurrence and 3 its product."""
     M, NT = prob.n_modes, prob.nt
     P = pairs if prob.raman else 0
     r = 1 if prob.raman else 0
@@ -294,20 +303,31 @@ def stage_flops(prob, pairs, n_terms, raman_path, recurrence_in_contract=False):
     if raman_path == 0:
         pair = P * (2 * fft + 12 * NT)
     else:
-        pair = P * NT * 24.0
-    contract = NT * (8.0 * n_terms * (1 + r) + 6.0 * pairs)
+        pair = P * NT * (12.0 if real else 24.0)
+    if merged is None:
+        contract = NT * (8.0 * n_terms * (1 + r) + 6.0 * pairs)
+    else:
+        contract = NT * ((5.0 if real else 10.0) * merged + (3.0 if real else 6.0) * pairs)
     if recurrence_in_contract:
-        contract += P * NT * 24.0
+        contract += P * NT * (12.0 if real else 24.0)
     nu = M * (2 * fft + 70.0 * NT)
     return {"pair": pair, "contract": contract, "nu": nu}
 
 
-def tc_mma_flops(prob, pairs):
+def tc_mma_flops(prob, pairs, real=False):
     """TF32 work the tensor-core contraction issues per solve and launch: per tile of 128
-    samples and chunk of 16 pair fields, 2 products (Re, Im) x 3 split terms (hi hi, hi lo,
-    lo hi) of 128 x 16 M x 16 MMA work, i.e. 2 * 3 * 2 * 16 ceil(P/16) * 16 M flops per sample."""
-    chunks = -(-pairs // 16)
-    return 2 * 3 * 2.0 * 16 * chunks * 16 * prob.n_modes * prob.nt
+    samples and chunk of 8 pair fields, 2 products (Re, Im; one in the real form) x 3 split terms
+    (hi hi, hi lo, lo hi) of 128 x 16 M x 8 MMA work, i.e. 2 * 3 * 2 * 8 ceil(P/8) * 16 M flops per
+    sample."""
+    chunks = -(-pairs // 8)
+    return (1 if real else 2) * 3 * 2.0 * 8 * chunks * 16 * prob.n_modes * prob.nt
+
+
+def tc_useful_flops(prob, pairs, real=False):
+    """... and what of it one unsplit product over (p, k) x pair fields needs: 2 M^2 P flops a sample
+    for each of the products, and sigma = sum_k U_k T_pk."""
+    M2 = prob.n_modes ** 2
+    return ((1 if real else 2) * 2.0 * M2 * pairs + (4.0 if real else 8.0) * M2) * prob.nt
 
 
 def tf32_peak_tflops():
@@ -360,14 +380,13 @@ def read_measured_peaks():
     return 6650.0, "fallback"
 
 
-def symmetric_in_lm(prob) -> bool:
-    """Q_pklm = Q_pkml for every entry, to 1e-12 of the largest."""
-    q = {}
-    for e in prob.coupling:
-        key = (int(e["p"]), int(e["k"]), int(e["l"]), int(e["m"]))
-        q[key] = q.get(key, 0.0) + float(e["value"])
-    top = max(abs(v) for v in q.values())
-    return all(abs(v - q.get((p, k, m, l), 0.0)) <= 1e-12 * top for (p, k, l, m), v in q.items())
+def batch_form(batch):
+    """(contraction over merged terms, real pair fields only) of a batch's first solve."""
+    import ctypes
+    import mm_propagation_b200 as mmp
+    sp, real = ctypes.c_uint32(0), ctypes.c_uint32(0)
+    mmp.lib().mmp_debug_batch_form(batch._ptr, 0, ctypes.byref(sp), ctypes.byref(real), None)
+    return bool(sp.value), bool(real.value)
 
 
 def read_ncu_traffic(kind: str, workload: str):
@@ -578,10 +597,12 @@ def ours_arm(args, dist):
     tc = bool(info.get("tensor_core_contraction", 0))
     pc = bool(info.get("contract_pair_chunk", 0))
     sr = bool(info.get("contract_sub_block", 0))
-    flops = stage_flops(probe, n_pairs, n_terms, raman_path, recurrence_in_contract=(raman_path == 2))
+    sp, real = batch_form(batch)
+    flops = stage_flops(probe, n_pairs, n_terms, raman_path, recurrence_in_contract=(raman_path == 2),
+                        merged=merged_terms(probe) if sp or sr else None, real=real)
     names = {"pair": ("k_pair", "k_raman_scan", "k_raman_agg (and k_raman_carry where it runs)")[raman_path],
              "contract": ("k_contract_tc" if tc else "k_contract_sr" if sr else "k_contract_pc" if pc
-                          else "k_contract_sp" if not info.get("dense_contraction") and info["contract_tile"] >= 64
+                          else "k_contract_sp" if sp
                           else "k_contract"), "nu": "k_nu"}
     share = {k: prof[k]["ms_per_launch"] * prof[k]["launches"] for k in prof}
     tot = sum(share.values())
@@ -606,12 +627,10 @@ def ours_arm(args, dist):
     tpeak, tpeak_src = tf32_peak_tflops()
     if tc and "contract" in kernels:
         # the dense contraction on the tensor cores: its issued TF32 MMA work (3 split products)
-        # and the useful GEMM work (8 M^4 NT per stage and solve) against the TF32 peak
+        # and what an unsplit product of the form that runs needs, against the TF32 peak
         kc = kernels["contract"]
-        tflops = tc_mma_flops(probe, n_pairs) * args.batch
-        if symmetric_in_lm(probe):  # the REAL form: one real product instead of two
-            tflops /= 2
-        useful = 8.0 * probe.n_modes ** 4 * probe.nt * args.batch
+        tflops = tc_mma_flops(probe, n_pairs, real) * args.batch
+        useful = tc_useful_flops(probe, n_pairs, real) * args.batch
         t = kc["ms_per_launch"] / 1e3
         t_tensor = tflops / (tpeak * 1e12)
         npeak = ncu_tf32_peak_tflops()
@@ -630,7 +649,7 @@ def ours_arm(args, dist):
                 "unit": "TFLOP/s", "frac": kd["tensor_frac"], "peak_source": tpeak_src,
                 "tensor_flops_per_launch": kd["tensor_flops_per_launch"],
                 "note": "achieved counts the issued TF32 MMA work (3 split products per product); "
-                        "frac_of_ncu_tf32_peak and useful_gemm_tflops (8 M^4 NT per stage and solve) beside it",
+                        "frac_of_ncu_tf32_peak and useful_gemm_tflops (the unsplit products) beside it",
                 "frac_of_ncu_tf32_peak": kd["tensor_frac_of_ncu_tf32_peak"],
                 "useful_gemm_tflops": kd["useful_gemm_tflops"]}
     elif kd["roofline_bound"] == "fp32":
