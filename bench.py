@@ -598,8 +598,11 @@ def ours_arm(args, dist):
     pc = bool(info.get("contract_pair_chunk", 0))
     sr = bool(info.get("contract_sub_block", 0))
     sp, real = batch_form(batch)
+    dense = bool(info.get("dense_contraction", 0))
     flops = stage_flops(probe, n_pairs, n_terms, raman_path, recurrence_in_contract=(raman_path == 2),
-                        merged=merged_terms(probe) if sp or sr else None, real=real)
+                        merged=merged_terms(probe) if sp or sr else 0 if dense else None, real=real)
+    if dense:  # the product over (p, k) x pair fields; on the tensor cores only sigma = sum_k U_k T_pk is FP32
+        flops["contract"] += (4.0 if real else 8.0) * probe.n_modes ** 2 * probe.nt if tc else tc_useful_flops(probe, n_pairs, real)
     names = {"pair": ("k_pair", "k_raman_scan", "k_raman_agg (and k_raman_carry where it runs)")[raman_path],
              "contract": ("k_contract_tc" if tc else "k_contract_sr" if sr else "k_contract_pc" if pc
                           else "k_contract_sp" if sp

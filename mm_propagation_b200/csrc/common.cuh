@@ -46,8 +46,8 @@ template <typename T> __device__ __forceinline__ c2<T> from_d2(double2 a);
 template <> __device__ __forceinline__ float2 from_d2<float>(double2 a) { return make_float2((float)a.x, (float)a.y); }
 template <> __device__ __forceinline__ double2 from_d2<double>(double2 a) { return a; }
 
-// Padded shared-memory index: one spare element per 32 keeps the Stockham
-// passes' strided stores free of bank conflicts for 8- and 16-byte elements.
+// Padded shared-memory index of k_raman_scan's staged row: one spare element per 32 spreads the
+// threads' strided samples over the banks for 8- and 16-byte elements.
 __host__ __device__ __forceinline__ int pad(int i) { return i + (i >> 5); }
 __host__ __device__ constexpr int padded_len(int n) { return n + (n >> 5); }
 

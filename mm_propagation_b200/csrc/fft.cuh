@@ -5,8 +5,8 @@
 //   first pass   thread i < B takes the A samples x[i + B r] straight from global memory (a
 //                warp's loads are consecutive), a radix-A butterfly in registers, the twiddles
 //                w_N^{i k_1}, and hands output k_1 to sub-row k_1 in shared memory;
-//   row passes   sub-row k_1 (B samples y_{k_1}) is transformed in place by B / A threads, up to
-//                8192 samples a warp or less: radices R_1, ..., R_m, each pass reading
+//   row passes   sub-row k_1 (B samples y_{k_1}) is transformed in place by B / A threads (rows of up
+//                to 8192 samples: one warp or less): radices R_1, ..., R_m, each pass reading
 //                and writing the same positions, so that one synchronisation of those
 //                threads separates two passes;
 //   last pass    leaves X[k_1 + A k_2] in registers, where the caller works on it.

@@ -23,7 +23,7 @@
 //                                   [last stage: psi_hat += h sum b_j N_hat_j, monitors],
 //                                   x_hat = psi_hat + h sum a_{i+1,j} N_hat_j,
 //                                   * E_{i+1} -> IFFT -> U for the next stage
-// Any other h_R takes k_pair (V -> FFT -> * H_R -> IFFT = R per pair field) instead of
+// Any other h_R takes k_pair (V -> FFT -> * H_R -> IFFT = R, a row per pair field) instead of
 // the first, and the contraction reads R as rows. k_prime makes U for stage 0 when a
 // propagate call starts. E_i = exp(i Im L_p(w) z) is never stored: the phase
 // Im L_p(w) * (z_n + c_i h) is evaluated in FP64, reduced in FP64 and only then passed
@@ -1690,7 +1690,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2)) k_contract_pc(c
 //            heaviest mode's; groups of similar length share a warp.
 // Shared memory bounds it: per term a lane reads W_q (16 bytes) and the term's record, and U_k
 // when k changes; per sub-block a slot reads two rows of U (REAL: four). Measured on a B200 at
-// 28 x 65536, 203 slots, 1060 merged terms, 8 solves, a launch: 519 us in the general form; REAL
+// 28 x 65536, 150 slots, 1060 merged terms, 8 solves, a launch: 519 us in the general form; REAL
 // form, which halves the phase-A chains and the FMAs of a term, 420 us; with four samples a
 // lane (half the W loads and records a sample; one U buffer keeps three CTAs an SM) 378 us, the
 // shared-memory pipe busy 75% of the time, issue 49%.
@@ -2071,7 +2071,7 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 3 : 1))
 // S <- lambda S + x sample after sample (the arithmetic of k_contract_sr's phase A without
 // the output), U arriving in sub-blocks of kSrSub samples through the same double buffer.
 // The contraction's tiles (tile_carry), or k_raman_carry, make the states entering the tiles of them.
-// Shared-memory reads of U bound it (l1tex 88% busy): 8 solves of 28 x 65536 with 203 slots, 105 us a
+// Shared-memory reads of U bound it (l1tex 88% busy): 8 solves of 28 x 65536 with 150 slots, 105 us a
 // launch; skipping the second row where a slot's two fields share a mode made it 134.
 template <typename T, bool REAL>
 __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
@@ -2195,11 +2195,12 @@ __global__ void __launch_bounds__(kSrThreads, (sizeof(T) == 4 ? 4 : 2))
 //      pointwise.)
 //   3. one warp per (p, 32 pairs): sigma = sum over p's merged terms of U_k (a Re W + i b Im W),
 //      terms as one record (a, b, positions of row k and row q), U_k read when k changes.
-// What bounds it: issue (62% of cycles on 28 warps), then the latency of the tile. Measured on a
+// What bounds it: the latency of the tile and of the states entering it (long_scoreboard stalls
+// first, 3.7 of 7 cycles an issued instruction, 28 warps an SM), then issue (53% of cycles). Measured on a
 // B200 against the scalar term loop over unmerged terms (k_contract<T, 0>), a launch: 32 solves
-// of 6 x 16384 (21 pair fields) 56 -> 44 us, 38.2 -> 27.8 million warp instructions; 128 of
-// 2 x 4096 29 -> 24 us; a step of one 6 x 8192 FP64 solve 112 -> 96 us. REAL form (11 slots for
-// the 21 pair fields): 45 -> 41 us.
+// of 6 x 16384 (16 pair fields) 56 -> 44 us, 38.2 -> 27.8 million warp instructions; 128 of
+// 2 x 4096 29 -> 24 us; a step of one 6 x 8192 FP64 solve 112 -> 96 us. REAL form (8 slots for
+// the 16 pair fields): 45 -> 41 us.
 template <typename T> struct LaneScan {
   using V = c2<T>;
   V lr2, li2, nli2, kr2, ki2;  // lambda and kappa, each component in both lanes
